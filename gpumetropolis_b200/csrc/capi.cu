@@ -134,17 +134,6 @@ const void* interp_kernel(int v) {
   }
 }
 
-void launch_interp(int v, dim3 grid, size_t smem, cudaStream_t st, const EvalProg& prog,
-                   const TmapDesc& tmap, const EvalArgs& E, const ChainArgs& A, int phase) {
-  switch (v) {
-    case V16x6: iter_kernel<16, 6><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-    case V8x8: iter_kernel<8, 8><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-    case V4x16: iter_kernel<4, 16><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-    default: iter_kernel<2, 32><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-  }
-  GPUM_CK(cudaGetLastError());
-}
-
 // Interpreter gradient kernels by width (1 + parameters, rounded up).
 int grad_width(uint32_t np) {
   const int w = 1 + (int)np;
@@ -161,16 +150,21 @@ const void* interp_grad_kernel(int W) {
   }
 }
 
-void launch_interp_grad(int W, dim3 grid, size_t smem, cudaStream_t st, const GradProg& prog,
-                        const TmapDesc& tmap, const EvalArgs& E, const ChainArgs& A, int phase) {
-  switch (W) {
-    case 9: iter_kernel_grad<9><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-    case 17: iter_kernel_grad<17><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-    case 33: iter_kernel_grad<33><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-    case 65: iter_kernel_grad<65><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-    default: iter_kernel_grad<129><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, phase); break;
-  }
-  GPUM_CK(cudaGetLastError());
+// Launch with programmatic dependent launch: the kernel may start while its
+// predecessor in the stream runs and waits for it itself (pdl_wait).  A step
+// of the sampling loop costs 2 kernels; their launch latencies overlap.
+void launch_pdl(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  GPUM_CK(cudaLaunchKernelExC(&cfg, fn, args));
 }
 
 int num_sms() {
@@ -267,7 +261,7 @@ struct gpum_b200_session {
   DBuf<double> state, prop, cur, last_eval, sd, temp, L, snap, zbuf, partials, pointwise,
       points, out64, gx, gy, mx, my, vbuf;
   DBuf<float> params, draws, draws_out;
-  DBuf<uint32_t> ctr, accepts, iter, tickets, ptape_i;
+  DBuf<uint32_t> ctr, accepts, iter, ptape_i;
   DBuf<double> ptape;
   EvalArgs E{};
   ChainArgs A{};
@@ -290,6 +284,9 @@ struct gpum_b200_session {
   gpum_b200_mlp* da_mlp = nullptr;
   int da_mlp_launches = 0;  // kernel launches per surrogate call
   DBuf<double> mom;  // draw moments scratch
+  DBuf<double> prior_v, prior_g;  // priors at a step's points, and their gradients
+  StepArgs step_args{};
+  size_t step_smem = 0;
   // Replica exchange on the device (0 = off).
   int pt_K = 0, pt_every = 0;
   DBuf<uint32_t> pt_att, pt_acc, pt_n;
@@ -479,8 +476,6 @@ struct gpum_b200_session {
                                    (int)geo.smem));
     params.ensure((size_t)np * geo.C_pad);
     partials.ensure((size_t)geo.NOB * geo.C_pad * kc.W);
-    tickets.ensure(geo.NCB);
-    GPUM_CK(cudaMemsetAsync(tickets.p, 0, sizeof(uint32_t) * geo.NCB, stream));
     E = EvalArgs{};
     E.n_obs = (int)n_obs;
     E.ncols = (int)(ext(kc) ? ncols_c : ncols);
@@ -495,7 +490,6 @@ struct gpum_b200_session {
     E.params = params.p;
     E.partials = partials.p;
     E.n_points = n;
-    E.tickets = tickets.p;
     E.err = d_err.p;
   }
 
@@ -510,7 +504,71 @@ struct gpum_b200_session {
     ++launches;
   }
 
-  void launch(int phase) { launch_with(geo, E, phase); }
+  // Warps per chain (or point) of the step and reduction kernels: as many as
+  // keep all of them in one wave (64 registers: 32 warps per SM).
+  static int warps_per_chain(int n) {
+    int w = kWarps;
+    while (w > 1 && (long long)n * w > 32ll * num_sms()) w /= 2;
+    return w;
+  }
+
+  // The geometry of the step kernel for the prepared run: 8 warps per block,
+  // fewer when the staged factors would not fit; none are staged above 96 KB
+  // per chain.
+  void setup_step() {
+    constexpr size_t kMax = 96 * 1024;
+    StepArgs& S = step_args;
+    S = StepArgs{};
+    S.partials = partials.p;
+    S.nob = geo.NOB;
+    S.C_pad = geo.C_pad;
+    S.Ws = kc.W;
+    S.W = A.mode == MODE_MALA ? 1 + (int)np : 1;
+    S.params = params.p;
+    S.wpc = warps_per_chain(n_chains);
+    S.wpb = kWarps;
+    S.stage_L = A.L && step_smem_doubles((int)np, S.W, S.wpc, true) * 8 <= kMax ? 1 : 0;
+    auto bytes = [&] {
+      return (size_t)(S.wpb / S.wpc) *
+             step_smem_doubles((int)np, S.W, S.wpc, S.stage_L != 0) * 8;
+    };
+    while (S.wpb > S.wpc && bytes() > kMax) S.wpb /= 2;
+    step_smem = bytes();
+    if (step_smem > 48 * 1024)
+      GPUM_CK(cudaFuncSetAttribute(step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)step_smem));
+  }
+
+  // The end of a step, after its evaluation has been launched.
+  void launch_step(int phase) {
+    step_args.phase = phase;
+    step_args.prior = E.prior_pts ? E.prior_out : nullptr;
+    step_args.prior_grad = E.prior_pts ? E.prior_grad : nullptr;
+    void* args[] = {(void*)&A, (void*)&step_args};
+    const int cpb = step_args.wpb / step_args.wpc;
+    launch_pdl((const void*)step_kernel, dim3((unsigned)((n_chains + cpb - 1) / cpb)),
+               dim3(32 * step_args.wpb), args, step_smem, stream);
+    ++launches;
+  }
+
+  // Evaluation and end of the start (PH_INIT, at the states) or of one
+  // iteration (PH_STEP, at the proposals); the evaluation's first row of CTAs
+  // computes the priors there.
+  void eval_and_step(int phase) {
+    E.prior_pts = prior_code.empty() ? nullptr : phase == PH_INIT ? A.state : A.prop;
+    launch_with(geo, E, phase, phase == PH_STEP);
+    launch_step(phase);
+  }
+
+  // Values w0 .. W - 1 of the n points of a batch, summed into out64.
+  void reduce(int n, int W, int w0) {
+    const int wpc = warps_per_chain(n), ppb = kWarps / wpc;
+    reduce_partials_kernel<<<(unsigned)((n + ppb - 1) / ppb), kThreads,
+                             sizeof(double) * kWarps * W, stream>>>(
+        partials.p, out64.p, geo.NOB, geo.C_pad, kc.W, n, W, w0, wpc);
+    GPUM_CK(cudaGetLastError());
+    ++launches;
+  }
 
   // One Metropolis iteration: for path-B DE the proposals of the generation
   // come first, in their own kernel (every chain reads the population).
@@ -521,7 +579,7 @@ struct gpum_b200_session {
       GPUM_CK(cudaGetLastError());
       ++launches;
     }
-    launch(PH_STEP);
+    eval_and_step(PH_STEP);
     if (pt_K > 0) {
       PtArgs P{pt_K, pt_every, A.iter, nullptr, nullptr, pt_n.p, pt_att.p, pt_acc.p,
                params.p, geo.C_pad};
@@ -531,19 +589,19 @@ struct gpum_b200_session {
     }
   }
 
-  void launch_with(const Geometry& g, EvalArgs& e, int phase) {
-    const dim3 grid(g.NCB, g.NOB);
-    if (kc.tc) {
-      void* args[] = {(void*)&tc_data.p, (void*)&e, (void*)&A, (void*)&phase};
-      GPUM_CK(cudaLaunchKernel(kc.fn, grid, dim3(kc.threads), args, g.smem, stream));
-    } else if (kc.compiled) {
-      void* args[] = {(void*)(ext(kc) ? &tmap_c : &tmap), (void*)&e, (void*)&A, (void*)&phase};
-      GPUM_CK(cudaLaunchKernel(kc.fn, grid, dim3(kThreads), args, g.smem, stream));
-    } else if (kc.grad_interp) {
-      launch_interp_grad(kc.W, grid, g.smem, stream, *gprog, tmap, e, A, phase);
-    } else {
-      launch_interp(variant, grid, g.smem, stream, *prog, tmap, e, A, phase);
-    }
+  // The evaluation kernel on geometry g; `pdl`: it may start while the
+  // previous kernel of the stream runs.
+  void launch_with(const Geometry& g, EvalArgs& e, int phase, bool pdl = false) {
+    const dim3 grid(g.NCB, g.NOB + (e.prior_pts ? 1 : 0)), block(kc.threads);
+    void* targs[] = {(void*)&tc_data.p, (void*)&e, (void*)&A, (void*)&phase};
+    void* cargs[] = {(void*)(ext(kc) ? &tmap_c : &tmap), (void*)&e, (void*)&A, (void*)&phase};
+    void* iargs[] = {kc.grad_interp ? (void*)gprog.get() : (void*)prog.get(), (void*)&tmap,
+                     (void*)&e, (void*)&A, (void*)&phase};
+    void** args = kc.tc ? targs : kc.compiled ? cargs : iargs;
+    if (pdl)
+      launch_pdl(kc.fn, grid, block, args, g.smem, stream);
+    else
+      GPUM_CK(cudaLaunchKernel(kc.fn, grid, block, args, g.smem, stream));
     ++launches;
   }
 
@@ -740,7 +798,8 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
   s->last_eval.ensure(C);
   s->ctr.ensure(C);
   s->accepts.ensure(C);
-  s->iter.ensure(g.NCB);
+  s->iter.ensure(C);
+  s->prior_v.ensure(C);
   s->draws.ensure(std::max<size_t>(1, (size_t)max_iter * np * g.C_pad));
   if (use_L) s->L.ensure((size_t)C * np * np);
   if (mala) {
@@ -749,6 +808,7 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
     s->mx.ensure(C * np);
     s->my.ensure(C * np);
     s->vbuf.ensure(C * np);
+    s->prior_g.ensure(C * np);
     if (!s->kc.compiled) {  // the interpreted prior's gradient tape
       const size_t npr = std::max<size_t>(s->prior_code.size() / 2, 1);
       s->ptape.ensure((size_t)C * 2 * npr);
@@ -765,7 +825,7 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
     GPUM_CK(cudaMemcpyAsync(s->L.p, L, sizeof(double) * C * np * np, cudaMemcpyHostToDevice, st));
   GPUM_CK(cudaMemsetAsync(s->ctr.p, 0, sizeof(uint32_t) * C, st));
   GPUM_CK(cudaMemsetAsync(s->accepts.p, 0, sizeof(uint32_t) * C, st));
-  GPUM_CK(cudaMemsetAsync(s->iter.p, 0, sizeof(uint32_t) * g.NCB, st));
+  GPUM_CK(cudaMemsetAsync(s->iter.p, 0, sizeof(uint32_t) * C, st));
   const int total = (int)(np * g.C_pad);
   points_to_params_kernel<<<(total + 255) / 256, 256, 0, st>>>(s->state.p, s->params.p, (int)C,
                                                                (int)np, g.C_pad);
@@ -835,7 +895,10 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
     A.rec_base = s->rec_count;
     A.rec_cap = s->rec_cap;
   }
-  s->launch(PH_INIT);
+  s->E.prior_out = s->prior_v.p;
+  s->E.prior_grad = mala ? s->prior_g.p : nullptr;
+  s->setup_step();
+  s->eval_and_step(PH_INIT);
   s->max_iter = max_iter;
   s->n_done = 0;
   s->prepared = true;
@@ -929,33 +992,24 @@ void batch(gpum_b200_session* s, const double* pts, size_t n_points, double* out
       if (s->ll.empty()) {
         GPUM_CK(cudaMemsetAsync(s->pointwise.p, 0, sizeof(double) * n * s->n_obs, s->stream));
       } else {
-        s->launch(PH_POINTWISE);
+        s->launch_with(s->geo, s->E, PH_POINTWISE);
       }
       GPUM_CK(cudaMemcpyAsync(out + p0 * s->n_obs, s->pointwise.p,
                               sizeof(double) * n * s->n_obs, cudaMemcpyDeviceToHost, s->stream));
     } else {
-      const int W = s->kc.W;
-      s->out64.ensure((size_t)n * W);
+      // Sums, or the gradient's np entries (the interpreter's gradient kernel
+      // pads its width, the entries past 1 + np are left out).
+      const int W = kind == B_GRAD ? 1 + (int)np : 1, w0 = kind == B_GRAD ? 1 : 0;
+      const size_t width = (size_t)(W - w0);
+      s->out64.ensure((size_t)n * width);
       if (s->ll.empty()) {
-        GPUM_CK(cudaMemsetAsync(s->out64.p, 0, sizeof(double) * n * W, s->stream));
+        GPUM_CK(cudaMemsetAsync(s->out64.p, 0, sizeof(double) * n * width, s->stream));
       } else {
-        s->launch(PH_EVAL);
-        reduce_partials_kernel<<<(n * W + 255) / 256, 256, 0, s->stream>>>(
-            s->partials.p, s->out64.p, s->geo.NOB, s->geo.C_pad, n, W);
-        GPUM_CK(cudaGetLastError());
-        ++s->launches;
+        s->launch_with(s->geo, s->E, PH_EVAL);
+        s->reduce(n, W, w0);
       }
-      if (kind == B_GRAD) {
-        std::vector<double> tmp((size_t)n * W);
-        GPUM_CK(cudaMemcpyAsync(tmp.data(), s->out64.p, sizeof(double) * n * W,
-                                cudaMemcpyDeviceToHost, s->stream));
-        GPUM_CK(cudaStreamSynchronize(s->stream));
-        for (int p = 0; p < n; ++p)
-          for (size_t j = 0; j < np; ++j) out[(p0 + p) * np + j] = tmp[(size_t)p * W + 1 + j];
-      } else {
-        GPUM_CK(cudaMemcpyAsync(out + p0, s->out64.p, sizeof(double) * n, cudaMemcpyDeviceToHost,
-                                s->stream));
-      }
+      GPUM_CK(cudaMemcpyAsync(out + p0 * width, s->out64.p, sizeof(double) * n * width,
+                              cudaMemcpyDeviceToHost, s->stream));
     }
     s->check_device_error();
   }
@@ -1080,6 +1134,7 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
   s->da_partials.ensure((size_t)max_nob * s->geo_da.C_pad);
   GPUM_CK(cudaMemsetAsync(s->da_params.p, 0, sizeof(float) * np * g.C_pad, st));
   s->E_da = s->E;
+  s->E_da.prior_pts = nullptr;  // the loop's own kernels compute the priors
   s->E_da.params = s->da_params.p;
   s->E_da.partials = s->da_partials.p;
   s->E_da.active = s->da_active.p;

@@ -1,18 +1,18 @@
 // common.cuh -- the per-iteration kernel skeleton shared by the interpreter
 // and the compiled (NVRTC) evaluation bodies, plus the accept/propose logic.
 //
-// One launch = one Metropolis iteration for every chain (the reference runs
-// a whole chain inside one CTA, src/rust/src/chain_kernel.rs:123-357; here
-// the data sum of every chain is spread over the whole GPU):
+// One launch evaluates one Metropolis iteration's proposals of every chain (the
+// reference runs a whole chain inside one CTA, src/rust/src/chain_kernel.rs
+// :123-357; here the data sum of every chain is spread over the whole GPU):
 //   grid.x = chain blocks of CG chains, grid.y = observation blocks;
 //   each CTA streams its observation tiles through shared memory with TMA
 //   (double-buffered, mbarrier completion, bounded waits) and evaluates its
 //   CG chains on every observation, so one tile read serves CG chains;
 //   per-thread compensated FP32 sums -> FP64 warp-shuffle tree -> FP64 sum
 //   over warps in fixed order -> FP64 partial per (obs block, chain, value);
-//   the last CTA of a chain block (atomic ticket, no spinning) sums the
-//   partials in obs-block order, adds the f64 prior, makes the tempered f64
-//   accept decision, records the draw and draws the next proposal.
+//   one more row of CTAs computes the chains' f64 priors meanwhile; the step
+//   kernel (kernels.cuh, step_kernel) then adds the partials up, makes the
+//   tempered f64 accept decision, records the draw and draws the next proposal.
 // Results are deterministic for a given launch geometry.
 #pragma once
 #include "device.cuh"
@@ -40,7 +40,7 @@ struct ChainArgs {
   double* last_eval;    // [C]   log posterior of the latest evaluated point
   uint32_t* ctr;        // [C]   triple32 counters
   uint32_t* accepts;    // [C]
-  uint32_t* iter;       // [NCB] iterations done, per chain block
+  uint32_t* iter;       // [C]   iterations done
   const double* sd;     // [C][np]
   const double* temp;   // [C]
   const double* L;      // [C][np][np] row-major lower factors, or nullptr
@@ -82,9 +82,13 @@ struct EvalArgs {
   double* partials;     // [NOB][C_pad][width]
   double* pointwise;    // [C][n_obs] (PH_POINTWISE)
   int n_points;         // chains/points that are real (rest padding)
-  uint32_t* tickets;    // [NCB]
   uint32_t* err;        // device error word
   const uint32_t* active;  // if set: only the first *active points are live
+  // A sampler step's priors (prior_block): the points [C][np], or nullptr (no
+  // prior, or not a step); the values [C] and, for MALA, the gradients [C][np]
+  const double* prior_pts;
+  double* prior_out;
+  double* prior_grad;
 };
 
 // Delayed acceptance evaluates the first `live` points of the compacted array
@@ -255,249 +259,26 @@ __device__ __forceinline__ Stream make_stream(const ChainArgs& A, int c) {
   return rs;
 }
 
-// -------------------------------------------------------------- MALA helpers
-// out = f * (1/2) M g, M = Ls Ls' (or diag sd^2), the whitened drift capped at
-// 2 sqrt(d) (MALTA; cpu_native.rs:617-651).
-__device__ inline void half_m_times(int np, const double* sd, const double* L, const double* g,
-                                    double* out, double* tmp) {
-  const double dmax = 2.0 * sqrt((double)np);
-  if (!L) {
-    for (int j = 0; j < np; ++j) tmp[j] = 0.5 * sd[j] * g[j];
-  } else {
-    for (int j = 0; j < np; ++j) {
-      double acc = 0.0;
-      for (int k = j; k < np; ++k) acc += L[(size_t)k * np + j] * g[k];
-      tmp[j] = 0.5 * acc;
-    }
-  }
-  double ss = 0.0;
-  for (int j = 0; j < np; ++j) ss += tmp[j] * tmp[j];
-  const double norm = sqrt(ss);
-  const double f = norm > dmax ? dmax / norm : 1.0;
-  if (!L) {
-    for (int j = 0; j < np; ++j) out[j] = f * sd[j] * tmp[j];
-  } else {
-    for (int k = 0; k < np; ++k) {
-      double acc = 0.0;
-      for (int j = 0; j <= k; ++j) acc += L[(size_t)k * np + j] * tmp[j];
-      out[k] = f * acc;
-    }
-  }
-}
-
-// -1/2 |Ls^{-1}(v - m)|^2 by forward substitution (cpu_native.rs:655-673).
-__device__ inline double log_q(int np, const double* sd, const double* L, const double* v,
-                               const double* m, double* tmp) {
-  double q = 0.0;
-  if (!L) {
-    for (int j = 0; j < np; ++j) {
-      const double r = (v[j] - m[j]) / sd[j];
-      q -= 0.5 * r * r;
-    }
-  } else {
-    for (int k = 0; k < np; ++k) {
-      double acc = v[k] - m[k];
-      for (int j = 0; j < k; ++j) acc -= L[(size_t)k * np + j] * tmp[j];
-      tmp[k] = acc / L[(size_t)k * np + k];
-      q -= 0.5 * tmp[k] * tmp[k];
-    }
-  }
-  return q;
-}
-
-// ------------------------------------------------------------- proposals
-// Next proposal of chain c into prop (f64) and params (f32).
-// Diagonal RWM chain_kernel.rs:212-223 / cpu_native.rs:726-735; Cholesky
-// RWM :224-249 / :736-753; DE on the frozen snapshot :250-295 / :754-784;
-// MALA :681-703 (mean from the cached gradient, then L z or sd * z).
-__device__ inline void propose(const ChainArgs& A, int c, Stream& rs, float* params, int C_pad) {
-  const int np = A.np;
-  const double* x = A.state + (size_t)c * np;
-  double* y = A.prop + (size_t)c * np;
-  const double* sd = A.sd + (size_t)c * np;
-  const double* L = A.L ? A.L + (size_t)c * np * np : nullptr;
-  if (A.mode == MODE_RWM) {
-    for (int j = 0; j < np; ++j) y[j] = x[j] + sd[j] * rs.normal();
-  } else if (A.mode == MODE_CHOL || A.mode == MODE_MALA) {
-    double* z = A.zbuf + (size_t)c * np;
-    const double* base = x;
-    if (A.mode == MODE_MALA) {
-      double* mx = A.mx + (size_t)c * np;
-      half_m_times(np, sd, L, A.gx + (size_t)c * np, mx, A.vbuf + (size_t)c * np);
-      for (int j = 0; j < np; ++j) mx[j] += x[j];
-      base = mx;
-    }
-    for (int j = 0; j < np; ++j) z[j] = rs.normal();
-    if (L) {
-      for (int k = 0; k < np; ++k) {
-        double acc = base[k];
-        for (int j = 0; j <= k; ++j) acc += L[(size_t)k * np + j] * z[j];
-        y[k] = acc;
-      }
-    } else {
-      for (int j = 0; j < np; ++j) y[j] = base[j] + sd[j] * z[j];
-    }
-  } else {
-    const int n = A.n_chains;
-    int a = (int)(rs.next() * (double)n);
-    if (a >= n) a = n - 1;
-    int b = (int)(rs.next() * (double)n);
-    if (b >= n) b = n - 1;
-    if (b == a) b = (b + 1) % n;
-    const double g = rs.next() < 0.1 ? 1.0 : A.gamma;
-    const double* pa = A.snap + (size_t)a * np;
-    const double* pb = A.snap + (size_t)b * np;
-    for (int j = 0; j < np; ++j) {
-      const double z = rs.normal();
-      const double diff = pa[j] - pb[j];
-      y[j] = x[j] + g * diff + A.de_noise * sd[j] * z;
-    }
-  }
-  for (int j = 0; j < np; ++j) params[(size_t)j * C_pad + c] = (float)y[j];
-}
-
-// Synchronous per-generation DE (path B, cpu_native.rs:400-506): the
-// difference vector comes from the current population, so this runs in its
-// own kernel after every chain's previous accept.  Partners a != c and
-// b != c, a (cpu_native.rs:430-440); g = 1 with probability 0.1, else gamma.
-__device__ inline void propose_desync(const ChainArgs& A, int c, Stream& rs, float* params,
-                                      int C_pad) {
-  const int n = A.n_chains, np = A.np;
-  int a = (int)(rs.next() * (double)n);
-  if (a >= n) a = n - 1;
-  if (a == c) a = (a + 1) % n;
-  int b = (int)(rs.next() * (double)n);
-  if (b >= n) b = n - 1;
-  while (b == c || b == a) b = (b + 1) % n;  // n >= 3 is checked by the host
-  const double g = rs.next() < 0.1 ? 1.0 : A.gamma;
-  const double* x = A.state + (size_t)c * np;
-  const double* pa = A.state + (size_t)a * np;
-  const double* pb = A.state + (size_t)b * np;
-  const double* sd = A.sd + (size_t)c * np;
-  double* y = A.prop + (size_t)c * np;
-  for (int j = 0; j < np; ++j) {
-    const double z = rs.normal();
-    y[j] = x[j] + g * (pa[j] - pb[j]) + A.de_noise * sd[j] * z;
-    params[(size_t)j * C_pad + c] = (float)y[j];
-  }
-}
-
-// Accept/reject + record + propose for chain c.  `ll` is the data-term sum;
-// with MALA the data-term gradient has been summed into A.gy (STEP) or A.gx
-// (INIT).  Prior::value(A, c, p) and Prior::value_grad(A, c, p, g) give the
-// f64 prior of chain c's point p (value_grad accumulates into g).
+// ------------------------------------------------------ priors of a step
+// The prior depends on the evaluation points only, so a step's launch carries
+// one extra row of CTAs (blockIdx.y == 0) that computes it beside the data
+// sums, one thread per chain: straight-line f64 code (65 divisions for the
+// 65-parameter model) that would otherwise sit in the serial path between
+// two evaluations.
 template <class Prior>
-__device__ inline void finalize_chain(const ChainArgs& A, int c, int cb, double ll, int phase,
-                                      float* params, int C_pad) {
-  const int np = A.np;
-  const uint32_t t = A.iter[cb];
-  Stream rs = make_stream(A, c);
-  const bool mala = A.mode == MODE_MALA;
-  double* x = A.state + (size_t)c * np;
-  const double bl = A.beta ? A.beta[c] * ll : ll;  // likelihood power
-  if (phase == PH_INIT) {
-    const double lp = bl + (mala ? Prior::value_grad(A, c, x, A.gx + (size_t)c * np)
-                                 : Prior::value(A, c, x));
-    A.cur[c] = lp;
-    A.last_eval[c] = lp;
-    if (A.n_iter > 0 && A.mode != MODE_DESYNC) {  // path B proposes in its own kernel
-      rs.it = 0;
-      propose(A, c, rs, params, C_pad);
-    }
-  } else {
-    const double* y = A.prop + (size_t)c * np;
-    const double plp = bl + (mala ? Prior::value_grad(A, c, y, A.gy + (size_t)c * np)
-                                  : Prior::value(A, c, y));
-    A.last_eval[c] = plp;
-    if (A.rec_ll) {
-      const uint64_t slot = A.rec_base + (uint64_t)t * A.n_chains + c;
-      if (slot < A.rec_cap) {
-        for (int j = 0; j < np; ++j) A.rec_theta[slot * np + j] = (float)y[j];
-        A.rec_ll[slot] = ll;
-      }
-    }
-    double lqd = 0.0;
-    if (mala) {
-      // q(x | y) - q(y | x) with the truncated drift at y (cpu_native.rs:704-710)
-      const double* sd = A.sd + (size_t)c * np;
-      const double* L = A.L ? A.L + (size_t)c * np * np : nullptr;
-      double* my = A.my + (size_t)c * np;
-      double* tmp = A.vbuf + (size_t)c * np;
-      half_m_times(np, sd, L, A.gy + (size_t)c * np, my, tmp);
-      for (int j = 0; j < np; ++j) my[j] += y[j];
-      lqd = log_q(np, sd, L, x, my, tmp) - log_q(np, sd, L, y, A.mx + (size_t)c * np, tmp);
-    }
-    double u;
-    if (A.rng == RNG_TRIPLE32) {
-      u = rs.next();
-    } else {
-      rs.it = t;
-      rs.k = 0xFFFF0000u;
-      u = rs.next();
-    }
-    // Tempered acceptance on the f64 totals (chain_kernel.rs:334,
-    // cpu_native.rs:792); MALA adds the proposal ratio and requires a
-    // finite proposal log density (cpu_native.rs:713-714).
-    const bool take = mala ? (isfinite(plp) && log(u) < (plp - A.cur[c]) / A.temp[c] + lqd)
-                           : (log(u) < (plp - A.cur[c]) / A.temp[c]);
-    if (take) {
-      for (int j = 0; j < np; ++j) x[j] = y[j];
-      if (mala) {
-        double* gx = A.gx + (size_t)c * np;
-        const double* gy = A.gy + (size_t)c * np;
-        for (int j = 0; j < np; ++j) gx[j] = gy[j];
-      }
-      A.cur[c] = plp;
-      A.accepts[c] += 1;
-    }
-    if (t < A.n_iter)
-      for (int j = 0; j < np; ++j) A.draws[((size_t)t * np + j) * C_pad + c] = (float)x[j];
-    if (t + 1 < A.n_iter && A.mode != MODE_DESYNC) {
-      rs.it = t + 1;
-      rs.k = 0;
-      propose(A, c, rs, params, C_pad);
-    }
-  }
-  A.ctr[c] = rs.ctr;
-}
-
-// The last CTA of chain block cb to write its partials (an atomic ticket, no
-// spinning) finishes the iteration for the block's CG chains: the partials
-// summed in observation-block order, then accept/reject, record and
-// propose.  Every one of the CTA's nthreads threads calls it.
-template <int W, class Prior>
-__device__ __forceinline__ void finish_chain_block(const EvalArgs& E, const ChainArgs& A, int cb,
-                                                   int CG, int phase, uint32_t* s_ticket,
-                                                   int nthreads) {
-  const int tid = threadIdx.x, np = E.np;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) *s_ticket = atomicAdd(&E.tickets[cb], 1u);
-  __syncthreads();
-  const uint32_t nob = gridDim.y;
-  if (*s_ticket != nob - 1) return;
-  __threadfence();
-  for (int cl = tid; cl < CG; cl += nthreads) {
+__device__ __forceinline__ void prior_block(const EvalArgs& E, const ChainArgs& A, int cb, int CG,
+                                            int nthreads) {
+  for (int cl = threadIdx.x; cl < CG; cl += nthreads) {
     const int c = cb * CG + cl;
     if (c >= A.n_chains) continue;
-    double ll = 0.0;
-    for (uint32_t o = 0; o < nob; ++o) ll += __ldcg(&E.partials[((size_t)o * E.C_pad + c) * W]);
-    if (A.mode == MODE_MALA) {
-      double* gsum = (phase == PH_INIT ? A.gx : A.gy) + (size_t)c * np;
-      const double b = A.beta ? A.beta[c] : 1.0;
-      for (int j = 0; j < np; ++j) {
-        double v = 0.0;
-        for (uint32_t o = 0; o < nob; ++o)
-          v += __ldcg(&E.partials[((size_t)o * E.C_pad + c) * W + 1 + j]);
-        gsum[j] = b * v;
-      }
+    const double* p = E.prior_pts + (size_t)c * A.np;
+    if (E.prior_grad) {
+      double* g = E.prior_grad + (size_t)c * A.np;
+      for (int j = 0; j < A.np; ++j) g[j] = 0.0;
+      E.prior_out[c] = Prior::value_grad(A, c, p, g);
+    } else {
+      E.prior_out[c] = Prior::value(A, c, p);
     }
-    finalize_chain<Prior>(A, c, cb, ll, phase, const_cast<float*>(E.params), E.C_pad);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    E.tickets[cb] = 0;
-    if (phase == PH_STEP) A.iter[cb] += 1;
   }
 }
 
@@ -505,14 +286,14 @@ __device__ __forceinline__ void finish_chain_block(const EvalArgs& E, const Chai
 // Shared-memory carve-up (the host's smem_bytes() must agree):
 //   2 data stages [ncols][T] f32 | params [np][CG] f32 (rounded to 4; none
 //   for chain-lane bodies, whose lanes read their parameters from global
-//   memory) | reduction [kWarps][G][width] f64 | 2 mbarriers | ticket.
+//   memory) | reduction [kWarps][G][width] f64 | 2 mbarriers.
 __host__ __device__ inline size_t skel_param_floats(int np, int CG, bool lanes) {
   return lanes ? 0 : (((size_t)np * CG + 3) & ~(size_t)3);
 }
 __host__ __device__ inline size_t skel_smem_bytes(int T, int ncols, int np, int CG, int G,
                                                   int width, bool lanes = false) {
   return 2 * (size_t)T * ncols * 4 + skel_param_floats(np, CG, lanes) * 4 +
-         (size_t)kWarps * G * width * 8 + 2 * 8 + 16;
+         (size_t)kWarps * G * width * 8 + 2 * 8;
 }
 
 // Body contract (G chains per thread):
@@ -542,7 +323,17 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   // Chain blocks vary fastest, so the CTAs that share an observation tile
   // run in the same wave and read it through L2 once.
   int cb = blockIdx.x, ob = blockIdx.y, tiles_per_cta = E.tiles_per_cta;
+  if (E.prior_pts) {
+    if (ob == 0) {
+      pdl_wait();
+      pdl_trigger();
+      prior_block<Prior>(E, A, cb, CG, kThreads);
+      return;
+    }
+    --ob;
+  }
   if (E.active) {  // delayed acceptance: geometry from the live count
+    pdl_wait();
     const int live = (int)*E.active;
     const int busy = (live + CG - 1) / CG;
     const int nob = da_obs_blocks(live, CG, (int)(gridDim.x * gridDim.y), E.ntiles,
@@ -561,14 +352,6 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   float* psm = xs + 2 * stage_floats;
   double* red = reinterpret_cast<double*>(psm + skel_param_floats(np, CG, kLanes));
   uint64_t* bars = reinterpret_cast<uint64_t*>(red + (size_t)kWarps * G * W);
-  uint32_t* s_ticket = reinterpret_cast<uint32_t*>(bars + 2);
-
-  if constexpr (!kLanes) {
-    for (int i = tid; i < np * CG; i += kThreads) {
-      const int p = i / CG, cl = i % CG;
-      psm[i] = E.params[(size_t)p * E.C_pad + (size_t)cb * CG + cl];
-    }
-  }
 
   const int t0 = ob * tiles_per_cta;
   const int t1 = min(t0 + tiles_per_cta, E.ntiles);
@@ -581,14 +364,22 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
     mbar_fence_init();
-  }
-  __syncthreads();
-  if (tid == 0 && staged) {
+    // The data does not change during a run: the first tiles are on their way
+    // before the previous step's proposals are waited for.
     for (int s = 0; s < 2 && s < nt; ++s) {
       mbar_expect_tx(&bars[s], tile_bytes);
       tma_load_2d(xs + s * stage_floats, tmap, &bars[s], (t0 + s) * T, 0);
     }
   }
+  pdl_wait();
+  pdl_trigger();
+  if constexpr (!kLanes) {
+    for (int i = tid; i < np * CG; i += kThreads) {
+      const int p = i / CG, cl = i % CG;
+      psm[i] = E.params[(size_t)p * E.C_pad + (size_t)cb * CG + cl];
+    }
+  }
+  __syncthreads();
   if constexpr (kLanes) {
     const float* pc = E.params + (size_t)cb * CG + (size_t)wc * 32 + lane;
     if constexpr (Body::kLanesAcc)
@@ -683,7 +474,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     // the CTA (the error bit is set) stops the tile loop for the whole CTA:
     // no more loads are issued, thread 0 waits (bounded) for the loads still
     // in flight into this CTA's stages, and the CTA goes on to the reduction
-    // and the ticket so the chain block's bookkeeping stays consistent.
+    // (its partial is written whatever happened).
     if (__syncthreads_or(gave_up)) {
       if (tid == 0 && staged) {
         mbar_wait_bounded(&bars[st], (uint32_t)((k >> 1) & 1));
@@ -729,20 +520,6 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     for (int o = 0; o < WO; ++o) v += red[((size_t)(o * E.WC + wcc) * G + g) * W + w];
     E.partials[((size_t)ob * E.C_pad + (size_t)cb * CG + cl) * W + w] = v;
   }
-  if (phase == PH_EVAL) return;
-  finish_chain_block<W, Prior>(E, A, cb, CG, phase, s_ticket, kThreads);
-}
-
-// Fixed-order sum of the partials of each point: out[p*W + w].
-static __global__ void reduce_partials_kernel(const double* __restrict__ partials,
-                                       double* __restrict__ out, int nob, int C_pad, int n,
-                                       int W) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * W) return;
-  const int c = i / W, w = i % W;
-  double v = 0.0;
-  for (int o = 0; o < nob; ++o) v += partials[((size_t)o * C_pad + c) * W + w];
-  out[i] = v;
 }
 
 }  // namespace gpum

@@ -445,8 +445,8 @@ gm_iter_grad(const __grid_constant__ gpum::TmapDesc tmap, gpum::EvalArgs E, gpum
 // acce[a] (the epilogue has read it).  Every
 // wait is bounded; one that runs out sets DEV_ERR_TC_TIMEOUT and a CTA-wide
 // abort flag, the roles leave their loops, the control thread waits (bounded)
-// for its MMAs and copies, and the CTA frees its tensor memory and finishes
-// the chain block's bookkeeping.
+// for its MMAs and copies, and the CTA frees its tensor memory and writes its
+// partial.
 //
 // Packed data (gm_tc_pack, once per session): per tile of TN observations
 // [hi: KP/4 chunks][TN][4] | [lo: same] | [tail: NTAIL][TN] floats, i.e. the
@@ -545,7 +545,17 @@ gm_iter_value_tc(const float* __restrict__ xt, gpum::EvalArgs E, gpum::ChainArgs
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int cb = blockIdx.x, ob = blockIdx.y, tiles_per_cta = E.tiles_per_cta;
+  if (E.prior_pts) {
+    if (ob == 0) {
+      pdl_wait();
+      pdl_trigger();
+      prior_block<JitPrior>(E, A, cb, kTcM, kTcThreads);
+      return;
+    }
+    --ob;
+  }
   if (E.active) {  // delayed acceptance: geometry from the live count
+    pdl_wait();
     const int live = (int)*E.active;
     const int busy = (live + kTcM - 1) / kTcM;
     const int nob = da_obs_blocks(live, kTcM, (int)(gridDim.x * gridDim.y), E.ntiles,
@@ -567,7 +577,7 @@ gm_iter_value_tc(const float* __restrict__ xt, gpum::EvalArgs E, gpum::ChainArgs
   uint64_t* accf = tempty + kTcST;
   uint64_t* acce = accf + 2;
   uint64_t* drain = acce + 2;
-  uint32_t* misc = reinterpret_cast<uint32_t*>(drain + 1);  // TMEM base, ticket, abort
+  uint32_t* misc = reinterpret_cast<uint32_t*>(drain + 1);  // TMEM base, -, abort
   volatile uint32_t* abort_flag = misc + 2;
 
   const int t0 = ob * tiles_per_cta;
@@ -575,7 +585,22 @@ gm_iter_value_tc(const float* __restrict__ xt, gpum::EvalArgs E, gpum::ChainArgs
   const int nt = max(t1 - t0, 0);
   const int chain0 = cb * kTcM;
 
-  if (tid == 0) {
+  // The control thread's copies: tile k's product columns into operand stage
+  // k % S, its tail columns into tail slot k % ST.
+  auto load_b = [&](int k) {
+    const int s = k % kTcS;
+    mbar_expect_tx(&bfull[s], kTcStageFloats * 4);
+    bulk_load(stg + (size_t)s * kTcStageFloats, xt + (size_t)(t0 + k) * kTcTileFloats,
+              kTcStageFloats * 4, &bfull[s]);
+  };
+  auto load_t = [&](int k) {
+    const int s = k % kTcST;
+    mbar_expect_tx(&tfull[s], kTcTailFloats * 4);
+    bulk_load(tls + (size_t)s * kTcTailFloats,
+              xt + (size_t)(t0 + k) * kTcTileFloats + kTcStageFloats, kTcTailFloats * 4,
+              &tfull[s]);
+  };
+  if (tid == 32 * kTcEpiWarps) {
     for (int s = 0; s < kTcS; ++s) {
       mbar_init(&bfull[s], 1);
       mbar_init(&bempty[s], 1);
@@ -591,8 +616,16 @@ gm_iter_value_tc(const float* __restrict__ xt, gpum::EvalArgs E, gpum::ChainArgs
     mbar_init(drain, 1);
     misc[2] = 0;
     mbar_fence_init();
+    // The packed data does not change during a run: the first tiles are on
+    // their way before the previous step's proposals are waited for.
+    for (int k = 0; k < kTcS && k < nt; ++k) load_b(k);
+    if (GM_TC_NTAIL > 0)
+      for (int k = 0; k < kTcST && k < nt; ++k) load_t(k);
   }
+  __syncwarp();
   if (warp == kTcEpiWarps) tmem_alloc(&misc[0], kTcTmemCols);
+  pdl_wait();
+  pdl_trigger();
   // The coefficient operand, one chain per thread: [hi | lo] in the
   // canonical layout (core matrix (k/4, r/8) at (k/4 * 16 + r/8) * 128 bytes).
   if (tid < kTcM) {
@@ -635,23 +668,8 @@ gm_iter_value_tc(const float* __restrict__ xt, gpum::EvalArgs E, gpum::ChainArgs
       constexpr uint32_t idesc = umma_idesc_tf32(kTcM, kTcTN);
       constexpr uint32_t lbo_a = (kTcM / 8) * 128, lbo_b = (kTcTN / 8) * 128;
       const uint32_t a_hi = smem_addr(As), a_lo = a_hi + (uint32_t)kTcKP * kTcM * 4;
-      auto load_b = [&](int k) {
-        const int s = k % kTcS;
-        mbar_expect_tx(&bfull[s], kTcStageFloats * 4);
-        bulk_load(stg + (size_t)s * kTcStageFloats, xt + (size_t)(t0 + k) * kTcTileFloats,
-                  kTcStageFloats * 4, &bfull[s]);
-      };
-      auto load_t = [&](int k) {
-        const int s = k % kTcST;
-        mbar_expect_tx(&tfull[s], kTcTailFloats * 4);
-        bulk_load(tls + (size_t)s * kTcTailFloats,
-                  xt + (size_t)(t0 + k) * kTcTileFloats + kTcStageFloats, kTcTailFloats * 4,
-                  &tfull[s]);
-      };
-      int nb = 0, ntl = 0;  // tiles whose operands / tail columns were issued
-      for (; nb < kTcS && nb < nt; ++nb) load_b(nb);
-      if (GM_TC_NTAIL > 0)
-        for (; ntl < kTcST && ntl < nt; ++ntl) load_t(ntl);
+      // tiles whose operands / tail columns were issued
+      int nb = min(kTcS, nt), ntl = GM_TC_NTAIL > 0 ? min(kTcST, nt) : 0;
       for (int k = 0; k < nt; ++k) {
         if (*abort_flag) break;
         const int s = k % kTcS, acc = k & 1;
@@ -812,7 +830,5 @@ gm_iter_value_tc(const float* __restrict__ xt, gpum::EvalArgs E, gpum::ChainArgs
     for (int pt = 1; pt < kTcParts; ++pt) v += red[pt * kTcM + tid];
     E.partials[(size_t)ob * E.C_pad + chain0 + tid] = v;
   }
-  if (phase == PH_EVAL) return;
-  finish_chain_block<1, JitPrior>(E, A, cb, kTcM, phase, &misc[1], kTcThreads);
 }
 #endif  // GM_TC

@@ -72,6 +72,18 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// Programmatic dependent launch: a kernel launched with the attribute starts
+// while its predecessor still runs and may do what does not depend on it;
+// pdl_wait returns once the predecessor has completed and its writes are
+// visible (at once without the attribute), pdl_trigger lets the successor
+// start.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Nanosecond clock of the GPU, for waits bounded in time as well as polls.
 __device__ __forceinline__ uint64_t gm_globaltimer() {
   uint64_t t;

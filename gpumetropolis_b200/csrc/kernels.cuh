@@ -251,6 +251,475 @@ iter_kernel_grad(const __grid_constant__ GradProg prog, const __grid_constant__ 
   run_iteration<1, W, InterpGradBody<W>, InterpPrior>(&tmap, E, A, phase, body);
 }
 
+// -------------------------------------------------------------- MALA helpers
+// out = f * (1/2) M g, M = Ls Ls' (or diag sd^2), the whitened drift capped at
+// 2 sqrt(d) (MALTA; cpu_native.rs:617-651).
+__device__ inline void half_m_times(int np, const double* sd, const double* L, const double* g,
+                                    double* out, double* tmp) {
+  const double dmax = 2.0 * sqrt((double)np);
+  if (!L) {
+    for (int j = 0; j < np; ++j) tmp[j] = 0.5 * sd[j] * g[j];
+  } else {
+    for (int j = 0; j < np; ++j) {
+      double acc = 0.0;
+      for (int k = j; k < np; ++k) acc += L[(size_t)k * np + j] * g[k];
+      tmp[j] = 0.5 * acc;
+    }
+  }
+  double ss = 0.0;
+  for (int j = 0; j < np; ++j) ss += tmp[j] * tmp[j];
+  const double norm = sqrt(ss);
+  const double f = norm > dmax ? dmax / norm : 1.0;
+  if (!L) {
+    for (int j = 0; j < np; ++j) out[j] = f * sd[j] * tmp[j];
+  } else {
+    for (int k = 0; k < np; ++k) {
+      double acc = 0.0;
+      for (int j = 0; j <= k; ++j) acc += L[(size_t)k * np + j] * tmp[j];
+      out[k] = f * acc;
+    }
+  }
+}
+
+// -1/2 |Ls^{-1}(v - m)|^2 by forward substitution (cpu_native.rs:655-673).
+__device__ inline double log_q(int np, const double* sd, const double* L, const double* v,
+                               const double* m, double* tmp) {
+  double q = 0.0;
+  if (!L) {
+    for (int j = 0; j < np; ++j) {
+      const double r = (v[j] - m[j]) / sd[j];
+      q -= 0.5 * r * r;
+    }
+  } else {
+    for (int k = 0; k < np; ++k) {
+      double acc = v[k] - m[k];
+      for (int j = 0; j < k; ++j) acc -= L[(size_t)k * np + j] * tmp[j];
+      tmp[k] = acc / L[(size_t)k * np + k];
+      q -= 0.5 * tmp[k] * tmp[k];
+    }
+  }
+  return q;
+}
+
+// ------------------------------------------------------------- proposals
+// Next proposal of chain c into prop (f64) and params (f32).
+// Diagonal RWM chain_kernel.rs:212-223 / cpu_native.rs:726-735; Cholesky
+// RWM :224-249 / :736-753; DE on the frozen snapshot :250-295 / :754-784;
+// MALA :681-703 (mean from the cached gradient, then L z or sd * z).
+__device__ inline void propose(const ChainArgs& A, int c, Stream& rs, float* params, int C_pad) {
+  const int np = A.np;
+  const double* x = A.state + (size_t)c * np;
+  double* y = A.prop + (size_t)c * np;
+  const double* sd = A.sd + (size_t)c * np;
+  const double* L = A.L ? A.L + (size_t)c * np * np : nullptr;
+  if (A.mode == MODE_RWM) {
+    for (int j = 0; j < np; ++j) y[j] = x[j] + sd[j] * rs.normal();
+  } else if (A.mode == MODE_CHOL || A.mode == MODE_MALA) {
+    double* z = A.zbuf + (size_t)c * np;
+    const double* base = x;
+    if (A.mode == MODE_MALA) {
+      double* mx = A.mx + (size_t)c * np;
+      half_m_times(np, sd, L, A.gx + (size_t)c * np, mx, A.vbuf + (size_t)c * np);
+      for (int j = 0; j < np; ++j) mx[j] += x[j];
+      base = mx;
+    }
+    for (int j = 0; j < np; ++j) z[j] = rs.normal();
+    if (L) {
+      for (int k = 0; k < np; ++k) {
+        double acc = base[k];
+        for (int j = 0; j <= k; ++j) acc += L[(size_t)k * np + j] * z[j];
+        y[k] = acc;
+      }
+    } else {
+      for (int j = 0; j < np; ++j) y[j] = base[j] + sd[j] * z[j];
+    }
+  } else {
+    const int n = A.n_chains;
+    int a = (int)(rs.next() * (double)n);
+    if (a >= n) a = n - 1;
+    int b = (int)(rs.next() * (double)n);
+    if (b >= n) b = n - 1;
+    if (b == a) b = (b + 1) % n;
+    const double g = rs.next() < 0.1 ? 1.0 : A.gamma;
+    const double* pa = A.snap + (size_t)a * np;
+    const double* pb = A.snap + (size_t)b * np;
+    for (int j = 0; j < np; ++j) {
+      const double z = rs.normal();
+      const double diff = pa[j] - pb[j];
+      y[j] = x[j] + g * diff + A.de_noise * sd[j] * z;
+    }
+  }
+  for (int j = 0; j < np; ++j) params[(size_t)j * C_pad + c] = (float)y[j];
+}
+
+// Synchronous per-generation DE (path B, cpu_native.rs:400-506): the
+// difference vector comes from the current population, so this runs in its
+// own kernel after every chain's previous accept.  Partners a != c and
+// b != c, a (cpu_native.rs:430-440); g = 1 with probability 0.1, else gamma.
+__device__ inline void propose_desync(const ChainArgs& A, int c, Stream& rs, float* params,
+                                      int C_pad) {
+  const int n = A.n_chains, np = A.np;
+  int a = (int)(rs.next() * (double)n);
+  if (a >= n) a = n - 1;
+  if (a == c) a = (a + 1) % n;
+  int b = (int)(rs.next() * (double)n);
+  if (b >= n) b = n - 1;
+  while (b == c || b == a) b = (b + 1) % n;  // n >= 3 is checked by the host
+  const double g = rs.next() < 0.1 ? 1.0 : A.gamma;
+  const double* x = A.state + (size_t)c * np;
+  const double* pa = A.state + (size_t)a * np;
+  const double* pb = A.state + (size_t)b * np;
+  const double* sd = A.sd + (size_t)c * np;
+  double* y = A.prop + (size_t)c * np;
+  for (int j = 0; j < np; ++j) {
+    const double z = rs.normal();
+    y[j] = x[j] + g * (pa[j] - pb[j]) + A.de_noise * sd[j] * z;
+    params[(size_t)j * C_pad + c] = (float)y[j];
+  }
+}
+
+// ------------------------------------------------- one chain, one warp
+// The i-th uniform (i >= 1) a chain's stream `rs` would return from its
+// current position, without advancing it: both streams are counter-based, so
+// the lanes of a warp can draw a chain's normals in parallel.
+__device__ __forceinline__ double stream_at(const Stream& rs, uint32_t i) {
+  if (rs.kind == RNG_TRIPLE32) return t32_uniform(rs.seedmix, rs.ctr + i);
+  const U4 r = philox4x32_10(U4{rs.k + i - 1u, rs.it, rs.chain, 0xB2000001u}, rs.seed,
+                             0x6A09E667u);
+  return u53(r.x, r.y);
+}
+__device__ __forceinline__ double stream_normal_at(const Stream& rs, uint32_t i0, int j) {
+  const double u1 = stream_at(rs, i0 + 2u * (uint32_t)j + 1u);
+  const double u2 = stream_at(rs, i0 + 2u * (uint32_t)j + 2u);
+  return sqrt(-2.0 * log(u1)) * cos(6.283185307179586 * u2);
+}
+
+__device__ __forceinline__ double warp_sum64(double v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+// half_m_times by the lanes of a warp, added to `at`: out = at + f (1/2) M g.
+// L has leading dimension ldL (shared or global memory); tmp: np doubles of
+// shared memory.
+__device__ __forceinline__ void half_m_warp(int np, const double* sd, const double* L, int ldL,
+                                            const double* g, const double* at, double* out,
+                                            double* tmp, int lane) {
+  double ss = 0.0;
+  for (int j = lane; j < np; j += 32) {
+    double v;
+    if (!L) {
+      v = 0.5 * sd[j] * g[j];
+    } else {
+      double acc = 0.0;
+      for (int k = j; k < np; ++k) acc += L[(size_t)k * ldL + j] * g[k];
+      v = 0.5 * acc;
+    }
+    tmp[j] = v;
+    ss += v * v;
+  }
+  const double norm = sqrt(warp_sum64(ss)), dmax = 2.0 * sqrt((double)np);
+  const double f = norm > dmax ? dmax / norm : 1.0;
+  __syncwarp();
+  for (int k = lane; k < np; k += 32) {
+    double v;
+    if (!L) {
+      v = f * sd[k] * tmp[k];
+    } else {
+      double acc = 0.0;
+      for (int j = 0; j <= k; ++j) acc += L[(size_t)k * ldL + j] * tmp[j];
+      v = f * acc;
+    }
+    out[k] = v + at[k];
+  }
+  __syncwarp();
+}
+
+// log_q(x | mx') - log_q(y | my'), the MALA proposal ratio, by the lanes of a
+// warp: r1 = x - my and r2 = y - mx through one forward substitution, column
+// by column (each row subtracts its terms in the serial order), so its serial
+// chain is np divisions long instead of np^2 products.  r1, r2: np doubles of
+// shared memory each.
+__device__ __forceinline__ double log_q_ratio_warp(int np, const double* sd, const double* L,
+                                                   int ldL, const double* x, const double* my,
+                                                   const double* y, const double* mx, double* r1,
+                                                   double* r2, int lane) {
+  double q = 0.0;
+  if (!L) {
+    for (int j = lane; j < np; j += 32) {
+      const double a = (x[j] - my[j]) / sd[j], b = (y[j] - mx[j]) / sd[j];
+      q += 0.5 * b * b - 0.5 * a * a;
+    }
+    return warp_sum64(q);
+  }
+  for (int j = lane; j < np; j += 32) {
+    r1[j] = x[j] - my[j];
+    r2[j] = y[j] - mx[j];
+  }
+  __syncwarp();
+  for (int j = 0; j < np; ++j) {
+    const double d = L[(size_t)j * ldL + j];
+    const double t1 = r1[j] / d, t2 = r2[j] / d;
+    for (int k = j + 1 + lane; k < np; k += 32) {
+      const double l = L[(size_t)k * ldL + j];
+      r1[k] -= l * t1;
+      r2[k] -= l * t2;
+    }
+    q += 0.5 * t2 * t2 - 0.5 * t1 * t1;
+    __syncwarp();
+  }
+  return q;
+}
+
+// propose() for chain c by the 32 lanes of a warp: the same draws, one
+// coordinate per lane.  L: the chain's factor with leading dimension ldL
+// (global or staged in shared memory), or nullptr; `sm` is this warp's
+// scratch of 2 np doubles.  Returns the stream advanced past the draws.
+__device__ inline Stream propose_warp(const ChainArgs& A, int c, Stream rs, float* params,
+                                      int C_pad, int lane, double* sm, const double* L, int ldL) {
+  const int np = A.np;
+  const double* x = A.state + (size_t)c * np;
+  double* y = A.prop + (size_t)c * np;
+  const double* sd = A.sd + (size_t)c * np;
+  uint32_t used = 2u * (uint32_t)np;
+  float* out = params + c;
+  if (A.mode == MODE_CHOL || A.mode == MODE_MALA) {
+    double* z = sm;
+    const double* base = x;
+    if (A.mode == MODE_MALA) {  // mean = x + f (1/2) M g (cpu_native.rs:617-651)
+      double* mx = A.mx + (size_t)c * np;
+      half_m_warp(np, sd, L, ldL, A.gx + (size_t)c * np, x, mx, z, lane);
+      base = mx;
+    }
+    for (int j = lane; j < np; j += 32) z[j] = stream_normal_at(rs, 0, j);
+    __syncwarp();
+    for (int k = lane; k < np; k += 32) {
+      double v;
+      if (L) {
+        v = base[k];
+        for (int j = 0; j <= k; ++j) v += L[(size_t)k * ldL + j] * z[j];
+      } else {
+        v = base[k] + sd[k] * z[k];
+      }
+      y[k] = v;
+      out[(size_t)k * C_pad] = (float)v;
+    }
+  } else {
+    const double *pa = x, *pb = x;
+    double g = 0.0, noise = 1.0;
+    uint32_t i0 = 0;
+    if (A.mode == MODE_DE) {  // the pair of the snapshot
+      const int n = A.n_chains;
+      int a = (int)(stream_at(rs, 1) * (double)n);
+      if (a >= n) a = n - 1;
+      int b = (int)(stream_at(rs, 2) * (double)n);
+      if (b >= n) b = n - 1;
+      if (b == a) b = (b + 1) % n;
+      g = stream_at(rs, 3) < 0.1 ? 1.0 : A.gamma;
+      pa = A.snap + (size_t)a * np;
+      pb = A.snap + (size_t)b * np;
+      noise = A.de_noise;
+      i0 = 3;
+    }
+    for (int j = lane; j < np; j += 32) {
+      const double z = stream_normal_at(rs, i0, j);
+      const double v = i0 ? x[j] + g * (pa[j] - pb[j]) + noise * sd[j] * z : x[j] + sd[j] * z;
+      y[j] = v;
+      out[(size_t)j * C_pad] = (float)v;
+    }
+    used += i0;
+  }
+  __syncwarp();
+  if (rs.kind == RNG_TRIPLE32) rs.ctr += used;
+  else rs.k += used;
+  return rs;
+}
+
+// ------------------------------------------------------------ partial sums
+// The sums over the observation blocks of chain c's first W of Ws values,
+// partials [nob][C_pad][Ws], by the `wpc` warps of a group (wi: this warp's
+// number in it); red: [wpc][W] doubles of shared memory.  With one value the threads
+// take the blocks, with several the lanes take the values (coalesced) and the
+// warps the blocks.  Every __syncthreads of the block is reached by all.
+__device__ __forceinline__ void group_partials(const double* __restrict__ partials, int nob,
+                                               int C_pad, int Ws, int W, int c, int wi,
+                                               int wpc, double* red, int lane) {
+  if (W == 1) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int o = wi * 32 + lane; o < nob; o += 32 * wpc)
+      v += __ldcg(&partials[((size_t)o * C_pad + c) * Ws]);
+    v = warp_sum64(v);
+    if (lane == 0) red[wi] = v;
+  } else {
+    for (int w = lane; w < W; w += 32) {
+      const double* p = partials + (size_t)c * Ws + w;
+      const size_t st = (size_t)C_pad * Ws;
+      double v = 0.0;
+#pragma unroll 8
+      for (int o = wi; o < nob; o += wpc) v += __ldcg(&p[(size_t)o * st]);
+      red[(size_t)wi * W + w] = v;
+    }
+  }
+}
+__device__ __forceinline__ double group_total(const double* red, int W, int w, int wpc) {
+  double v = red[w];
+  for (int i = 1; i < wpc; ++i) v += red[(size_t)i * W + w];
+  return v;
+}
+
+// Sums of each point's values w0 .. W - 1 into out[point][W - w0]: one group of
+// wpc warps per point.  A single thread per value over all observation blocks
+// took 25 us for 250 points of 18 values.
+static __global__ void __launch_bounds__(kThreads)
+reduce_partials_kernel(const double* __restrict__ partials, double* __restrict__ out, int nob,
+                       int C_pad, int Ws, int n, int W, int w0, int wpc) {
+  extern __shared__ double rsm[];  // [8][W]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wi = warp % wpc, c = (int)blockIdx.x * (kWarps / wpc) + warp / wpc;
+  double* red = rsm + (size_t)(warp / wpc) * wpc * W;
+  if (c < n) group_partials(partials, nob, C_pad, Ws, W, c, wi, wpc, red, lane);
+  __syncthreads();
+  if (wi != 0 || c >= n) return;
+  for (int w = w0 + lane; w < W; w += 32)
+    out[(size_t)c * (W - w0) + w - w0] = group_total(red, W, w, wpc);
+}
+
+// ------------------------------------------------------------- a step's end
+// What a Metropolis step does after the evaluation of its proposals: the
+// partial sums added up, the f64 prior, the accept decision on the f64 totals
+// (MALA with the proposal ratio), the draw, the next proposal.  `wpc` warps
+// per chain: all of them add the chain's partials, the first one does the
+// rest, a coordinate per lane.
+//
+// It is bound by latency (the loads, log and cos in f64, np steps of the
+// Langevin substitution), not by any rate.  Run by one thread per chain in the
+// last CTA of each chain block it took 30 us at 1,024 chains x 17 parameters,
+// 144 us at 2,048 x 65 (DE) and 620 us at 2,048 x 24 (MALA with a factor) of
+// every iteration, on at most a few SMs.  The factor is staged in shared
+// memory before the wait for the evaluation, when it fits.
+struct StepArgs {
+  const double* partials;    // [nob][C_pad][Ws], W values of each used
+  int nob, C_pad, Ws, W;
+  const double* prior;       // [C], or nullptr: no prior
+  const double* prior_grad;  // [C][np] (MALA)
+  float* params;             // [np][C_pad] evaluation points of the next step
+  int phase;                 // PH_INIT or PH_STEP
+  int wpc;                   // warps per chain: 1, 2, 4 or 8
+  int wpb;                   // warps per block
+  int stage_L;               // 1: factors staged in shared memory
+};
+// Doubles of shared memory per chain: partial sums, 3 np scratch (the factor's
+// leading dimension is odd, so a column of it spreads over the banks).
+__host__ __device__ inline int step_ld(int np) { return np | 1; }
+__host__ __device__ inline size_t step_smem_doubles(int np, int W, int wpc, bool stage_L) {
+  return (size_t)wpc * W + 3 * (size_t)np + (stage_L ? (size_t)np * step_ld(np) : 0);
+}
+
+static __global__ void __launch_bounds__(kThreads) step_kernel(ChainArgs A, StepArgs S) {
+  extern __shared__ double ssm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wpc = S.wpc, wi = warp % wpc, grp = warp / wpc;
+  const int c = (int)blockIdx.x * (S.wpb / wpc) + grp;
+  const int np = A.np;
+  double* red = ssm + (size_t)grp * step_smem_doubles(np, S.W, wpc, S.stage_L != 0);
+  double* tmp = red + (size_t)wpc * S.W;  // [3][np]
+  const bool live = c < A.n_chains;
+  const double* L = A.L && live ? A.L + (size_t)c * np * np : nullptr;
+  int ldL = np;
+  if (L && S.stage_L) {  // set by the host before the run: no wait needed
+    double* Ls = tmp + 3 * np;
+    ldL = step_ld(np);
+    for (int i = wi * 32 + lane; i < np * np; i += 32 * wpc)
+      Ls[(i / np) * ldL + i % np] = L[i];
+    L = Ls;
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (live) group_partials(S.partials, S.nob, S.C_pad, S.Ws, S.W, c, wi, wpc, red, lane);
+  __syncthreads();
+  if (wi != 0 || !live) return;
+
+  const size_t o = (size_t)c * np;
+  const bool mala = A.mode == MODE_MALA;
+  double* x = A.state + o;
+  const double* sd = A.sd + o;
+  const uint32_t t = A.iter[c];
+  Stream rs = make_stream(A, c);
+  const double b = A.beta ? A.beta[c] : 1.0;  // likelihood power
+  const double ll = group_total(red, S.W, 0, wpc);
+  const double lp = (A.beta ? b * ll : ll) + (S.prior ? S.prior[c] : 0.0);
+  if (mala) {
+    double* g = (S.phase == PH_INIT ? A.gx : A.gy) + o;
+    for (int j = lane; j < np; j += 32) {
+      const double v = b * group_total(red, S.W, 1 + j, wpc);
+      g[j] = S.prior_grad ? v + S.prior_grad[o + j] : v;
+    }
+    __syncwarp();
+  }
+  if (S.phase == PH_INIT) {
+    if (lane == 0) {
+      A.cur[c] = lp;
+      A.last_eval[c] = lp;
+    }
+    if (A.n_iter == 0 || A.mode == MODE_DESYNC) return;  // path B proposes in its own kernel
+    rs.it = 0;
+  } else {
+    const double* y = A.prop + o;
+    const double cur = A.cur[c];
+    double lqd = 0.0;
+    if (mala) {
+      // q(x | y) - q(y | x) with the truncated drift at y (cpu_native.rs:704-710)
+      double* my = A.my + o;
+      half_m_warp(np, sd, L, ldL, A.gy + o, y, my, tmp, lane);
+      lqd = log_q_ratio_warp(np, sd, L, ldL, x, my, y, A.mx + o, tmp, tmp + np, lane);
+    }
+    if (A.rng != RNG_TRIPLE32) {
+      rs.it = t;
+      rs.k = 0xFFFF0000u;
+    }
+    const double u = rs.next();
+    // Tempered acceptance on the f64 totals (chain_kernel.rs:334,
+    // cpu_native.rs:792); MALA adds the proposal ratio and requires a
+    // finite proposal log density (cpu_native.rs:713-714).
+    const bool take = mala ? (isfinite(lp) && log(u) < (lp - cur) / A.temp[c] + lqd)
+                           : (log(u) < (lp - cur) / A.temp[c]);
+    if (A.rec_ll) {
+      const uint64_t slot = A.rec_base + (uint64_t)t * A.n_chains + c;
+      if (slot < A.rec_cap) {
+        for (int j = lane; j < np; j += 32) A.rec_theta[slot * np + j] = (float)y[j];
+        if (lane == 0) A.rec_ll[slot] = ll;
+      }
+    }
+    for (int j = lane; j < np; j += 32) {
+      const double v = take ? y[j] : x[j];
+      if (take) {
+        x[j] = v;
+        if (mala) A.gx[o + j] = A.gy[o + j];
+      }
+      if (t < A.n_iter) A.draws[((size_t)t * np + j) * S.C_pad + c] = (float)v;
+    }
+    if (lane == 0) {
+      A.last_eval[c] = lp;
+      if (take) {
+        A.cur[c] = lp;
+        A.accepts[c] += 1;
+      }
+      A.iter[c] = t + 1;
+    }
+    __syncwarp();
+    if (t + 1 >= A.n_iter || A.mode == MODE_DESYNC) {
+      if (lane == 0) A.ctr[c] = rs.ctr;
+      return;
+    }
+    rs.it = t + 1;
+    rs.k = 0;
+  }
+  rs = propose_warp(A, c, rs, S.params, S.C_pad, lane, tmp, L, ldL);
+  if (lane == 0) A.ctr[c] = rs.ctr;
+}
+
 // ------------------------------------------------------------- helpers
 // Row-major f64 rows [r0, r0+nr) -> column-major f32 [ncols][ld].
 static __global__ void convert_rows_kernel(const double* __restrict__ src, float* __restrict__ dst,
@@ -631,113 +1100,6 @@ static __global__ void da_pack_kernel(ChainArgs A, DaArgs D) {
   D.params[(size_t)j * D.C_pad + D.slot[c]] = (float)A.prop[i];
 }
 
-// The i-th uniform (i >= 1) a chain's stream `rs` would return from its
-// current position, without advancing it: both streams are counter-based, so
-// the lanes of a warp can draw a chain's normals in parallel.
-__device__ __forceinline__ double stream_at(const Stream& rs, uint32_t i) {
-  if (rs.kind == RNG_TRIPLE32) return t32_uniform(rs.seedmix, rs.ctr + i);
-  const U4 r = philox4x32_10(U4{rs.k + i - 1u, rs.it, rs.chain, 0xB2000001u}, rs.seed,
-                             0x6A09E667u);
-  return u53(r.x, r.y);
-}
-__device__ __forceinline__ double stream_normal_at(const Stream& rs, uint32_t i0, int j) {
-  const double u1 = stream_at(rs, i0 + 2u * (uint32_t)j + 1u);
-  const double u2 = stream_at(rs, i0 + 2u * (uint32_t)j + 2u);
-  return sqrt(-2.0 * log(u1)) * cos(6.283185307179586 * u2);
-}
-
-// propose() for chain c by the 32 lanes of a warp: the same draws, the same
-// arithmetic per coordinate (each lane runs one coordinate's loops in the
-// serial order; the drift norm is summed by lane 0 in coordinate order), so
-// the proposal equals the serial one bit for bit.  `sm` is this warp's
-// scratch of 2 np doubles.  Returns the stream advanced past the draws.
-__device__ inline Stream propose_warp(const ChainArgs& A, int c, Stream rs, float* params,
-                                      int C_pad, int lane, double* sm) {
-  const int np = A.np;
-  const double* x = A.state + (size_t)c * np;
-  double* y = A.prop + (size_t)c * np;
-  const double* sd = A.sd + (size_t)c * np;
-  const double* L = A.L ? A.L + (size_t)c * np * np : nullptr;
-  uint32_t used = 2u * (uint32_t)np;
-  if (A.mode == MODE_RWM) {
-    for (int j = lane; j < np; j += 32) y[j] = x[j] + sd[j] * stream_normal_at(rs, 0, j);
-  } else if (A.mode == MODE_CHOL || A.mode == MODE_MALA) {
-    double* z = sm;
-    double* base = sm + np;
-    if (A.mode == MODE_MALA) {
-      // mean = x + f (1/2) M g (half_m_times, cpu_native.rs:617-651)
-      const double* gx = A.gx + (size_t)c * np;
-      double* tmp = z;  // reused for z below, after the mean is built
-      for (int j = lane; j < np; j += 32) {
-        double acc = 0.0;
-        if (!L) {
-          tmp[j] = 0.5 * sd[j] * gx[j];
-        } else {
-          for (int k = j; k < np; ++k) acc += L[(size_t)k * np + j] * gx[k];
-          tmp[j] = 0.5 * acc;
-        }
-      }
-      __syncwarp();
-      double f = 1.0;
-      if (lane == 0) {
-        double ss = 0.0;
-        for (int j = 0; j < np; ++j) ss += tmp[j] * tmp[j];
-        const double norm = sqrt(ss), dmax = 2.0 * sqrt((double)np);
-        f = norm > dmax ? dmax / norm : 1.0;
-      }
-      f = __shfl_sync(0xffffffffu, f, 0);
-      double* mx = A.mx + (size_t)c * np;
-      for (int k = lane; k < np; k += 32) {
-        double out;
-        if (!L) {
-          out = f * sd[k] * tmp[k];
-        } else {
-          double acc = 0.0;
-          for (int j = 0; j <= k; ++j) acc += L[(size_t)k * np + j] * tmp[j];
-          out = f * acc;
-        }
-        mx[k] = out + x[k];
-        base[k] = mx[k];
-      }
-    } else {
-      for (int k = lane; k < np; k += 32) base[k] = x[k];
-    }
-    __syncwarp();
-    for (int j = lane; j < np; j += 32) z[j] = stream_normal_at(rs, 0, j);
-    __syncwarp();
-    for (int k = lane; k < np; k += 32) {
-      if (L) {
-        double acc = base[k];
-        for (int j = 0; j <= k; ++j) acc += L[(size_t)k * np + j] * z[j];
-        y[k] = acc;
-      } else {
-        y[k] = base[k] + sd[k] * z[k];
-      }
-    }
-  } else {  // DE on the snapshot
-    const int n = A.n_chains;
-    int a = (int)(stream_at(rs, 1) * (double)n);
-    if (a >= n) a = n - 1;
-    int b = (int)(stream_at(rs, 2) * (double)n);
-    if (b >= n) b = n - 1;
-    if (b == a) b = (b + 1) % n;
-    const double g = stream_at(rs, 3) < 0.1 ? 1.0 : A.gamma;
-    const double* pa = A.snap + (size_t)a * np;
-    const double* pb = A.snap + (size_t)b * np;
-    for (int j = lane; j < np; j += 32) {
-      const double zj = stream_normal_at(rs, 3, j);
-      const double diff = pa[j] - pb[j];
-      y[j] = x[j] + g * diff + A.de_noise * sd[j] * zj;
-    }
-    used += 3u;
-  }
-  for (int j = lane; j < np; j += 32) params[(size_t)j * C_pad + c] = (float)y[j];
-  __syncwarp();
-  if (rs.kind == RNG_TRIPLE32) rs.ctr += used;
-  else rs.k += used;
-  return rs;
-}
-
 // Stage 2 for the survivors, the draw for every chain, the next proposal.
 // One warp per chain: the lanes add the chain's observation-block partials in
 // a fixed lane-strided order and a fixed shuffle tree (deterministic), lane 0
@@ -799,7 +1161,8 @@ static __global__ void da_finalize_kernel(ChainArgs A, DaArgs D, const double* _
   if (t + 1 < A.n_iter) {
     rs.it = t + 1;
     rs.k = 0;
-    rs = propose_warp(A, c, rs, D.full, D.C_pad, lane, fin_sm + (size_t)(threadIdx.x >> 5) * 2 * np);
+    rs = propose_warp(A, c, rs, D.full, D.C_pad, lane, fin_sm + (size_t)(threadIdx.x >> 5) * 2 * np,
+                      A.L ? A.L + (size_t)c * np * np : nullptr, np);
   }
   if (lane == 0) A.ctr[c] = rs.ctr;
 }

@@ -243,7 +243,6 @@ extern "C" int gpum_b200_loglik_batch_noalloc(
   E.params = d_params;
   E.partials = d_part;
   E.n_points = n;
-  E.tickets = nullptr;  // PH_EVAL takes no ticket
   E.err = d_err;
   ChainArgs A{};
 
@@ -258,7 +257,8 @@ extern "C" int gpum_b200_loglik_batch_noalloc(
     case 4: iter_kernel<4, 16><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, PH_EVAL); break;
     default: iter_kernel<2, 32><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, PH_EVAL); break;
   }
-  reduce_partials_kernel<<<(n + 255) / 256, 256, 0, st>>>(d_part, d_out, nob, C_pad, n, 1);
+  reduce_partials_kernel<<<(n + kWarps - 1) / kWarps, kThreads, sizeof(double) * kWarps, st>>>(
+      d_part, d_out, nob, C_pad, 1, n, 1, 0, 1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     if (err && err_len) std::snprintf(err, err_len, "launch failed: %s", cudaGetErrorString(e));
