@@ -184,7 +184,7 @@ struct KernelChoice {
   const void* fn = nullptr;  // __global__ pointer or cudaKernel_t
   int G = 8;                 // chains per thread (per warp for a chain-lane body)
   int W = 1;                 // values per chain (1, or 1 + np with the gradient)
-  bool lanes = false;        // chain-lane body: G = 32 chains per warp group
+  bool lanes = false;        // chain-lane body: G = 32 or 64 chains per warp group
   bool grad_interp = false;  // the interpreter engine's gradient (tape) kernel
   bool tc = false;           // the compiled engine's tensor-core value kernel
   int threads = kThreads;    // threads per CTA
@@ -384,8 +384,10 @@ struct gpum_b200_session {
   bool ext(const KernelChoice& k) const { return k.compiled && cm.n_mat > 0; }
 
   // `pointwise`: per-observation output, which the tensor-core value kernel
-  // does not write.
-  KernelChoice choose(bool need_grad, bool pointwise = false) {
+  // does not write.  Gradients of more than 256 points run two chains per lane:
+  // its eight warps of 64 then share no chain, as the eight of 32 share none
+  // above 224, so every chain's FP32 blocks are the same on either kernel.
+  KernelChoice choose(int n, bool need_grad, bool pointwise = false) {
     KernelChoice k;
     // Gradients: the compiled engine's adjoint unless the interpreter engine
     // was chosen or NVRTC cannot build the model; then the interpreted tape.
@@ -414,6 +416,10 @@ struct gpum_b200_session {
       k.fn = need_grad ? (const void*)cm.k_grad : (const void*)cm.k_value;
       k.lanes = need_grad ? cm.lanes_grad : cm.lanes;
       k.G = k.lanes ? 32 : (need_grad ? cm.GG : cm.G);
+      if (need_grad && cm.k_grad2 && n > 256) {
+        k.fn = (const void*)cm.k_grad2;
+        k.G = 64;
+      }
       k.W = need_grad ? 1 + (int)np : 1;
       if (!need_grad && !pointwise && tc_ok) {
         k.tc = true;
@@ -469,7 +475,7 @@ struct gpum_b200_session {
 
   // Evaluation-argument block for `n` points (params in `params`).
   void setup_eval(int n, bool need_grad, bool pointwise = false) {
-    kc = choose(need_grad, pointwise);
+    kc = choose(n, need_grad, pointwise);
     geo = geometry(n, kc);
     if (geo.smem + static_smem(kc.fn) > 48 * 1024)
       GPUM_CK(cudaFuncSetAttribute(kc.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,

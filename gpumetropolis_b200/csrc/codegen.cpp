@@ -13,6 +13,7 @@
 //   float  gm_value_grad(d, p, h, float* gp, float* gh)  gp/gh accumulated
 //   void   gm_value_grad4l(const float* xo, int nv, p, h, float* gp, float* gh,
 //                          float* out)  four observations, chain-lane body
+//   void   gm_value_grad4l2(xo, nv, p, h, gp, gh, out)  for two chains
 //   void   gm_hoist_grad(const float* p, const float* gh, float* gp)
 //   double gm_prior(const double* p)
 //   double gm_prior_grad(const double* p, double* g)     g accumulated
@@ -903,11 +904,24 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
   // (forward as gm_value_grad, no value rewrites).  The reverse sweep reloads
   // the data columns it needs (gm_lds4v) rather than keeping the forward's
   // loads live.  Observations k >= nv (a partial last quad) read observation
-  // 0's data and enter the sweep with adjoint 0.
-  s << "__device__ __forceinline__ void gm_value_grad4l(const float* __restrict__ xo, int nv, "
-       "const float* __restrict__ p, const float* __restrict__ h, float* __restrict__ gp, "
-       "float* __restrict__ gh, float* __restrict__ out) {\n";
-  {
+  // 0's data and enter the sweep with adjoint 0.  gm_value_grad4l2: the same
+  // for two chains, each with the arithmetic of the first form in its order,
+  // so that one load of a column serves both.
+  for (int CH = 1; CH <= 2; ++CH) {
+    const bool two = CH == 2;
+    s << "__device__ __forceinline__ void gm_value_grad4l" << (two ? "2" : "")
+      << "(const float* __restrict__ xo, int nv, "
+      << (two ? "const float (&p)[2][GM_NP], const float (&h)[2][GM_NH], float (&gp)[2][GM_NP], "
+                "float (&gh)[2][GM_NH], float (&out)[2][4]) {\n"
+              : "const float* __restrict__ p, const float* __restrict__ h, "
+                "float* __restrict__ gp, float* __restrict__ gh, float* __restrict__ out) {\n");
+    // element j of chain c's array; lane (chain c, observation k) of a value
+    auto elem = [&](const char* arr, int c, int j) {
+      return std::string(arr) + (two ? "[" + std::to_string(c) + "]" : "") + "[" +
+             std::to_string(j) + "]";
+    };
+    const int NL = 4 * CH;  // value lanes: l = 4 c + k
+    auto sfx = [&](int l) { return "_" + std::to_string(l); };
     std::vector<char> fl(N, 0), rl(N, 0);
     auto data4 = [&](int i, int k, bool reload) -> std::string {
       std::vector<char>& L = reload ? rl : fl;
@@ -924,47 +938,50 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
       }
       return q + "_" + std::to_string(k);
     };
-    auto ref4g = [&](int i, int k, bool reload) -> std::string {
+    auto ref4g = [&](int i, int l, bool reload) -> std::string {
       const Node& x = g.n[i];
-      if (x.op == O_C || x.op == O_P) return name[i];
-      if (hslot[i] >= 0) return "h[" + std::to_string(hslot[i]) + "]";
-      if (dslot[i] >= 0) return data4(i, k, reload);
-      return name[i] + "_" + std::to_string(k);
+      if (x.op == O_C) return name[i];
+      if (x.op == O_P) return elem("p", l / 4, (int)x.arg);
+      if (hslot[i] >= 0) return elem("h", l / 4, hslot[i]);
+      if (dslot[i] >= 0) return data4(i, l % 4, reload);
+      return name[i] + sfx(l);
     };
     for (int i = 0; i < N; ++i) {
       if (!live[i] || !is_pd(i)) continue;
       const Node& x = g.n[i];
-      std::string a[4], b[4];
-      for (int k = 0; k < 4; ++k) {
-        a[k] = ref4g(x.a, k, false);
-        if (x.b >= 0) b[k] = ref4g(x.b, k, false);
+      std::vector<std::string> av(NL), bv(NL);
+      for (int l = 0; l < NL; ++l) {
+        av[l] = ref4g(x.a, l, false);
+        if (x.b >= 0) bv[l] = ref4g(x.b, l, false);
       }
-      const std::string rb = recip(i) >= 0 ? "h[" + std::to_string(recip(i)) + "]" : "";
-      for (int k = 0; k < 4; ++k)
-        s << "  const float " << name[i] << "_" << k << " = "
-          << (rb.empty() ? op_expr(g, i, a[k], b[k], true) : "(" + a[k] + " * " + rb + ")")
+      for (int l = 0; l < NL; ++l)
+        s << "  const float " << name[i] << sfx(l) << " = "
+          << (recip(i) < 0 ? op_expr(g, i, av[l], bv[l], true)
+                           : "(" + av[l] + " * " + elem("h", l / 4, recip(i)) + ")")
           << ";\n";
     }
     for (int i = 0; i < N; ++i)
       if (live[i] && is_pd(i))
-        for (int k = 0; k < 4; ++k) s << "  float g" << i << "_" << k << " = 0.0f;\n";
+        for (int l = 0; l < NL; ++l) s << "  float g" << i << sfx(l) << " = 0.0f;\n";
     std::vector<char> has_adj(N, 0);
-    auto sink4 = [&](int c, const std::string* e) {
+    auto sink4 = [&](int c, const std::vector<std::string>& e) {
       if (c < 0 || !(g.n[c].dep & DEP_P)) return;
-      for (int k = 0; k < 4; ++k) {
-        if (g.n[c].op == O_P) s << "  gp[" << g.n[c].arg << "] += " << e[k] << ";\n";
-        else if (hslot[c] >= 0) s << "  gh[" << hslot[c] << "] += " << e[k] << ";\n";
+      for (int l = 0; l < NL; ++l) {
+        if (g.n[c].op == O_P)
+          s << "  " << elem("gp", l / 4, (int)g.n[c].arg) << " += " << e[l] << ";\n";
+        else if (hslot[c] >= 0)
+          s << "  " << elem("gh", l / 4, hslot[c]) << " += " << e[l] << ";\n";
         else
-          s << "  g" << c << "_" << k << (has_adj[c] ? " += " : " = ") << e[k] << ";\n";
+          s << "  g" << c << sfx(l) << (has_adj[c] ? " += " : " = ") << e[l] << ";\n";
       }
       if (g.n[c].op != O_P && hslot[c] < 0) has_adj[c] = 1;
     };
     if (root >= 0 && (g.n[root].dep & DEP_P)) {
-      std::string w[4];
-      for (int k = 0; k < 4; ++k)
-        w[k] = k == 0 ? "1.0f" : "(nv > " + std::to_string(k) + " ? 1.0f : 0.0f)";
+      std::vector<std::string> w(NL);
+      for (int l = 0; l < NL; ++l)
+        w[l] = l % 4 == 0 ? "1.0f" : "(nv > " + std::to_string(l % 4) + " ? 1.0f : 0.0f)";
       if (is_pd(root)) {
-        for (int k = 0; k < 4; ++k) s << "  g" << root << "_" << k << " = " << w[k] << ";\n";
+        for (int l = 0; l < NL; ++l) s << "  g" << root << sfx(l) << " = " << w[l] << ";\n";
         has_adj[root] = 1;
       } else {
         sink4(root, w);
@@ -973,24 +990,22 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
     for (int i = N - 1; i >= 0; --i) {
       if (!live[i] || !is_pd(i)) continue;
       const Node& x = g.n[i];
-      std::vector<std::vector<std::pair<int, std::string>>> ce(4);
-      for (int k = 0; k < 4; ++k) {
-        const std::string G = "g" + std::to_string(i) + "_" + std::to_string(k);
-        const std::string v = name[i] + "_" + std::to_string(k);
-        ce[k] = adjoints(g, i, G, v, ref4g(x.a, k, true), x.b >= 0 ? ref4g(x.b, k, true) : "",
-                         true, recip(i) >= 0 ? "h[" + std::to_string(recip(i)) + "]" : "");
-      }
+      std::vector<std::vector<std::pair<int, std::string>>> ce(NL);
+      for (int l = 0; l < NL; ++l)
+        ce[l] = adjoints(g, i, "g" + std::to_string(i) + sfx(l), name[i] + sfx(l),
+                         ref4g(x.a, l, true), x.b >= 0 ? ref4g(x.b, l, true) : "", true,
+                         recip(i) >= 0 ? elem("h", l / 4, recip(i)) : "");
       for (size_t j = 0; j < ce[0].size(); ++j) {
-        std::string e[4];
-        for (int k = 0; k < 4; ++k) e[k] = ce[k][j].second;
+        std::vector<std::string> e(NL);
+        for (int l = 0; l < NL; ++l) e[l] = ce[l][j].second;
         sink4(ce[0][j].first, e);
       }
     }
-    for (int k = 0; k < 4; ++k)
-      s << "  out[" << k << "] = " << (root < 0 ? std::string("0.0f") : ref4g(root, k, false))
-        << ";\n";
+    for (int l = 0; l < NL; ++l)
+      s << "  " << (two ? elem("out", l / 4, l % 4) : "out[" + std::to_string(l) + "]") << " = "
+        << (root < 0 ? std::string("0.0f") : ref4g(root, l, false)) << ";\n";
+    s << "  (void)xo; (void)nv; (void)p; (void)h; (void)gp; (void)gh;\n}\n";
   }
-  s << "  (void)xo; (void)nv; (void)p; (void)h; (void)gp; (void)gh;\n}\n";
 
   // Chain rule through the hoisted parameter-only nodes, once per chain.
   s << "__device__ __forceinline__ void gm_hoist_grad(const float* __restrict__ p, "

@@ -298,8 +298,9 @@ __host__ __device__ inline size_t skel_smem_bytes(int T, int ncols, int np, int 
 
 // Body contract (G chains per thread):
 //   bool kChainLanes                       false: lanes are observations (below);
-//                                          true: lanes are chains, G = 32 counts
-//                                          the chains of a warp, and the body has
+//                                          true: lanes are chains, G counts the
+//                                          chains of a warp (32 kLaneChains: lane
+//                                          l holds l, l + 32, ...), the body has
 //                                          begin_lanes(pc, C_pad), eval4(xo, nv),
 //                                          last4(k) instead of begin/eval/last
 //   bool kLanesAcc (chain lanes)           true: the body accumulates values
@@ -381,7 +382,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   }
   __syncthreads();
   if constexpr (kLanes) {
-    const float* pc = E.params + (size_t)cb * CG + (size_t)wc * 32 + lane;
+    const float* pc = E.params + (size_t)cb * CG + (size_t)wc * G + lane;
     if constexpr (Body::kLanesAcc)
       body.begin_lanes_acc(pc, E.C_pad, red + ((size_t)warp * G + lane) * W);
     else
@@ -495,8 +496,12 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   // tree), then the WO warps that share a chain group, in warp order.
 #pragma unroll
   for (int w = 0; w < W; ++w) {
-    if constexpr (kLanes) {  // each lane holds its own chain's sum (G == 32)
-      if (!Body::kLanesAcc || w == 0) red[((size_t)warp * G + lane) * W + w] = body.total(0, w);
+    if constexpr (kLanes) {  // each lane holds its own chains' sums
+      if (!Body::kLanesAcc || w == 0) {
+#pragma unroll
+        for (int c = 0; c < Body::kLaneChains; ++c)
+          red[((size_t)warp * G + 32 * c + lane) * W + w] = body.total(c, w);
+      }
     } else {
       double tot[G];
 #pragma unroll

@@ -199,6 +199,7 @@ constexpr int kValueG = GM_G;
 struct JitLanes {
   static constexpr bool kChainLanes = true;
   static constexpr bool kLanesAcc = false;
+  static constexpr int kLaneChains = 1;
   static constexpr int kObsPerEval = 4;
   static constexpr int kTileObs = GM_T;
   float p[GM_NP];
@@ -255,57 +256,78 @@ constexpr int kValueG = GM_G;
 // own FP64 row of the reduction buffer in shared memory (acc, W = 1 + np
 // values, zeroed at the start), hoisted-value adjoints into FP64 registers,
 // and pushed through the hoisted nodes once at the end.
+//
+// CH = 2: two chains per lane (chains l and l + 32 of a warp's 64).  A column
+// load is the limit at CH = 1 (a broadcast 16-byte load occupies the shared-
+// memory pipe for 2.2 cycles and feeds 4 multiply-adds; 48 of them per four
+// observations of the 24-parameter Poisson model are 106 of the 145 cycles
+// that those took), so here each feeds 8.
+template <int CH>
 struct JitLanesG {
   static constexpr bool kChainLanes = true;
   static constexpr bool kLanesAcc = true;
+  static constexpr int kLaneChains = CH;
   static constexpr int kObsPerEval = 4;
   static constexpr int kTileObs = GM_T;
-  float p[GM_NP];
-  float h[GM_NH];
-  float gp[GM_NP];
-  float gh[GM_NH];
-  double ghd[GM_NH];
-  double* acc;
-  double s;
-  float part;
+  float p[CH][GM_NP];
+  float h[CH][GM_NH];
+  float gp[CH][GM_NP];
+  float gh[CH][GM_NH];
+  double ghd[CH][GM_NH];
+  double* acc[CH];
+  double s[CH];
+  float part[CH];
   int cnt;
-  float lastv[4];
+  float lastv[CH][4];
 
+  // row: the first chain's values; the second's are 32 rows further.
   __device__ __forceinline__ void begin_lanes_acc(const float* pc, int C_pad, double* row) {
 #pragma unroll
-    for (int j = 0; j < GM_NP; ++j) {
-      p[j] = pc[(size_t)j * C_pad];
-      gp[j] = 0.0f;
-    }
-    gm_hoist(p, h);
+    for (int c = 0; c < CH; ++c) {
 #pragma unroll
-    for (int j = 0; j < GM_NH; ++j) {
-      gh[j] = 0.0f;
-      ghd[j] = 0.0;
+      for (int j = 0; j < GM_NP; ++j) {
+        p[c][j] = pc[(size_t)j * C_pad + 32 * c];
+        gp[c][j] = 0.0f;
+      }
+      gm_hoist(p[c], h[c]);
+#pragma unroll
+      for (int j = 0; j < GM_NH; ++j) {
+        gh[c][j] = 0.0f;
+        ghd[c][j] = 0.0;
+      }
+      acc[c] = row + (size_t)32 * c * (1 + GM_NP);
+      for (int w = 0; w < 1 + GM_NP; ++w) acc[c][w] = 0.0;
+      s[c] = 0.0;
+      part[c] = 0.0f;
     }
-    acc = row;
-    for (int w = 0; w < 1 + GM_NP; ++w) acc[w] = 0.0;
-    s = 0.0;
-    part = 0.0f;
     cnt = 0;
   }
 
+  __device__ __forceinline__ void quad(const float* xo, int nv) {
+    if constexpr (CH == 2) gm_value_grad4l2(xo, nv, p, h, gp, gh, lastv);
+    else gm_value_grad4l(xo, nv, p[0], h[0], gp[0], gh[0], lastv[0]);
+  }
+
   __device__ __forceinline__ void eval4(const float* xo, int nv) {
-    float v[4];
-    if (nv == 4) gm_value_grad4l(xo, 4, p, h, gp, gh, v);
-    else gm_value_grad4l(xo, nv, p, h, gp, gh, v);
+    if (nv == 4) quad(xo, 4);
+    else quad(xo, nv);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) lastv[k] = v[k];
-    if (nv == 4) {
-      part = ((part + v[0]) + v[1]) + (v[2] + v[3]);
-    } else {
+    for (int c = 0; c < CH; ++c) {
+      const float(&v)[4] = lastv[c];
+      if (nv == 4) {
+        part[c] = ((part[c] + v[0]) + v[1]) + (v[2] + v[3]);
+      } else {
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
-        if (k < nv) part += v[k];
+        for (int k = 0; k < 3; ++k)
+          if (k < nv) part[c] += v[k];
+      }
     }
     if (++cnt == 2) {
-      s += (double)part;
-      part = 0.0f;
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        s[c] += (double)part[c];
+        part[c] = 0.0f;
+      }
       cnt = 0;
     }
   }
@@ -313,36 +335,42 @@ struct JitLanesG {
   // After each tile: the tile's FP32 adjoints into the FP64 accumulators.
   __device__ __forceinline__ void flush_tile() {
 #pragma unroll
-    for (int j = 0; j < GM_NP; ++j) {
-      acc[1 + j] += (double)gp[j];
-      gp[j] = 0.0f;
-    }
+    for (int c = 0; c < CH; ++c) {
 #pragma unroll
-    for (int j = 0; j < GM_NH; ++j) {
-      ghd[j] += (double)gh[j];
-      gh[j] = 0.0f;
+      for (int j = 0; j < GM_NP; ++j) {
+        acc[c][1 + j] += (double)gp[c][j];
+        gp[c][j] = 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < GM_NH; ++j) {
+        ghd[c][j] += (double)gh[c][j];
+        gh[c][j] = 0.0f;
+      }
     }
   }
 
-  __device__ __forceinline__ float last4(int k) const { return lastv[k]; }
+  __device__ __forceinline__ float last4(int k) const { return lastv[0][k]; }
 
   __device__ __forceinline__ void end() {
     flush_tile();
-    float ghf[GM_NH], gx[GM_NP];
 #pragma unroll
-    for (int j = 0; j < GM_NH; ++j) ghf[j] = (float)ghd[j];
+    for (int c = 0; c < CH; ++c) {
+      float ghf[GM_NH], gx[GM_NP];
 #pragma unroll
-    for (int j = 0; j < GM_NP; ++j) gx[j] = 0.0f;
-    gm_hoist_grad(p, ghf, gx);
+      for (int j = 0; j < GM_NH; ++j) ghf[j] = (float)ghd[c][j];
 #pragma unroll
-    for (int j = 0; j < GM_NP; ++j) acc[1 + j] += (double)gx[j];
+      for (int j = 0; j < GM_NP; ++j) gx[j] = 0.0f;
+      gm_hoist_grad(p[c], ghf, gx);
+#pragma unroll
+      for (int j = 0; j < GM_NP; ++j) acc[c][1 + j] += (double)gx[j];
+    }
   }
 
-  __device__ __forceinline__ double total(int, int w) const {
-    return w == 0 ? s + (double)part : acc[w];
+  __device__ __forceinline__ double total(int c, int w) const {
+    return w == 0 ? s[c] + (double)part[c] : acc[c][w];
   }
 };
-using GradBody = JitLanesG;
+using GradBody = JitLanesG<1>;
 constexpr int kGradG = 32;  // chains per warp group, as the host counts them
 #else
 using GradBody = JitBody<GM_GG, true>;
@@ -414,6 +442,18 @@ gm_iter_grad(const __grid_constant__ gpum::TmapDesc tmap, gpum::EvalArgs E, gpum
                                                                             phase,
                                                                         body);
 }
+
+#if GM_GRAD2
+// The gradient kernel with two chains per lane (64 per warp), for batches that
+// fill its eight warps.
+extern "C" __global__ void __launch_bounds__(gpum::kThreads, 1)
+gm_iter_grad2(const __grid_constant__ gpum::TmapDesc tmap, gpum::EvalArgs E, gpum::ChainArgs A,
+              int phase) {
+  gpum::JitLanesG<2> body;
+  gpum::run_iteration<64, 1 + GM_NP, gpum::JitLanesG<2>, gpum::JitPrior>(&tmap, E, A, phase,
+                                                                          body);
+}
+#endif
 
 #if GM_TC
 // ----------------------------------------------------------------------------

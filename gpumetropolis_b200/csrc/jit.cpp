@@ -198,6 +198,8 @@ bool jit_value_lanes(const GenModel& gm, bool pair) {
 
 bool jit_grad_lanes(const GenModel& gm) { return gm.np + std::max(gm.n_hoist, 1) <= 100; }
 
+bool jit_grad_two(const GenModel& gm) { return gm.np + std::max(gm.n_hoist, 1) <= 34; }
+
 std::string jit_source(const GenModel& gm, int G, int GG, bool pair) {
   const bool lanes = jit_value_lanes(gm, pair);
   const bool lanes_grad = jit_grad_lanes(gm);
@@ -205,6 +207,7 @@ std::string jit_source(const GenModel& gm, int G, int GG, bool pair) {
   s += "#include \"device.cuh\"\n";
   s += "#define GM_LANES " + std::string(lanes ? "1" : "0") + "\n";
   s += "#define GM_LANESG " + std::string(lanes_grad ? "1" : "0") + "\n";
+  s += "#define GM_GRAD2 " + std::string(jit_grad_two(gm) ? "1" : "0") + "\n";
   s += "#define GM_PAIR " + std::string(pair ? "1" : "0") + "\n";
   s += "#define GM_G " + std::to_string(G) + "\n";
   s += "#define GM_GG " + std::to_string(GG) + "\n";
@@ -262,6 +265,12 @@ int jit_compile(const GenModel& gm, CompiledModel* out, std::string* err) {
       cudaLibraryGetKernel(&e.model.k_mat, e.lib, "gm_materialize") != cudaSuccess ||
       cudaLibraryGetKernel(&e.model.k_prior, e.lib, "gm_prior_batch") != cudaSuccess) {
     *err = "compiled model is missing its kernels";
+    cudaLibraryUnload(e.lib);
+    return 1;
+  }
+  if (jit_grad_two(gm) &&
+      cudaLibraryGetKernel(&e.model.k_grad2, e.lib, "gm_iter_grad2") != cudaSuccess) {
+    *err = "compiled model is missing its two-chain gradient kernel";
     cudaLibraryUnload(e.lib);
     return 1;
   }

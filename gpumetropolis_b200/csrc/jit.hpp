@@ -15,6 +15,7 @@ namespace gpum {
 struct CompiledModel {
   cudaKernel_t k_value = nullptr;   // gm_iter_value
   cudaKernel_t k_grad = nullptr;    // gm_iter_grad
+  cudaKernel_t k_grad2 = nullptr;   // gm_iter_grad2 (two chains per lane), or nullptr
   cudaKernel_t k_mat = nullptr;     // gm_materialize (extra data columns)
   cudaKernel_t k_prior = nullptr;   // gm_prior_batch (f64 prior, optional gradient)
   int n_mat = 0;                    // materialized data-only operations
@@ -47,6 +48,12 @@ bool jit_value_lanes(const GenModel& gm, bool pair);
 // + hoisted values (values and adjoints in registers) stay within 100; wider
 // ones take the scalar body (GG chains per thread, lanes over observations).
 bool jit_grad_lanes(const GenModel& gm);
+
+// Whether the two-chains-per-lane gradient kernel is built: its registers hold
+// twice the parameters, hoisted values and their adjoints, 136 at 34, which
+// leaves room for the loaded columns; its FP64 rows are 138 KB of shared memory
+// at 33 parameters.
+bool jit_grad_two(const GenModel& gm);
 
 // Returns 0 and a loaded model, or 1 with a message (NVRTC missing, compile
 // error, load error).

@@ -20,9 +20,13 @@ RWM, DE, CHOL, MALA = 0, 1, 2, 3
     (3, 70, 1185, MALA, 2), (3, 70, 2369, CHOL, 2), (3, 70, 4737, RWM, 2),
     (23, 70, 9, MALA, 2), (23, 70, 601, MALA, 0), (119, 70, 3, MALA, 2), (119, 70, 5, CHOL, 2),
     (3, 300001, 2, RWM, 2), (3, 300001, 2, MALA, 0),
+    # the gradient kernel with two chains per lane: from 257 chains, up to 33
+    # parameters (its last column of chains empty, half full, full)
+    (23, 1027, 256, MALA, 2), (23, 1027, 257, MALA, 2), (23, 258, 512, MALA, 2),
+    (32, 70, 545, MALA, 2), (33, 70, 545, MALA, 2),
 ])
 def test_step_follows_the_oracle(gpu, p, n_obs, C, mode, engine):
-    n_iter = 8 if n_obs < 1000 else 2
+    n_iter = 8 if n_obs < 1000 else 2 if n_obs > 2000 else 4
     w = W.make("logistic", n_obs=n_obs, p=p)
     m = w.model
     d = m.n_params
@@ -44,7 +48,8 @@ def test_step_follows_the_oracle(gpu, p, n_obs, C, mode, engine):
     o = o.reshape((n_iter, C, d), order="F")
     # A decision can differ only where |log ratio - log u| is inside the error
     # of the two data sums, 1e-6 of sum |l_i| each (about 0.5 n_obs): at 70
-    # observations below 1e-4 per step, 8e-4 per chain.  With 300,001 it is
+    # observations below 1e-4 per step, 8e-4 per chain, at 1,027 below 1e-3 per
+    # step at the bar and below 1e-4 at the 1e-7 that such sums have.  With 300,001 it is
     # 0.6 of a log unit at the bar (1e-8 of the sum in practice), so those
     # runs are two chains by two steps and compared as they are.
     same = np.all(np.isclose(g, o, rtol=1e-5, atol=1e-4 * scale * np.sqrt(d)), axis=(0, 2))
