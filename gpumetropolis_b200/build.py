@@ -16,7 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgpum_b200.so")
 SOURCES = ["capi.cu", "program.cpp", "codegen.cpp", "jit.cpp", "noalloc.cu", "mlp.cu"]
 HEADERS = ["device.cuh", "interp.cuh", "kernels.cuh", "common.cuh", "compiled.cuh",
-           "program.hpp", "codegen.hpp", "jit.hpp", "tc_gemm.cuh"]
+           "program.hpp", "codegen.hpp", "jit.hpp", "tc_gemm.cuh", "staging.hpp"]
 # Headers the compiled engine hands to NVRTC at run time, embedded as strings.
 EMBED = [("kEmbeddedDevice", "device.cuh"), ("kEmbeddedCommon", "common.cuh"),
          ("kEmbeddedCompiled", "compiled.cuh")]
@@ -82,7 +82,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             objs = list(ex.map(compile_one, SOURCES))
         tmp = LIB + f".{os.getpid()}.tmp"
         subprocess.run([nvcc(), *host_compiler(), *ARCH, "--shared", "-o", tmp, *objs,
-                        "-lcudart", "-ldl"], check=True)
+                        "-lcudart", "-ldl", "-lpthread"], check=True)
     os.replace(tmp, LIB)
     return LIB
 

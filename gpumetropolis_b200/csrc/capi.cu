@@ -32,6 +32,7 @@
 #include "jit.hpp"
 #include "kernels.cuh"
 #include "program.hpp"
+#include "staging.hpp"
 
 using namespace gpum;
 
@@ -82,14 +83,29 @@ struct DBuf {
     if (count <= n && p) return;
     release();
     if (count == 0) count = 1;
-    GPUM_CK(cudaMalloc(&p, count * sizeof(T)));
+    GPUM_CK(dev_alloc((void**)&p, count * sizeof(T)));
     n = count;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p && own) dev_free(p, n * sizeof(T));
     p = nullptr;
     n = 0;
+    own = true;
   }
+  bool own = true;
+  // `count` elements of the slab at *at (nullptr: only the size), advancing it.
+  void carve(char* slab, size_t* at, size_t count) {
+    if (slab) {
+      release();
+      p = reinterpret_cast<T*>(slab + *at);
+      n = count;
+      own = false;
+    }
+    *at += (count * sizeof(T) + 255) & ~(size_t)255;
+  }
+  DBuf() = default;
+  DBuf(const DBuf&) = delete;
+  DBuf& operator=(const DBuf&) = delete;
   ~DBuf() { release(); }
 };
 
@@ -258,9 +274,12 @@ struct gpum_b200_session {
   int n_chains = 0;
   uint32_t max_iter = 0, n_done = 0;
   bool prepared = false;
-  DBuf<double> state, prop, cur, last_eval, sd, temp, L, snap, zbuf, partials, pointwise,
-      points, out64, gx, gy, mx, my, vbuf;
-  DBuf<float> params, draws, draws_out;
+  // The chains' arrays are carved out of one allocation (run_arrays).
+  DBuf<char> slab;
+  DBuf<double> state, prop, cur, last_eval, sd, temp, L, snap, zbuf, partials, points, out64, gx,
+      gy, mx, my, vbuf;
+  DBuf<RunVars> vars;
+  DBuf<float> params, pointwise, draws, draws_out;
   DBuf<uint32_t> ctr, accepts, iter, ptape_i;
   DBuf<double> ptape;
   EvalArgs E{};
@@ -268,6 +287,25 @@ struct gpum_b200_session {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   int graph_len = 0;
+  // Everything the captured launches depend on, compared as bytes; a run whose
+  // key differs captures anew.
+  struct GraphKey {
+    ChainArgs A;
+    EvalArgs E;
+    StepArgs S;
+    Geometry g;
+    const void* fn;
+    size_t step_smem;
+    int pt_K, pt_every;
+    void *pt_att, *pt_acc, *pt_n;
+  };
+  std::vector<char> graph_key;
+  // The evaluation set up last (sizes and kernel, no pointers to inputs).
+  int set_n = -1;
+  bool set_grad = false, set_pw = false;
+  // Pinned block: inputs of a small run or batch, and small results.
+  char* pin = nullptr;
+  cudaEvent_t pin_read = nullptr;  // the last kernel that reads the inputs is done
   uint64_t graph_launches = 0;  // kernel nodes per graph replay
   uint64_t launches = 0;
   // Training pairs for the surrogate (exact runs only).
@@ -296,7 +334,36 @@ struct gpum_b200_session {
 
   ~gpum_b200_session() {
     drop_graph();
-    if (stream) cudaStreamDestroy(stream);
+    if (pin_read) cudaEventDestroy(pin_read);
+    if (stream) {
+      cudaStreamSynchronize(stream);  // before the pinned block goes back
+      cudaStreamDestroy(stream);
+    }
+    pinned_small().give(pin);
+  }
+
+  // The input part of the pinned block, free to write, when it holds `bytes`;
+  // inputs_read() after the kernel that reads it.
+  double* pinned_inputs(size_t bytes) {
+    if (!pin || bytes > kSmallIn) return nullptr;
+    GPUM_CK(cudaEventSynchronize(pin_read));
+    return reinterpret_cast<double*>(pin);
+  }
+  void inputs_read() { GPUM_CK(cudaEventRecord(pin_read, stream)); }
+  // The result part, for `bytes`; its user waits for the stream.
+  char* pinned_results(size_t bytes) { return pin && bytes <= kSmallOut ? pin + kSmallIn : nullptr; }
+
+  // A result of n values to the host: through the pinned block when small,
+  // directly to pinned or moderate destinations, in parallel chunks to large
+  // pageable ones (from about 2 MB the threads pay).
+  template <class T>
+  void result_to_host(T* dst, const T* src, size_t n) {
+    const size_t bytes = n * sizeof(T);
+    if (bytes > (2u << 20) && !host_is_pinned(dst)) {
+      GPUM_CK(copy_to_host(dst, src, n, stream));
+    } else {
+      GPUM_CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
+    }
   }
 
   void drop_graph() {
@@ -304,6 +371,49 @@ struct gpum_b200_session {
     if (graph) cudaGraphDestroy(graph);
     gexec = nullptr;
     graph = nullptr;
+    graph_key.clear();
+  }
+
+  std::vector<char> current_key() const {
+    GraphKey k;
+    std::memset((void*)&k, 0, sizeof k);
+    k.A = A;
+    k.A.n_iter = k.A.seed = 0;  // in vars
+    k.A.gamma = k.A.de_noise = 0.0;
+    k.A.rec_base = 0;
+    k.A.draws = nullptr;
+    k.E = E;
+    k.S = step_args;
+    k.S.phase = 0;
+    k.E.prior_pts = nullptr;
+    k.g = geo;
+    k.fn = kc.fn;
+    k.step_smem = step_smem;
+    k.pt_K = pt_K;
+    k.pt_every = pt_every;
+    k.pt_att = pt_att.p;
+    k.pt_acc = pt_acc.p;
+    k.pt_n = pt_n.p;
+    const char* b = reinterpret_cast<const char*>(&k);
+    return std::vector<char>(b, b + sizeof k);
+  }
+
+  // The chains' arrays of a run of C chains in one allocation.
+  void run_arrays(size_t C, bool mala) {
+    for (char* base = nullptr;;) {
+      size_t at = 0;
+      for (auto* b : {&state, &prop, &snap, &sd, &zbuf}) b->carve(base, &at, C * np);
+      for (auto* b : {&temp, &cur, &last_eval, &prior_v}) b->carve(base, &at, C);
+      for (auto* b : {&ctr, &accepts, &iter}) b->carve(base, &at, C);
+      vars.carve(base, &at, 1);
+      for (auto* b : {&gx, &gy, &mx, &my, &vbuf, &prior_g}) {
+        if (mala) b->carve(base, &at, C * np);
+        else if (!b->own) b->release();  // of a slab that may be gone
+      }
+      if (base) return;
+      slab.ensure(at);
+      base = slab.p;
+    }
   }
 
   // Builds the compiled engine once; false (with cm_error) when NVRTC is
@@ -480,6 +590,9 @@ struct gpum_b200_session {
     uint32_t e = 0;
     GPUM_CK(cudaMemcpyAsync(&e, d_err.p, sizeof e, cudaMemcpyDeviceToHost, stream));
     GPUM_CK(cudaStreamSynchronize(stream));
+    report_device_error(e);
+  }
+  void report_device_error(uint32_t e) {
     if (e) {
       GPUM_CK(cudaMemsetAsync(d_err.p, 0, sizeof(uint32_t), stream));
       throw Failure{GPUM_ERR_DEVICE, "a kernel reported a device-side failure (code " +
@@ -489,11 +602,17 @@ struct gpum_b200_session {
 
   // Evaluation-argument block for `n` points (params in `params`).
   void setup_eval(int n, bool need_grad, bool pointwise = false) {
-    kc = choose(n, need_grad, pointwise);
-    geo = geometry(n, kc);
-    if (geo.smem + static_smem(kc.fn) > 48 * 1024)
-      GPUM_CK(cudaFuncSetAttribute(kc.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)geo.smem));
+    if (n != set_n || need_grad != set_grad || pointwise != set_pw) {
+      set_n = -1;  // unless all of it succeeds
+      kc = choose(n, need_grad, pointwise);
+      geo = geometry(n, kc);
+      if (geo.smem + static_smem(kc.fn) > 48 * 1024)
+        GPUM_CK(cudaFuncSetAttribute(kc.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)geo.smem));
+      set_n = n;
+      set_grad = need_grad;
+      set_pw = pointwise;
+    }
     params.ensure((size_t)np * geo.C_pad);
     partials.ensure((size_t)geo.NOB * geo.C_pad * kc.W);
     E = EvalArgs{};
@@ -514,13 +633,21 @@ struct gpum_b200_session {
   }
 
   void upload_points(const double* pts, int n) {
-    points.ensure((size_t)n * np);
-    GPUM_CK(cudaMemcpyAsync(points.p, pts, sizeof(double) * n * np, cudaMemcpyHostToDevice,
-                            stream));
+    const size_t bytes = sizeof(double) * n * np;
+    const double* src = nullptr;
+    if (double* in = pinned_inputs(bytes)) {
+      std::memcpy(in, pts, bytes);
+      src = in;
+    } else {
+      points.ensure((size_t)n * np);
+      GPUM_CK(cudaMemcpyAsync(points.p, pts, bytes, cudaMemcpyHostToDevice, stream));
+      src = points.p;
+    }
     const int total = (int)(np * geo.C_pad);
-    points_to_params_kernel<<<(total + 255) / 256, 256, 0, stream>>>(points.p, params.p, n,
-                                                                     (int)np, geo.C_pad);
+    points_to_params_kernel<<<(total + 255) / 256, 256, 0, stream>>>(src, params.p, n, (int)np,
+                                                                     geo.C_pad);
     GPUM_CK(cudaGetLastError());
+    if (src != points.p) inputs_read();
     ++launches;
   }
 
@@ -580,13 +707,18 @@ struct gpum_b200_session {
     launch_step(phase);
   }
 
-  // Values w0 .. W - 1 of the n points of a batch, summed into out64.
-  void reduce(int n, int W, int w0) {
+  // Values w0 .. W - 1 of the n points of a batch, summed into dst (device or
+  // pinned host memory); err_out (pinned), when given, receives the error word.
+  void reduce(int n, int W, int w0, double* dst, uint32_t* err_out) {
     const int wpc = warps_per_chain(n), ppb = kWarps / wpc;
-    reduce_partials_kernel<<<(unsigned)((n + ppb - 1) / ppb), kThreads,
-                             sizeof(double) * kWarps * W, stream>>>(
-        partials.p, out64.p, geo.NOB, geo.C_pad, kc.W, n, W, w0, wpc);
-    GPUM_CK(cudaGetLastError());
+    const double* part = partials.p;
+    const uint32_t* err = d_err.p;
+    int nob = geo.NOB, C_pad = geo.C_pad, Ws = kc.W;
+    void* args[] = {(void*)&part, (void*)&dst, (void*)&nob, (void*)&C_pad, (void*)&Ws,
+                    (void*)&n,    (void*)&W,   (void*)&w0,  (void*)&wpc,   (void*)&err,
+                    (void*)&err_out};
+    launch_pdl((const void*)reduce_partials_kernel, dim3((unsigned)((n + ppb - 1) / ppb)),
+               dim3(kThreads), args, sizeof(double) * kWarps * W, stream);
     ++launches;
   }
 
@@ -735,6 +867,8 @@ gpum_b200_session* create_session(const uint32_t* code, size_t n_code, const dou
   s->prior_consts.assign(prior_consts, prior_consts + n_prior_consts);
 
   GPUM_CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+  GPUM_CK(cudaEventCreateWithFlags(&s->pin_read, cudaEventDisableTiming));
+  s->pin = pinned_small().take();
   s->d_err.ensure(1);
   GPUM_CK(cudaMemsetAsync(s->d_err.p, 0, sizeof(uint32_t), s->stream));
   s->d_prior_code.ensure(std::max<size_t>(n_prior, 2));
@@ -803,54 +937,21 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
           GPUM_ERR_UNSUPPORTED);
 
   s->settle_recording();
-  s->drop_graph();
   s->prepared = false;
   s->n_chains = (int)C;
   s->setup_eval((int)C, mala);
   const Geometry& g = s->geo;
-  s->state.ensure(C * np);
-  s->prop.ensure(C * np);
-  s->snap.ensure(C * np);
-  s->sd.ensure(C * np);
-  s->zbuf.ensure(C * np);
-  s->temp.ensure(C);
-  s->cur.ensure(C);
-  s->last_eval.ensure(C);
-  s->ctr.ensure(C);
-  s->accepts.ensure(C);
-  s->iter.ensure(C);
-  s->prior_v.ensure(C);
+  s->run_arrays(C, mala);
   s->draws.ensure(std::max<size_t>(1, (size_t)max_iter * np * g.C_pad));
   if (use_L) s->L.ensure((size_t)C * np * np);
-  if (mala) {
-    s->gx.ensure(C * np);
-    s->gy.ensure(C * np);
-    s->mx.ensure(C * np);
-    s->my.ensure(C * np);
-    s->vbuf.ensure(C * np);
-    s->prior_g.ensure(C * np);
-    if (!s->kc.compiled) {  // the interpreted prior's gradient tape
-      const size_t npr = std::max<size_t>(s->prior_code.size() / 2, 1);
-      s->ptape.ensure((size_t)C * 2 * npr);
-      s->ptape_i.ensure((size_t)C * 2 * npr);
-    }
+  if (mala && !s->kc.compiled) {  // the interpreted prior's gradient tape
+    const size_t npr = std::max<size_t>(s->prior_code.size() / 2, 1);
+    s->ptape.ensure((size_t)C * 2 * npr);
+    s->ptape_i.ensure((size_t)C * 2 * npr);
   }
   cudaStream_t st = s->stream;
-  GPUM_CK(cudaMemcpyAsync(s->state.p, init, sizeof(double) * C * np, cudaMemcpyHostToDevice, st));
-  GPUM_CK(cudaMemcpyAsync(s->snap.p, s->state.p, sizeof(double) * C * np,
-                          cudaMemcpyDeviceToDevice, st));
-  GPUM_CK(cudaMemcpyAsync(s->sd.p, sd, sizeof(double) * C * np, cudaMemcpyHostToDevice, st));
-  GPUM_CK(cudaMemcpyAsync(s->temp.p, temps, sizeof(double) * C, cudaMemcpyHostToDevice, st));
   if (use_L)
     GPUM_CK(cudaMemcpyAsync(s->L.p, L, sizeof(double) * C * np * np, cudaMemcpyHostToDevice, st));
-  GPUM_CK(cudaMemsetAsync(s->ctr.p, 0, sizeof(uint32_t) * C, st));
-  GPUM_CK(cudaMemsetAsync(s->accepts.p, 0, sizeof(uint32_t) * C, st));
-  GPUM_CK(cudaMemsetAsync(s->iter.p, 0, sizeof(uint32_t) * C, st));
-  const int total = (int)(np * g.C_pad);
-  points_to_params_kernel<<<(total + 255) / 256, 256, 0, st>>>(s->state.p, s->params.p, (int)C,
-                                                               (int)np, g.C_pad);
-  GPUM_CK(cudaGetLastError());
-  ++s->launches;
 
   ChainArgs& A = s->A;
   A = ChainArgs{};
@@ -882,6 +983,7 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
   A.prior_consts = s->d_prior_consts.p;
   A.n_prior = (int)(s->prior_code.size() / 2);
   A.zbuf = s->zbuf.p;
+  A.vars = s->vars.p;
   if (mala) {
     A.gx = s->gx.p;
     A.gy = s->gy.p;
@@ -905,9 +1007,6 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
     s->pt_att.ensure(C);
     s->pt_acc.ensure(C);
     s->pt_n.ensure(1);
-    GPUM_CK(cudaMemsetAsync(s->pt_att.p, 0, sizeof(uint32_t) * C, st));
-    GPUM_CK(cudaMemsetAsync(s->pt_acc.p, 0, sizeof(uint32_t) * C, st));
-    GPUM_CK(cudaMemsetAsync(s->pt_n.p, 0, sizeof(uint32_t), st));
   }
   if (s->rec_cap > 0) {
     A.rec_theta = s->rec_theta.p;
@@ -915,6 +1014,35 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
     A.rec_base = s->rec_count;
     A.rec_cap = s->rec_cap;
   }
+  RunInit R{};
+  if (double* in = s->pinned_inputs(sizeof(double) * (2 * C * np + C))) {
+    std::memcpy(in, init, sizeof(double) * C * np);
+    std::memcpy(in + C * np, sd, sizeof(double) * C * np);
+    std::memcpy(in + 2 * C * np, temps, sizeof(double) * C);
+    R.init = in;
+    R.sd = in + C * np;
+    R.temp = in + 2 * C * np;
+  } else {
+    GPUM_CK(cudaMemcpyAsync(s->state.p, init, sizeof(double) * C * np, cudaMemcpyHostToDevice,
+                            st));
+    GPUM_CK(cudaMemcpyAsync(s->sd.p, sd, sizeof(double) * C * np, cudaMemcpyHostToDevice, st));
+    GPUM_CK(cudaMemcpyAsync(s->temp.p, temps, sizeof(double) * C, cudaMemcpyHostToDevice, st));
+    R.init = s->state.p;
+    R.sd = s->sd.p;
+    R.temp = s->temp.p;
+  }
+  R.vars = RunVars{max_iter, seed, gamma, de_noise, A.rec_base, A.draws};
+  R.d_vars = s->vars.p;
+  if (s->pt_K > 0) {
+    R.pt_att = s->pt_att.p;
+    R.pt_acc = s->pt_acc.p;
+    R.pt_n = s->pt_n.p;
+  }
+  run_init_kernel<<<(unsigned)(((size_t)np * g.C_pad + 255) / 256), 256, 0, st>>>(
+      A, R, s->params.p, s->snap.p, s->sd.p, s->temp.p, g.C_pad);
+  GPUM_CK(cudaGetLastError());
+  s->inputs_read();
+  ++s->launches;
   s->E.prior_out = s->prior_v.p;
   s->E.prior_grad = mala ? s->prior_g.p : nullptr;
   s->setup_step();
@@ -929,6 +1057,7 @@ void advance(gpum_b200_session* s, uint32_t n) {
   require((uint64_t)s->n_done + n <= s->max_iter, "advance beyond the prepared max_iter");
   if (n == 0) return;
   constexpr int kGraphLen = 32;
+  if (n >= (uint32_t)kGraphLen && s->gexec && s->graph_key != s->current_key()) s->drop_graph();
   if (n >= (uint32_t)kGraphLen && !s->gexec) {
     GPUM_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     const uint64_t before = s->launches;
@@ -945,9 +1074,10 @@ void advance(gpum_b200_session* s, uint32_t n) {
     GPUM_CK(cudaStreamEndCapture(s->stream, &s->graph));
     GPUM_CK(cudaGraphInstantiate(&s->gexec, s->graph, 0));
     s->graph_len = kGraphLen;
+    s->graph_key = s->current_key();
   }
   uint32_t left = n;
-  while (s->gexec && left >= (uint32_t)s->graph_len) {
+  while (n >= (uint32_t)kGraphLen && s->gexec && left >= (uint32_t)s->graph_len) {
     GPUM_CK(cudaGraphLaunch(s->gexec, s->stream));
     s->launches += s->graph_launches;
     left -= s->graph_len;
@@ -959,12 +1089,27 @@ void advance(gpum_b200_session* s, uint32_t n) {
 void fetch(gpum_b200_session* s, float* out_draws, float* out_accept, double* out_last,
            uint32_t* n_done) {
   require(s && s->prepared, "session has no prepared run");
-  s->check_device_error();
   const uint32_t n = s->n_done;
   const int C = s->n_chains;
   const size_t np = s->np;
   if (n_done) *n_done = n;
+  if (!out_draws && !out_accept && !out_last) return;  // the count alone: nothing to wait for
   cudaStream_t st = s->stream;
+  // The small results first, so that a failed run copies no draws: the error
+  // word, the log posteriors and the acceptance counts, one wait for all.
+  std::vector<char> own;
+  char* r = s->pinned_results((size_t)C * 12 + 8);
+  if (!r) {
+    own.resize((size_t)C * 12 + 8);
+    r = own.data();
+  }
+  uint32_t* err = reinterpret_cast<uint32_t*>(r);
+  double* last = reinterpret_cast<double*>(r + 8);
+  uint32_t* acc = reinterpret_cast<uint32_t*>(r + 8 + (size_t)C * 8);
+  GPUM_CK(cudaMemcpyAsync(err, s->d_err.p, sizeof *err, cudaMemcpyDeviceToHost, st));
+  GPUM_CK(cudaMemcpyAsync(acc, s->accepts.p, sizeof(uint32_t) * C, cudaMemcpyDeviceToHost, st));
+  if (out_last)
+    GPUM_CK(cudaMemcpyAsync(last, s->cur.p, sizeof(double) * C, cudaMemcpyDeviceToHost, st));
   if (out_draws && n > 0) {
     s->draws_out.ensure((size_t)n * C * np);
     dim3 grid((C + 31) / 32, (n + 31) / 32, (unsigned)np);
@@ -972,15 +1117,22 @@ void fetch(gpum_b200_session* s, float* out_draws, float* out_accept, double* ou
                                                       (int)np, C, s->geo.C_pad);
     GPUM_CK(cudaGetLastError());
     ++s->launches;
-    GPUM_CK(cudaMemcpyAsync(out_draws, s->draws_out.p, sizeof(float) * n * C * np,
-                            cudaMemcpyDeviceToHost, st));
+    const size_t nd = (size_t)n * C * np;
+    char* dr = s->pinned_results((size_t)C * 12 + 8 + nd * sizeof(float));
+    if (dr) {  // small draws share the wait
+      dr += ((size_t)C * 12 + 8);
+      GPUM_CK(cudaMemcpyAsync(dr, s->draws_out.p, sizeof(float) * nd, cudaMemcpyDeviceToHost, st));
+      GPUM_CK(cudaStreamSynchronize(st));
+      std::memcpy(out_draws, dr, sizeof(float) * nd);
+    } else {
+      s->result_to_host(out_draws, s->draws_out.p, nd);
+      GPUM_CK(cudaStreamSynchronize(st));
+    }
+  } else {
+    GPUM_CK(cudaStreamSynchronize(st));
   }
-  std::vector<uint32_t> acc(C);
-  GPUM_CK(cudaMemcpyAsync(acc.data(), s->accepts.p, sizeof(uint32_t) * C,
-                          cudaMemcpyDeviceToHost, st));
-  if (out_last)
-    GPUM_CK(cudaMemcpyAsync(out_last, s->cur.p, sizeof(double) * C, cudaMemcpyDeviceToHost, st));
-  GPUM_CK(cudaStreamSynchronize(st));
+  s->report_device_error(*err);
+  if (out_last) std::memcpy(out_last, last, sizeof(double) * C);
   if (out_accept)
     for (int c = 0; c < C; ++c) out_accept[c] = n == 0 ? 0.0f : (float)acc[c] / (float)n;
 }
@@ -995,7 +1147,6 @@ void batch(gpum_b200_session* s, const double* pts, size_t n_points, double* out
   require(n_points <= (1u << 24), "more than 2^24 points", GPUM_ERR_UNSUPPORTED);
   s->settle_recording();
   s->prepared = false;  // the evaluation buffers are reused
-  s->drop_graph();
   const size_t np = s->np;
   size_t chunk = n_points;
   if (kind == B_POINTWISE && s->n_obs > 0)
@@ -1007,31 +1158,42 @@ void batch(gpum_b200_session* s, const double* pts, size_t n_points, double* out
     s->A = ChainArgs{};
     if (kind == B_POINTWISE) {
       if (s->n_obs == 0) continue;
-      s->pointwise.ensure((size_t)n * s->n_obs);
+      // f32 on the device and over the bus, as they are computed; widened by
+      // the host threads that copy them out.
+      const size_t nv = (size_t)n * s->n_obs;
+      s->pointwise.ensure(nv);
       s->E.pointwise = s->pointwise.p;
       if (s->ll.empty()) {
-        GPUM_CK(cudaMemsetAsync(s->pointwise.p, 0, sizeof(double) * n * s->n_obs, s->stream));
+        GPUM_CK(cudaMemsetAsync(s->pointwise.p, 0, sizeof(float) * nv, s->stream));
       } else {
-        s->launch_with(s->geo, s->E, PH_POINTWISE);
+        s->launch_with(s->geo, s->E, PH_POINTWISE, true);
       }
-      GPUM_CK(cudaMemcpyAsync(out + p0 * s->n_obs, s->pointwise.p,
-                              sizeof(double) * n * s->n_obs, cudaMemcpyDeviceToHost, s->stream));
+      GPUM_CK(copy_to_host(out + p0 * s->n_obs, s->pointwise.p, nv, s->stream));
+      s->check_device_error();
     } else {
       // Sums, or the gradient's np entries (the interpreter's gradient kernel
       // pads its width, the entries past 1 + np are left out).
       const int W = kind == B_GRAD ? 1 + (int)np : 1, w0 = kind == B_GRAD ? 1 : 0;
-      const size_t width = (size_t)(W - w0);
-      s->out64.ensure((size_t)n * width);
+      const size_t width = (size_t)(W - w0), nv = (size_t)n * width;
       if (s->ll.empty()) {
-        GPUM_CK(cudaMemsetAsync(s->out64.p, 0, sizeof(double) * n * width, s->stream));
-      } else {
-        s->launch_with(s->geo, s->E, PH_EVAL);
-        s->reduce(n, W, w0);
+        std::fill(out + p0 * width, out + p0 * width + nv, 0.0);
+        s->check_device_error();
+        continue;
       }
-      GPUM_CK(cudaMemcpyAsync(out + p0 * width, s->out64.p, sizeof(double) * n * width,
-                              cudaMemcpyDeviceToHost, s->stream));
+      s->launch_with(s->geo, s->E, PH_EVAL, true);
+      if (char* r = s->pinned_results(8 + nv * sizeof(double))) {
+        // few values: the reduction writes them and the error word to the host
+        s->reduce(n, W, w0, reinterpret_cast<double*>(r + 8), reinterpret_cast<uint32_t*>(r));
+        GPUM_CK(cudaStreamSynchronize(s->stream));
+        s->report_device_error(*reinterpret_cast<volatile uint32_t*>(r));
+        std::memcpy(out + p0 * width, r + 8, nv * sizeof(double));
+      } else {
+        s->out64.ensure(nv);
+        s->reduce(n, W, w0, s->out64.p, nullptr);
+        s->result_to_host(out + p0 * width, s->out64.p, nv);
+        s->check_device_error();
+      }
     }
-    s->check_device_error();
   }
 }
 
@@ -1193,6 +1355,7 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
   GPUM_CK(cudaGetLastError());
   ++s->launches;
 
+  s->drop_graph();  // of the exact run
   constexpr uint32_t kDaGraphLen = 16;
   uint32_t left = n_iter;
   if (n_iter >= kDaGraphLen) {
@@ -1304,6 +1467,7 @@ int gpum_b200_session_set_engine(gpum_b200_session* s, int engine, char* err, si
     if (engine == GPUM_ENGINE_COMPILED && !s->compiled_available())
       throw Failure{GPUM_ERR_UNSUPPORTED, "compiled engine unavailable: " + s->cm_error};
     s->engine = engine;
+    s->set_n = -1;
     s->drop_graph();
     s->prepared = false;
   });
@@ -1533,9 +1697,19 @@ int gpum_b200_session_draw_moments(gpum_b200_session* s, uint32_t t0, uint32_t n
                                                     pmean, pm2);
     GPUM_CK(cudaGetLastError());
     s->launches += 3;
-    GPUM_CK(cudaMemcpyAsync(chain_mean, dmean, sizeof(double) * C * np, cudaMemcpyDeviceToHost,
-                            st));
-    GPUM_CK(cudaMemcpyAsync(chain_m2, dm2, sizeof(double) * C * np, cudaMemcpyDeviceToHost, st));
+    const size_t cn = (size_t)C * np, all = 2 * cn + np + (size_t)np * np;
+    if (char* r = s->pinned_results(all * sizeof(double))) {
+      const double* h = reinterpret_cast<const double*>(r);
+      GPUM_CK(cudaMemcpyAsync(r, dmean, all * sizeof(double), cudaMemcpyDeviceToHost, st));
+      GPUM_CK(cudaStreamSynchronize(st));
+      std::memcpy(chain_mean, h, cn * sizeof(double));
+      std::memcpy(chain_m2, h + cn, cn * sizeof(double));
+      std::memcpy(pool_mean, h + 2 * cn, np * sizeof(double));
+      std::memcpy(pool_m2, h + 2 * cn + np, sizeof(double) * np * np);
+      return;
+    }
+    GPUM_CK(cudaMemcpyAsync(chain_mean, dmean, sizeof(double) * cn, cudaMemcpyDeviceToHost, st));
+    GPUM_CK(cudaMemcpyAsync(chain_m2, dm2, sizeof(double) * cn, cudaMemcpyDeviceToHost, st));
     GPUM_CK(cudaMemcpyAsync(pool_mean, pmean, sizeof(double) * np, cudaMemcpyDeviceToHost, st));
     GPUM_CK(cudaMemcpyAsync(pool_m2, pm2, sizeof(double) * np * np, cudaMemcpyDeviceToHost, st));
     GPUM_CK(cudaStreamSynchronize(st));
@@ -1547,9 +1721,12 @@ int gpum_b200_session_state(gpum_b200_session* s, double* out_state, char* err,
   return guard(err, err_len, [&] {
     require(s && s->prepared, "session has no prepared run");
     require(out_state != nullptr, "output pointer is NULL");
-    GPUM_CK(cudaMemcpyAsync(out_state, s->state.p, sizeof(double) * s->n_chains * s->np,
-                            cudaMemcpyDeviceToHost, s->stream));
+    const size_t bytes = sizeof(double) * s->n_chains * s->np;
+    char* r = s->pinned_results(bytes);
+    GPUM_CK(cudaMemcpyAsync(r ? r : (char*)out_state, s->state.p, bytes, cudaMemcpyDeviceToHost,
+                            s->stream));
     GPUM_CK(cudaStreamSynchronize(s->stream));
+    if (r) std::memcpy(out_state, r, bytes);
   });
 }
 

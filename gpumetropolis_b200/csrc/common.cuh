@@ -31,6 +31,17 @@ enum Phase : int { PH_EVAL = 0, PH_INIT = 1, PH_STEP = 2, PH_POINTWISE = 3 };
 enum RngKind : int { RNG_TRIPLE32 = 0, RNG_PHILOX = 1 };
 enum ModeKind : int { MODE_RWM = 0, MODE_DE = 1, MODE_CHOL = 2, MODE_MALA = 3, MODE_DESYNC = 4 };
 
+// What differs from one prepared run of a session to the next while its
+// buffers and sizes stay: kept in device memory, so that the captured graph of
+// the iterations serves every batch of an adaptive warmup (capturing,
+// instantiating and destroying one took 0.4 ms per batch).
+struct RunVars {
+  uint32_t n_iter, seed;
+  double gamma, de_noise;
+  uint64_t rec_base;
+  float* draws;
+};
+
 // Chain state of a run, all device pointers.
 struct ChainArgs {
   int n_chains, np;
@@ -73,6 +84,7 @@ struct ChainArgs {
   // chain a tape of n_prior values, adjoints and operand indices.
   double* ptape;        // [C][2][n_prior]
   uint32_t* ptape_i;    // [C][2][n_prior]
+  const RunVars* vars;  // n_iter, seed, gamma, de_noise, rec_base and draws of the run
 };
 
 struct EvalArgs {
@@ -80,7 +92,7 @@ struct EvalArgs {
   int width;            // values per (chain, obs block): 1, or 1 + np with the gradient
   const float* params;  // [np][C_pad] evaluation points (f32)
   double* partials;     // [NOB][C_pad][width]
-  double* pointwise;    // [C][n_obs] (PH_POINTWISE)
+  float* pointwise;     // [C][n_obs] (PH_POINTWISE)
   int n_points;         // chains/points that are real (rest padding)
   uint32_t* err;        // device error word
   const uint32_t* active;  // if set: only the first *active points are live
@@ -413,7 +425,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
           if (c < E.n_points) {
 #pragma unroll
             for (int q = 0; q < 4; ++q)  // constant indices keep the values in registers
-              if (q < nv) E.pointwise[(size_t)c * E.n_obs + obs0 + o + q] = (double)body.last4(q);
+              if (q < nv) E.pointwise[(size_t)c * E.n_obs + obs0 + o + q] = body.last4(q);
           }
         }
       }
@@ -431,8 +443,8 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
             const int c = cb * CG + wc * G + g;
             if (c < E.n_points) {
               const float2 lv = body.last2(g);
-              E.pointwise[(size_t)c * E.n_obs + obs] = (double)lv.x;
-              if (v1) E.pointwise[(size_t)c * E.n_obs + obs + 1] = (double)lv.y;
+              E.pointwise[(size_t)c * E.n_obs + obs] = lv.x;
+              if (v1) E.pointwise[(size_t)c * E.n_obs + obs + 1] = lv.y;
             }
           }
         }
@@ -466,7 +478,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
 #pragma unroll
           for (int g = 0; g < G; ++g) {
             const int c = cb * CG + wc * G + g;
-            if (c < E.n_points) E.pointwise[(size_t)c * E.n_obs + obs] = (double)body.last(g);
+            if (c < E.n_points) E.pointwise[(size_t)c * E.n_obs + obs] = body.last(g);
           }
         }
       }

@@ -378,6 +378,17 @@ __device__ inline void propose_desync(const ChainArgs& A, int c, Stream& rs, flo
   }
 }
 
+// The run's own values into a kernel's argument block.
+__device__ __forceinline__ void load_vars(ChainArgs& A) {
+  const RunVars v = *A.vars;
+  A.n_iter = v.n_iter;
+  A.seed = v.seed;
+  A.gamma = v.gamma;
+  A.de_noise = v.de_noise;
+  A.rec_base = v.rec_base;
+  A.draws = v.draws;
+}
+
 // ------------------------------------------------- one chain, one warp
 // The i-th uniform (i >= 1) a chain's stream `rs` would return from its
 // current position, without advancing it: both streams are counter-based, so
@@ -572,10 +583,15 @@ __device__ __forceinline__ double group_total(const double* red, int W, int w, i
 // Sums of each point's values w0 .. W - 1 into out[point][W - w0]: one group of
 // wpc warps per point.  A single thread per value over all observation blocks
 // took 25 us for 250 points of 18 values.
+// out and err_out may be pinned host memory; err_out, when given, receives
+// the session's device error word.
 static __global__ void __launch_bounds__(kThreads)
 reduce_partials_kernel(const double* __restrict__ partials, double* __restrict__ out, int nob,
-                       int C_pad, int Ws, int n, int W, int w0, int wpc) {
+                       int C_pad, int Ws, int n, int W, int w0, int wpc,
+                       const uint32_t* __restrict__ err, uint32_t* __restrict__ err_out) {
   extern __shared__ double rsm[];  // [8][W]
+  pdl_wait();
+  if (err_out && blockIdx.x == 0 && threadIdx.x == 0) *err_out = __ldcg(err);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wi = warp % wpc, c = (int)blockIdx.x * (kWarps / wpc) + warp / wpc;
   double* red = rsm + (size_t)(warp / wpc) * wpc * W;
@@ -635,6 +651,7 @@ static __global__ void __launch_bounds__(kThreads) step_kernel(ChainArgs A, Step
       Ls[(i / np) * ldL + i % np] = L[i];
     L = Ls;
   }
+  load_vars(A);  // as the factors
   pdl_wait();
   pdl_trigger();
   if (live) group_partials(S.partials, S.nob, S.C_pad, S.Ws, S.W, c, wi, wpc, red, lane);
@@ -731,13 +748,54 @@ static __global__ void convert_rows_kernel(const double* __restrict__ src, float
 }
 
 // f64 chain-major points [C][np] -> f32 [np][C_pad]; pad chains copy chain 0.
+// pts may be pinned host memory.
 static __global__ void points_to_params_kernel(const double* __restrict__ pts, float* __restrict__ params,
                                         int n, int np, int C_pad) {
+  pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np * C_pad) return;
   const int j = i / C_pad, c = i % C_pad;
   const int src = c < n ? c : 0;
   params[i] = (float)pts[(size_t)src * np + j];
+}
+
+// The start of a run in one launch: states, DE snapshot, proposal scales,
+// temperatures, evaluation points, counters and the run's values.  init, sd
+// and temp may be pinned host memory or the state arrays themselves.
+struct RunInit {
+  const double *init, *sd, *temp;
+  RunVars vars;
+  RunVars* d_vars;
+  uint32_t *pt_att, *pt_acc, *pt_n;  // or nullptr
+};
+static __global__ void run_init_kernel(ChainArgs A, RunInit R, float* __restrict__ params,
+                                       double* snap, double* sd, double* temp, int C_pad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int np = A.np;
+  if (i >= np * C_pad) return;
+  const int j = i / C_pad, c = i % C_pad;
+  const bool live = c < A.n_chains;
+  const double x = R.init[(size_t)(live ? c : 0) * np + j];
+  params[i] = (float)x;
+  if (!live) return;
+  const size_t o = (size_t)c * np + j;
+  const double s = R.sd[o];
+  A.state[o] = x;
+  snap[o] = x;
+  sd[o] = s;
+  if (j != 0) return;
+  temp[c] = R.temp[c];
+  A.ctr[c] = 0;
+  A.accepts[c] = 0;
+  A.iter[c] = 0;
+  if (R.pt_att) {
+    R.pt_att[c] = 0;
+    R.pt_acc[c] = 0;
+  }
+  if (c == 0) {
+    *R.d_vars = R.vars;
+    if (R.pt_n) R.pt_n[0] = 0;
+  }
 }
 
 // Internal draws [n_iter][np][C_pad] -> the reference layout, column-major
@@ -874,6 +932,7 @@ struct PtArgs {
 };
 
 static __global__ void pt_exchange_kernel(ChainArgs A, PtArgs P) {
+  load_vars(A);
   const uint32_t t = P.iter[0];  // iterations done (all chain blocks agree here)
   if (t == 0 || t % (uint32_t)P.every != 0 || t >= A.n_iter) return;
   const uint32_t s = t / (uint32_t)P.every;  // exchange number, from 1
@@ -929,6 +988,7 @@ static __global__ void pt_exchange_kernel(ChainArgs A, PtArgs P) {
 static __global__ void desync_propose_kernel(ChainArgs A, float* params, int C_pad) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= A.n_chains) return;
+  load_vars(A);
   const uint32_t t = A.iter[0];
   if (t >= A.n_iter) return;
   Stream rs = make_stream(A, c);

@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "../../include/gpum_b200.h"
+#include "staging.hpp"
 #include "tc_gemm.cuh"
 
 using namespace gpum;
@@ -60,15 +61,14 @@ template <class T>
 struct Buf {
   T* p = nullptr;
   size_t n = 0;
+  static size_t bytes(size_t count) { return std::max<size_t>(count, 1) * sizeof(T); }
   void alloc(size_t count) {
-    if (p) cudaFree(p);
+    dev_free(p, bytes(n));
     p = nullptr;
-    MLP_CK(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)));
+    MLP_CK(dev_alloc((void**)&p, bytes(count)));
     n = count;
   }
-  ~Buf() {
-    if (p) cudaFree(p);
-  }
+  ~Buf() { dev_free(p, bytes(n)); }
 };
 
 // ----------------------------------------------------------------- kernels

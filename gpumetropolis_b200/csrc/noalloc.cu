@@ -258,7 +258,7 @@ extern "C" int gpum_b200_loglik_batch_noalloc(
     default: iter_kernel<2, 32><<<grid, kThreads, smem, st>>>(prog, tmap, E, A, PH_EVAL); break;
   }
   reduce_partials_kernel<<<(n + kWarps - 1) / kWarps, kThreads, sizeof(double) * kWarps, st>>>(
-      d_part, d_out, nob, C_pad, 1, n, 1, 0, 1);
+      d_part, d_out, nob, C_pad, 1, n, 1, 0, 1, nullptr, nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     if (err && err_len) std::snprintf(err, err_len, "launch failed: %s", cudaGetErrorString(e));
