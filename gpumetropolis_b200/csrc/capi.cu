@@ -39,7 +39,7 @@ using namespace gpum;
 namespace gpum {
 // Surrogate inference on device parameters (mlp.cu).
 int mlp_infer(gpum_b200_mlp* m, const double* theta, int n, int d, double* out, cudaStream_t st,
-              std::string* err);
+              std::string* err, bool pdl);
 int mlp_infer_launches(const gpum_b200_mlp* m, int n);
 int mlp_infer_grad(gpum_b200_mlp* m, const double* theta, int n, int d, double* out_val,
                    double* out_grad, cudaStream_t st, std::string* err);
@@ -170,17 +170,7 @@ const void* interp_grad_kernel(int W) {
 // predecessor in the stream runs and waits for it itself (pdl_wait).  A step
 // of the sampling loop costs 2 kernels; their launch latencies overlap.
 void launch_pdl(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  GPUM_CK(cudaLaunchKernelExC(&cfg, fn, args));
+  GPUM_CK(launch_dependent(fn, grid, block, args, smem, st));
 }
 
 int num_sms() {
@@ -314,7 +304,7 @@ struct gpum_b200_session {
   uint64_t rec_cap = 0, rec_count = 0;
   // Delayed acceptance.
   DBuf<double> sll_x, sll_y, prior_x, prior_y, da_partials, da_gs, da_tvals, da_tadj;
-  DBuf<uint32_t> da_flag, da_slot, da_active, da_iter, da_stage1, da_tlhs, da_trhs;
+  DBuf<uint32_t> da_flag, da_slot, da_active, da_stage1, da_tlhs, da_trhs;
   DBuf<float> da_params;
   Geometry geo_da{};
   EvalArgs E_da{};
@@ -1210,37 +1200,48 @@ void launch_prior(gpum_b200_session* s, double* pts, double* out) {
   int n = s->n_chains;
   double* grad = s->A.mode == MODE_MALA ? s->D.gs : nullptr;
   void* args[] = {(void*)&pts, (void*)&n, (void*)&out, (void*)&grad};
-  GPUM_CK(cudaLaunchKernel((const void*)s->cm.k_prior, dim3((unsigned)((n + 127) / 128)),
-                           dim3(128), args, 0, s->stream));
+  launch_pdl((const void*)s->cm.k_prior, dim3((unsigned)((n + 127) / 128)), dim3(128), args, 0,
+             s->stream);
   ++s->launches;
 }
 
 void da_step(gpum_b200_session* s) {
   const int C = s->n_chains, np = (int)s->np;
+  cudaStream_t st = s->stream;
+  // The prior first: the surrogate's kernel stages its network meanwhile.
+  const bool screen = s->D.prior_ready && s->A.mode != MODE_MALA && C <= kScreenChains;
+  if (screen) launch_prior(s, s->prop.p, s->prior_y.p);
   std::string e;
   const int rc = s->A.mode == MODE_MALA
                      ? mlp_infer_grad(s->da_mlp, s->prop.p, C, np, s->sll_y.p, s->D.gs,
                                       s->stream, &e)
-                     : mlp_infer(s->da_mlp, s->prop.p, C, np, s->sll_y.p, s->stream, &e);
+                     : mlp_infer(s->da_mlp, s->prop.p, C, np, s->sll_y.p, s->stream, &e, true);
   if (rc != GPUM_OK) throw Failure{rc, "surrogate: " + e};
-  cudaStream_t st = s->stream;
-  if (s->D.prior_ready) launch_prior(s, s->prop.p, s->prior_y.p);
-  // 64-thread blocks spread the per-chain f64 work (prior, proposal) over
-  // more SMs; finalize runs one warp per chain.
-  const unsigned cb = (unsigned)((C + 63) / 64);
-  da_stage1_kernel<<<cb, 64, 0, st>>>(s->A, s->D);
-  da_compact_kernel<<<1, 1024, 0, st>>>(s->A, s->D);
-  da_pack_kernel<<<(unsigned)(((size_t)C * np + 255) / 256), 256, 0, st>>>(s->A, s->D);
-  GPUM_CK(cudaGetLastError());
-  s->launch_with(s->geo_da, s->E_da, PH_EVAL);
-  da_finalize_kernel<<<(unsigned)((C + 7) / 8), 256, (size_t)8 * 2 * np * sizeof(double), st>>>(
-      s->A, s->D, s->da_partials.p, s->geo_da.CG, s->geo_da.NCB * s->geo_da.NOB,
-      s->geo_da.ntiles, s->geo_da.C_pad);
-  da_tick_kernel<<<1, 32, 0, st>>>(s->D);
-  GPUM_CK(cudaGetLastError());
-  s->launches += 5 + (uint64_t)s->da_mlp_launches;  // launch_prior counts itself
+  void* ad[] = {(void*)&s->A, (void*)&s->D};
+  if (screen) {
+    launch_pdl((const void*)da_screen_kernel, dim3(1), dim3(kScreenThreads), ad, 0, st);
+    s->launches += 1;
+  } else {
+    if (s->D.prior_ready) launch_prior(s, s->prop.p, s->prior_y.p);
+    // 64-thread blocks spread the per-chain f64 work (prior, drift) over SMs
+    const unsigned cb = (unsigned)((C + 63) / 64);
+    da_stage1_kernel<<<cb, 64, 0, st>>>(s->A, s->D);
+    da_compact_kernel<<<1, 1024, 0, st>>>(s->A, s->D);
+    da_pack_kernel<<<(unsigned)(((size_t)C * np + 255) / 256), 256, 0, st>>>(s->A, s->D);
+    GPUM_CK(cudaGetLastError());
+    s->launches += 3;
+  }
+  s->launch_with(s->geo_da, s->E_da, PH_EVAL, true);
+  const double* part = s->da_partials.p;
+  int CG = s->geo_da.CG, total = s->geo_da.NCB * s->geo_da.NOB, ntiles = s->geo_da.ntiles,
+      cp = s->geo_da.C_pad;
+  void* af[] = {(void*)&s->A, (void*)&s->D, (void*)&part, (void*)&CG, (void*)&total,
+                (void*)&ntiles, (void*)&cp};
+  launch_pdl((const void*)da_finalize_kernel, dim3((unsigned)((C + 7) / 8)), dim3(256), af,
+             (size_t)8 * 2 * np * sizeof(double), st);
+  s->launches += 1 + (uint64_t)s->da_mlp_launches;  // launch_prior counts itself
   if (s->pt_K > 0) {  // exchanges on the exact log posteriors, caches swapped along
-    PtArgs P{s->pt_K,   s->pt_every,  s->D.iter, s->D.sll_x, s->D.prior_x,
+    PtArgs P{s->pt_K,   s->pt_every,  s->A.iter, s->D.sll_x, s->D.prior_x,
              s->pt_n.p, s->pt_att.p, s->pt_acc.p, s->D.full,  s->D.C_pad};
     pt_exchange_kernel<<<(unsigned)((C + 127) / 128), 128, 0, st>>>(s->A, P);
     GPUM_CK(cudaGetLastError());
@@ -1297,7 +1298,6 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
   s->da_slot.ensure(C);
   s->da_stage1.ensure(C);
   s->da_active.ensure(1);
-  s->da_iter.ensure(1);
   s->da_params.ensure((size_t)np * g.C_pad);
   // The exact evaluation runs a fixed 1-D grid of one CTA per resident slot
   // (at least one per chain block); the kernel splits it into (live chain
@@ -1328,7 +1328,6 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
   D.flag = s->da_flag.p;
   D.slot = s->da_slot.p;
   D.active = s->da_active.p;
-  D.iter = s->da_iter.p;
   D.stage1 = s->da_stage1.p;
   D.params = s->da_params.p;
   D.full = s->params.p;
@@ -1342,7 +1341,7 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
   s->da_mlp_launches = 0;
   std::string e;
   int rc = lang ? mlp_infer_grad(mlp, s->state.p, (int)C, np, s->sll_x.p, D.gs, st, &e)
-                : mlp_infer(mlp, s->state.p, (int)C, np, s->sll_x.p, st, &e);
+                : mlp_infer(mlp, s->state.p, (int)C, np, s->sll_x.p, st, &e, false);
   if (rc != GPUM_OK) throw Failure{rc, "surrogate: " + e};
   s->da_mlp_launches = lang ? mlp_infer_grad_launches(mlp, (int)C)
                             : mlp_infer_launches(mlp, (int)C);
@@ -2054,7 +2053,7 @@ int gpum_b200_session_train_surrogate(gpum_b200_session* s, gpum_b200_mlp* m,
     if (n_ho > 0) {  // residual spread of the trained network on the held-out pairs
       DBuf<double> pred;
       pred.ensure(n_ho);
-      rc = mlp_infer(m, ho_th.p, (int)n_ho, d, pred.p, st, &e);
+      rc = mlp_infer(m, ho_th.p, (int)n_ho, d, pred.p, st, &e, false);
       if (rc != GPUM_OK) throw Failure{rc, e};
       std::vector<double> hpred(n_ho), hll(n_ho);
       GPUM_CK(cudaMemcpyAsync(hpred.data(), pred.p, n_ho * sizeof(double),

@@ -405,6 +405,8 @@ extern "C" __global__ void gm_materialize(float* __restrict__ cols, long long n_
 // acceptance reads these instead of interpreting the prior per chain.
 extern "C" __global__ void gm_prior_batch(const double* __restrict__ x, int n,
                                           double* __restrict__ out, double* __restrict__ grad) {
+  gpum::pdl_wait();
+  gpum::pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double* p = x + (size_t)i * GM_NP;

@@ -84,6 +84,24 @@ __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+#ifndef __CUDACC_RTC__
+// Host side: a launch with the programmatic dependent launch attribute.
+inline cudaError_t launch_dependent(const void* fn, dim3 grid, dim3 block, void** args,
+                                    size_t smem, cudaStream_t st) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+#endif
+
 // Nanosecond clock of the GPU, for waits bounded in time as well as polls.
 __device__ __forceinline__ uint64_t gm_globaltimer() {
   uint64_t t;

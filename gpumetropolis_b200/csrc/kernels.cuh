@@ -1006,7 +1006,6 @@ struct DaArgs {
   uint32_t* flag;    // [C] stage 1 accepted this iteration
   uint32_t* slot;    // [C] position in the compacted evaluation
   uint32_t* active;  // [1] stage-1 acceptances this iteration
-  uint32_t* iter;    // [1] iterations done
   uint32_t* stage1;  // [C] stage-1 acceptance counts
   float* params;     // [np][C_pad] compacted evaluation points
   float* full;       // [np][C_pad] scratch for propose()
@@ -1050,7 +1049,6 @@ __device__ __forceinline__ double da_uniform(Stream& rs, uint32_t t, uint32_t k)
 // draws its first proposal again, now with that drift.
 static __global__ void da_setup_kernel(ChainArgs A, DaArgs D) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c == 0) D.iter[0] = 0;
   if (c >= A.n_chains) return;
   const double* x = A.state + (size_t)c * A.np;
   if (A.mode == MODE_MALA) {
@@ -1081,7 +1079,7 @@ static __global__ void da_setup_kernel(ChainArgs A, DaArgs D) {
 static __global__ void da_stage1_kernel(ChainArgs A, DaArgs D) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= A.n_chains) return;
-  const uint32_t t = D.iter[0];
+  const uint32_t t = A.iter[c];
   const int np = A.np;
   const double* y = A.prop + (size_t)c * np;
   double py, lqd = 0.0;
@@ -1160,6 +1158,64 @@ static __global__ void da_pack_kernel(ChainArgs A, DaArgs D) {
   D.params[(size_t)j * D.C_pad + D.slot[c]] = (float)A.prop[i];
 }
 
+// Stage 1, the compaction and the packing in one block, for a symmetric
+// proposal whose priors are ready (prior_y): up to kScreenChains chains, two a
+// thread.  Apart they were three launches of 3.7, 2.0 and 1.8 us and the gaps
+// between them, each too short to fill the GPU.
+constexpr int kScreenThreads = 1024, kScreenChains = 2 * kScreenThreads;
+static __global__ void __launch_bounds__(kScreenThreads) da_screen_kernel(ChainArgs A, DaArgs D) {
+  __shared__ uint32_t sums[2][32];
+  __shared__ uint16_t who[kScreenChains];  // slot -> chain
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();
+  pdl_trigger();
+  uint32_t f[2], below[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int c = i * kScreenThreads + tid;
+    f[i] = 0;
+    if (c < A.n_chains) {
+      Stream rs = make_stream(A, c);
+      const double u = da_uniform(rs, A.iter[c], 0xFFFF0001u);
+      const double a1 =
+          ((D.sll_y[c] + D.prior_y[c]) - (D.sll_x[c] + D.prior_x[c])) / A.temp[c];
+      f[i] = log(u) < a1 ? 1u : 0u;
+      D.flag[c] = f[i];
+      A.ctr[c] = rs.ctr;
+    }
+    const uint32_t b = __ballot_sync(0xffffffffu, f[i] != 0);
+    below[i] = __popc(b & ((1u << lane) - 1u));
+    if (lane == 0) sums[i][warp] = __popc(b);
+  }
+  __syncthreads();
+  // survivors before each warp, in chain order
+  if (warp < 2) {
+    uint32_t v = sums[warp][lane];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, v, off);
+      if (lane >= off) v += x;
+    }
+    sums[warp][lane] = v;  // inclusive
+  }
+  __syncthreads();
+  const uint32_t first = sums[0][31], live = first + sums[1][31];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int c = i * kScreenThreads + tid;
+    if (!f[i]) continue;
+    const uint32_t k = (i ? first : 0u) + (warp > 0 ? sums[i][warp - 1] : 0u) + below[i];
+    D.slot[c] = k;
+    who[k] = (uint16_t)c;
+  }
+  if (tid == 0) D.active[0] = live;
+  __syncthreads();
+  for (uint32_t i = tid; i < live * (uint32_t)A.np; i += kScreenThreads) {
+    const uint32_t k = i % live, j = i / live;
+    D.params[(size_t)j * D.C_pad + k] = (float)A.prop[(size_t)who[k] * A.np + j];
+  }
+}
+
 // Stage 2 for the survivors, the draw for every chain, the next proposal.
 // One warp per chain: the lanes add the chain's observation-block partials in
 // a fixed lane-strided order and a fixed shuffle tree (deterministic), lane 0
@@ -1168,6 +1224,8 @@ static __global__ void da_finalize_kernel(ChainArgs A, DaArgs D, const double* _
                                           int CG, int total, int ntiles, int C_pad_eval) {
   const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_trigger();
   if (c >= A.n_chains) return;
   const bool live = D.flag[c] != 0;
   double ll = 0.0;
@@ -1181,7 +1239,7 @@ static __global__ void da_finalize_kernel(ChainArgs A, DaArgs D, const double* _
   }
   extern __shared__ double fin_sm[];  // [warps per block][2 np]
   const int np = A.np;
-  const uint32_t t = D.iter[0];
+  const uint32_t t = A.iter[c];
   double* x = A.state + (size_t)c * np;
   const double* y = A.prop + (size_t)c * np;
   Stream rs = make_stream(A, c);
@@ -1224,11 +1282,10 @@ static __global__ void da_finalize_kernel(ChainArgs A, DaArgs D, const double* _
     rs = propose_warp(A, c, rs, D.full, D.C_pad, lane, fin_sm + (size_t)(threadIdx.x >> 5) * 2 * np,
                       A.L ? A.L + (size_t)c * np * np : nullptr, np);
   }
-  if (lane == 0) A.ctr[c] = rs.ctr;
-}
-
-static __global__ void da_tick_kernel(DaArgs D) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) D.iter[0] += 1;
+  if (lane == 0) {
+    A.ctr[c] = rs.ctr;
+    A.iter[c] = t + 1;
+  }
 }
 
 }  // namespace gpum

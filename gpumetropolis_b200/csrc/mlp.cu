@@ -312,24 +312,34 @@ __global__ void mlp_input_grad(const float* __restrict__ dX, int n, int d, int d
 //   X = transform(theta) -> shared (bf16, K-major core matrices)
 //   Z1 = X W1^T  (tcgen05, M = 128, N = H, K = 64, accumulators in TMEM)
 //   A1 = silu(Z1 + b1) -> shared (bf16, the K-major A operand of layer 2)
-//   Z2 = A1 W2^T (tcgen05, K = H in 64-wide slices; each W2 slice staged in
-//        shared memory, the next one prefetched into registers meanwhile)
+//   Z2 = A1 W2^T (tcgen05, K = H; W2 staged whole at H = 128, in 64-wide K
+//        slices through registers at H = 256, where it does not fit)
 //   y  = silu(Z2 + b2) . w3 + b3 (four column-quarter partials added in
 //        order);  out = y * ysd + ymean   (f64)
-// Shared memory: X 16 KB | W1 H x 64 | A1 (H / 64) x 16 KB | W2 slice H x 64.
-// The whitening scratch (centred inputs, 128 x 64 f32) and the head
+// Shared memory: X 16 KB | W1 H x 64 | A1 (H / 64) x 16 KB | W2 | whitening
+// matrix d x 64 | b1, b2, w3.  The centred inputs (128 x 64 f32) and the head
 // partials live in A1's space when it is free.  Waits are bounded; a timeout
 // sets the error word and skips the epilogues.
+//
+// Bound by latency, 8 CTAs at 1,024 rows: the network's weights do not depend
+// on the launch before it, so all of them are staged before the wait for that
+// launch's proposals, and the whitening runs 16 independent sums per thread
+// over shared memory.  1,024 rows, d = 17, H = 128 in the two-stage loop: 19.4 us
+// before, 10.9 now, part of it beside the prior's kernel.
 constexpr int kInfRows = 128;
 constexpr int kInfThreads = 512;
 
+__host__ __device__ constexpr size_t mlp_infer_w2_bytes(int H) {
+  return (size_t)H * (H == 128 ? 128 : 64) * 2;
+}
 __host__ __device__ constexpr size_t mlp_infer_smem(int H) {
   return (size_t)kInfRows * 64 * 2 + (size_t)H * 64 * 2 + (size_t)(H / 64) * kInfRows * 64 * 2 +
-         (size_t)H * 64 * 2 + 64;
+         mlp_infer_w2_bytes(H) + 64 * 64 * 4 + (size_t)3 * H * 4 + 64;
 }
 
+template <int H>
 __global__ void __launch_bounds__(kInfThreads, 1)
-mlp_infer_fused(const double* __restrict__ theta, int n, int d, int H,
+mlp_infer_fused(const double* __restrict__ theta, int n, int d,
                 const float* __restrict__ xmean, const float* __restrict__ xinv,
                 const float* __restrict__ xw, const bf16* __restrict__ W1h,
                 const float* __restrict__ b1, const bf16* __restrict__ W2h,
@@ -338,23 +348,56 @@ mlp_infer_fused(const double* __restrict__ theta, int n, int d, int H,
                 uint32_t* err) {
   extern __shared__ __align__(1024) unsigned char fsm[];
   constexpr int kSlice = kInfRows * 64 * 2;  // one 128 x 64 bf16 slice
+  constexpr bool kWhole = H == 128;          // W2 staged whole
+  constexpr int KH = H / 64;
   unsigned char* sx = fsm;
   unsigned char* sw1 = sx + kSlice;
   unsigned char* sa1 = sw1 + (size_t)H * 128;
-  unsigned char* sw2 = sa1 + (size_t)(H / 64) * kSlice;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sw2 + (size_t)H * 128);
+  unsigned char* sw2 = sa1 + (size_t)KH * kSlice;
+  float* sxw = reinterpret_cast<float*>(sw2 + mlp_infer_w2_bytes(H));  // [j][64]: xw[k][j]
+  float* sb1 = sxw + 64 * 64;
+  float* sb2 = sb1 + H;
+  float* sw3 = sb2 + H;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sw3 + H);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rloc = (warp & 3) * 32 + lane;  // this thread's TMEM lane = row
   const int quarter = warp >> 2;            // hidden-column quarter
   const int row0 = blockIdx.x * kInfRows;
-  const int KH = H / 64;
 
   if (warp == 0) tmem_alloc(tslot, 256);
   if (tid == 0) {
     mbar_init(bar, 1);
     mbar_fence_init();
   }
+  // The network: W1 (H x 64) and, at H = 128, W2 in their K-major layouts, the
+  // whitening matrix transposed, the per-column operands.
+  for (int i = tid; i < H * 8; i += kInfThreads) {
+    const int r = i >> 3, c8 = (i & 7) * 8;
+    *reinterpret_cast<uint4*>(sw1 + kmajor_offset(r, c8, H)) =
+        *reinterpret_cast<const uint4*>(W1h + (size_t)r * 64 + c8);
+  }
+  if constexpr (kWhole) {
+    for (int i = tid; i < H * H / 8; i += kInfThreads) {
+      const int r = i / (H / 8), c8 = (i % (H / 8)) * 8;
+      *reinterpret_cast<uint4*>(sw2 + (size_t)(c8 / 64) * H * 128 +
+                                kmajor_offset(r, c8 % 64, H)) =
+          *reinterpret_cast<const uint4*>(W2h + (size_t)r * H + c8);
+    }
+  }
+  if (xw)
+    for (int i = tid; i < 64 * d; i += kInfThreads) {
+      const int k = i % 64, j = i / 64;
+      sxw[j * 64 + k] = k < d ? xw[(size_t)k * d + j] : 0.0f;
+    }
+  for (int i = tid; i < H; i += kInfThreads) {
+    sb1[i] = b1[i];
+    sb2[i] = b2[i];
+    sw3[i] = w3[i];
+  }
+  const float b3v = b3[0];
+  pdl_wait();
+  pdl_trigger();
 
   // Inputs: row rloc, input columns [16 quarter, 16 quarter + 16).  The
   // centred values go to a swizzled scratch (conflict-free column access).
@@ -366,39 +409,45 @@ mlp_infer_fused(const double* __restrict__ theta, int n, int d, int H,
     for (int j = quarter; j < d; j += 4)
       cen[rloc * 64 + ((j + rloc) & 63)] = live ? (float)th[j] - xmean[j] : 0.0f;
     __syncthreads();
-    for (int k8 = quarter * 16; k8 < quarter * 16 + 16; k8 += 8) {
-      __align__(16) bf16 v8[8];
+    float v[16];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int k = k8 + q;
-        float v = 0.0f;
-        if (live && k < d) {
-          if (xw) {
-            const float* wr = xw + (size_t)k * d;
-            for (int j = 0; j < d; ++j) v = fmaf(wr[j], cen[rloc * 64 + ((j + rloc) & 63)], v);
-          } else {
-            v = cen[rloc * 64 + ((k + rloc) & 63)] * xinv[k];
+    for (int q = 0; q < 16; ++q) v[q] = 0.0f;
+    const int k0 = quarter * 16;
+    if (live && k0 < d) {
+      if (xw) {
+        for (int j = 0; j < d; ++j) {
+          const float c = cen[rloc * 64 + ((j + rloc) & 63)];
+          const float4* w4 = reinterpret_cast<const float4*>(sxw + j * 64 + k0);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 w = w4[q];
+            v[4 * q] = fmaf(w.x, c, v[4 * q]);
+            v[4 * q + 1] = fmaf(w.y, c, v[4 * q + 1]);
+            v[4 * q + 2] = fmaf(w.z, c, v[4 * q + 2]);
+            v[4 * q + 3] = fmaf(w.w, c, v[4 * q + 3]);
           }
         }
-        v8[q] = __float2bfloat16(v);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+          if (k0 + q < d) v[q] = cen[rloc * 64 + ((k0 + q + rloc) & 63)] * xinv[k0 + q];
       }
-      *reinterpret_cast<uint4*>(sx + kmajor_offset(rloc, k8, kInfRows)) =
-          *reinterpret_cast<const uint4*>(v8);
     }
-  }
-  // W1 (H x 64) into its K-major layout.
-  for (int i = tid; i < H * 8; i += kInfThreads) {
-    const int r = i >> 3, c8 = (i & 7) * 8;
-    *reinterpret_cast<uint4*>(sw1 + kmajor_offset(r, c8, H)) =
-        *reinterpret_cast<const uint4*>(W1h + (size_t)r * 64 + c8);
+    __align__(16) bf16 v8[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v8[q] = __float2bfloat16(k0 + q < d ? v[q] : 0.0f);
+    *reinterpret_cast<uint4*>(sx + kmajor_offset(rloc, k0, kInfRows)) =
+        *reinterpret_cast<const uint4*>(v8);
+    *reinterpret_cast<uint4*>(sx + kmajor_offset(rloc, k0 + 8, kInfRows)) =
+        *reinterpret_cast<const uint4*>(v8 + 8);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tslot;
-  const uint32_t idesc = umma_idesc_bf16(kInfRows, H);
-  const uint32_t lbo_x = (kInfRows / 8) * 128, lbo_h = (uint32_t)(H / 8) * 128;
+  constexpr uint32_t idesc = umma_idesc_bf16(kInfRows, H);
+  constexpr uint32_t lbo_x = (kInfRows / 8) * 128, lbo_h = (uint32_t)(H / 8) * 128;
   if (tid == 0) {
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
@@ -407,43 +456,39 @@ mlp_infer_fused(const double* __restrict__ theta, int n, int d, int H,
                 kk > 0 ? 1u : 0u);
     umma_commit(bar);
   }
-  // W2 slice prefetch into registers while layer 1 runs (H x 64 per slice).
-  constexpr int kMaxPf = 256 * 8 / kInfThreads;  // 4 chunks per thread at H = 256
-  uint4 pf[kMaxPf];
-  const int npf = H * 8 / kInfThreads;
+  // At H = 256: W2 slice prefetch into registers while layer 1 runs.
+  constexpr int npf = kWhole ? 1 : H * 8 / kInfThreads;
+  uint4 pf[npf];
   auto load_w2 = [&](int s) {
 #pragma unroll
-    for (int q = 0; q < kMaxPf; ++q) {
-      if (q < npf) {
-        const int i = tid + q * kInfThreads, r = i >> 3, c8 = (i & 7) * 8;
-        pf[q] = *reinterpret_cast<const uint4*>(W2h + (size_t)r * H + s * 64 + c8);
-      }
+    for (int q = 0; q < npf; ++q) {
+      const int i = tid + q * kInfThreads, r = i >> 3, c8 = (i & 7) * 8;
+      pf[q] = *reinterpret_cast<const uint4*>(W2h + (size_t)r * H + s * 64 + c8);
     }
   };
   auto store_w2 = [&]() {
 #pragma unroll
-    for (int q = 0; q < kMaxPf; ++q) {
-      if (q < npf) {
-        const int i = tid + q * kInfThreads, r = i >> 3, c8 = (i & 7) * 8;
-        *reinterpret_cast<uint4*>(sw2 + kmajor_offset(r, c8, H)) = pf[q];
-      }
+    for (int q = 0; q < npf; ++q) {
+      const int i = tid + q * kInfThreads, r = i >> 3, c8 = (i & 7) * 8;
+      *reinterpret_cast<uint4*>(sw2 + kmajor_offset(r, c8, H)) = pf[q];
     }
   };
-  load_w2(0);
+  if constexpr (!kWhole) load_w2(0);
   int ok = mbar_wait_bounded(bar, 0u) ? 1 : 0;
   ok = __syncthreads_and(ok);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-  const int cq = H / 4;  // hidden columns per quarter (64 or 32)
+  constexpr int cq = H / 4;  // hidden columns per quarter (64 or 32)
   const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   if (ok) {
     // Layer-1 epilogue: A1 = silu(Z1 + b1) as bf16 into the layer-2 A operand.
+#pragma unroll
     for (int c = quarter * cq; c < quarter * cq + cq; c += 16) {
       float v[16];
       tmem_ld16(trow + (uint32_t)c, v);
       __align__(16) bf16 a8[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) a8[j] = __float2bfloat16(silu(v[j] + b1[c + j]));
+      for (int j = 0; j < 16; ++j) a8[j] = __float2bfloat16(silu(v[j] + sb1[c + j]));
       unsigned char* base = sa1 + (size_t)(c / 64) * kSlice;
       *reinterpret_cast<uint4*>(base + kmajor_offset(rloc, c % 64, kInfRows)) =
           *reinterpret_cast<const uint4*>(a8);
@@ -451,23 +496,31 @@ mlp_infer_fused(const double* __restrict__ theta, int n, int d, int H,
           *reinterpret_cast<const uint4*>(a8 + 8);
     }
   }
-  // Layer 2 over the K slices of A1 / W2.
-  for (int s = 0; s < KH && ok; ++s) {
-    store_w2();
+  // Layer 2: K slices of A1 and W2, each step's products committed together.
+  constexpr int kSteps = kWhole ? 1 : KH, kPer = KH / kSteps;
+  for (int s = 0; s < kSteps && ok; ++s) {
+    if constexpr (!kWhole) store_w2();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (tid == 0) {
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
+      for (int kk = 0; kk < 4 * kPer; ++kk) {
+        const int sl = s * kPer + kk / 4, k4 = kk % 4;
         umma_bf16(tmem,
-                  umma_smem_desc(smem_addr(sa1 + (size_t)s * kSlice) + 2 * kk * lbo_x, lbo_x, 128),
-                  umma_smem_desc(smem_addr(sw2) + 2 * kk * lbo_h, lbo_h, 128), idesc,
-                  (s > 0 || kk > 0) ? 1u : 0u);
+                  umma_smem_desc(smem_addr(sa1 + (size_t)sl * kSlice) + 2 * k4 * lbo_x, lbo_x,
+                                 128),
+                  umma_smem_desc(smem_addr(sw2 + (kWhole ? (size_t)sl * H * 128 : 0)) +
+                                     2 * k4 * lbo_h,
+                                 lbo_h, 128),
+                  idesc, (s > 0 || kk > 0) ? 1u : 0u);
+      }
       umma_commit(bar);
     }
-    if (s + 1 < KH) load_w2(s + 1);
+    if constexpr (!kWhole) {
+      if (s + 1 < kSteps) load_w2(s + 1);
+    }
     ok = mbar_wait_bounded(bar, (uint32_t)((s + 1) & 1)) ? 1 : 0;
     ok = __syncthreads_and(ok);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -477,11 +530,12 @@ mlp_infer_fused(const double* __restrict__ theta, int n, int d, int H,
   float* part = reinterpret_cast<float*>(sa1);
   if (ok) {
     float acc = 0.0f;
+#pragma unroll
     for (int c = quarter * cq; c < quarter * cq + cq; c += 16) {
       float v[16];
       tmem_ld16(trow + (uint32_t)c, v);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) acc = fmaf(silu(v[j] + b2[c + j]), w3[c + j], acc);
+      for (int j = 0; j < 16; ++j) acc = fmaf(silu(v[j] + sb2[c + j]), sw3[c + j], acc);
     }
     part[quarter * kInfRows + rloc] = acc;
   } else if (tid == 0) {
@@ -492,7 +546,7 @@ mlp_infer_fused(const double* __restrict__ theta, int n, int d, int H,
     const int row = row0 + rloc;
     const float y = ((part[rloc] + part[kInfRows + rloc]) + part[2 * kInfRows + rloc]) +
                     part[3 * kInfRows + rloc];
-    if (row < n) out[row] = (double)(y + b3[0]) * ysd + ymean;
+    if (row < n) out[row] = (double)(y + b3v) * ysd + ymean;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -737,9 +791,11 @@ int mlp_infer_launches(const gpum_b200_mlp* m, int n) {
 }
 
 // Surrogate log-likelihood of n f64 parameter vectors (device, chain-major)
-// into out (device), enqueued on `st`.  Used by the delayed-acceptance loop.
+// into out (device), enqueued on `st`.  Used by the delayed-acceptance loop
+// (`pdl`: the fused kernel may start while the launch before it runs; the
+// network has not been changed by that launch).
 int mlp_infer(gpum_b200_mlp* m, const double* theta, int n, int d, double* out, cudaStream_t st,
-              std::string* err) {
+              std::string* err, bool pdl) {
   if (!m || d != m->d) {
     *err = "surrogate input width does not match the model's parameter count";
     return GPUM_ERR_INVALID;
@@ -750,16 +806,27 @@ int mlp_infer(gpum_b200_mlp* m, const double* theta, int n, int d, double* out, 
   try {
     if (m->fused_inference()) {
       const size_t smem = mlp_infer_smem(m->H);
+      const void* fn = m->H == 128 ? (const void*)mlp_infer_fused<128>
+                                   : (const void*)mlp_infer_fused<256>;
       if (!m->infer_smem_set) {
-        MLP_CK(cudaFuncSetAttribute(mlp_infer_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+        MLP_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         m->infer_smem_set = true;
       }
       if (n > 0) {
-        mlp_infer_fused<<<(unsigned)((n + kInfRows - 1) / kInfRows), kInfThreads, smem, st>>>(
-            theta, n, d, m->H, m->xmean.p, m->xinv.p, m->xw_or_null(), m->W1h.p, m->b1p(),
-            m->W2h.p, m->b2p(), m->w3p(), m->b3p(), m->ysd, m->ymean, out, m->err.p);
-        MLP_CK(cudaGetLastError());
+        const float *xmean = m->xmean.p, *xinv = m->xinv.p, *xw = m->xw_or_null(), *b1 = m->b1p(),
+                    *b2 = m->b2p(), *w3 = m->w3p(), *b3 = m->b3p();
+        const bf16 *W1 = m->W1h.p, *W2 = m->W2h.p;
+        uint32_t* e = m->err.p;
+        void* args[] = {(void*)&theta, (void*)&n,  (void*)&d,  (void*)&xmean, (void*)&xinv,
+                        (void*)&xw,    (void*)&W1, (void*)&b1, (void*)&W2,    (void*)&b2,
+                        (void*)&w3,    (void*)&b3, (void*)&m->ysd, (void*)&m->ymean,
+                        (void*)&out,   (void*)&e};
+        const dim3 grid((unsigned)((n + kInfRows - 1) / kInfRows));
+        if (pdl) {
+          MLP_CK(launch_dependent(fn, grid, dim3(kInfThreads), args, smem, st));
+        } else {
+          MLP_CK(cudaLaunchKernel(fn, grid, dim3(kInfThreads), args, smem, st));
+        }
       }
       m->st = keep;
       return GPUM_OK;
@@ -1104,7 +1171,7 @@ int gpum_b200_mlp_predict(gpum_b200_mlp* m, const double* theta, size_t n, doubl
     MLP_CK(cudaMemcpyAsync(dth.p, theta, n * m->d * sizeof(double), cudaMemcpyHostToDevice,
                            m->st));
     std::string e;
-    const int rc = gpum::mlp_infer(m, dth.p, (int)n, m->d, dout.p, m->st, &e);
+    const int rc = gpum::mlp_infer(m, dth.p, (int)n, m->d, dout.p, m->st, &e, false);
     if (rc != GPUM_OK) throw MlpFail{rc, e};
     MLP_CK(cudaMemcpyAsync(out, dout.p, n * sizeof(double), cudaMemcpyDeviceToHost, m->st));
     MLP_CK(cudaStreamSynchronize(m->st));

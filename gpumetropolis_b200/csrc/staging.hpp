@@ -166,11 +166,13 @@ inline void convert_copy(double* dst, const float* src, size_t n) {
 // the 26 MB 1.45.)
 template <class To, class From>
 cudaError_t copy_to_host(To* dst, const From* src, size_t n, cudaStream_t st) {
+  // The threads poll for chunks, so they start when there is something to copy.
+  cudaError_t e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return e;
   const size_t per = kChunkPinned / sizeof(From), chunks = (n + per - 1) / per;
   const size_t want = std::min<size_t>(kChunkBlocks, std::max<size_t>(chunks, 1));
   std::vector<char*> blocks;
   std::vector<cudaEvent_t> ev;
-  cudaError_t e = cudaSuccess;
   while (blocks.size() < want) {
     char* p = pinned_chunks().take();
     if (!p) break;
