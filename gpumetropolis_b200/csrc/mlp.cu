@@ -11,14 +11,15 @@
 //
 // One training step on a batch of B rows (B, H multiples of 128, H <= 512;
 // the input width padded to dp, a multiple of 64) is seven kernels, captured
-// once per train() call as a CUDA graph and replayed:
-//   gather   X (bf16, row-major and transposed), targets t
+// four steps at a time as a CUDA graph and replayed:
+//   gather   X (bf16, row-major and transposed), targets t: of the next step,
+//            into the other of two buffers, on a second stream
 //   GEMM1    Z1 = X W1^T + b1; A1 = silu(Z1) (row-major and transposed)
 //   GEMM2    Z2 = A1 W2^T + b2 with the head fused into its epilogue (one
 //            CTA holds whole rows): y = silu(Z2) w3 + b3, r = y - t, dy =
 //            2r/B, dZ2 = dy w3 silu'(Z2) (both layouts); per-CTA column sums
 //            for w3's and b2's gradients, row sums for b3's and the loss
-//   GEMM3    dW2 = dZ2^T A1, split K into fixed partials
+//   GEMM3    dW2 = dZ2^T A1, split K into fixed partials (second stream)
 //   GEMM4    dZ1 = (dZ2 W2) * silu'(Z1) (transposed); per-CTA sums for b1's
 //   GEMM5    dW1 = dZ1^T X, split K into fixed partials
 //   adam     every gradient from its partials in a fixed order, then Adam
@@ -115,12 +116,13 @@ __device__ __forceinline__ void mlp_input_row(Src theta_at, bool live, int d, in
 // transposed) and standardised targets, one warp per row, kGatherRows rows
 // per block.
 // idx_mode 0: rows 0..n-1 in order (inference / gradient check);
-//          1: Philox-random rows of the training set at step ctr[0].
+//          1: Philox-random rows of the training set at step ctr[0] + ahead.
 constexpr int kGatherRows = 8;
 
 __global__ void mlp_gather(const float* __restrict__ theta, const double* __restrict__ ll,
                            size_t n, int d, int dp, int B, int idx_mode, uint32_t seed,
-                           const uint32_t* __restrict__ ctr, const float* __restrict__ xmean,
+                           const uint32_t* __restrict__ ctr, uint32_t ahead,
+                           const float* __restrict__ xmean,
                            const float* __restrict__ xinv, const float* __restrict__ xw,
                            float ymean, float yinv, bf16* __restrict__ Xh,
                            bf16* __restrict__ XTh, float* __restrict__ t) {
@@ -128,7 +130,8 @@ __global__ void mlp_gather(const float* __restrict__ theta, const double* __rest
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * kGatherRows + warp;
   if (row >= B) return;  // whole warps leave; no block-wide barrier follows
-  size_t src = idx_mode ? pick(seed, ctr[0], (uint32_t)row, (uint32_t)n) : (size_t)row;
+  size_t src = idx_mode ? pick(seed, ctr[0] + ahead, (uint32_t)row, (uint32_t)n)
+                        : (size_t)row;
   const bool live = src < n;
   if (!live) src = 0;
   const float* th = theta + src * d;
@@ -173,43 +176,73 @@ struct GradParts {
   int nct;
 };
 
+// p[0] + p[st] + ... of n values in order, sixteen loads in flight (one after
+// the other they were half of the kernel's 8.3 us).
+__device__ __forceinline__ float sum_in_order(const float* __restrict__ p, size_t st, int n) {
+  float g = 0.0f;
+  int z = 0;
+  for (; z + 16 <= n; z += 16) {
+    float v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = __ldcg(p + (size_t)(z + k) * st);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) g += v[k];
+  }
+  for (; z < n; ++z) g += __ldcg(p + (size_t)z * st);
+  return g;
+}
+
+// A learning-rate schedule in device memory: stage k runs to step ends[k]
+// (from the first step of the call).
+struct Schedule {
+  const uint32_t* ends;
+  const float* lrs;
+  int n;
+};
+__device__ __forceinline__ float lr_at(const Schedule& S, uint32_t step) {
+  int lo = 0, hi = S.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    if (step < S.ends[mid]) hi = mid;
+    else lo = mid + 1;
+  }
+  return S.lrs[lo];
+}
+
 // Every gradient from its partials (fixed order) into G; with `apply`, Adam
-// (learning rate *lr_p, device memory, so a captured step serves every stage
-// of a schedule) at step ctr[0] + 1 on the master weights and their BF16 copies (W1h, W2h
+// at step ctr[0] + 1 on the master weights and their BF16 copies (W1h, W2h
 // and the transposed W1Th, W2Th), the loss of the step into
-// loss_hist[ctr[0] - loss_base]; mlp_step_done then advances ctr[0].
+// loss_hist[ctr[0] - loss_base]; the last block to finish (a ticket, ctr[1])
+// advances ctr[0], which every block has read by then.
 __global__ void mlp_reduce_adam(MlpLayout L, GradParts Gp, float* __restrict__ P,
                                 float* __restrict__ Mm, float* __restrict__ V,
                                 float* __restrict__ G, bf16* __restrict__ W1h,
                                 bf16* __restrict__ W1Th, bf16* __restrict__ W2h,
-                                bf16* __restrict__ W2Th, const float* __restrict__ lr_p,
+                                bf16* __restrict__ W2Th, Schedule sched,
                                 int apply, uint32_t* __restrict__ ctr, float* __restrict__ loss,
                                 uint32_t loss_base, uint32_t loss_cap) {
   const uint32_t step = *reinterpret_cast<volatile const uint32_t*>(ctr);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int H = L.H, dp = L.dp;
+  pdl_trigger();
   if (i < L.n) {
     float g = 0.0f;
     if (i < L.ob1) {
-      for (int z = 0; z < Gp.S1; ++z) g += Gp.pW1[(size_t)z * H * dp + i];
+      g = sum_in_order(Gp.pW1 + i, (size_t)H * dp, Gp.S1);
     } else if (i < L.oW2) {
-      const size_t j = i - L.ob1;
-      for (int c = 0; c < Gp.nct; ++c) g += Gp.colb1[(size_t)c * H + j];
+      g = sum_in_order(Gp.colb1 + (i - L.ob1), H, Gp.nct);
     } else if (i < L.ob2) {
-      const size_t k = i - L.oW2;
-      for (int z = 0; z < Gp.S2; ++z) g += Gp.pW2[(size_t)z * H * H + k];
+      g = sum_in_order(Gp.pW2 + (i - L.oW2), (size_t)H * H, Gp.S2);
     } else if (i < L.ow3) {
-      const size_t j = i - L.ob2;
-      for (int c = 0; c < Gp.nct; ++c) g += Gp.colhead[((size_t)Gp.nct + c) * H + j];
+      g = sum_in_order(Gp.colhead + (size_t)Gp.nct * H + (i - L.ob2), H, Gp.nct);
     } else if (i < L.ob3) {
-      const size_t j = i - L.ow3;
-      for (int c = 0; c < Gp.nct; ++c) g += Gp.colhead[(size_t)c * H + j];
+      g = sum_in_order(Gp.colhead + (i - L.ow3), H, Gp.nct);
     } else {
-      for (int c = 0; c < Gp.nct; ++c) g += Gp.rowpart[c];
+      g = sum_in_order(Gp.rowpart, 1, Gp.nct);
     }
     G[i] = g;
     if (apply) {
-      const float lr = *lr_p;
+      const float lr = lr_at(sched, step - loss_base);
       const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
       const float t = (float)(step + 1);
       const float c1 = 1.0f - powf(b1, t), c2 = 1.0f - powf(b2, t);
@@ -230,17 +263,17 @@ __global__ void mlp_reduce_adam(MlpLayout L, GradParts Gp, float* __restrict__ P
     }
   }
   if (i == 0 && loss) {
-    float s = 0.0f;
-    for (int c = 0; c < Gp.nct; ++c) s += Gp.rowpart[Gp.nct + c];
+    const float s = sum_in_order(Gp.rowpart + Gp.nct, 1, Gp.nct);
     const uint32_t slot = step - loss_base;
     if (slot < loss_cap) loss[slot] = s;
   }
-}
-
-// The step counter advances after the reduction (a kernel of its own: every
-// block of the reduction has read the counter by then).
-__global__ void mlp_step_done(uint32_t* __restrict__ ctr) {
-  if (threadIdx.x == 0) ctr[0] += 1;
+  if (apply) {
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&ctr[1], 1u) == gridDim.x - 1) {
+      ctr[1] = 0;
+      ctr[0] = step + 1;
+    }
+  }
 }
 
 __global__ void mlp_init_weights(float* __restrict__ w, size_t n, int fan_in, int cols_live,
@@ -568,13 +601,16 @@ struct gpum_b200_mlp {
   Buf<float> P, Mm, V, G;
   Buf<bf16> W1h, W1Th, W2h, W2Th;
   // batch work buffers
-  Buf<bf16> Xh, XTh, A1h, A1Th, dZ2h, dZ2Th, dZ1Th;
-  Buf<float> Z1, t, yhat, dX;
+  // the batch in two buffers: a step's gather runs during the step before
+  Buf<bf16> Xh[2], XTh[2], A1h, A1Th, dZ2h, dZ2Th, dZ1Th;
+  Buf<float> Z1, t[2], yhat, dX;
   // gradient partials: split K (weights), per-CTA columns / rows (biases, head, loss)
   Buf<float> pW1, pW2, colhead, colb1, rowpart;
   int S1 = 1, S2 = 1;
-  Buf<uint32_t> ctr;   // [step, unused]
-  Buf<float> lr;       // [1] the current learning rate
+  Buf<uint32_t> ctr;   // [step, ticket of the reduction]
+  Buf<float> lrs;      // learning rates of a call's stages
+  Buf<uint32_t> ends;  // and the steps they end at
+  Schedule sched{};
   Buf<float> losses;   // per-step sums of squared residuals of one train() call
   // normaliser
   Buf<float> xmean, xinv, xw;  // xw: d x d whitening, used when `whiten`
@@ -583,7 +619,7 @@ struct gpum_b200_mlp {
   float ymean = 0.0f, yinv = 1.0f, ysd = 1.0f;
   Buf<uint32_t> err;
   bool infer_smem_set = false;
-  bool gemm_smem_set[16] = {};  // per (BN, epilogue) instantiation
+  bool gemm_smem_set[20] = {};  // per (BN, epilogue) instantiation
 
   float* W1p() const { return P.p + L.oW1; }
   float* b1p() const { return P.p + L.ob1; }
@@ -596,26 +632,41 @@ struct gpum_b200_mlp {
   bool fused_inference() const { return dp == 64 && (H == 128 || H == 256); }
 
   ~gpum_b200_mlp() {
+    if (st2) cudaStreamSynchronize(st2);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (st2) cudaStreamDestroy(st2);
     if (st) cudaStreamDestroy(st);
   }
 
+  // `pdl`: may start while the kernel before it in the stream runs.
   template <int BN, int EPI>
-  void gemm(const GemmArgs& a, int S) {
+  void gemm(const GemmArgs& a, int S, bool pdl = false) {
     const size_t smem = tc_gemm_smem<BN>();
     // Set once per instantiation, so later launches (possibly under stream
     // capture) make no non-stream API calls.
-    constexpr int slot = (BN == 64 ? 0 : BN == 128 ? 1 : BN == 256 ? 2 : 3) * 4 + EPI;
+    constexpr int slot =
+        (BN == 64 ? 0 : BN == 128 ? 1 : BN == 256 ? 2 : BN == 512 ? 3 : 4) * 4 + EPI;
+    const void* fn = (const void*)tc_gemm_kernel<BN, EPI>;
     if (!gemm_smem_set[slot]) {
-      MLP_CK(cudaFuncSetAttribute(tc_gemm_kernel<BN, EPI>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      MLP_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       gemm_smem_set[slot] = true;
     }
     dim3 grid(a.N / BN, a.M / kGemmBM, S);
-    tc_gemm_kernel<BN, EPI><<<grid, kGemmThreads, smem, st>>>(a);
-    MLP_CK(cudaGetLastError());
+    void* args[] = {(void*)&a};
+    if (pdl) {
+      MLP_CK(launch_dependent(fn, grid, dim3(kGemmThreads<EPI>), args, smem, st));
+    } else {
+      MLP_CK(cudaLaunchKernel(fn, grid, dim3(kGemmThreads<EPI>), args, smem, st));
+    }
+  }
+  // A layer's output in tiles of a quarter of its width: at batch 4096 and H =
+  // 128 that is 128 CTAs instead of 32.
+  template <int EPI>
+  void gemm_quarter(const GemmArgs& a, bool pdl) {
+    if (H == 128) gemm<32, EPI>(a, 1, pdl);
+    else if (H == 256) gemm<64, EPI>(a, 1, pdl);
+    else gemm<128, EPI>(a, 1, pdl);
   }
 
   GemmArgs args(const bf16* A, const bf16* Bm, int M, int N, int K) const {
@@ -630,15 +681,17 @@ struct gpum_b200_mlp {
     return a;
   }
 
-  // Layer 1 (SiLU epilogue) and layer 2 with the head, for `rows` rows in Xh;
-  // targets in t for the first n_live rows (nullptr: inference, r = 0).
-  void forward(int rows, int n_live, const float* targets, int unit_dy = 0) {
-    GemmArgs a1 = args(Xh.p, W1h.p, rows, H, dp);
+  // Layer 1 (SiLU epilogue) and layer 2 with the head, for `rows` rows in
+  // Xh[xb]; targets in t for the first n_live rows (nullptr: inference, r = 0).
+  // `pdl`: layer 1 may start while the kernel before it runs.
+  void forward(int rows, int n_live, const float* targets, int unit_dy = 0, int xb = 0,
+               bool pdl = false) {
+    GemmArgs a1 = args(Xh[xb].p, W1h.p, rows, H, dp);
     a1.C = Z1.p;
     a1.bias = b1p();
     a1.act = A1h.p;
     a1.actT = targets ? A1Th.p : nullptr;
-    gemm<128, EPI_SILU>(a1, 1);
+    gemm_quarter<EPI_SILU>(a1, pdl);
     GemmArgs a2 = args(A1h.p, W2h.p, rows, H, H);
     a2.bias = b2p();
     a2.w3 = w3p();
@@ -651,53 +704,46 @@ struct gpum_b200_mlp {
     a2.actT = targets ? dZ2Th.p : nullptr;
     a2.unit_dy = unit_dy;
     a2.yhat = yhat.p;
-    if (H == 128) gemm<128, EPI_HEAD>(a2, 1);
-    else if (H == 256) gemm<256, EPI_HEAD>(a2, 1);
-    else gemm<512, EPI_HEAD>(a2, 1);
+    if (H == 128) gemm<128, EPI_HEAD>(a2, 1, true);
+    else if (H == 256) gemm<256, EPI_HEAD>(a2, 1, true);
+    else gemm<512, EPI_HEAD>(a2, 1, true);
   }
 
   // Weight gradients and b1's (after forward() with targets), then the
   // reduction of every gradient into G, with Adam when `apply`.
   void backward_and_update(int apply, float* loss_hist, uint32_t loss_base,
-                           uint32_t loss_cap) {
-    GemmArgs g3 = args(dZ2Th.p, A1Th.p, H, H, B);  // dW2 = dZ2^T A1
-    g3.C = pW2.p;
-    g3.kz = B / S2;
+                           uint32_t loss_cap, int xb = 0) {
     // dW2 on the second stream, concurrent with dZ1 and dW1 (both only read
     // dZ2); the reduction waits for both.  Under stream capture the fork and
     // join become graph edges.
-    const bool fork = st2 != nullptr;
-    if (fork) {
-      MLP_CK(cudaEventRecord(ev_fork, st));
-      MLP_CK(cudaStreamWaitEvent(st2, ev_fork, 0));
-      cudaStream_t keep = st;
-      st = st2;
-      try {
-        gemm<64, EPI_STORE>(g3, S2);
-      } catch (...) {
-        st = keep;
-        throw;
-      }
-      st = keep;
-      MLP_CK(cudaEventRecord(ev_join, st2));
-    } else {
+    GemmArgs g3 = args(dZ2Th.p, A1Th.p, H, H, B);  // dW2 = dZ2^T A1
+    g3.C = pW2.p;
+    g3.kz = B / S2;
+    MLP_CK(cudaEventRecord(ev_fork, st));
+    MLP_CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+    std::swap(st, st2);
+    try {
       gemm<64, EPI_STORE>(g3, S2);
+    } catch (...) {
+      std::swap(st, st2);
+      throw;
     }
+    std::swap(st, st2);
+    MLP_CK(cudaEventRecord(ev_join, st2));
     GemmArgs g4 = args(dZ2h.p, W2Th.p, B, H, H);   // dZ1 = (dZ2 W2) * silu'(Z1)
     g4.Zprev = Z1.p;
     g4.actT = dZ1Th.p;
     g4.colpart = colb1.p;
-    gemm<128, EPI_DSILU>(g4, 1);
-    GemmArgs g5 = args(dZ1Th.p, XTh.p, H, dp, B);  // dW1 = dZ1^T X
+    gemm_quarter<EPI_DSILU>(g4, true);
+    GemmArgs g5 = args(dZ1Th.p, XTh[xb].p, H, dp, B);  // dW1 = dZ1^T X
     g5.C = pW1.p;
     g5.kz = B / S1;
-    gemm<64, EPI_STORE>(g5, S1);
-    if (fork) MLP_CK(cudaStreamWaitEvent(st, ev_join, 0));
+    gemm<64, EPI_STORE>(g5, S1, true);
+    MLP_CK(cudaStreamWaitEvent(st, ev_join, 0));
     GradParts gp{pW1.p, S1, pW2.p, S2, colhead.p, colb1.p, rowpart.p, B / kGemmBM};
     mlp_reduce_adam<<<blocks(L.n), 256, 0, st>>>(L, gp, P.p, Mm.p, V.p, G.p, W1h.p, W1Th.p,
-                                                  W2h.p, W2Th.p, lr.p, apply, ctr.p, loss_hist,
+                                                  W2h.p, W2Th.p, sched, apply, ctr.p, loss_hist,
                                                   loss_base, loss_cap);
-    if (apply) mlp_step_done<<<1, 32, 0, st>>>(ctr.p);
     MLP_CK(cudaGetLastError());
   }
 
@@ -711,10 +757,10 @@ struct gpum_b200_mlp {
     GemmArgs g4 = args(dZ2h.p, W2Th.p, rows, H, H);  // dZ1 = (dZ2 W2) * silu'(Z1)
     g4.Zprev = Z1.p;
     g4.act = A1Th.p;
-    gemm<128, EPI_DSILU>(g4, 1);
+    gemm_quarter<EPI_DSILU>(g4, true);
     GemmArgs g5 = args(A1Th.p, W1Th.p, rows, dp, H);  // dX = dZ1 W1
     g5.C = dX.p;
-    gemm<64, EPI_STORE>(g5, 1);
+    gemm<64, EPI_STORE>(g5, 1, true);
     mlp_input_grad<<<blocks((size_t)n * 32), 256, 0, st>>>(dX.p, n, d_in, dp, xinv.p,
                                                            xw_or_null(), ysd, out_grad);
     MLP_CK(cudaGetLastError());
@@ -754,14 +800,26 @@ void need(bool ok, const char* msg, int code = GPUM_ERR_INVALID) {
   if (!ok) throw MlpFail{code, msg};
 }
 
-// Upload host pairs (theta f64 -> f32, ll f64) into device buffers.
+__global__ void mlp_narrow(const double* __restrict__ x, size_t n, float* __restrict__ out) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (float)x[i];
+}
+
+// Upload host pairs (theta f64 -> f32 on the device, ll f64) into device
+// buffers, the parameters through 16 MB of staging.
 void upload_pairs(gpum_b200_mlp* m, const double* theta, const double* ll, size_t n,
                   Buf<float>& dth, Buf<double>& dll) {
-  std::vector<float> th((size_t)n * m->d);
-  for (size_t i = 0; i < th.size(); ++i) th[i] = (float)theta[i];
-  dth.alloc(th.size());
-  MLP_CK(cudaMemcpyAsync(dth.p, th.data(), th.size() * sizeof(float), cudaMemcpyHostToDevice,
-                         m->st));
+  const size_t total = n * m->d, per = std::min<size_t>(total, (size_t)2 << 20);
+  Buf<double> stage;
+  stage.alloc(per);
+  dth.alloc(total);
+  for (size_t at = 0; at < total; at += per) {
+    const size_t k = std::min(per, total - at);
+    MLP_CK(cudaMemcpyAsync(stage.p, theta + at, k * sizeof(double), cudaMemcpyHostToDevice,
+                           m->st));
+    mlp_narrow<<<blocks(k), 256, 0, m->st>>>(stage.p, k, dth.p + at);
+    MLP_CK(cudaGetLastError());
+  }
   if (ll) {
     dll.alloc(n);
     MLP_CK(cudaMemcpyAsync(dll.p, ll, n * sizeof(double), cudaMemcpyHostToDevice, m->st));
@@ -835,7 +893,7 @@ int mlp_infer(gpum_b200_mlp* m, const double* theta, int n, int d, double* out, 
       const int rows = std::min(m->B, n - r0);
       const int Mi = (rows + kGemmBM - 1) / kGemmBM * kGemmBM;  // rows padded to the tile
       mlp_gather64<<<Mi, 128, 0, st>>>(theta + (size_t)r0 * d, rows, d, m->dp, Mi, m->xmean.p,
-                                       m->xinv.p, m->xw_or_null(), m->Xh.p);
+                                       m->xinv.p, m->xw_or_null(), m->Xh[0].p);
       m->forward(Mi, Mi, nullptr);
       mlp_unscale<<<blocks(rows), 256, 0, st>>>(m->yhat.p, rows, m->ysd, m->ymean, out + r0);
       MLP_CK(cudaGetLastError());
@@ -866,7 +924,7 @@ int mlp_infer_grad(gpum_b200_mlp* m, const double* theta, int n, int d, double* 
       const int rows = std::min(m->B, n - r0);
       const int Mi = (rows + kGemmBM - 1) / kGemmBM * kGemmBM;
       mlp_gather64<<<Mi, 128, 0, st>>>(theta + (size_t)r0 * d, rows, d, m->dp, Mi, m->xmean.p,
-                                       m->xinv.p, m->xw_or_null(), m->Xh.p);
+                                       m->xinv.p, m->xw_or_null(), m->Xh[0].p);
       MLP_CK(cudaGetLastError());
       m->value_grad(Mi, rows, d, out_val + r0, out_grad + (size_t)r0 * d);
     }
@@ -930,12 +988,14 @@ int gpum_b200_mlp_create(uint32_t d, uint32_t hidden, uint32_t batch, uint32_t s
     m->W1Th.alloc((size_t)dp * H);
     m->W2h.alloc((size_t)H * H);
     m->W2Th.alloc((size_t)H * H);
-    m->Xh.alloc((size_t)B * dp);
-    m->XTh.alloc((size_t)dp * B);
+    for (int k = 0; k < 2; ++k) {
+      m->Xh[k].alloc((size_t)B * dp);
+      m->XTh[k].alloc((size_t)dp * B);
+      m->t[k].alloc(B);
+    }
     for (auto* b : {&m->A1h, &m->dZ2h}) b->alloc((size_t)B * H);
     for (auto* b : {&m->A1Th, &m->dZ2Th, &m->dZ1Th}) b->alloc((size_t)H * B);
     m->Z1.alloc((size_t)B * H);
-    m->t.alloc(B);
     m->yhat.alloc(B);
     m->dX.alloc((size_t)B * dp);
     m->S2 = split_k(B, (H / 128) * (H / 64), sms, 16);
@@ -947,7 +1007,6 @@ int gpum_b200_mlp_create(uint32_t d, uint32_t hidden, uint32_t batch, uint32_t s
     m->colb1.alloc((size_t)nct * H);
     m->rowpart.alloc((size_t)2 * nct);
     m->ctr.alloc(2);
-    m->lr.alloc(1);
     m->xmean.alloc(d);
     m->xinv.alloc(d);
     m->xw.alloc((size_t)d * d);
@@ -1056,54 +1115,72 @@ void train_on_device(gpum_b200_mlp* m, const float* dth, const double* dll, size
                      float* out_loss) {
   m->losses.alloc(total);
   const uint32_t base = m->steps_done;
-  // One step: its kernels read the step from the device counter the
-  // reduction advances and the learning rate from device memory, so one
-  // captured CUDA graph serves all steps of all stages.
-  auto one_step = [&] {
-    mlp_gather<<<m->B / kGatherRows, 32 * kGatherRows, 0, m->st>>>(
-        dth, dll, n_pairs, m->d, m->dp, m->B, 1, m->seed, m->ctr.p, m->xmean.p,
-        m->xinv.p, m->xw_or_null(), m->ymean, m->yinv, m->Xh.p, m->XTh.p, m->t.p);
-    MLP_CK(cudaGetLastError());
-    m->forward(m->B, m->B, m->t.p);
-    m->backward_and_update(1, m->losses.p, base, (uint32_t)total);
-  };
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  bool first = true;
-  cudaError_t le = cudaSuccess;
-  for (uint32_t k = 0; k < n_stages && le == cudaSuccess; ++k) {
+  // The schedule in device memory: one captured graph serves all its steps.
+  std::vector<uint32_t> ends;
+  std::vector<float> rates;
+  uint32_t at = 0;
+  for (uint32_t k = 0; k < n_stages; ++k) {
     if (steps[k] == 0) continue;
-    const float lr_f = (float)lrs[k];
-    MLP_CK(cudaMemcpyAsync(m->lr.p, &lr_f, sizeof lr_f, cudaMemcpyHostToDevice, m->st));
-    MLP_CK(cudaStreamSynchronize(m->st));  // lr_f is a stack value
-    uint32_t left = steps[k];
-    if (first) {
-      one_step();  // eagerly: sets every kernel attribute outside capture
-      first = false;
-      --left;
-    }
-    if (left > 0 && !exec) {
-      MLP_CK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
-      try {
-        one_step();
-      } catch (...) {
-        cudaGraph_t g2 = nullptr;
-        cudaStreamEndCapture(m->st, &g2);
-        if (g2) cudaGraphDestroy(g2);
-        throw;
-      }
-      MLP_CK(cudaStreamEndCapture(m->st, &graph));
-      const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-      if (ie != cudaSuccess) {
-        cudaGraphDestroy(graph);
-        MLP_CK(ie);
-      }
-    }
-    for (; left > 0 && le == cudaSuccess; --left) le = cudaGraphLaunch(exec, m->st);
+    at += steps[k];
+    ends.push_back(at);
+    rates.push_back((float)lrs[k]);
   }
-  if (exec) cudaGraphExecDestroy(exec);
-  if (graph) cudaGraphDestroy(graph);
-  MLP_CK(le);
+  m->ends.alloc(ends.size());
+  m->lrs.alloc(rates.size());
+  MLP_CK(cudaMemcpyAsync(m->ends.p, ends.data(), ends.size() * sizeof(uint32_t),
+                         cudaMemcpyHostToDevice, m->st));
+  MLP_CK(cudaMemcpyAsync(m->lrs.p, rates.data(), rates.size() * sizeof(float),
+                         cudaMemcpyHostToDevice, m->st));
+  m->sched = Schedule{m->ends.p, m->lrs.p, (int)ends.size()};
+  auto gather = [&](cudaStream_t st, int xb, uint32_t ahead) {
+    mlp_gather<<<m->B / kGatherRows, 32 * kGatherRows, 0, st>>>(
+        dth, dll, n_pairs, m->d, m->dp, m->B, 1, m->seed, m->ctr.p, ahead, m->xmean.p,
+        m->xinv.p, m->xw_or_null(), m->ymean, m->yinv, m->Xh[xb].p, m->XTh[xb].p, m->t[xb].p);
+    MLP_CK(cudaGetLastError());
+  };
+  // One step on the batch in buffer xb; the next step's batch is gathered into
+  // the other one meanwhile, on the second stream before dW2, so the reduction
+  // that advances the step counter waits for it.
+  auto one_step = [&](int xb) {
+    MLP_CK(cudaEventRecord(m->ev_fork, m->st));
+    MLP_CK(cudaStreamWaitEvent(m->st2, m->ev_fork, 0));
+    gather(m->st2, xb ^ 1, 1);
+    m->forward(m->B, m->B, m->t[xb].p, 0, xb, true);
+    m->backward_and_update(1, m->losses.p, base, (uint32_t)total, xb);
+  };
+  gather(m->st, 0, 0);
+  uint64_t done = 0;
+  int xb = 0;
+  auto eager = [&](uint64_t n) {
+    for (; n > 0; --n, ++done, xb ^= 1) one_step(xb);
+  };
+  // The first step sets every kernel attribute outside capture; the others
+  // before the capture keep the GPU busy while the graph is built (1.1 ms for
+  // eight steps, half of it for four, which replay as fast).
+  constexpr uint64_t kGraphSteps = 4;  // even: a replay begins on the buffer it ends on
+  constexpr uint64_t kFirst = 12;
+  eager(std::min<uint64_t>(total, kFirst));
+  if (total - done >= 2 * kGraphSteps) {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    MLP_CK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
+    try {
+      for (uint64_t k = 0; k < kGraphSteps; ++k) one_step(xb ^ (int)(k & 1));
+    } catch (...) {
+      cudaGraph_t g2 = nullptr;
+      cudaStreamEndCapture(m->st, &g2);
+      if (g2) cudaGraphDestroy(g2);
+      throw;
+    }
+    MLP_CK(cudaStreamEndCapture(m->st, &graph));
+    cudaError_t le = cudaGraphInstantiate(&exec, graph, 0);
+    for (; le == cudaSuccess && total - done >= kGraphSteps; done += kGraphSteps)
+      le = cudaGraphLaunch(exec, m->st);
+    if (exec) cudaGraphExecDestroy(exec);
+    cudaGraphDestroy(graph);
+    MLP_CK(le);
+  }
+  eager(total - done);
   m->steps_done += (uint32_t)total;
   std::vector<float> losses(total);
   MLP_CK(cudaMemcpyAsync(losses.data(), m->losses.p, total * sizeof(float),
@@ -1214,11 +1291,11 @@ int gpum_b200_mlp_gradients(gpum_b200_mlp* m, const double* theta, const double*
     Buf<float> loss1;
     loss1.alloc(1);
     mlp_gather<<<m->B / kGatherRows, 32 * kGatherRows, 0, m->st>>>(
-        dth.p, dll.p, n, m->d, m->dp, m->B, 0, 0, m->ctr.p,
+        dth.p, dll.p, n, m->d, m->dp, m->B, 0, 0, m->ctr.p, 0,
                                         m->xmean.p, m->xinv.p, m->xw_or_null(), m->ymean,
-                                        m->yinv, m->Xh.p, m->XTh.p, m->t.p);
+                                        m->yinv, m->Xh[0].p, m->XTh[0].p, m->t[0].p);
     MLP_CK(cudaGetLastError());
-    m->forward(m->B, (int)n, m->t.p);
+    m->forward(m->B, (int)n, m->t[0].p);
     // loss slot: the device step counter is not advanced without `apply`
     uint32_t step = 0;
     MLP_CK(cudaMemcpyAsync(&step, m->ctr.p, sizeof step, cudaMemcpyDeviceToHost, m->st));

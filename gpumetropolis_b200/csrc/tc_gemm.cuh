@@ -3,18 +3,24 @@
 //
 //   C[M x N] (f32) = A[M x K] (bf16, row-major) . B[N x K]^T (bf16, row-major)
 //
-// One CTA (256 threads) owns a 128 x BN output tile (BN in {64, 128, 256,
-// 512}; 512 is two N = 256 MMAs side by side in tensor memory).  Per 64-wide
-// K step the CTA copies its A and B slices into shared memory in the
-// canonical K-major, no-swizzle core-matrix layout (8 rows x 16 bytes per
-// core matrix), one elected thread issues the tcgen05.mma (M=128, N<=256,
-// K=16) into TMEM accumulators and commits them to an mbarrier, and the CTA
-// waits (bounded) before reusing shared memory; the next slice's global loads
-// are in flight meanwhile.  The epilogue reads TMEM with tcgen05.ld: warp w
-// owns lanes 32 (w % 4) .. 32 (w % 4) + 31 (rows) and column half w / 4, and
-// applies one of the fused epilogues of the surrogate's training step
-// (GemmEpi).  M, N and K must be multiples of
-// 128, BN and 64 (callers pad with zeros).
+// One CTA (256 threads, 512 for the head's epilogue) owns a 128 x BN output
+// tile (BN in {32, 64, 128, 256, 512}; 512 is two N = 256 MMAs side by side in
+// tensor memory).  K goes through shared memory in stages of up to two 64-wide
+// slices, each in the canonical K-major, no-swizzle core-matrix layout (8 rows
+// x 16 bytes per core matrix), two stages deep: cp.async fills a stage while
+// one elected thread's tcgen05.mma (M=128, N<=256, K=16) work on the other
+// into TMEM accumulators, committed to an mbarrier per stage (bounded waits).
+// The epilogue reads TMEM with tcgen05.ld: warp w owns lanes 32 (w % 4) .. 32
+// (w % 4) + 31 (rows) and column part w / 4, and applies one of the fused
+// epilogues of the surrogate's training step (GemmEpi).  M, N and K must be
+// multiples of 128, BN and 64 (callers pad with zeros).
+// The kernels of a step are bound by their latency, not by a rate (at batch
+// 4096 and H = 128 one has 0.07 to 0.13 GFLOP), so a tile is as narrow as
+// fills the GPU, the K of most of them is one stage with one wait, and the
+// set-up runs before the wait for the kernel before (programmatic dependent
+// launch).  A training step (d = 17, H = 128, batch 4096): 62 us with 32-CTA
+// tiles, one slice per stage through registers and the gather in the chain, 39
+// now.
 // Split K (EPI_STORE only): with gridDim.z = S > 1, CTA z reduces K columns
 // [z*kz, z*kz + kz) into its own partial C + z*M*N; the consumer adds the S
 // partials in order, which keeps the result deterministic.
@@ -26,8 +32,7 @@
 namespace gpum {
 
 constexpr int kGemmBM = 128;
-constexpr int kGemmBK = 64;
-constexpr int kGemmThreads = 256;
+constexpr int kGemmBK = 64;  // one slice of K
 
 enum DevErrGemm : uint32_t { DEV_ERR_MMA_TIMEOUT = 1u << 1 };
 
@@ -107,7 +112,7 @@ __device__ __forceinline__ float warp_sum(float x) {
 }
 
 // Fused epilogues of the surrogate's training step (one thread = one row and
-// one half of the tile's columns):
+// one part of the tile's columns):
 //   EPI_STORE  C = acc (+ bias), f32; with gridDim.z > 1 a split-K partial
 //   EPI_SILU   Z = acc + bias -> C (f32); A = silu(Z) -> act (bf16, row-major)
 //              and actT (bf16, transposed [N][M])
@@ -123,6 +128,12 @@ __device__ __forceinline__ float warp_sum(float x) {
 //              and act (bf16 row-major, optional); per CTA the column sums
 //              of dZ1 (b1's gradient) -> colpart[gridDim.y][N] (optional)
 enum GemmEpi : int { EPI_STORE = 0, EPI_SILU = 1, EPI_HEAD = 2, EPI_DSILU = 3 };
+
+// Slices per stage and threads of an instantiation.
+template <int BN>
+constexpr int kGemmSlices = BN == 512 ? 1 : 2;
+template <int EPI>
+constexpr int kGemmThreads = EPI == EPI_HEAD ? 512 : 256;
 
 struct GemmArgs {
   const __nv_bfloat16* A;
@@ -147,10 +158,22 @@ struct GemmArgs {
 
 template <int BN>
 constexpr size_t tc_gemm_smem() {
-  // A slice | B slice | column-sum scratch [2][4 lane quarters][BN] | row
-  // partials [2 halves][128] | bias, w3 [2][BN] | barrier, slot
-  return (size_t)kGemmBM * kGemmBK * 2 + (size_t)BN * kGemmBK * 2 + (size_t)2 * 4 * BN * 4 +
-         2 * 128 * 4 + (size_t)2 * BN * 4 + 16 + 16 + 1024;
+  // two stages of A and B slices | column-sum scratch [2][4 lane quarters][BN]
+  // | row partials [2 halves][128] | bias, w3 [2][BN] | barriers, slot
+  return (size_t)2 * kGemmSlices<BN> * (kGemmBM + BN) * kGemmBK * 2 + (size_t)2 * 4 * BN * 4 +
+         2 * 128 * 4 + (size_t)2 * BN * 4 + 32 + 1024;
+}
+
+// 16 bytes from global to shared memory, asynchronously (cp.async).
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // Stores 16 bf16 values of one row (32 bytes).
@@ -168,20 +191,22 @@ __device__ __forceinline__ void store_bf16x16(__nv_bfloat16* dst, const float (&
 }
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(kGemmThreads, 1) tc_gemm_kernel(const GemmArgs g) {
-  static_assert(BN == 64 || BN == 128 || BN == 256 || BN == 512, "BN");
+__global__ void __launch_bounds__(kGemmThreads<EPI>, 1) tc_gemm_kernel(const GemmArgs g) {
+  static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256 || BN == 512, "BN");
+  constexpr int kThr = kGemmThreads<EPI>;
   constexpr int kMmaN = BN < 256 ? BN : 256;          // N of one MMA
   constexpr int kNMma = BN / kMmaN;                   // MMAs side by side
   constexpr uint32_t kTmemCols = BN <= 32 ? 32 : (uint32_t)BN;
+  constexpr int kSl = kGemmSlices<BN>;
+  constexpr uint32_t kABytes = kGemmBM * kGemmBK * 2, kBBytes = BN * kGemmBK * 2;  // a slice
+  constexpr uint32_t kStage = kSl * (kABytes + kBBytes);
   extern __shared__ __align__(1024) unsigned char gsm[];
-  unsigned char* sa = gsm;                                  // 128 x 64 bf16 = 16 KB
-  unsigned char* sb = gsm + kGemmBM * kGemmBK * 2;          // BN x 64 bf16
-  float* red = reinterpret_cast<float*>(sb + BN * kGemmBK * 2);  // [2][4][BN]
-  float* ypart = red + 2 * 4 * BN;                                // [2][128]
-  float* s_bias = ypart + 2 * 128;                                 // [BN]
-  float* s_w3 = s_bias + BN;                                       // [BN]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(s_w3 + BN);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
+  float* red = reinterpret_cast<float*>(gsm + 2 * kStage);  // [2][4][BN]
+  float* ypart = red + 2 * 4 * BN;                          // [2][128]
+  float* s_bias = ypart + 2 * 128;                          // [BN]
+  float* s_w3 = s_bias + BN;                                // [BN]
+  uint64_t* bar = reinterpret_cast<uint64_t*>(s_w3 + BN);   // [2] stages, [1] drain
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 3);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int M = g.M, N = g.N, K = g.K;
   const int m0 = blockIdx.y * kGemmBM, n0 = blockIdx.x * BN;
@@ -191,100 +216,105 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tc_gemm_kernel(const GemmArgs
 
   if (warp == 0) tmem_alloc(tslot, kTmemCols);
   if (tid == 0) {
-    mbar_init(bar, 1);
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_init(&bar[2], 1);
     mbar_fence_init();
   }
-  // the epilogue's per-column operands, read by every row: staged once
-  for (int i = tid; i < BN; i += kGemmThreads) {
-    s_bias[i] = g.bias ? g.bias[n0 + i] : 0.0f;
-    s_w3[i] = g.w3 ? g.w3[n0 + i] : 0.0f;
-  }
+  // The next kernel of the step allocates tensor memory too and may start once
+  // every CTA has triggered: only after this CTA has its own, or the two could
+  // wait for each other.
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tslot;
-  constexpr uint32_t idesc = umma_idesc_bf16(kGemmBM, kMmaN);
-  const uint32_t sa_addr = smem_addr(sa), sb_addr = smem_addr(sb);
-  const uint32_t lbo_a = (kGemmBM / 8) * 128, lbo_b = (BN / 8) * 128;
-  bool ok = true;
-  uint32_t fail_parity = 0;  // phase of the commit a wait gave up on
+  pdl_wait();
+  pdl_trigger();
 
-  // Staging: each thread owns kLA + kLB 16-byte chunks of a K slice.  All
-  // global loads of a slice are issued back to back into registers, and the
-  // next slice is loaded while the tensor core works on the current one.
   constexpr int kChunks = kGemmBK / 8;  // 16-byte chunks per row of a slice
-  constexpr int kLA = kGemmBM * kChunks / kGemmThreads;
-  constexpr int kLB = BN * kChunks / kGemmThreads;
-  static_assert(kGemmBM * kChunks % kGemmThreads == 0 && BN * kChunks % kGemmThreads == 0, "");
-  uint4 ra[kLA], rb[kLB];
-  auto load_slice = [&](int k0) {
+  const uint32_t base = smem_addr(gsm);
+  const int nsl = (kend - kbeg) / kGemmBK, nst = (nsl + kSl - 1) / kSl;
+  auto load_stage = [&](int st) {
+    const uint32_t sa = base + (uint32_t)(st & 1) * kStage, sb = sa + kSl * kABytes;
 #pragma unroll
-    for (int q = 0; q < kLA; ++q) {
-      const int i = tid + q * kGemmThreads, r = i / kChunks, c8 = (i % kChunks) * 8;
-      ra[q] = *reinterpret_cast<const uint4*>(A + (size_t)(m0 + r) * K + k0 + c8);
+    for (int q = 0; q < kSl; ++q) {
+      const int sl = st * kSl + q;
+      if (sl >= nsl) break;
+      const int k0 = kbeg + sl * kGemmBK;
+      for (int i = tid; i < kGemmBM * kChunks; i += kThr) {
+        const int r = i / kChunks, c8 = (i % kChunks) * 8;
+        cp_async16(sa + q * kABytes + kmajor_offset(r, c8, kGemmBM),
+                   A + (size_t)(m0 + r) * K + k0 + c8);
+      }
+      for (int i = tid; i < BN * kChunks; i += kThr) {
+        const int r = i / kChunks, c8 = (i % kChunks) * 8;
+        cp_async16(sb + q * kBBytes + kmajor_offset(r, c8, BN),
+                   B + (size_t)(n0 + r) * K + k0 + c8);
+      }
     }
-#pragma unroll
-    for (int q = 0; q < kLB; ++q) {
-      const int i = tid + q * kGemmThreads, r = i / kChunks, c8 = (i % kChunks) * 8;
-      rb[q] = *reinterpret_cast<const uint4*>(B + (size_t)(n0 + r) * K + k0 + c8);
-    }
+    cp_async_commit();
   };
-  auto store_slice = [&]() {
-#pragma unroll
-    for (int q = 0; q < kLA; ++q) {
-      const int i = tid + q * kGemmThreads, r = i / kChunks, c8 = (i % kChunks) * 8;
-      *reinterpret_cast<uint4*>(sa + kmajor_offset(r, c8, kGemmBM)) = ra[q];
-    }
-#pragma unroll
-    for (int q = 0; q < kLB; ++q) {
-      const int i = tid + q * kGemmThreads, r = i / kChunks, c8 = (i % kChunks) * 8;
-      *reinterpret_cast<uint4*>(sb + kmajor_offset(r, c8, BN)) = rb[q];
-    }
-  };
-  if (kbeg < kend) load_slice(kbeg);
-
-  for (int k0 = kbeg, it = 0; k0 < kend; k0 += kGemmBK, ++it) {
-    store_slice();
-    // Generic-proxy smem writes must be visible to the tensor core's async proxy.
+  if (nst > 0) load_stage(0);
+  if (nst > 1) load_stage(1);
+  // the epilogue's per-column operands, read by every row: staged once
+  for (int i = tid; i < BN; i += kThr) {
+    s_bias[i] = g.bias ? g.bias[n0 + i] : 0.0f;
+    s_w3[i] = g.w3 ? g.w3[n0 + i] : 0.0f;
+  }
+  constexpr uint32_t idesc = umma_idesc_bf16(kGemmBM, kMmaN);
+  constexpr uint32_t lbo_a = (kGemmBM / 8) * 128, lbo_b = (BN / 8) * 128;
+  bool ok = true;
+  for (int it = 0; it < nst; ++it) {
+    if (it + 1 < nst) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    // Shared-memory writes must be visible to the tensor core's async proxy.
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t sa = base + (uint32_t)(it & 1) * kStage, sb = sa + kSl * kABytes;
 #pragma unroll
-      for (int kk = 0; kk < kGemmBK / 16; ++kk) {
-        const uint64_t ad = umma_smem_desc(sa_addr + 2 * kk * lbo_a, lbo_a, 128);
+      for (int q = 0; q < kSl; ++q) {
+        if (it * kSl + q >= nsl) break;
 #pragma unroll
-        for (int h = 0; h < kNMma; ++h) {
-          // rows [h * 256, h * 256 + 256) of the B slice: 32 row groups further
-          const uint64_t bd =
-              umma_smem_desc(sb_addr + 2 * kk * lbo_b + h * (kMmaN / 8) * 128, lbo_b, 128);
-          umma_bf16(tmem + (uint32_t)(h * kMmaN), ad, bd, idesc,
-                    (k0 > kbeg || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < kGemmBK / 16; ++kk) {
+          const uint64_t ad = umma_smem_desc(sa + q * kABytes + 2 * kk * lbo_a, lbo_a, 128);
+#pragma unroll
+          for (int h = 0; h < kNMma; ++h) {
+            // rows [h * 256, h * 256 + 256) of the B slice: 32 row groups further
+            const uint64_t bd = umma_smem_desc(
+                sb + q * kBBytes + 2 * kk * lbo_b + h * (kMmaN / 8) * 128, lbo_b, 128);
+            umma_bf16(tmem + (uint32_t)(h * kMmaN), ad, bd, idesc,
+                      (it > 0 || q > 0 || kk > 0) ? 1u : 0u);
+          }
         }
       }
-      umma_commit(bar);
+      umma_commit(&bar[it & 1]);
     }
-    if (k0 + kGemmBK < kend) load_slice(k0 + kGemmBK);  // overlaps the MMAs
     __syncwarp();
-    fail_parity = (uint32_t)(it & 1);
-    if (!mbar_wait_bounded(bar, fail_parity)) {
-      ok = false;
-      if (lane == 0) atomicOr(g.err, DEV_ERR_MMA_TIMEOUT);
+    // The stage is free, or the last product done.  A wait that gives up in
+    // any thread ends the K loop and skips the epilogue in every thread.
+    if (it + 2 < nst || it + 1 == nst) {
+      if (!mbar_wait_bounded(&bar[it & 1], (uint32_t)((it >> 1) & 1))) {
+        ok = false;
+        if (lane == 0) atomicOr(g.err, DEV_ERR_MMA_TIMEOUT);
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      ok = __syncthreads_and(ok) != 0;
+      if (!ok) break;
+      if (it + 2 < nst) load_stage(it + 2);
     }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // block-uniform: a wait that gave up in any thread ends the K loop and
-    // skips the epilogue in every thread
-    ok = __syncthreads_and(ok) != 0;
-    if (!ok) break;
   }
+  if (!ok) cp_async_wait<0>();  // no copy is left when the block ends
 
   // Epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows) and the
-  // columns [cb, ce) of its half of the tile, 16 at a time.
-  const int quarter = warp & 3, half = warp >> 2;
+  // columns [cb, ce) of its part of the tile, 16 at a time.
+  const int quarter = warp & 3, part = warp >> 2;
   const int row = m0 + quarter * 32 + lane;
   const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-  constexpr int kHalf = BN / 2;
-  const int cb = half * kHalf, ce = cb + kHalf;
+  constexpr int kCols = BN / (kThr / 128);
+  const int cb = part * kCols, ce = cb + kCols;
   if (ok) {
     if constexpr (EPI == EPI_STORE || EPI == EPI_SILU) {
       float* C = g.C + (size_t)blockIdx.z * M * N;
@@ -313,19 +343,41 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tc_gemm_kernel(const GemmArgs
         }
       }
     } else if constexpr (EPI == EPI_HEAD) {
-      // pass 1: the prediction of this row, its two column halves added in order
-      float yp = 0.0f;
-#pragma unroll 1
-      for (int c = cb; c < ce; c += 16) {
-        float v[16];
-        tmem_ld16(trow + (uint32_t)c, v);
+      // pass 1: the prediction of this row: two column halves, each a chain of
+      // products in column order over two parts (the odd part goes on from the
+      // even one's sum), added in order
+      {
+        // up to 64 activations in registers while the even parts' sums form
+        // (128 at H = 512 would spill: there the odd parts start afterwards)
+        constexpr int kKeep = kCols <= 64 ? kCols : 16;
+        float sv[kKeep];
+        auto act = [&](int c) {  // columns cb + c .. + 15 into sv[c % kKeep ..]
+          float v[16];
+          tmem_ld16(trow + (uint32_t)(cb + c), v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) yp = fmaf(silu(v[j] + s_bias[c + j]), s_w3[c + j], yp);
+          for (int j = 0; j < 16; ++j) sv[c % kKeep + j] = silu(v[j] + s_bias[cb + c + j]);
+        };
+        float* mine = &ypart[(part >> 1) * 128 + quarter * 32 + lane];
+        if constexpr (kKeep == kCols) {
+#pragma unroll
+          for (int c = 0; c < kCols; c += 16) act(c);
+        }
+        auto chain = [&](float yp) {
+#pragma unroll
+          for (int c = 0; c < kCols; c += 16) {
+            if constexpr (kKeep != kCols) act(c);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) yp = fmaf(sv[c % kKeep + j], s_w3[cb + c + j], yp);
+          }
+          *mine = yp;
+        };
+        if (!(part & 1)) chain(0.0f);
+        __syncthreads();
+        if (part & 1) chain(*mine);
       }
-      ypart[half * 128 + quarter * 32 + lane] = yp;
       __syncthreads();
       const float y = (ypart[quarter * 32 + lane] + ypart[128 + quarter * 32 + lane]) + g.b3[0];
-      if (g.yhat && half == 0) g.yhat[row] = y;
+      if (g.yhat && part == 0) g.yhat[row] = y;
       const bool live = row < g.n_live;
       const float r = (live && g.t) ? y - g.t[row] : 0.0f;
       const float dy = g.unit_dy ? 1.0f : 2.0f * r / (float)g.n_live;
@@ -359,7 +411,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tc_gemm_kernel(const GemmArgs
       const float sdy = warp_sum(dy), sr2 = warp_sum(r * r);
       __syncthreads();
       if (g.colpart) {
-        for (int i = tid; i < 2 * BN; i += kGemmThreads) {
+        for (int i = tid; i < 2 * BN; i += kThr) {
           const int q = i / BN, n = i % BN;
           const float* rq = red + (size_t)q * 4 * BN;
           g.colpart[((size_t)q * gridDim.y + blockIdx.y) * N + n] =
@@ -367,7 +419,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tc_gemm_kernel(const GemmArgs
         }
       }
       if (g.rowpart) {
-        if (half == 0 && lane == 0) {
+        if (part == 0 && lane == 0) {
           ypart[quarter] = sdy;
           ypart[4 + quarter] = sr2;
         }
@@ -404,28 +456,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tc_gemm_kernel(const GemmArgs
       }
       if (g.colpart) {
         __syncthreads();
-        for (int n = tid; n < BN; n += kGemmThreads)
+        for (int n = tid; n < BN; n += kThr)
           g.colpart[(size_t)blockIdx.y * N + n0 + n] =
               ((red[n] + red[BN + n]) + red[2 * BN + n]) + red[3 * BN + n];
       }
     }
   }
   // After a wait that gave up, give the MMAs in flight one more bounded wait
-  // before the tensor memory is released.
-  if (!ok && tid == 0) mbar_wait_bounded(bar, fail_parity);
+  // (a commit of their own) before the tensor memory is released.
+  if (!ok && tid == 0) {
+    umma_commit(&bar[2]);
+    mbar_wait_bounded(&bar[2], 0u);
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
-}
-
-// out[i] = sum_z part[z*n + i], z in order.
-static __global__ void tc_splitk_sum(const float* __restrict__ part, int S, size_t n,
-                                     float* __restrict__ out) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float t = 0.0f;
-  for (int z = 0; z < S; ++z) t += part[(size_t)z * n + i];
-  out[i] = t;
 }
 
 }  // namespace gpum
