@@ -609,6 +609,7 @@ struct gpum_b200_session {
     E.n_obs = (int)n_obs;
     E.ncols = (int)(ext(kc) ? ncols_c : ncols);
     E.T = kc.tc ? cm.tc_tn : (ext(kc) ? T_c : T);
+    E.U = stage_tiles(E.T, E.ncols);
     E.ntiles = geo.ntiles;
     E.tiles_per_cta = geo.tiles_per_cta;
     E.CG = geo.CG;

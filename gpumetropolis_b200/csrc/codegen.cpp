@@ -418,7 +418,8 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
     const std::string lw =
         w.op == O_C ? (paired ? "gm2(" + flit(std::log(w.c)) + ")" : flit(std::log(w.c)))
                     : hname + "[" + std::to_string(lslot[e.weight]) + "]";
-    if (paired) return std::string(e.sign > 0 ? "gm2_add(" : "gm2_sub(") + a + ", " + lw + ")";
+    if (paired)
+      return "gm2_add(" + a + ", " + (e.sign > 0 ? lw : "gm2_neg(" + lw + ")") + ")";
     return "(" + a + (e.sign > 0 ? " + " : " - ") + lw + ")";
   };
 
@@ -714,11 +715,51 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
       nsp_fold[i] = 1;
       nsp_skip[a] = nsp_skip[b] = 1;
     }
+    // Exact folds of the paired code (an FFMA2, FMUL2 or FADD2 takes two issue
+    // slots each; an operand that does not depend on the observation is
+    // computed outside the loop):
+    //   -a * r            = a * -r (r a hoisted reciprocal; neg_fold)
+    //   a - p             = a + -p (p a parameter, hoisted value or constant;
+    //                       a not a product, which the compiler would contract
+    //                       with the sum into one rounding)
+    //   c + a / 2^k       = fma(a, 2^-k, c) for a constant |c| >= 2^-60: the
+    //                       scaled a is exact unless it is below 2^-126, where
+    //                       the sum is c either way (pow2_fold)
+    auto invariant = [&](int i) { return i >= 0 && (g.n[i].dep & DEP_D) == 0; };
+    auto product = [&](int i) {
+      const uint32_t op = g.n[i].op;
+      return op == O_MUL || op == O_DIV || op == O_POW || op == O_NEG;
+    };
+    std::vector<char> neg_fold(N, 0), fold_skip(N, 0);
+    std::vector<int> pow2_fold(N, -1);
+    for (int i = 0; i < N; ++i) {
+      if (!live[i] || !is_pd(i) || fused[i] || nsp_fold[i] || lse[i] || softplus_arg[i] >= 0)
+        continue;
+      const Node& x = g.n[i];
+      if (recip(i) >= 0) {
+        if (is_pd(x.a) && g.n[x.a].op == O_NEG && uses[x.a] == 1 && x.a != root) {
+          neg_fold[i] = 1;
+          fold_skip[x.a] = 1;
+        }
+      } else if (x.op == O_ADD) {
+        for (int m : {x.a, x.b}) {
+          const int o = m == x.a ? x.b : x.a;
+          if (!is_pd(m) || fused[m] || g.n[m].op != O_DIV || recip(m) >= 0 || uses[m] != 1 ||
+              m == root || g.n[o].op != O_C || !(std::fabs(g.n[o].c) >= 0x1p-60) ||
+              !std::isfinite((float)g.n[o].c) || pow2_recip(g, g.n[m].b).empty() ||
+              !(std::fabs(g.n[g.n[m].b].c) > 1.0))
+            continue;
+          pow2_fold[i] = m;
+          fold_skip[m] = 1;
+          break;
+        }
+      }
+    }
     // The paired value of node i with the references R (rewrites included);
     // value_node(i): whether the paired value function evaluates node i.
     auto value_node = [&](int i) {
       return live[i] && is_pd(i) && !fused[i] && !softplus_inner[i] && !nsp_skip[i] &&
-             !lse_skip[i];
+             !lse_skip[i] && !fold_skip[i];
     };
     auto value2_expr = [&](int i, const std::function<std::string(int)>& R) -> std::string {
       const Node& x = g.n[i];
@@ -730,7 +771,15 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
         return "gm2_fma_nsoftplus(" + R(m.a) + ", " + R(m.b) + ", " + R(softplus_arg[x.b]) + ")";
       }
       if (softplus_arg[i] >= 0) return "gm2_softplus(" + R(softplus_arg[i]) + ")";
+      if (neg_fold[i])
+        return "gm2_mul(" + R(g.n[x.a].a) + ", gm2_neg(hh[" + std::to_string(recip(i)) + "]))";
       if (recip(i) >= 0) return "gm2_mul(" + R(x.a) + ", hh[" + std::to_string(recip(i)) + "])";
+      if (pow2_fold[i] >= 0) {
+        const int m = pow2_fold[i], o = m == x.a ? x.b : x.a;
+        return "gm2_fma(" + R(g.n[m].a) + ", gm2(" + pow2_recip(g, g.n[m].b) + "), " + R(o) + ")";
+      }
+      if (x.op == O_SUB && invariant(x.b) && !invariant(x.a) && !product(x.a))
+        return "gm2_add(" + R(x.a) + ", gm2_neg(" + R(x.b) + "))";
       if (x.op == O_ADD && (fused[x.a] || (x.b >= 0 && fused[x.b]))) {
         const int m = fused[x.a] ? x.a : x.b, o = fused[x.a] ? x.b : x.a;
         return "gm2_fma(" + R(g.n[m].a) + ", " + R(g.n[m].b) + ", " + R(o) + ")";

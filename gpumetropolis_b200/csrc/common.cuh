@@ -89,6 +89,7 @@ struct ChainArgs {
 
 struct EvalArgs {
   int n_obs, ncols, T, ntiles, tiles_per_cta, CG, WC, C_pad, np;
+  int U;                // tiles per stage (stage_tiles)
   int width;            // values per (chain, obs block): 1, or 1 + np with the gradient
   const float* params;  // [np][C_pad] evaluation points (f32)
   double* partials;     // [NOB][C_pad][width]
@@ -295,8 +296,18 @@ __device__ __forceinline__ void prior_block(const EvalArgs& E, const ChainArgs& 
 }
 
 // --------------------------------------------------------- kernel skeleton
+// Tiles per stage: a narrow model's tile is a KB or two (a TMA box is at most
+// 256 observations), so a stage holds as many as 16 KB do and the CTA's barrier
+// and wait come once for all of them.  With the folds of the generated code
+// (codegen.cpp) 40 steps of 2,048 chains x 2^18 observations of the one-column
+// mixture went from 24.5 to 20.9 ms.
+__host__ __device__ inline int stage_tiles(int T, int ncols) {
+  const int bytes = T * ncols * 4;
+  const int u = bytes > 0 ? (16 << 10) / bytes : 1;
+  return u < 1 ? 1 : (u > 8 ? 8 : u);
+}
 // Shared-memory carve-up (the host's smem_bytes() must agree):
-//   2 data stages [ncols][T] f32 | params [np][CG] f32 (rounded to 4; none
+//   2 data stages [U][ncols][T] f32 | params [np][CG] f32 (rounded to 4; none
 //   for chain-lane bodies, whose lanes read their parameters from global
 //   memory) | reduction [kWarps][G][width] f64 | 2 mbarriers.
 __host__ __device__ inline size_t skel_param_floats(int np, int CG, bool lanes) {
@@ -304,7 +315,7 @@ __host__ __device__ inline size_t skel_param_floats(int np, int CG, bool lanes) 
 }
 __host__ __device__ inline size_t skel_smem_bytes(int T, int ncols, int np, int CG, int G,
                                                   int width, bool lanes = false) {
-  return 2 * (size_t)T * ncols * 4 + skel_param_floats(np, CG, lanes) * 4 +
+  return 2 * (size_t)stage_tiles(T, ncols) * T * ncols * 4 + skel_param_floats(np, CG, lanes) * 4 +
          (size_t)kWarps * G * width * 8 + 2 * 8;
 }
 
@@ -359,7 +370,8 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   const int WO = kWarps / E.WC;
   const int wc = warp % E.WC, wo = warp / E.WC;
 
-  const size_t stage_floats = (size_t)T * ncols;
+  const size_t tile_floats = (size_t)T * ncols, stage_floats = E.U * tile_floats;
+  const int U = E.U;
   float* xs = reinterpret_cast<float*>(smem_raw);
   constexpr bool kLanes = Body::kChainLanes;
   float* psm = xs + 2 * stage_floats;
@@ -369,7 +381,15 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   const int t0 = ob * tiles_per_cta;
   const int t1 = min(t0 + tiles_per_cta, E.ntiles);
   const int nt = max(t1 - t0, 0);
-  const uint32_t tile_bytes = (uint32_t)(stage_floats * sizeof(float));
+  const int nst = (nt + U - 1) / U;  // stages
+  // Stage s of this CTA: tiles t0 + s U .. into buffer s % 2.
+  auto load_stage = [&](int s) {
+    const int n = min(U, nt - s * U);
+    float* dst = xs + (s & 1) * stage_floats;
+    mbar_expect_tx(&bars[s & 1], (uint32_t)(n * tile_floats * sizeof(float)));
+    for (int u = 0; u < n; ++u)
+      tma_load_2d(dst + u * tile_floats, tmap, &bars[s & 1], (t0 + s * U + u) * T, 0);
+  };
   // No tiles (or no data columns): the tensor map is never touched.
   const bool staged = ncols > 0 && nt > 0;
   if (tid == 0 && staged) {
@@ -379,10 +399,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     mbar_fence_init();
     // The data does not change during a run: the first tiles are on their way
     // before the previous step's proposals are waited for.
-    for (int s = 0; s < 2 && s < nt; ++s) {
-      mbar_expect_tx(&bars[s], tile_bytes);
-      tma_load_2d(xs + s * stage_floats, tmap, &bars[s], (t0 + s) * T, 0);
-    }
+    for (int s = 0; s < 2 && s < nst; ++s) load_stage(s);
   }
   pdl_wait();
   pdl_trigger();
@@ -403,82 +420,85 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     body.begin(psm + wc * G, CG);
   }
 
-  for (int k = 0; k < nt; ++k) {
+  for (int k = 0; k < nst; ++k) {
     const int st = k & 1;
-    const float* tile = xs + st * stage_floats;
     int gave_up = 0;
     if (staged && !mbar_wait_bounded(&bars[st], (uint32_t)((k >> 1) & 1))) {
       gave_up = 1;
       if (lane == 0) atomicOr(E.err, DEV_ERR_TMA_TIMEOUT);
     }
-    const int obs0 = (t0 + k) * T;
-    if constexpr (kLanes) {
-      // quads of observations (o .. o + 3), the WO warps of a chain group
-      // taking every WO-th quad; all lanes read the same addresses
-      for (int o = 4 * wo; o < T; o += 4 * WO) {
-        const long long left = (long long)E.n_obs - (obs0 + o);
-        if (left <= 0) break;
-        const int nv = left >= 4 ? 4 : (int)left;
-        body.eval4(tile + o, nv);
-        if (phase == PH_POINTWISE) {
-          const int c = cb * CG + wc * 32 + lane;
-          if (c < E.n_points) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)  // constant indices keep the values in registers
-              if (q < nv) E.pointwise[(size_t)c * E.n_obs + obs0 + o + q] = body.last4(q);
-          }
-        }
-      }
-      if constexpr (Body::kLanesAcc) body.flush_tile();
-    } else if constexpr (Body::kObsPerEval == 2) {
-      // observation pairs (2 pi, 2 pi + 1); T is even, so each pair is
-      // 8-byte aligned in every column of the tile
-      auto pair = [&](int pi) {
-        const int obs = obs0 + 2 * pi;
-        const bool v0 = obs < E.n_obs, v1 = obs + 1 < E.n_obs;
-        body.eval2(tile + 2 * pi, T, v0, v1);
-        if (phase == PH_POINTWISE && v0) {
-#pragma unroll
-          for (int g = 0; g < G; ++g) {
-            const int c = cb * CG + wc * G + g;
+    const int nu = min(U, nt - k * U);
+    for (int u = 0; u < nu; ++u) {
+      const float* tile = xs + st * stage_floats + u * tile_floats;
+      const int obs0 = (t0 + k * U + u) * T;
+      if constexpr (kLanes) {
+        // quads of observations (o .. o + 3), the WO warps of a chain group
+        // taking every WO-th quad; all lanes read the same addresses
+        for (int o = 4 * wo; o < T; o += 4 * WO) {
+          const long long left = (long long)E.n_obs - (obs0 + o);
+          if (left <= 0) break;
+          const int nv = left >= 4 ? 4 : (int)left;
+          body.eval4(tile + o, nv);
+          if (phase == PH_POINTWISE) {
+            const int c = cb * CG + wc * 32 + lane;
             if (c < E.n_points) {
-              const float2 lv = body.last2(g);
-              E.pointwise[(size_t)c * E.n_obs + obs] = lv.x;
-              if (v1) E.pointwise[(size_t)c * E.n_obs + obs + 1] = lv.y;
+  #pragma unroll
+              for (int q = 0; q < 4; ++q)  // constant indices keep the values in registers
+                if (q < nv) E.pointwise[(size_t)c * E.n_obs + obs0 + o + q] = body.last4(q);
             }
           }
         }
-      };
-      constexpr int kT = Body::kTileObs;  // compile-time tile height, or 0
-      if (kT > 0 && kT % 64 == 0 && WO == 1) {
-        // every warp covers the tile: a fixed trip count, unrolled so the
-        // compiler can overlap one pair's loads with another's arithmetic
-        bool done = false;
-        if constexpr (kT > 0) {
-          if (phase != PH_POINTWISE && obs0 + kT <= E.n_obs) {  // a full tile
-#pragma unroll
-            for (int it = 0; it < kT / 64; ++it) body.eval2_full(tile + 2 * (lane + 32 * it));
-            body.flush();
-            done = true;
+        if constexpr (Body::kLanesAcc) body.flush_tile();
+      } else if constexpr (Body::kObsPerEval == 2) {
+        // observation pairs (2 pi, 2 pi + 1); T is even, so each pair is
+        // 8-byte aligned in every column of the tile
+        auto pair = [&](int pi) {
+          const int obs = obs0 + 2 * pi;
+          const bool v0 = obs < E.n_obs, v1 = obs + 1 < E.n_obs;
+          body.eval2(tile + 2 * pi, T, v0, v1);
+          if (phase == PH_POINTWISE && v0) {
+  #pragma unroll
+            for (int g = 0; g < G; ++g) {
+              const int c = cb * CG + wc * G + g;
+              if (c < E.n_points) {
+                const float2 lv = body.last2(g);
+                E.pointwise[(size_t)c * E.n_obs + obs] = lv.x;
+                if (v1) E.pointwise[(size_t)c * E.n_obs + obs + 1] = lv.y;
+              }
+            }
           }
-        }
-        if (!done) {
-#pragma unroll
-          for (int it = 0; it < (kT > 0 ? kT : 64) / 64; ++it) pair(lane + 32 * it);
+        };
+        constexpr int kT = Body::kTileObs;  // compile-time tile height, or 0
+        if (kT > 0 && kT % 64 == 0 && WO == 1) {
+          // every warp covers the tile: a fixed trip count, unrolled so the
+          // compiler can overlap one pair's loads with another's arithmetic
+          bool done = false;
+          if constexpr (kT > 0) {
+            if (phase != PH_POINTWISE && obs0 + kT <= E.n_obs) {  // a full tile
+  #pragma unroll
+              for (int it = 0; it < kT / 64; ++it) body.eval2_full(tile + 2 * (lane + 32 * it));
+              body.flush();
+              done = true;
+            }
+          }
+          if (!done) {
+  #pragma unroll
+            for (int it = 0; it < (kT > 0 ? kT : 64) / 64; ++it) pair(lane + 32 * it);
+          }
+        } else {
+          for (int pi = lane + 32 * wo; 2 * pi < T; pi += 32 * WO) pair(pi);
         }
       } else {
-        for (int pi = lane + 32 * wo; 2 * pi < T; pi += 32 * WO) pair(pi);
-      }
-    } else {
-      for (int ol = lane + 32 * wo; ol < T; ol += 32 * WO) {
-        const int obs = obs0 + ol;
-        const bool valid = obs < E.n_obs;
-        body.eval(tile + ol, T, valid);
-        if (phase == PH_POINTWISE && valid) {
-#pragma unroll
-          for (int g = 0; g < G; ++g) {
-            const int c = cb * CG + wc * G + g;
-            if (c < E.n_points) E.pointwise[(size_t)c * E.n_obs + obs] = body.last(g);
+        for (int ol = lane + 32 * wo; ol < T; ol += 32 * WO) {
+          const int obs = obs0 + ol;
+          const bool valid = obs < E.n_obs;
+          body.eval(tile + ol, T, valid);
+          if (phase == PH_POINTWISE && valid) {
+  #pragma unroll
+            for (int g = 0; g < G; ++g) {
+              const int c = cb * CG + wc * G + g;
+              if (c < E.n_points) E.pointwise[(size_t)c * E.n_obs + obs] = body.last(g);
+            }
           }
         }
       }
@@ -491,15 +511,12 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     if (__syncthreads_or(gave_up)) {
       if (tid == 0 && staged) {
         mbar_wait_bounded(&bars[st], (uint32_t)((k >> 1) & 1));
-        if (k + 1 < nt) mbar_wait_bounded(&bars[st ^ 1], (uint32_t)(((k + 1) >> 1) & 1));
+        if (k + 1 < nst) mbar_wait_bounded(&bars[st ^ 1], (uint32_t)(((k + 1) >> 1) & 1));
       }
       __syncthreads();
       break;
     }
-    if (tid == 0 && staged && k + 2 < nt) {
-      mbar_expect_tx(&bars[st], tile_bytes);
-      tma_load_2d(xs + st * stage_floats, tmap, &bars[st], (t0 + k + 2) * T, 0);
-    }
+    if (tid == 0 && staged && k + 2 < nst) load_stage(k + 2);
   }
   if (phase == PH_POINTWISE) return;
   body.end();

@@ -412,11 +412,11 @@ __device__ __forceinline__ float gm_softplus(float a) {
 // for LOG(c1 EXP(a) + c2 EXP(b)) with positive parameter-only weights (p = a
 // + log c1, q = b + log c2): no exponential of the terms themselves, so no
 // FP32 underflow to log(0) where the reference's f64 sum is still finite.
-// NaN propagates; both terms -inf gives -inf.
+// NaN propagates (through the max); two terms -inf give -inf + log1p(u), where
+// the NaN of their difference became u = 0 (gm_log1p_nexp's fmaxf returns its
+// other operand), so -inf again without a test.
 __device__ __forceinline__ float gm_logaddexp(float p, float q) {
-  const float m = gm_max_nan(p, q);
-  const float r = m + gm_log1p_nexp(p - q);
-  return m < -3.402823466e38f ? m : r;  // m is -inf
+  return gm_max_nan(p, q) + gm_log1p_nexp(p - q);
 }
 
 // ------------------------------------------------- paired FP32 arithmetic
@@ -473,8 +473,7 @@ __device__ __forceinline__ float2 gm2_softplus(float2 a) {
 // Paired gm_logaddexp.
 __device__ __forceinline__ float2 gm2_logaddexp(float2 p, float2 q) {
   const float2 m = make_float2(gm_max_nan(p.x, q.x), gm_max_nan(p.y, q.y));
-  const float2 r = __fadd2_rn(m, gm2_log1p_nexp(__ffma2_rn(q, gm2(-1.0f), p)));
-  return make_float2(m.x < -3.402823466e38f ? m.x : r.x, m.y < -3.402823466e38f ? m.y : r.y);
+  return __fadd2_rn(m, gm2_log1p_nexp(__ffma2_rn(q, gm2(-1.0f), p)));
 }
 // x * y - softplus(a) as FFMA2(x, y, min(-a, 0) - log1p(e^-|a|)), the NaN-
 // propagating min giving -max(a, 0): one rounding fewer than the product and

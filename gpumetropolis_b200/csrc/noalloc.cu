@@ -233,6 +233,7 @@ extern "C" int gpum_b200_loglik_batch_noalloc(
   E.n_obs = (int)n_obs;
   E.ncols = (int)n_cols;
   E.T = T;
+  E.U = stage_tiles(T, (int)n_cols);
   E.ntiles = ntiles;
   E.tiles_per_cta = tiles_per_cta;
   E.CG = CG;
