@@ -284,7 +284,7 @@ struct gpum_b200_session {
     EvalArgs E;
     StepArgs S;
     Geometry g;
-    const void* fn;
+    const void *fn, *step_fn;
     size_t step_smem;
     int pt_K, pt_every;
     void *pt_att, *pt_acc, *pt_n;
@@ -312,9 +312,11 @@ struct gpum_b200_session {
   gpum_b200_mlp* da_mlp = nullptr;
   int da_mlp_launches = 0;  // kernel launches per surrogate call
   DBuf<double> mom;  // draw moments scratch
-  DBuf<double> prior_v, prior_g;  // priors at a step's points, and their gradients
+  // priors at a step's points, their gradients, and the step's draws
+  DBuf<double> prior_v, prior_g, side_lu, side_z, side_inc;
   StepArgs step_args{};
   size_t step_smem = 0;
+  const void* step_fn = nullptr;
   // Replica exchange on the device (0 = off).
   int pt_K = 0, pt_every = 0;
   DBuf<uint32_t> pt_att, pt_acc, pt_n;
@@ -378,6 +380,7 @@ struct gpum_b200_session {
     k.E.prior_pts = nullptr;
     k.g = geo;
     k.fn = kc.fn;
+    k.step_fn = step_fn;
     k.step_smem = step_smem;
     k.pt_K = pt_K;
     k.pt_every = pt_every;
@@ -392,8 +395,9 @@ struct gpum_b200_session {
   void run_arrays(size_t C, bool mala) {
     for (char* base = nullptr;;) {
       size_t at = 0;
-      for (auto* b : {&state, &prop, &snap, &sd, &zbuf}) b->carve(base, &at, C * np);
-      for (auto* b : {&temp, &cur, &last_eval, &prior_v}) b->carve(base, &at, C);
+      for (auto* b : {&state, &prop, &snap, &sd, &zbuf, &side_z, &side_inc})
+        b->carve(base, &at, C * np);
+      for (auto* b : {&temp, &cur, &last_eval, &prior_v, &side_lu}) b->carve(base, &at, C);
       for (auto* b : {&ctr, &accepts, &iter}) b->carve(base, &at, C);
       vars.carve(base, &at, 1);
       for (auto* b : {&gx, &gy, &mx, &my, &vbuf, &prior_g}) {
@@ -643,11 +647,27 @@ struct gpum_b200_session {
   }
 
   // Warps per chain (or point) of the step and reduction kernels: as many as
-  // keep all of them in one wave (64 registers: 32 warps per SM).
+  // keep all of them in one wave (80 registers: 24 warps per SM).
   static int warps_per_chain(int n) {
     int w = kWarps;
-    while (w > 1 && (long long)n * w > 32ll * num_sms()) w /= 2;
+    while (w > 1 && (long long)n * w > 24ll * num_sms()) w /= 2;
     return w;
+  }
+
+  // Whether the evaluation's side rows make a step's draws: where the step
+  // kernel gives a chain all eight warps, i.e. the chains are few.  With more
+  // chains its warps draw as fast as they decide, while each side CTA would
+  // hold an SM's shared memory (2,048 x 65 DE on 2^18 observations: 14.1 ms
+  // for 20 steps, 13.4 with the draws in the step kernel; 8 Gaussian chains:
+  // 5.0 us per step, 6.2).
+  bool side_draws() const {
+    return A.mode != MODE_DESYNC && warps_per_chain(n_chains) == kWarps;
+  }
+  // The row of the priors, and the rows of the normals: one a thread, up to
+  // eight rows.
+  int side_rows() const {
+    if (!side_draws()) return prior_code.empty() ? 0 : 1;
+    return 1 + (int)std::min(8ll, ((long long)geo.CG * np + kc.threads - 1) / kc.threads);
   }
 
   // The geometry of the step kernel for the prepared run: 8 warps per block,
@@ -665,15 +685,19 @@ struct gpum_b200_session {
     S.params = params.p;
     S.wpc = warps_per_chain(n_chains);
     S.wpb = kWarps;
-    S.stage_L = A.L && step_smem_doubles((int)np, S.W, S.wpc, true) * 8 <= kMax ? 1 : 0;
+    S.stage_L = A.L && (A.mode == MODE_MALA || !side_draws()) &&
+                        step_smem_doubles((int)np, S.W, S.wpc, true) * 8 <= kMax
+                    ? 1
+                    : 0;
     auto bytes = [&] {
       return (size_t)(S.wpb / S.wpc) *
              step_smem_doubles((int)np, S.W, S.wpc, S.stage_L != 0) * 8;
     };
     while (S.wpb > S.wpc && bytes() > kMax) S.wpb /= 2;
     step_smem = bytes();
+    step_fn = side_draws() ? (const void*)step_kernel<false> : (const void*)step_kernel<true>;
     if (step_smem > 48 * 1024)
-      GPUM_CK(cudaFuncSetAttribute(step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      GPUM_CK(cudaFuncSetAttribute(step_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)step_smem));
   }
 
@@ -682,16 +706,19 @@ struct gpum_b200_session {
     step_args.phase = phase;
     step_args.prior = E.prior_pts ? E.prior_out : nullptr;
     step_args.prior_grad = E.prior_pts ? E.prior_grad : nullptr;
+    step_args.lu = E.side_lu;
+    step_args.z = E.side_z;
+    step_args.inc = E.side_inc;
     void* args[] = {(void*)&A, (void*)&step_args};
     const int cpb = step_args.wpb / step_args.wpc;
-    launch_pdl((const void*)step_kernel, dim3((unsigned)((n_chains + cpb - 1) / cpb)),
+    launch_pdl(step_fn, dim3((unsigned)((n_chains + cpb - 1) / cpb)),
                dim3(32 * step_args.wpb), args, step_smem, stream);
     ++launches;
   }
 
   // Evaluation and end of the start (PH_INIT, at the states) or of one
-  // iteration (PH_STEP, at the proposals); the evaluation's first row of CTAs
-  // computes the priors there.
+  // iteration (PH_STEP, at the proposals); the evaluation's side rows compute
+  // the priors there and the step's draws.
   void eval_and_step(int phase) {
     E.prior_pts = prior_code.empty() ? nullptr : phase == PH_INIT ? A.state : A.prop;
     launch_with(geo, E, phase, phase == PH_STEP);
@@ -735,7 +762,7 @@ struct gpum_b200_session {
   // The evaluation kernel on geometry g; `pdl`: it may start while the
   // previous kernel of the stream runs.
   void launch_with(const Geometry& g, EvalArgs& e, int phase, bool pdl = false) {
-    const dim3 grid(g.NCB, g.NOB + (e.prior_pts ? 1 : 0)), block(kc.threads);
+    const dim3 grid(g.NCB, g.NOB + e.side_rows), block(kc.threads);
     void* targs[] = {(void*)&tc_data.p, (void*)&e, (void*)&A, (void*)&phase};
     void* cargs[] = {(void*)(ext(kc) ? &tmap_c : &tmap), (void*)&e, (void*)&A, (void*)&phase};
     void* iargs[] = {kc.grad_interp ? (void*)gprog.get() : (void*)prog.get(), (void*)&tmap,
@@ -1036,6 +1063,12 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
   ++s->launches;
   s->E.prior_out = s->prior_v.p;
   s->E.prior_grad = mala ? s->prior_g.p : nullptr;
+  s->E.side_rows = s->side_rows();
+  if (s->side_draws()) {
+    s->E.side_lu = s->side_lu.p;
+    s->E.side_z = s->side_z.p;
+    s->E.side_inc = use_L || A.mode == MODE_DE ? s->side_inc.p : nullptr;
+  }
   s->setup_step();
   s->eval_and_step(PH_INIT);
   s->max_iter = max_iter;
@@ -1317,7 +1350,7 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
   s->da_partials.ensure((size_t)max_nob * s->geo_da.C_pad);
   GPUM_CK(cudaMemsetAsync(s->da_params.p, 0, sizeof(float) * np * g.C_pad, st));
   s->E_da = s->E;
-  s->E_da.prior_pts = nullptr;  // the loop's own kernels compute the priors
+  s->E_da.side_rows = 0;  // the loop's own kernels compute priors and draws
   s->E_da.params = s->da_params.p;
   s->E_da.partials = s->da_partials.p;
   s->E_da.active = s->da_active.p;

@@ -10,8 +10,8 @@
 //   CG chains on every observation, so one tile read serves CG chains;
 //   per-thread compensated FP32 sums -> FP64 warp-shuffle tree -> FP64 sum
 //   over warps in fixed order -> FP64 partial per (obs block, chain, value);
-//   one more row of CTAs computes the chains' f64 priors meanwhile; the step
-//   kernel (kernels.cuh, step_kernel) then adds the partials up, makes the
+//   side rows of CTAs compute the chains' f64 priors and draws meanwhile; the
+//   step kernel (kernels.cuh, step_kernel) then adds the partials up, makes the
 //   tempered f64 accept decision, records the draw and draws the next proposal.
 // Results are deterministic for a given launch geometry.
 #pragma once
@@ -97,11 +97,18 @@ struct EvalArgs {
   int n_points;         // chains/points that are real (rest padding)
   uint32_t* err;        // device error word
   const uint32_t* active;  // if set: only the first *active points are live
-  // A sampler step's priors (prior_block): the points [C][np], or nullptr (no
-  // prior, or not a step); the values [C] and, for MALA, the gradients [C][np]
+  // A sampler step's side rows (side_block; 0: not a step): the points [C][np]
+  // of the priors, or nullptr without a prior; the values [C] and, for MALA,
+  // the gradients [C][np]; the logs of the acceptance uniforms [C], normals
+  // [C][np], and L z or the DE differences [C][np], or nullptr (the step
+  // kernel draws)
+  int side_rows;
   const double* prior_pts;
   double* prior_out;
   double* prior_grad;
+  double* side_lu;
+  double* side_z;
+  double* side_inc;
 };
 
 // Delayed acceptance evaluates the first `live` points of the compacted array
@@ -272,26 +279,121 @@ __device__ __forceinline__ Stream make_stream(const ChainArgs& A, int c) {
   return rs;
 }
 
-// ------------------------------------------------------ priors of a step
-// The prior depends on the evaluation points only, so a step's launch carries
-// one extra row of CTAs (blockIdx.y == 0) that computes it beside the data
-// sums, one thread per chain: straight-line f64 code (65 divisions for the
-// 65-parameter model) that would otherwise sit in the serial path between
-// two evaluations.
+// The run's own values into a kernel's argument block.
+__device__ __forceinline__ void load_vars(ChainArgs& A) {
+  const RunVars v = *A.vars;
+  A.n_iter = v.n_iter;
+  A.seed = v.seed;
+  A.gamma = v.gamma;
+  A.de_noise = v.de_noise;
+  A.rec_base = v.rec_base;
+  A.draws = v.draws;
+}
+
+// The i-th uniform (i >= 1) a chain's stream `rs` would return from its
+// current position, without advancing it: both streams are counter-based, so
+// a chain's draws can be made by many threads.
+__device__ __forceinline__ double stream_at(const Stream& rs, uint32_t i) {
+  if (rs.kind == RNG_TRIPLE32) return t32_uniform(rs.seedmix, rs.ctr + i);
+  const U4 r = philox4x32_10(U4{rs.k + i - 1u, rs.it, rs.chain, 0xB2000001u}, rs.seed,
+                             0x6A09E667u);
+  return u53(r.x, r.y);
+}
+__device__ __forceinline__ double stream_normal_at(const Stream& rs, uint32_t i0, int j) {
+  const double u1 = stream_at(rs, i0 + 2u * (uint32_t)j + 1u);
+  const double u2 = stream_at(rs, i0 + 2u * (uint32_t)j + 2u);
+  return sqrt(-2.0 * log(u1)) * cos(6.283185307179586 * u2);
+}
+// The stream of chain c for this step's acceptance uniform, and, past it, for
+// the next proposal's draws (advance_stream: past those, too).
+__device__ __forceinline__ Stream accept_stream(const ChainArgs& A, int c, uint32_t t) {
+  Stream rs = make_stream(A, c);
+  if (A.rng != RNG_TRIPLE32) {
+    rs.it = t;
+    rs.k = 0xFFFF0000u;
+  }
+  return rs;
+}
+__device__ __forceinline__ Stream propose_stream(const ChainArgs& A, int c, bool step,
+                                                 uint32_t t) {
+  Stream rs = make_stream(A, c);
+  if (step) {
+    if (A.rng == RNG_TRIPLE32) rs.ctr += 1u;  // the acceptance uniform
+    rs.it = t + 1;
+  }
+  return rs;
+}
+
+// The DE difference of a chain's next proposal, coordinate j, from the pair of
+// the snapshot that its stream draws first.
+__device__ __forceinline__ double de_difference(const ChainArgs& A, const Stream& rs, int j) {
+  const int n = A.n_chains, np = A.np;
+  int a = (int)(stream_at(rs, 1) * (double)n);
+  if (a >= n) a = n - 1;
+  int b = (int)(stream_at(rs, 2) * (double)n);
+  if (b >= n) b = n - 1;
+  if (b == a) b = (b + 1) % n;
+  const double g = stream_at(rs, 3) < 0.1 ? 1.0 : A.gamma;
+  return g * (A.snap[(size_t)a * np + j] - A.snap[(size_t)b * np + j]);
+}
+
+// ------------------------------------------ the side of a step's evaluation
+// What the end of a step needs besides the data sums depends on the points, the
+// counters and the factors only, so extra rows of CTAs (blockIdx.y <
+// E.side_rows) compute it beside the evaluation.  Row 0: the f64 priors
+// (straight-line code, 65 divisions for the 65-parameter model), one thread
+// per chain.  With E.side_z (few chains, where an iteration is a chain of
+// latencies and SMs are free) also the logs of the acceptance uniforms, and
+// the other rows, a share of the chain block's chains each, the next
+// proposals' normals and L z or the DE differences: in the step kernel they
+// were 2 of the 6.2 us of an iteration of 8 Gaussian chains.  (Inlined: as a
+// function of its own it returned wrong values in the tensor-core kernel.)
 template <class Prior>
-__device__ __forceinline__ void prior_block(const EvalArgs& E, const ChainArgs& A, int cb, int CG,
-                                            int nthreads) {
-  for (int cl = threadIdx.x; cl < CG; cl += nthreads) {
-    const int c = cb * CG + cl;
-    if (c >= A.n_chains) continue;
-    const double* p = E.prior_pts + (size_t)c * A.np;
-    if (E.prior_grad) {
-      double* g = E.prior_grad + (size_t)c * A.np;
-      for (int j = 0; j < A.np; ++j) g[j] = 0.0;
-      E.prior_out[c] = Prior::value_grad(A, c, p, g);
-    } else {
-      E.prior_out[c] = Prior::value(A, c, p);
+__device__ __forceinline__ void side_block(const EvalArgs& E, ChainArgs A, int cb, int CG,
+                                           int phase, int nthreads) {
+  load_vars(A);
+  const int np = A.np;
+  const bool step = phase == PH_STEP;
+  if (blockIdx.y == 0) {
+    for (int cl = threadIdx.x; cl < CG; cl += nthreads) {
+      const int c = cb * CG + cl;
+      if (c >= A.n_chains) continue;
+      if (step && E.side_z) E.side_lu[c] = log(stream_at(accept_stream(A, c, A.iter[c]), 1u));
+      if (!E.prior_pts) continue;
+      const double* p = E.prior_pts + (size_t)c * np;
+      if (E.prior_grad) {
+        double* g = E.prior_grad + (size_t)c * np;
+        for (int j = 0; j < np; ++j) g[j] = 0.0;
+        E.prior_out[c] = Prior::value_grad(A, c, p, g);
+      } else {
+        E.prior_out[c] = Prior::value(A, c, p);
+      }
     }
+    return;
+  }
+  const int rows = E.side_rows - 1, row = (int)blockIdx.y - 1, per = (CG + rows - 1) / rows;
+  const int c0 = cb * CG + row * per;
+  const int n = min(min(per, CG - row * per), A.n_chains - c0);  // may be <= 0
+  const bool de = A.mode == MODE_DE;
+  for (int i = threadIdx.x; i < n * np; i += nthreads) {
+    const int c = c0 + i / np, j = i % np;
+    const uint32_t t = step ? A.iter[c] : 0u;
+    if ((step ? t + 1 : 0u) >= A.n_iter) continue;  // no proposal follows
+    const size_t o = (size_t)c * np + j;
+    const Stream rs = propose_stream(A, c, step, t);
+    E.side_z[o] = stream_normal_at(rs, de ? 3u : 0u, j);
+    if (de) E.side_inc[o] = de_difference(A, rs, j);
+  }
+  if (!A.L) return;
+  __syncthreads();  // uniform: the chains' normals are this block's own
+  for (int i = threadIdx.x; i < n * np; i += nthreads) {
+    const int c = c0 + i / np, k = i % np;
+    const double* L = A.L + ((size_t)c * np + k) * np;
+    const double* z = E.side_z + (size_t)c * np;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int j = 0; j <= k; ++j) acc += L[j] * z[j];
+    E.side_inc[(size_t)c * np + k] = acc;
   }
 }
 
@@ -347,14 +449,14 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   // Chain blocks vary fastest, so the CTAs that share an observation tile
   // run in the same wave and read it through L2 once.
   int cb = blockIdx.x, ob = blockIdx.y, tiles_per_cta = E.tiles_per_cta;
-  if (E.prior_pts) {
-    if (ob == 0) {
+  if (E.side_rows) {
+    if (ob < E.side_rows) {
       pdl_wait();
       pdl_trigger();
-      prior_block<Prior>(E, A, cb, CG, kThreads);
+      side_block<Prior>(E, A, cb, CG, phase, kThreads);
       return;
     }
-    --ob;
+    ob -= E.side_rows;
   }
   if (E.active) {  // delayed acceptance: geometry from the live count
     pdl_wait();

@@ -587,14 +587,14 @@ gm_iter_value_tc(const float* __restrict__ xt, gpum::EvalArgs E, gpum::ChainArgs
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int cb = blockIdx.x, ob = blockIdx.y, tiles_per_cta = E.tiles_per_cta;
-  if (E.prior_pts) {
-    if (ob == 0) {
+  if (E.side_rows) {
+    if (ob < E.side_rows) {
       pdl_wait();
       pdl_trigger();
-      prior_block<JitPrior>(E, A, cb, kTcM, kTcThreads);
+      side_block<JitPrior>(E, A, cb, kTcM, phase, kTcThreads);
       return;
     }
-    --ob;
+    ob -= E.side_rows;
   }
   if (E.active) {  // delayed acceptance: geometry from the live count
     pdl_wait();

@@ -378,33 +378,7 @@ __device__ inline void propose_desync(const ChainArgs& A, int c, Stream& rs, flo
   }
 }
 
-// The run's own values into a kernel's argument block.
-__device__ __forceinline__ void load_vars(ChainArgs& A) {
-  const RunVars v = *A.vars;
-  A.n_iter = v.n_iter;
-  A.seed = v.seed;
-  A.gamma = v.gamma;
-  A.de_noise = v.de_noise;
-  A.rec_base = v.rec_base;
-  A.draws = v.draws;
-}
-
 // ------------------------------------------------- one chain, one warp
-// The i-th uniform (i >= 1) a chain's stream `rs` would return from its
-// current position, without advancing it: both streams are counter-based, so
-// the lanes of a warp can draw a chain's normals in parallel.
-__device__ __forceinline__ double stream_at(const Stream& rs, uint32_t i) {
-  if (rs.kind == RNG_TRIPLE32) return t32_uniform(rs.seedmix, rs.ctr + i);
-  const U4 r = philox4x32_10(U4{rs.k + i - 1u, rs.it, rs.chain, 0xB2000001u}, rs.seed,
-                             0x6A09E667u);
-  return u53(r.x, r.y);
-}
-__device__ __forceinline__ double stream_normal_at(const Stream& rs, uint32_t i0, int j) {
-  const double u1 = stream_at(rs, i0 + 2u * (uint32_t)j + 1u);
-  const double u2 = stream_at(rs, i0 + 2u * (uint32_t)j + 2u);
-  return sqrt(-2.0 * log(u1)) * cos(6.283185307179586 * u2);
-}
-
 __device__ __forceinline__ double warp_sum64(double v) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -605,47 +579,306 @@ reduce_partials_kernel(const double* __restrict__ partials, double* __restrict__
 // ------------------------------------------------------------- a step's end
 // What a Metropolis step does after the evaluation of its proposals: the
 // partial sums added up, the f64 prior, the accept decision on the f64 totals
-// (MALA with the proposal ratio), the draw, the next proposal.  `wpc` warps
-// per chain: all of them add the chain's partials, the first one does the
-// rest, a coordinate per lane.
+// (MALA with the proposal ratio), the draw, the next proposal.  `wpc` warps per
+// chain: all of them add the chain's partials, the first one does the rest, a
+// coordinate per lane; the step's draws come from the evaluation's side rows or
+// are made first.
 //
-// It is bound by latency (the loads, log and cos in f64, np steps of the
-// Langevin substitution), not by any rate.  Run by one thread per chain in the
-// last CTA of each chain block it took 30 us at 1,024 chains x 17 parameters,
-// 144 us at 2,048 x 65 (DE) and 620 us at 2,048 x 24 (MALA with a factor) of
-// every iteration, on at most a few SMs.  The factor is staged in shared
-// memory before the wait for the evaluation, when it fits.
+// It is bound by latency (dependent loads, with MALA np steps of the
+// substitution), not by any rate.  Run by one thread per chain in the last CTA
+// of each chain block it took 30 us at 1,024 chains x 17 parameters, 144 us at
+// 2,048 x 65 (DE) and 620 us at 2,048 x 24 (MALA with a factor) of every
+// iteration, on at most a few SMs.  Up to 32 parameters lane j keeps coordinate
+// j in registers, loaded while the partials are; MALA's factor is staged in
+// shared memory before the wait for the evaluation, when it fits.
+// Per iteration: 8 Gaussian chains on 20,000 observations 10.0 us with the
+// last-CTA end, 6.2 with this kernel drawing for itself, 4.5 with the side
+// rows' draws; MALA with a factor, 2,048 x 24 on 256 observations, 620 us to 78.
 struct StepArgs {
   const double* partials;    // [nob][C_pad][Ws], W values of each used
   int nob, C_pad, Ws, W;
   const double* prior;       // [C], or nullptr: no prior
-  const double* prior_grad;  // [C][np] (MALA)
+  const double* prior_grad;  // [C][np] (MALA), or nullptr
+  const double* lu;          // [C] logs of the acceptance uniforms
+  const double* z;           // [C][np] normals of the next proposal, or nullptr:
+                             // all three drawn here
+  const double* inc;         // [C][np] L z, or DE differences
   float* params;             // [np][C_pad] evaluation points of the next step
   int phase;                 // PH_INIT or PH_STEP
   int wpc;                   // warps per chain: 1, 2, 4 or 8
   int wpb;                   // warps per block
   int stage_L;               // 1: factors staged in shared memory
 };
-// Doubles of shared memory per chain: partial sums, 3 np scratch (the factor's
+// Doubles of shared memory per chain: partial sums, 4 np scratch (the factor's
 // leading dimension is odd, so a column of it spreads over the banks).
 __host__ __device__ inline int step_ld(int np) { return np | 1; }
 __host__ __device__ inline size_t step_smem_doubles(int np, int W, int wpc, bool stage_L) {
-  return (size_t)wpc * W + 3 * (size_t)np + (stage_L ? (size_t)np * step_ld(np) : 0);
+  return (size_t)wpc * W + 4 * (size_t)np + (stage_L ? (size_t)np * step_ld(np) : 0);
 }
 
-static __global__ void __launch_bounds__(kThreads) step_kernel(ChainArgs A, StepArgs S) {
+// The next proposal's coordinate from its mean: RWM and diagonal MALA mean + sd
+// z, with a factor mean + L z, DE (x + g (x_a - x_b)) + noise sd z.
+__device__ __forceinline__ double next_point(const ChainArgs& A, double mean, double sd, double z,
+                                             double inc) {
+  if (A.L) return mean + inc;
+  if (A.mode == MODE_DE) return (mean + inc) + (A.de_noise * sd) * z;
+  return mean + sd * z;
+}
+// Draws of a step from the triple32 counter: the uniform and the proposal's.
+__device__ __forceinline__ uint32_t draws_used(const ChainArgs& A, bool step, bool more) {
+  return (step ? 1u : 0u) +
+         (more ? 2u * (uint32_t)A.np + (A.mode == MODE_DE ? 3u : 0u) : 0u);
+}
+
+// The draws of chain c's step by its first warp: the log of the acceptance
+// uniform, and into z and inc (np doubles of shared memory each) the next
+// proposal's normals and L z or the DE differences.
+__device__ __forceinline__ double draw_warp(const ChainArgs& A, int c, bool step, uint32_t t,
+                                            const double* L, int ldL, double* z, double* inc,
+                                            int lane) {
+  const int np = A.np;
+  const double lu = step ? log(stream_at(accept_stream(A, c, t), 1u)) : 0.0;
+  if (A.mode == MODE_DESYNC || (step ? t + 1 : 0u) >= A.n_iter) return lu;
+  const Stream rs = propose_stream(A, c, step, t);
+  const bool de = A.mode == MODE_DE;
+  for (int j = lane; j < np; j += 32) {
+    z[j] = stream_normal_at(rs, de ? 3u : 0u, j);
+    if (de) inc[j] = de_difference(A, rs, j);
+  }
+  __syncwarp();
+  if (L)
+    for (int k = lane; k < np; k += 32) {
+      double acc = 0.0;
+      for (int j = 0; j <= k; ++j) acc += L[(size_t)k * ldL + j] * z[j];
+      inc[k] = acc;
+    }
+  __syncwarp();
+  return lu;
+}
+
+// The drift at `at` for up to 32 parameters, this lane's coordinate of the mean
+// at + f (1/2) M g (M = L L' or diag sd^2, the whitened drift capped at 2
+// sqrt(np): MALTA; cpu_native.rs:617-651).  sg, st: np doubles of shared memory.
+__device__ __forceinline__ double mean_lane(int np, double sd, const double* L, int ldL, double g,
+                                            double at, double* sg, double* st, int lane) {
+  const bool on = lane < np;
+  if (on) sg[lane] = g;
+  __syncwarp();
+  double v = 0.0;
+  if (on) {
+    if (!L) {
+      v = 0.5 * sd * g;
+    } else {
+      for (int k = lane; k < np; ++k) v += L[(size_t)k * ldL + lane] * sg[k];
+      v *= 0.5;
+    }
+    st[lane] = v;
+  }
+  const double norm = sqrt(warp_sum64(v * v)), dmax = 2.0 * sqrt((double)np);
+  const double f = norm > dmax ? dmax / norm : 1.0;
+  __syncwarp();
+  double d = 0.0;
+  if (on) {
+    if (!L) {
+      d = f * sd * v;
+    } else {
+      for (int j = 0; j <= lane; ++j) d += L[(size_t)lane * ldL + j] * st[j];
+      d *= f;
+    }
+  }
+  return d + at;
+}
+
+// A chain's state as lane `lane` of its first warp holds it, np <= 32.
+struct LaneState {
+  double x, y, sd, mx, z, inc, cur, temp, prior, lu;
+  uint32_t t, ctr;
+};
+__device__ __forceinline__ LaneState load_lane(const ChainArgs& A, const StepArgs& S, int c,
+                                               int lane) {
+  const size_t o = (size_t)c * A.np + lane;
+  const bool on = lane < A.np, step = S.phase == PH_STEP;
+  LaneState P;
+  P.t = A.iter[c];
+  P.ctr = A.ctr[c];
+  P.temp = A.temp[c];
+  P.cur = step ? A.cur[c] : 0.0;
+  P.lu = step && S.z ? S.lu[c] : 0.0;
+  P.prior = S.prior ? S.prior[c] : 0.0;
+  P.x = on ? A.state[o] : 0.0;
+  P.y = on && step ? A.prop[o] : 0.0;
+  P.sd = on ? A.sd[o] : 1.0;
+  P.z = on && S.z ? S.z[o] : 0.0;
+  P.inc = on && S.inc ? S.inc[o] : 0.0;
+  P.mx = on && step && A.mode == MODE_MALA ? A.mx[o] : 0.0;
+  return P;
+}
+
+__device__ __forceinline__ void finish_lane(const ChainArgs& A, const StepArgs& S, int c,
+                                            int lane, const double* L, int ldL,
+                                            const LaneState& P, const double* red, double* sg,
+                                            double* st) {
+  const int np = A.np;
+  const size_t o = (size_t)c * np + lane;
+  const bool on = lane < np, step = S.phase == PH_STEP, mala = A.mode == MODE_MALA;
+  const double b = A.beta ? A.beta[c] : 1.0;  // likelihood power
+  const double ll = group_total(red, S.W, 0, S.wpc);
+  const double lp = (A.beta ? b * ll : ll) + P.prior;
+  double g = 0.0, mean = 0.0;
+  if (mala) {
+    if (on) {
+      g = b * group_total(red, S.W, 1 + lane, S.wpc);
+      if (S.prior_grad) g += S.prior_grad[o];
+    }
+    mean = mean_lane(np, P.sd, L, ldL, g, step ? P.y : P.x, sg, st, lane);
+  }
+  bool take = true;  // the start: the mean is the state's
+  double xn = P.x;
+  if (step) {
+    double lqd = 0.0;
+    if (mala) {
+      // q(x | y) - q(y | x) with the truncated drift at y (cpu_native.rs:704-710):
+      // both residuals through one forward substitution, column by column
+      double r1 = P.x - mean, r2 = P.y - P.mx;
+      if (!L) {
+        const double u1 = r1 / P.sd, u2 = r2 / P.sd;
+        lqd = warp_sum64(on ? 0.5 * u2 * u2 - 0.5 * u1 * u1 : 0.0);
+      } else {
+        for (int j = 0; j < np; ++j) {
+          const double d = L[(size_t)j * ldL + j];
+          const double t1 = __shfl_sync(0xffffffffu, r1, j) / d;
+          const double t2 = __shfl_sync(0xffffffffu, r2, j) / d;
+          if (on && lane > j) {
+            const double l = L[(size_t)lane * ldL + j];
+            r1 -= l * t1;
+            r2 -= l * t2;
+          }
+          lqd += 0.5 * t2 * t2 - 0.5 * t1 * t1;
+        }
+      }
+    }
+    // Tempered acceptance on the f64 totals (chain_kernel.rs:334,
+    // cpu_native.rs:792); MALA adds the proposal ratio and requires a
+    // finite proposal log density (cpu_native.rs:713-714).
+    take = mala ? (isfinite(lp) && P.lu < (lp - P.cur) / P.temp + lqd)
+                : (P.lu < (lp - P.cur) / P.temp);
+    if (take) xn = P.y;
+  }
+  const bool more = A.mode != MODE_DESYNC && (step ? P.t + 1 : 0u) < A.n_iter;
+  if (more && on) {
+    // a rejected proposal leaves the state, and with it its drift, as it was
+    const double y = next_point(A, mala ? (take ? mean : P.mx) : xn, P.sd, P.z, P.inc);
+    S.params[(size_t)lane * S.C_pad + c] = (float)y;
+    A.prop[o] = y;
+  }
+  if (step && on) {
+    if (take) A.state[o] = xn;
+    if (P.t < A.n_iter) A.draws[((size_t)P.t * np + lane) * S.C_pad + c] = (float)xn;
+  }
+  if (step && A.rec_ll) {
+    const uint64_t slot = A.rec_base + (uint64_t)P.t * A.n_chains + c;
+    if (slot < A.rec_cap) {
+      if (on) A.rec_theta[slot * np + lane] = (float)P.y;
+      if (lane == 0) A.rec_ll[slot] = ll;
+    }
+  }
+  if (mala && take && on) {
+    A.gx[o] = g;  // a replica exchange moves it with the state
+    A.mx[o] = mean;
+  }
+  if (lane == 0) {
+    A.last_eval[c] = lp;
+    if (take) A.cur[c] = lp;
+    if (step) {
+      if (take) A.accepts[c] += 1;
+      A.iter[c] = P.t + 1;
+    }
+    A.ctr[c] = P.ctr + (A.rng == RNG_TRIPLE32 ? draws_used(A, step, more) : 0u);
+  }
+}
+
+// The same for any number of parameters, lane j taking j, j + 32, ...
+__device__ inline void finish_wide(const ChainArgs& A, const StepArgs& S, int c, int lane,
+                                   const double* L, int ldL, double lu, const double* z,
+                                   const double* inc, const double* red, double* tmp) {
+  const int np = A.np;
+  const size_t o = (size_t)c * np;
+  const bool step = S.phase == PH_STEP, mala = A.mode == MODE_MALA;
+  double* x = A.state + o;
+  double* y = A.prop + o;
+  const double* sd = A.sd + o;
+  const uint32_t t = A.iter[c];
+  const double b = A.beta ? A.beta[c] : 1.0;  // likelihood power
+  const double ll = group_total(red, S.W, 0, S.wpc);
+  const double lp = (A.beta ? b * ll : ll) + (S.prior ? S.prior[c] : 0.0);
+  double* gy = mala ? A.gy + o : nullptr;
+  double* my = mala ? A.my + o : nullptr;
+  if (mala) {
+    for (int j = lane; j < np; j += 32) {
+      const double v = b * group_total(red, S.W, 1 + j, S.wpc);
+      gy[j] = S.prior_grad ? v + S.prior_grad[o + j] : v;
+    }
+    __syncwarp();
+    half_m_warp(np, sd, L, ldL, gy, step ? y : x, my, tmp, lane);
+  }
+  bool take = true;  // the start: the mean is the state's
+  if (step) {
+    const double lqd =
+        mala ? log_q_ratio_warp(np, sd, L, ldL, x, my, y, A.mx + o, tmp, tmp + np, lane) : 0.0;
+    const double cur = A.cur[c], temp = A.temp[c];
+    take = mala ? (isfinite(lp) && lu < (lp - cur) / temp + lqd) : (lu < (lp - cur) / temp);
+  }
+  const bool more = A.mode != MODE_DESYNC && (step ? t + 1 : 0u) < A.n_iter;
+  const uint64_t slot = A.rec_base + (uint64_t)t * A.n_chains + c;
+  const bool rec = step && A.rec_ll && slot < A.rec_cap;
+  for (int j = lane; j < np; j += 32) {
+    const double yj = step ? y[j] : 0.0;
+    const double xn = step && take ? yj : x[j];
+    if (step) {
+      if (take) x[j] = xn;
+      if (t < A.n_iter) A.draws[((size_t)t * np + j) * S.C_pad + c] = (float)xn;
+      if (rec) A.rec_theta[slot * np + j] = (float)yj;
+    }
+    if (mala && take) {
+      A.gx[o + j] = gy[j];
+      A.mx[o + j] = my[j];
+    }
+    if (more) {
+      const double v =
+          next_point(A, mala ? (take ? my[j] : A.mx[o + j]) : xn, sd[j], z[j], inc[j]);
+      y[j] = v;
+      S.params[(size_t)j * S.C_pad + c] = (float)v;
+    }
+  }
+  if (lane == 0) {
+    A.last_eval[c] = lp;
+    if (take) A.cur[c] = lp;
+    if (rec) A.rec_ll[slot] = ll;
+    if (step) {
+      if (take) A.accepts[c] += 1;
+      A.iter[c] = t + 1;
+    }
+    if (A.rng == RNG_TRIPLE32) A.ctr[c] += draws_used(A, step, more);
+  }
+}
+
+// kDraw: the step's draws are made here (many chains: 80 registers, three CTAs
+// per SM), else by the side rows (few: no spills on the way of each iteration).
+template <bool kDraw>
+static __global__ void __launch_bounds__(kThreads, kDraw ? 3 : 2)
+step_kernel(ChainArgs A, StepArgs S) {
   extern __shared__ double ssm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wpc = S.wpc, wi = warp % wpc, grp = warp / wpc;
   const int c = (int)blockIdx.x * (S.wpb / wpc) + grp;
   const int np = A.np;
   double* red = ssm + (size_t)grp * step_smem_doubles(np, S.W, wpc, S.stage_L != 0);
-  double* tmp = red + (size_t)wpc * S.W;  // [3][np]
+  double* tmp = red + (size_t)wpc * S.W;  // [4][np]
   const bool live = c < A.n_chains;
   const double* L = A.L && live ? A.L + (size_t)c * np * np : nullptr;
   int ldL = np;
   if (L && S.stage_L) {  // set by the host before the run: no wait needed
-    double* Ls = tmp + 3 * np;
+    double* Ls = tmp + 4 * np;
     ldL = step_ld(np);
     for (int i = wi * 32 + lane; i < np * np; i += 32 * wpc)
       Ls[(i / np) * ldL + i % np] = L[i];
@@ -654,87 +887,33 @@ static __global__ void __launch_bounds__(kThreads) step_kernel(ChainArgs A, Step
   load_vars(A);  // as the factors
   pdl_wait();
   pdl_trigger();
+  LaneState P;
+  const bool narrow = np <= 32, step = S.phase == PH_STEP, first = wi == 0 && live;
+  if (narrow && first) P = load_lane(A, S, c, lane);
+  double lu = 0.0;
+  const double *z = tmp + 2 * np, *inc = tmp + 3 * np;
+  if constexpr (kDraw) {
+    if (L && S.stage_L) __syncthreads();  // the factors are staged
+    if (first) lu = draw_warp(A, c, step, A.iter[c], L, ldL, tmp + 2 * np, tmp + 3 * np, lane);
+  } else if (first && !narrow) {
+    const size_t o = (size_t)c * np;
+    lu = S.lu[c];
+    z = S.z + o;
+    inc = S.inc ? S.inc + o : z;  // unused without differences
+  }
   if (live) group_partials(S.partials, S.nob, S.C_pad, S.Ws, S.W, c, wi, wpc, red, lane);
   __syncthreads();
-  if (wi != 0 || !live) return;
-
-  const size_t o = (size_t)c * np;
-  const bool mala = A.mode == MODE_MALA;
-  double* x = A.state + o;
-  const double* sd = A.sd + o;
-  const uint32_t t = A.iter[c];
-  Stream rs = make_stream(A, c);
-  const double b = A.beta ? A.beta[c] : 1.0;  // likelihood power
-  const double ll = group_total(red, S.W, 0, wpc);
-  const double lp = (A.beta ? b * ll : ll) + (S.prior ? S.prior[c] : 0.0);
-  if (mala) {
-    double* g = (S.phase == PH_INIT ? A.gx : A.gy) + o;
-    for (int j = lane; j < np; j += 32) {
-      const double v = b * group_total(red, S.W, 1 + j, wpc);
-      g[j] = S.prior_grad ? v + S.prior_grad[o + j] : v;
+  if (!first) return;
+  if (narrow) {
+    if constexpr (kDraw) {
+      P.lu = lu;
+      P.z = lane < np ? z[lane] : 0.0;
+      P.inc = lane < np ? inc[lane] : 0.0;
     }
-    __syncwarp();
-  }
-  if (S.phase == PH_INIT) {
-    if (lane == 0) {
-      A.cur[c] = lp;
-      A.last_eval[c] = lp;
-    }
-    if (A.n_iter == 0 || A.mode == MODE_DESYNC) return;  // path B proposes in its own kernel
-    rs.it = 0;
+    finish_lane(A, S, c, lane, L, ldL, P, red, tmp, tmp + np);
   } else {
-    const double* y = A.prop + o;
-    const double cur = A.cur[c];
-    double lqd = 0.0;
-    if (mala) {
-      // q(x | y) - q(y | x) with the truncated drift at y (cpu_native.rs:704-710)
-      double* my = A.my + o;
-      half_m_warp(np, sd, L, ldL, A.gy + o, y, my, tmp, lane);
-      lqd = log_q_ratio_warp(np, sd, L, ldL, x, my, y, A.mx + o, tmp, tmp + np, lane);
-    }
-    if (A.rng != RNG_TRIPLE32) {
-      rs.it = t;
-      rs.k = 0xFFFF0000u;
-    }
-    const double u = rs.next();
-    // Tempered acceptance on the f64 totals (chain_kernel.rs:334,
-    // cpu_native.rs:792); MALA adds the proposal ratio and requires a
-    // finite proposal log density (cpu_native.rs:713-714).
-    const bool take = mala ? (isfinite(lp) && log(u) < (lp - cur) / A.temp[c] + lqd)
-                           : (log(u) < (lp - cur) / A.temp[c]);
-    if (A.rec_ll) {
-      const uint64_t slot = A.rec_base + (uint64_t)t * A.n_chains + c;
-      if (slot < A.rec_cap) {
-        for (int j = lane; j < np; j += 32) A.rec_theta[slot * np + j] = (float)y[j];
-        if (lane == 0) A.rec_ll[slot] = ll;
-      }
-    }
-    for (int j = lane; j < np; j += 32) {
-      const double v = take ? y[j] : x[j];
-      if (take) {
-        x[j] = v;
-        if (mala) A.gx[o + j] = A.gy[o + j];
-      }
-      if (t < A.n_iter) A.draws[((size_t)t * np + j) * S.C_pad + c] = (float)v;
-    }
-    if (lane == 0) {
-      A.last_eval[c] = lp;
-      if (take) {
-        A.cur[c] = lp;
-        A.accepts[c] += 1;
-      }
-      A.iter[c] = t + 1;
-    }
-    __syncwarp();
-    if (t + 1 >= A.n_iter || A.mode == MODE_DESYNC) {
-      if (lane == 0) A.ctr[c] = rs.ctr;
-      return;
-    }
-    rs.it = t + 1;
-    rs.k = 0;
+    finish_wide(A, S, c, lane, L, ldL, lu, z, inc, red, tmp);
   }
-  rs = propose_warp(A, c, rs, S.params, S.C_pad, lane, tmp, L, ldL);
-  if (lane == 0) A.ctr[c] = rs.ctr;
 }
 
 // ------------------------------------------------------------- helpers
