@@ -10,7 +10,7 @@
 //
 // Pinned and device allocations cost 1 to 5 ms and 40 to 150 us a call, more
 // than a short run, so both come from process-wide pools that keep what is
-// given back: 1 MB of small blocks, 8 MB of large ones and 64 MB of device
+// given back: 2 MB of small blocks, 8 MB of large ones and 64 MB of device
 // memory at most, until the process ends.  Demand beyond that falls back to the
 // driver.  Every function here is safe to call from several threads.
 #pragma once
@@ -29,10 +29,10 @@
 
 namespace gpum {
 
-constexpr size_t kSmallPinned = 64 << 10;  // a session's block
-constexpr size_t kSmallIn = 40 << 10;      // of it, for the host's inputs
+constexpr size_t kSmallPinned = 128 << 10;  // a session's block
+constexpr size_t kSmallIn = 64 << 10;       // of it, for the host's inputs
 constexpr size_t kSmallOut = kSmallPinned - kSmallIn;
-constexpr size_t kChunkPinned = 1 << 20;   // a block of a large transfer
+constexpr size_t kChunkPinned = 1 << 20;    // a block of a large transfer
 constexpr int kSmallBlocks = 16, kChunkBlocks = 8;
 
 // One pinned allocation, made at the first use, in equal blocks.
