@@ -436,6 +436,7 @@ __host__ __device__ inline size_t skel_smem_bytes(int T, int ncols, int np, int 
 //   void begin(const float* pc0, int CG)   pc0 = this thread's first chain in
 //                                          the [np][CG] parameter tile
 //   void eval(const float* xo, int T, bool valid)  one observation
+//   kRounds == 2: eval_rounds(xo, xs, T, v0, v1) takes two, at xo and xo + xs
 //   float last(int g)                      value of the last eval (pointwise)
 //   void end()                             after the last observation
 //   double total(int g, int w)             w = 0 value, 1.. gradient entries
@@ -589,6 +590,24 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
           }
         } else {
           for (int pi = lane + 32 * wo; 2 * pi < T; pi += 32 * WO) pair(pi);
+        }
+      } else if constexpr (Body::kRounds == 2) {
+        // two of a lane's observations per call (the host chooses this body
+        // where 64 WO divides T)
+        for (int ol = lane + 32 * wo; ol < T; ol += 64 * WO) {
+          const int obs = obs0 + ol, xs = 32 * WO;
+          const bool v0 = obs < E.n_obs, v1 = obs + xs < E.n_obs;
+          body.eval_rounds(tile + ol, xs, T, v0, v1);
+          if (phase == PH_POINTWISE) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+              const int c = cb * CG + wc * G + g;
+              if (c >= E.n_points) continue;
+              float* out = E.pointwise + (size_t)c * E.n_obs + obs;
+              if (v0) out[0] = body.last(g, 0);
+              if (v1) out[xs] = body.last(g, 1);
+            }
+          }
         }
       } else {
         for (int ol = lane + 32 * wo; ol < T; ol += 32 * WO) {

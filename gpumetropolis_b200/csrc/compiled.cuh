@@ -39,6 +39,7 @@ template <int G, bool GRAD>
 struct JitBody {
   static constexpr bool kChainLanes = false;
   static constexpr int kObsPerEval = 1;
+  static constexpr int kRounds = 1;
   float p[G][GM_NP];
   float h[G][GM_NH];
   Acc64 acc[G];

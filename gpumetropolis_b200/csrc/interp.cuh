@@ -32,74 +32,106 @@ struct __align__(16) EvalProg {
 
 enum HeavyKind : int { H_NONE = -1, H_DIV = 0, H_POW = 1, H_LGAMMA = 2 };
 
-// The G parameters of this thread's chains for one parameter index, as G/2
-// pairs: one broadcast 16- or 8-byte shared load per 4 or 2 chains.
-template <int G>
+// A thread's G values are G chains at one observation (O = 1) or G/2 chains at
+// two (O = 2: the lower half of the pairs at the first, the upper at the
+// second).  A parameter load (a broadcast 16 bytes, 2.2 cycles of the shared-
+// memory pipe, per four chains) is what a term of a linear predictor costs:
+// at O = 2 it serves twice the observations.
+
+// The G/O parameters of this thread's chains for one parameter index, as
+// pairs, for every observation: one broadcast 16- or 8-byte shared load per 4 or
+// 2 chains.
+template <int G, int O>
 __device__ __forceinline__ void load_params2(const float* __restrict__ p,
                                              float2 (&v)[G / 2]) {
-  if constexpr (G % 4 == 0) {
+  constexpr int C = G / O;
+  if constexpr (C % 4 == 0) {
 #pragma unroll
-    for (int g = 0; g < G; g += 4) {
+    for (int g = 0; g < C; g += 4) {
       const float4 q = *reinterpret_cast<const float4*>(p + g);
       v[g / 2] = make_float2(q.x, q.y);
       v[g / 2 + 1] = make_float2(q.z, q.w);
     }
   } else {
 #pragma unroll
-    for (int g = 0; g < G; g += 2) v[g / 2] = *reinterpret_cast<const float2*>(p + g);
+    for (int g = 0; g < C; g += 2) v[g / 2] = *reinterpret_cast<const float2*>(p + g);
   }
+#pragma unroll
+  for (int h = C / 2; h < G / 2; ++h) v[h] = v[h - C / 2];
 }
 
-// acc += sum over n terms of param[p_k] * x[col_k] for the G chains, in term
-// order (one FFMA2 per chain pair and term).  The narrower variants load two
-// terms ahead of their multiply-adds to overlap the loads' latency.
-template <int G>
+// acc += sum over n terms of param[p_k] * x[col_k] for the G values, in term
+// order (one FFMA2 per pair and term).  The narrower variants load two terms
+// ahead of their multiply-adds to overlap the loads' latency.  xs: the second
+// observation is at xo + xs.
+template <int G, int O>
 __device__ __forceinline__ void gpum_dot(float2 (&acc)[G / 2], const uint32_t* __restrict__ tm,
-                                         uint32_t n, const float* __restrict__ xo, int T,
+                                         uint32_t n, const float* __restrict__ xo, int xs, int T,
                                          const float* __restrict__ pc0, int CG) {
-  constexpr int H = G / 2;
+  constexpr int H = G / 2, HP = H / O;
+  auto x = [&](uint32_t t, float2 (&v)[O]) {
+    const float* p = xo + (size_t)(t >> 11) * T;
+    v[0] = gm2(p[0]);
+    if constexpr (O == 2) v[1] = gm2(p[xs]);
+  };
   uint32_t k = 0;
-  if constexpr (H <= 4) {
+  if constexpr (O == 2) {
+    for (; k + 4 <= n; k += 4) {
+      float2 v[4][O], p[4][H];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t tq = tm[k + q];
+        x(tq, v[q]);
+        load_params2<G, O>(pc0 + (size_t)(tq & 0x7FFu) * CG, p[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int h = 0; h < H; ++h) acc[h] = gm2_fma(p[q][h], v[q][h / HP], acc[h]);
+    }
+  } else if constexpr (HP <= 4) {
     for (; k + 2 <= n; k += 2) {
       const uint32_t ta = tm[k], tb = tm[k + 1];
-      const float2 va = gm2(xo[(size_t)(ta >> 11) * T]), vb = gm2(xo[(size_t)(tb >> 11) * T]);
-      float2 pa[H], pb[H];
-      load_params2<G>(pc0 + (size_t)(ta & 0x7FFu) * CG, pa);
-      load_params2<G>(pc0 + (size_t)(tb & 0x7FFu) * CG, pb);
+      float2 va[O], vb[O], pa[H], pb[H];
+      x(ta, va);
+      x(tb, vb);
+      load_params2<G, O>(pc0 + (size_t)(ta & 0x7FFu) * CG, pa);
+      load_params2<G, O>(pc0 + (size_t)(tb & 0x7FFu) * CG, pb);
 #pragma unroll
-      for (int h = 0; h < H; ++h) acc[h] = gm2_fma(pa[h], va, acc[h]);
+      for (int h = 0; h < H; ++h) acc[h] = gm2_fma(pa[h], va[h / HP], acc[h]);
 #pragma unroll
-      for (int h = 0; h < H; ++h) acc[h] = gm2_fma(pb[h], vb, acc[h]);
+      for (int h = 0; h < H; ++h) acc[h] = gm2_fma(pb[h], vb[h / HP], acc[h]);
     }
   }
   for (; k < n; ++k) {
     const uint32_t tw = tm[k];
-    const float2 v = gm2(xo[(size_t)(tw >> 11) * T]);
-    float2 pv[H];
-    load_params2<G>(pc0 + (size_t)(tw & 0x7FFu) * CG, pv);
+    float2 v[O], pv[H];
+    x(tw, v);
+    load_params2<G, O>(pc0 + (size_t)(tw & 0x7FFu) * CG, pv);
 #pragma unroll
-    for (int h = 0; h < H; ++h) acc[h] = gm2_fma(pv[h], v, acc[h]);
+    for (int h = 0; h < H; ++h) acc[h] = gm2_fma(pv[h], v[h / HP], acc[h]);
   }
 }
 
-// Interpret the program once for G chains at one observation.  The stack
-// holds the chains as pairs, so the arithmetic runs on sm_100's two-wide
+// Interpret the program once for G values.  The stack holds them as pairs of
+// chains, so the arithmetic runs on sm_100's two-wide
 // FP32 instructions (FADD2, FMUL2, FFMA2; subtraction and negation as exact
 // FFMA2 / FMUL2 by -1), which round each half exactly like the scalar
 // instruction: the values are those of one chain per instruction.
 //   s  : slot S, chains 2h and 2h+1 in s[S][h]
-//   xo : this lane's observation inside the tile; column j is at xo[j*T]
+//   xo : this lane's observation inside the tile; column j is at xo[j*T], the
+//        second observation's at xo[j*T + xs]
 //   pc0: this thread's first chain in the param tile; param p, chain g at
 //        pc0[p*CG + g]  (16-byte aligned; G is a multiple of 2)
 //   hsm: this thread's operand scratch for the shared expensive ops, 2*G
 //        floats at a stride of kInterpThreads (the block's thread count)
-template <int G, int D>
+template <int G, int D, int O>
 __device__ __forceinline__ void interp_run(const EvalProg& pg, float2 (&s)[D][G / 2],
-                                           const float* __restrict__ xo, int T,
+                                           const float* __restrict__ xo, int xs, int T,
                                            const float* __restrict__ pc0, int CG,
                                            float* __restrict__ hsm) {
   static_assert(G % 2 == 0, "chains are processed in pairs");
-  constexpr int H = G / 2;
+  constexpr int H = G / 2, HP = H / O;
   const uint32_t n = pg.n_uops;
   // Saved subtrees (K_SAVEk / K_LOADk): registers, since every case names
   // its save index at compile time.  The sixteen-chain variant keeps one, the
@@ -115,7 +147,8 @@ __device__ __forceinline__ void interp_run(const EvalProg& pg, float2 (&s)[D][G 
     const uint32_t a1 = w >> 22;
     int hk = H_NONE, hs = 0;
 
-#define GPUM_XD(a) xo[(size_t)(a) * T]
+// within a loop over the pairs h: the column's value at pair h's observation
+#define GPUM_XD(a) xo[(size_t)(a) * T + (O == 2 && h >= HP ? xs : 0)]
 #define GPUM_HA(g) hsm[(g) * kInterpThreads]
 #define GPUM_HB(g) hsm[(G + (g)) * kInterpThreads]
 #define GPUM_UN(S, EXPR)                                                               \
@@ -143,7 +176,7 @@ __device__ __forceinline__ void interp_run(const EvalProg& pg, float2 (&s)[D][G 
 #define GPUM_SLOT(S)                                                                   \
   case S * NKIND + K_PUSH_C: GPUM_UN(S, gm2(pg.cst[a0]))                               \
   case S * NKIND + K_PUSH_P:                                                           \
-    if constexpr (S < D) load_params2<G>(pc0 + (size_t)a0 * CG, s[S]);                 \
+    if constexpr (S < D) load_params2<G, O>(pc0 + (size_t)a0 * CG, s[S]);                 \
     break;                                                                             \
   case S * NKIND + K_PUSH_D: GPUM_UN(S, gm2(GPUM_XD(a0)))                              \
   case S * NKIND + K_ADD:                                                              \
@@ -175,21 +208,21 @@ __device__ __forceinline__ void interp_run(const EvalProg& pg, float2 (&s)[D][G 
   case S * NKIND + K_ADD_P:                                                            \
     if constexpr (S < D) {                                                             \
       float2 pv[H];                                                                    \
-      load_params2<G>(pc0 + (size_t)a0 * CG, pv);                                      \
+      load_params2<G, O>(pc0 + (size_t)a0 * CG, pv);                                      \
       _Pragma("unroll") for (int h = 0; h < H; ++h) s[S][h] = gm2_add(s[S][h], pv[h]); \
     }                                                                                  \
     break;                                                                             \
   case S * NKIND + K_SUB_P:                                                            \
     if constexpr (S < D) {                                                             \
       float2 pv[H];                                                                    \
-      load_params2<G>(pc0 + (size_t)a0 * CG, pv);                                      \
+      load_params2<G, O>(pc0 + (size_t)a0 * CG, pv);                                      \
       _Pragma("unroll") for (int h = 0; h < H; ++h) s[S][h] = gm2_sub(s[S][h], pv[h]); \
     }                                                                                  \
     break;                                                                             \
   case S * NKIND + K_MUL_P:                                                            \
     if constexpr (S < D) {                                                             \
       float2 pv[H];                                                                    \
-      load_params2<G>(pc0 + (size_t)a0 * CG, pv);                                      \
+      load_params2<G, O>(pc0 + (size_t)a0 * CG, pv);                                      \
       _Pragma("unroll") for (int h = 0; h < H; ++h) s[S][h] = gm2_mul(s[S][h], pv[h]); \
     }                                                                                  \
     break;                                                                             \
@@ -200,8 +233,8 @@ __device__ __forceinline__ void interp_run(const EvalProg& pg, float2 (&s)[D][G 
       _Pragma("unroll") for (int h = 0; h < H; ++h) {                                  \
         GPUM_HA(2 * h) = s[S][h].x;                                                    \
         GPUM_HA(2 * h + 1) = s[S][h].y;                                                \
-        GPUM_HB(2 * h) = pp[2 * h];                                                    \
-        GPUM_HB(2 * h + 1) = pp[2 * h + 1];                                            \
+        GPUM_HB(2 * h) = pp[2 * (h % HP)];                                             \
+        GPUM_HB(2 * h + 1) = pp[2 * (h % HP) + 1];                                     \
       }                                                                                \
       hk = ((w & kCaseMask) == S * NKIND + K_DIV_P) ? H_DIV : H_POW;                   \
       hs = S;                                                                          \
@@ -220,19 +253,19 @@ __device__ __forceinline__ void interp_run(const EvalProg& pg, float2 (&s)[D][G 
   case S * NKIND + K_SQR: GPUM_UN(S, gm2_mul(s[S][h], s[S][h]))                        \
   case S * NKIND + K_FMA_PD:                                                           \
     if constexpr (S < D) {                                                             \
-      const float2 v = gm2(GPUM_XD(a1));                                               \
       float2 pv[H];                                                                    \
-      load_params2<G>(pc0 + (size_t)a0 * CG, pv);                                      \
-      _Pragma("unroll") for (int h = 0; h < H; ++h) s[S][h] = gm2_fma(pv[h], v, s[S][h]); \
+      load_params2<G, O>(pc0 + (size_t)a0 * CG, pv);                                      \
+      _Pragma("unroll") for (int h = 0; h < H; ++h)                                     \
+        s[S][h] = gm2_fma(pv[h], gm2(GPUM_XD(a1)), s[S][h]);                           \
     }                                                                                  \
     break;                                                                             \
   case S * NKIND + K_DOTP:                                                             \
-    if constexpr (S < D) load_params2<G>(pc0 + (size_t)(pg.term[a0] & 0x7FFu) * CG, s[S]); \
+    if constexpr (S < D) load_params2<G, O>(pc0 + (size_t)(pg.term[a0] & 0x7FFu) * CG, s[S]); \
     [[fallthrough]];                                                                   \
   case S * NKIND + K_DOT:                                                              \
     if constexpr (S < D) {                                                             \
       const uint32_t t0 = a0 + ((w & kCaseMask) == S * NKIND + K_DOTP ? 1u : 0u);      \
-      gpum_dot<G>(s[S], pg.term + t0, a1 & kDotCount, xo, T, pc0, CG);                 \
+      gpum_dot<G, O>(s[S], pg.term + t0, a1 & kDotCount, xo, xs, T, pc0, CG);          \
       if (a1 & kDotSave) {                                                             \
         if constexpr (NS > 0) {                                                        \
           _Pragma("unroll") for (int h = 0; h < H; ++h) sv[0][h] = s[S][h];            \
@@ -256,7 +289,7 @@ __device__ __forceinline__ void interp_run(const EvalProg& pg, float2 (&s)[D][G 
   case S * NKIND + K_MUL_P1:                                                           \
     if constexpr (S + 1 < D) {                                                         \
       float2 pv[H];                                                                    \
-      load_params2<G>(pc0 + (size_t)a0 * CG, pv);                                      \
+      load_params2<G, O>(pc0 + (size_t)a0 * CG, pv);                                      \
       const uint32_t kd = (w & kCaseMask) - S * NKIND;                                 \
       if (kd == K_ADD_P1) {                                                            \
         _Pragma("unroll") for (int h = 0; h < H; ++h) s[S][h] = gm2_add(pv[h], s[S + 1][h]); \

@@ -9,35 +9,48 @@
 
 namespace gpum {
 
-template <int G, int D>
+// G values per thread: G chains (O = 1), or G/2 chains at two observations of a
+// lane at once (O = 2).  Either way a lane's observations are added in the same
+// order.
+template <int G, int D, int O>
 struct InterpBody {
   static constexpr bool kChainLanes = false;
   static constexpr int kObsPerEval = 1;
+  static constexpr int kRounds = O;
+  static constexpr int kChains = G / O;
   const EvalProg& pg;
   const float* pc0;
   int CG;
   float* hsm;
   float2 s[D][G / 2];  // chain pairs
-  Comp acc[G];
+  Comp acc[kChains];
   __device__ InterpBody(const EvalProg& p, float* h) : pg(p), pc0(nullptr), CG(0), hsm(h) {}
   __device__ __forceinline__ void begin(const float* p0, int cg) {
     pc0 = p0;
     CG = cg;
 #pragma unroll
-    for (int g = 0; g < G; ++g) acc[g].init();
+    for (int g = 0; g < kChains; ++g) acc[g].init();
   }
-  __device__ __forceinline__ void eval(const float* xo, int T, bool valid) {
-    interp_run<G, D>(pg, s, xo, T, pc0, CG, hsm);
-    if (valid) {
+  __device__ __forceinline__ void add(int round) {
 #pragma unroll
-      for (int h = 0; h < G / 2; ++h) {
-        acc[2 * h].add(s[0][h].x);
-        acc[2 * h + 1].add(s[0][h].y);
-      }
+    for (int h = 0; h < kChains / 2; ++h) {
+      acc[2 * h].add(s[0][round * (kChains / 2) + h].x);
+      acc[2 * h + 1].add(s[0][round * (kChains / 2) + h].y);
     }
   }
-  __device__ __forceinline__ float last(int g) const {
-    return (g & 1) ? s[0][g >> 1].y : s[0][g >> 1].x;
+  __device__ __forceinline__ void eval(const float* xo, int T, bool valid) {
+    interp_run<G, D, O>(pg, s, xo, 0, T, pc0, CG, hsm);
+    if (valid) add(0);
+  }
+  // The observations at xo and xo + xs.
+  __device__ __forceinline__ void eval_rounds(const float* xo, int xs, int T, bool v0, bool v1) {
+    interp_run<G, D, O>(pg, s, xo, xs, T, pc0, CG, hsm);
+    if (v0) add(0);
+    if (v1) add(O - 1);
+  }
+  __device__ __forceinline__ float last(int g, int round = 0) const {
+    const float2 v = s[0][round * (kChains / 2) + (g >> 1)];
+    return (g & 1) ? v.y : v.x;
   }
   __device__ __forceinline__ void end() {}
   __device__ __forceinline__ double total(int g, int) const { return acc[g].total(); }
@@ -61,14 +74,14 @@ struct InterpPrior {
 // The widest variants (sixteen chains per thread over a six-deep stack, eight
 // over eight: 96 and 64 stack registers) keep their stacks in registers at one
 // CTA per SM; the others fit two.
-template <int G, int D>
+template <int G, int D, int O = 1>
 __global__ void __launch_bounds__(kThreads, (G >= 8 ? 1 : 2))
 iter_kernel(const __grid_constant__ EvalProg prog, const __grid_constant__ TmapDesc tmap,
             EvalArgs E, ChainArgs A, int phase) {
   static_assert(kThreads == kInterpThreads, "the operand scratch is laid out per thread");
   __shared__ float hsm[2 * G * kInterpThreads];
-  InterpBody<G, D> body(prog, hsm + threadIdx.x);
-  run_iteration<G, 1, InterpBody<G, D>, InterpPrior>(&tmap, E, A, phase, body);
+  InterpBody<G, D, O> body(prog, hsm + threadIdx.x);
+  run_iteration<G / O, 1, InterpBody<G, D, O>, InterpPrior>(&tmap, E, A, phase, body);
 }
 
 // ------------------------------------------------------- failure self-test
@@ -112,6 +125,7 @@ template <int W>
 struct InterpGradBody {
   static constexpr bool kChainLanes = false;
   static constexpr int kObsPerEval = 1;
+  static constexpr int kRounds = 1;
   static constexpr int kNp = W - 1;
   const GradProg& pg;
   const float* pc0;

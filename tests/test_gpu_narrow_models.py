@@ -64,3 +64,22 @@ def test_folds_match_the_oracle(gpu, text):
     # the terms' absolute sum, here at most 4 |ref| + 4
     assert np.max(np.abs(got - ref) / (4 * np.abs(ref) + 4)) <= 12 * 2.0 ** -24
     assert np.max(np.abs(tot - got.sum(axis=1)) / np.abs(got).sum(axis=1)) <= 1e-6
+
+
+@pytest.mark.parametrize("p,n_obs,n_points", [(3, 255, 70), (3, 513, 12), (3, 257, 9), (5, 64, 57),
+                                              (40, 300, 70), (40, 300, 9)])
+def test_interpreter_at_two_observations(gpu, p, n_obs, n_points):
+    # eight chains at two observations per thread where the tile (256, or 128
+    # and less for 41 columns) leaves every lane two, sixteen chains elsewhere
+    w = W.make("logistic", n_obs=n_obs, p=p)
+    m = w.model
+    pts = w.truth["beta"] + np.random.default_rng(1).normal(0, 0.1, (n_points, m.n_params))
+    args = (m.loglik.code, m.loglik.consts, m.n_params, w.data, m.n_cols, n_obs, pts)
+    with gpu.Session(m.loglik.code, m.loglik.consts, m.prior.code, m.prior.consts, m.n_params,
+                     w.data, m.n_cols, n_obs, engine=0) as s:
+        got, tot = s.loglik_pointwise(pts), s.loglik_batch(pts)
+    ref = O.loglik_pointwise(*args)
+    # an f32 linear predictor of p + 1 terms of size below 4, two roundings each
+    assert np.max(np.abs(got - ref)) <= 2 * (p + 8) * 4 * 2.0 ** -23
+    ref = O.loglik_batch(*args)
+    assert np.max(np.abs(tot - ref) / np.abs(ref)) <= 1e-6
