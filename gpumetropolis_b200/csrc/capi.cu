@@ -491,6 +491,10 @@ struct gpum_b200_session {
   // does not write.  Gradients of more than 256 points run two chains per lane:
   // its eight warps of 64 then share no chain, as the eight of 32 share none
   // above 224, so every chain's FP32 blocks are the same on either kernel.
+  // From 33 to 256 points its form with four warps shares a chain among as many
+  // warps as the eight of 32 do (4, 2 or 1).  The kernel on 65,537 observations,
+  // eight warps of 32 -> four of 64: 250 points of 17 parameters 96 -> 83 us, of
+  // 24 83 -> 66, 100 points of 24 43 -> 35, 64 of 17 28 -> 25.
   KernelChoice choose(int n, bool need_grad, bool pointwise = false) {
     KernelChoice k;
     // Gradients: the compiled engine's adjoint unless the interpreter engine
@@ -523,6 +527,10 @@ struct gpum_b200_session {
       if (need_grad && cm.k_grad2 && n > 256) {
         k.fn = (const void*)cm.k_grad2;
         k.G = 64;
+      } else if (need_grad && cm.k_grad2h && n > 32) {
+        k.fn = (const void*)cm.k_grad2h;
+        k.G = 64;
+        k.threads = 128;
       }
       k.W = need_grad ? 1 + (int)np : 1;
       if (!need_grad && !pointwise && tc_ok) {
@@ -557,7 +565,7 @@ struct gpum_b200_session {
     g.G = k.G;
     const int groups = (n + g.G - 1) / g.G;
     g.WC = 1;
-    while (!k.tc && g.WC < kWarps && g.WC < groups) g.WC *= 2;
+    while (!k.tc && g.WC < k.threads / 32 && g.WC < groups) g.WC *= 2;
     g.CG = g.WC * g.G;
     g.NCB = (n + g.CG - 1) / g.CG;
     g.C_pad = g.NCB * g.CG;
@@ -565,7 +573,7 @@ struct gpum_b200_session {
     g.ntiles = (int)((n_obs + Tk - 1) / Tk);
     g.smem = k.tc ? tc_smem_bytes(cm.tc_kp, cm.tc_ntail, cm.tc_tn, cm.tc_stages)
                   : skel_smem_bytes(Tk, (int)(ext(k) ? ncols_c : ncols), (int)np, g.CG, g.G,
-                                    k.W, k.lanes);
+                                    k.W, k.lanes, k.threads / 32);
     int occ = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, k.threads, g.smem);
     if (occ < 1) occ = 1;

@@ -416,9 +416,10 @@ __host__ __device__ inline size_t skel_param_floats(int np, int CG, bool lanes) 
   return lanes ? 0 : (((size_t)np * CG + 3) & ~(size_t)3);
 }
 __host__ __device__ inline size_t skel_smem_bytes(int T, int ncols, int np, int CG, int G,
-                                                  int width, bool lanes = false) {
+                                                  int width, bool lanes = false,
+                                                  int warps = kWarps) {
   return 2 * (size_t)stage_tiles(T, ncols) * T * ncols * 4 + skel_param_floats(np, CG, lanes) * 4 +
-         (size_t)kWarps * G * width * 8 + 2 * 8;
+         (size_t)warps * G * width * 8 + 2 * 8;
 }
 
 // Body contract (G chains per thread):
@@ -440,8 +441,8 @@ __host__ __device__ inline size_t skel_smem_bytes(int T, int ncols, int np, int 
 //   float last(int g)                      value of the last eval (pointwise)
 //   void end()                             after the last observation
 //   double total(int g, int w)             w = 0 value, 1.. gradient entries
-//   W (compile time) = E.width values reduced per chain
-template <int G, int W, class Body, class Prior>
+//   W (compile time) = E.width values reduced per chain; NW warps per CTA
+template <int G, int W, class Body, class Prior, int NW = kWarps>
 __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalArgs& E,
                                               const ChainArgs& A, int phase, Body& body) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -454,7 +455,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     if (ob < E.side_rows) {
       pdl_wait();
       pdl_trigger();
-      side_block<Prior>(E, A, cb, CG, phase, kThreads);
+      side_block<Prior>(E, A, cb, CG, phase, 32 * NW);
       return;
     }
     ob -= E.side_rows;
@@ -470,7 +471,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     cb = id % busy;
     ob = id / busy;
   }
-  const int WO = kWarps / E.WC;
+  const int WO = NW / E.WC;
   const int wc = warp % E.WC, wo = warp / E.WC;
 
   const size_t tile_floats = (size_t)T * ncols, stage_floats = E.U * tile_floats;
@@ -479,7 +480,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   constexpr bool kLanes = Body::kChainLanes;
   float* psm = xs + 2 * stage_floats;
   double* red = reinterpret_cast<double*>(psm + skel_param_floats(np, CG, kLanes));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(red + (size_t)kWarps * G * W);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(red + (size_t)NW * G * W);
 
   const int t0 = ob * tiles_per_cta;
   const int t1 = min(t0 + tiles_per_cta, E.ntiles);
@@ -507,7 +508,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
   pdl_wait();
   pdl_trigger();
   if constexpr (!kLanes) {
-    for (int i = tid; i < np * CG; i += kThreads) {
+    for (int i = tid; i < np * CG; i += 32 * NW) {
       const int p = i / CG, cl = i % CG;
       psm[i] = E.params[(size_t)p * E.C_pad + (size_t)cb * CG + cl];
     }
@@ -668,7 +669,7 @@ __device__ __forceinline__ void run_iteration(const TmapDesc* tmap, const EvalAr
     }
   }
   __syncthreads();
-  for (int i = tid; i < CG * W; i += kThreads) {
+  for (int i = tid; i < CG * W; i += 32 * NW) {
     const int cl = i / W, w = i % W;
     const int wcc = cl / G, g = cl % G;
     double v = 0.0;

@@ -447,14 +447,21 @@ gm_iter_grad(const __grid_constant__ gpum::TmapDesc tmap, gpum::EvalArgs E, gpum
 }
 
 #if GM_GRAD2
-// The gradient kernel with two chains per lane (64 per warp), for batches that
-// fill its eight warps.
+// The gradient kernel with two chains per lane (64 per warp): eight warps for
+// batches above 256 points, four (two CTAs per SM) for those above 32.
 extern "C" __global__ void __launch_bounds__(gpum::kThreads, 1)
 gm_iter_grad2(const __grid_constant__ gpum::TmapDesc tmap, gpum::EvalArgs E, gpum::ChainArgs A,
               int phase) {
   gpum::JitLanesG<2> body;
   gpum::run_iteration<64, 1 + GM_NP, gpum::JitLanesG<2>, gpum::JitPrior>(&tmap, E, A, phase,
                                                                           body);
+}
+extern "C" __global__ void __launch_bounds__(128, 2)
+gm_iter_grad2h(const __grid_constant__ gpum::TmapDesc tmap, gpum::EvalArgs E, gpum::ChainArgs A,
+               int phase) {
+  gpum::JitLanesG<2> body;
+  gpum::run_iteration<64, 1 + GM_NP, gpum::JitLanesG<2>, gpum::JitPrior, 4>(&tmap, E, A, phase,
+                                                                             body);
 }
 #endif
 

@@ -269,8 +269,9 @@ int jit_compile(const GenModel& gm, CompiledModel* out, std::string* err) {
     return 1;
   }
   if (jit_grad_two(gm) &&
-      cudaLibraryGetKernel(&e.model.k_grad2, e.lib, "gm_iter_grad2") != cudaSuccess) {
-    *err = "compiled model is missing its two-chain gradient kernel";
+      (cudaLibraryGetKernel(&e.model.k_grad2, e.lib, "gm_iter_grad2") != cudaSuccess ||
+       cudaLibraryGetKernel(&e.model.k_grad2h, e.lib, "gm_iter_grad2h") != cudaSuccess)) {
+    *err = "compiled model is missing its two-chain gradient kernels";
     cudaLibraryUnload(e.lib);
     return 1;
   }

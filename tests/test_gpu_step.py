@@ -64,6 +64,25 @@ def test_step_follows_the_oracle(gpu, p, n_obs, C, mode, engine):
     assert 0.0 <= acc.min() and acc.max() <= 1.0
 
 
+# The gradient kernel of four warps at the edges of its shared chains and of its
+# range; values and gradient 3, 16 and 17 wide (sums of several observation
+# blocks side by side up to 16).
+@pytest.mark.parametrize("p,n_obs,n_points", [(1, 515, 32), (1, 2049, 33), (1, 300001, 64),
+                                              (14, 515, 65), (14, 9001, 128), (14, 2049, 256),
+                                              (15, 9001, 129), (15, 70, 257)])
+def test_gradient_sums(gpu, p, n_obs, n_points):
+    w = W.make("logistic", n_obs=n_obs, p=p)
+    m = w.model
+    pts = w.truth["beta"] + np.random.default_rng(4).normal(0, 0.1, (n_points, m.n_params))
+    keep = np.unique(np.linspace(0, n_points - 1, 40).astype(int))
+    prog = (m.loglik.code, m.loglik.consts, m.n_params, w.data, m.n_cols, w.n_obs)
+    with gpu.Session(m.loglik.code, m.loglik.consts, m.prior.code, m.prior.consts, m.n_params,
+                     w.data, m.n_cols, w.n_obs) as s:
+        g = s.grad_batch(pts).reshape(n_points, -1)
+    og, oa = O.grad_abs_batch(*prog, pts[keep])
+    assert np.max(np.abs(g[keep] - og) / oa) <= 1e-5
+
+
 @pytest.mark.parametrize("n_obs,n_points", [(70, 1), (70, 593), (300001, 3), (9001, 4737)])
 @pytest.mark.parametrize("engine", [2, 0])
 def test_batch_sums(gpu, n_obs, n_points, engine):
