@@ -35,6 +35,11 @@ struct GenModel {
   // the kernel adds one control warp.
   bool tc = false;
   int tc_k = 0, tc_kp = 0, tc_ntail = 0, tc_tn = 0, tc_stages = 0, tc_warps = 8;
+  // Whether the two-chains-per-lane gradient is generated: its registers hold
+  // twice the parameters, hoisted values and their adjoints, 136 at 34, which
+  // leaves room for the loaded columns; its FP64 rows are 138 KB of shared
+  // memory at 33 parameters.
+  bool grad_two() const { return np + (n_hoist > 1 ? n_hoist : 1) <= 34; }
 };
 
 // Dynamic shared memory of the tensor-core value kernel: `stages` stages of

@@ -198,8 +198,6 @@ bool jit_value_lanes(const GenModel& gm, bool pair) {
 
 bool jit_grad_lanes(const GenModel& gm) { return gm.np + std::max(gm.n_hoist, 1) <= 100; }
 
-bool jit_grad_two(const GenModel& gm) { return gm.np + std::max(gm.n_hoist, 1) <= 34; }
-
 std::string jit_source(const GenModel& gm, int G, int GG, bool pair) {
   const bool lanes = jit_value_lanes(gm, pair);
   const bool lanes_grad = jit_grad_lanes(gm);
@@ -207,7 +205,7 @@ std::string jit_source(const GenModel& gm, int G, int GG, bool pair) {
   s += "#include \"device.cuh\"\n";
   s += "#define GM_LANES " + std::string(lanes ? "1" : "0") + "\n";
   s += "#define GM_LANESG " + std::string(lanes_grad ? "1" : "0") + "\n";
-  s += "#define GM_GRAD2 " + std::string(jit_grad_two(gm) ? "1" : "0") + "\n";
+  s += "#define GM_GRAD2 " + std::string(gm.grad_two() ? "1" : "0") + "\n";
   s += "#define GM_PAIR " + std::string(pair ? "1" : "0") + "\n";
   s += "#define GM_G " + std::to_string(G) + "\n";
   s += "#define GM_GG " + std::to_string(GG) + "\n";
@@ -215,7 +213,6 @@ std::string jit_source(const GenModel& gm, int G, int GG, bool pair) {
   // hoisted values) <= 40 broadcast pairs) fit in 80 registers without
   // spills: three CTAs, 24 warps per SM.
   const int w = gm.np + std::max(gm.n_hoist, 1);
-  // Paired gradient body of at most 25 parameters + hoisted values: two CTAs.
   s += "#define GM_GRAD_CTAS 1\n";  // the gradient bodies keep up to 255 registers
   // Chain lanes: two CTAs while parameters + hoisted values stay within 80.
   s += "#define GM_VALUE_CTAS " +
@@ -268,7 +265,7 @@ int jit_compile(const GenModel& gm, CompiledModel* out, std::string* err) {
     cudaLibraryUnload(e.lib);
     return 1;
   }
-  if (jit_grad_two(gm) &&
+  if (gm.grad_two() &&
       (cudaLibraryGetKernel(&e.model.k_grad2, e.lib, "gm_iter_grad2") != cudaSuccess ||
        cudaLibraryGetKernel(&e.model.k_grad2h, e.lib, "gm_iter_grad2h") != cudaSuccess)) {
     *err = "compiled model is missing its two-chain gradient kernels";

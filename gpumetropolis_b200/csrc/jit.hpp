@@ -50,12 +50,6 @@ bool jit_value_lanes(const GenModel& gm, bool pair);
 // ones take the scalar body (GG chains per thread, lanes over observations).
 bool jit_grad_lanes(const GenModel& gm);
 
-// Whether the two-chains-per-lane gradient kernel is built: its registers hold
-// twice the parameters, hoisted values and their adjoints, 136 at 34, which
-// leaves room for the loaded columns; its FP64 rows are 138 KB of shared memory
-// at 33 parameters.
-bool jit_grad_two(const GenModel& gm);
-
 // Returns 0 and a loaded model, or 1 with a message (NVRTC missing, compile
 // error, load error).
 int jit_compile(const GenModel& gm, CompiledModel* out, std::string* err);
