@@ -33,6 +33,7 @@ constexpr size_t kSmallPinned = 128 << 10;  // a session's block
 constexpr size_t kSmallIn = 64 << 10;       // of it, for the host's inputs
 constexpr size_t kSmallOut = kSmallPinned - kSmallIn;
 constexpr size_t kChunkPinned = 1 << 20;    // a block of a large transfer
+constexpr size_t kThreadedCopy = 4 * kChunkPinned;  // transfers moved by several threads
 constexpr int kSmallBlocks = 16, kChunkBlocks = 8;
 
 // One pinned allocation, made at the first use, in equal blocks.
@@ -160,16 +161,20 @@ inline void convert_copy(double* dst, const float* src, size_t n) {
 // n device values into pageable host memory after the work already enqueued
 // on `st` (f32 values may widen to f64 on the way, which is exact); returns
 // when they have arrived.  The calling thread keeps a ring of pinned blocks
-// filled by the copy engine and hands each to up to five threads that move
-// them on.  (Threads that each copied and moved their own blocks took 0.75 to
-// 1.5 ms for 13 MB widened to 26, this ring 0.6 to 0.7, the driver's staging of
-// the 26 MB 1.45.)
+// filled by the copy engine.  Below 4 MB it moves them on itself, in pieces of
+// 512 KB (1.5 MB widened to 3: 143 us; 1 MB pieces and two threads, whose start
+// takes as long as the copy, 290; the driver's staging of the 3 MB 187).  Above,
+// it hands blocks of 1 MB to up to five threads (4 MB to 8: 261 us, alone 360;
+// 13 MB to 26: 0.53 to 0.67 ms, alone 1.25, the driver 1.33; threads that each
+// copied and moved their own blocks 0.75 to 1.5).
 template <class To, class From>
 cudaError_t copy_to_host(To* dst, const From* src, size_t n, cudaStream_t st) {
   // The threads poll for chunks, so they start when there is something to copy.
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return e;
-  const size_t per = kChunkPinned / sizeof(From), chunks = (n + per - 1) / per;
+  const bool alone = n * sizeof(From) < kThreadedCopy;
+  const size_t per = (alone ? kChunkPinned / 2 : kChunkPinned) / sizeof(From);
+  const size_t chunks = (n + per - 1) / per;
   const size_t want = std::min<size_t>(kChunkBlocks, std::max<size_t>(chunks, 1));
   std::vector<char*> blocks;
   std::vector<cudaEvent_t> ev;
@@ -209,7 +214,7 @@ cudaError_t copy_to_host(To* dst, const From* src, size_t n, cudaStream_t st) {
     }
   };
   std::vector<std::thread> threads;
-  if (e == cudaSuccess && chunks > 1) {
+  if (e == cudaSuccess && !alone) {
     const size_t cores = std::max(1u, std::thread::hardware_concurrency() / 2);
     const size_t nt = std::min<size_t>(std::min<size_t>(5, cores), chunks);
     threads.reserve(nt);

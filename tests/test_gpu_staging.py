@@ -37,6 +37,19 @@ def test_pointwise_blocks(gpu, n_obs, n_points):
     assert np.max(np.abs(got.ravel() - ref)) <= 1e-5 * max(1.0, np.max(np.abs(ref)))
 
 
+@pytest.mark.parametrize("n_obs", [BLOCK // 2 - 1, BLOCK // 2, BLOCK // 2 + 1, 4 * BLOCK - 1,
+                                   4 * BLOCK, 4 * BLOCK + 1])
+def test_pointwise_pieces(gpu, n_obs):
+    """Half-block pieces below four blocks, whole blocks and threads from there."""
+    w = W.make("gaussian", n_obs=n_obs)
+    m = w.model
+    pts = np.array([[3.25]])
+    with _session(gpu, w) as s:
+        got = s.loglik_pointwise(pts)
+    ref = O.loglik_pointwise(m.loglik.code, m.loglik.consts, 1, w.data, 1, n_obs, pts)
+    assert np.max(np.abs(got - ref)) <= 1e-5 * max(1.0, np.max(np.abs(ref)))
+
+
 def test_pointwise_from_two_threads(gpu):
     w = W.make("gaussian", n_obs=BLOCK + 5)
     pts = np.linspace(3.0, 4.0, 12).reshape(-1, 1)
