@@ -305,8 +305,16 @@ struct JitLanesG {
   }
 
   __device__ __forceinline__ void quad(const float* xo, int nv) {
-    if constexpr (CH == 2) gm_value_grad4l2(xo, nv, p, h, gp, gh, lastv);
-    else gm_value_grad4l(xo, nv, p[0], h[0], gp[0], gh[0], lastv[0]);
+    // The data's last, partial quad: chain by chain with the one-chain form.
+    // Its adjoints carry weights, and a sum of two weighted products has two
+    // ways to become a multiply-add: the compiler chose another one in the
+    // two-chain form (a gradient 2e-6 off the one-chain kernel's).
+    if (CH == 1 || nv < 4) {
+#pragma unroll
+      for (int c = 0; c < CH; ++c) gm_value_grad4l(xo, nv, p[c], h[c], gp[c], gh[c], lastv[c]);
+    } else {
+      if constexpr (CH == 2) gm_value_grad4l2(xo, 4, p, h, gp, gh, lastv);
+    }
   }
 
   __device__ __forceinline__ void eval4(const float* xo, int nv) {

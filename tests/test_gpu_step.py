@@ -83,6 +83,22 @@ def test_gradient_sums(gpu, p, n_obs, n_points):
     assert np.max(np.abs(g[keep] - og) / oa) <= 1e-5
 
 
+# A partial quad is one warp's, however many share a chain: gradients with two
+# chains per lane equal those with one bit for bit.
+@pytest.mark.parametrize("n_obs", [1, 2, 3])
+@pytest.mark.parametrize("n_points", [60, 300])
+def test_partial_quad_of_two_chains(gpu, n_obs, n_points):
+    w = W.make("logistic", n_obs=n_obs, p=16)
+    m = w.model
+    pts = np.random.default_rng(0).normal(0, 0.5, (n_points, m.n_params))
+    with gpu.Session(m.loglik.code, m.loglik.consts, m.prior.code, m.prior.consts, m.n_params,
+                     w.data, m.n_cols, w.n_obs) as s:
+        two = s.grad_batch(pts).reshape(n_points, -1)
+        one = np.concatenate([s.grad_batch(pts[k:k + 20]).reshape(20, -1)
+                              for k in range(0, n_points, 20)])
+    assert np.array_equal(two, one)
+
+
 @pytest.mark.parametrize("n_obs,n_points", [(70, 1), (70, 593), (300001, 3), (9001, 4737)])
 @pytest.mark.parametrize("engine", [2, 0])
 def test_batch_sums(gpu, n_obs, n_points, engine):
