@@ -562,6 +562,43 @@ struct gpum_b200_session {
     return k;
   }
 
+  // Whether a chain's sums are the same, up to FP64 rounding, however its tiles
+  // are divided among observation blocks: every FP32 block of terms ends with
+  // its tile.  Not so for the chain-lane bodies where a warp's quads of a tile
+  // are odd (blocks of two quads), for the scalar bodies (blocks across tiles)
+  // and the interpreter's gradient, nor for gradients with hoisted values, whose
+  // chain rule is FP32 once per observation block.
+  bool sums_follow_tiles(const KernelChoice& k, int Tk, int WO) const {
+    if (k.grad_interp) return false;
+    if (!k.compiled || k.tc) return true;  // compensated, or FP64 per tile
+    if (k.W > 1 && gm.n_hoist > 0) return false;
+    if (k.lanes) return Tk / 4 / WO % 2 == 0;
+    return k.W == 1 && cm.pair;
+  }
+
+  // Those kernels keep the division into four waves of CTAs (for two chains per
+  // lane: of the one-chain kernel's), so that their results do not move by FP32
+  // roundings when the geometry of the others changes: 41 points x 71,864
+  // observations of the 65-parameter Student-t model differed by 8e-7.
+  void four_waves(int n, const KernelChoice& k, int Tk, Geometry& g) const {
+    int NCB = g.NCB, slots = 0, occ = 1;
+    const void* fn = k.fn;
+    size_t smem = g.smem;
+    if (k.W > 1 && k.G == 64) {
+      int WC = 1;
+      while (WC < kWarps && WC < (n + 31) / 32) WC *= 2;
+      NCB = (n + 32 * WC - 1) / (32 * WC);
+      fn = (const void*)cm.k_grad;
+      smem = skel_smem_bytes(Tk, (int)(ext(k) ? ncols_c : ncols), (int)np, 32 * WC, 32, k.W, true);
+    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, fn == k.fn ? k.threads : kThreads,
+                                                  smem);
+    slots = num_sms() * std::max(occ, 1);
+    const int nob = std::min(std::max(1, 4 * slots / NCB), std::max(1, g.ntiles));
+    g.tiles_per_cta = g.ntiles > 0 ? (g.ntiles + nob - 1) / nob : 0;
+    g.NOB = g.ntiles > 0 ? (g.ntiles + g.tiles_per_cta - 1) / g.tiles_per_cta : 1;
+  }
+
   Geometry geometry(int n, const KernelChoice& k) const {
     Geometry g{};
     g.G = k.G;
@@ -580,6 +617,10 @@ struct gpum_b200_session {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, k.threads, g.smem);
     if (occ < 1) occ = 1;
     const int slots = num_sms() * occ;
+    if (!sums_follow_tiles(k, Tk, k.threads / 32 / g.WC)) {
+      four_waves(n, k, Tk, g);
+      return g;
+    }
     // Observation blocks: up to four waves of CTAs, the count whose waves x
     // (tiles per CTA + one tile's time for a CTA's start and end) is smallest.
     // Fewer waves pay the start less often, more waves fill the last one
