@@ -1,4 +1,5 @@
-// kernels.cuh -- the interpreter engine's per-iteration kernel, and helper
+// kernels.cuh -- the interpreter engine's evaluation kernels, the sums of partials,
+// the end of a step (step_kernel), exchanges, the two-stage loop, and helper
 // kernels (data layout, points, draws layout).
 //
 // The evaluation body here is the register-stack interpreter (interp.cuh):
@@ -956,8 +957,8 @@ static __global__ void convert_rows_kernel(const double* __restrict__ src, float
 
 // f64 chain-major points [C][np] -> f32 [np][C_pad]; pad chains copy chain 0.
 // pts may be pinned host memory.
-static __global__ void points_to_params_kernel(const double* __restrict__ pts, float* __restrict__ params,
-                                        int n, int np, int C_pad) {
+static __global__ void points_to_params_kernel(const double* __restrict__ pts,
+                                        float* __restrict__ params, int n, int np, int C_pad) {
   pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np * C_pad) return;
@@ -1427,7 +1428,8 @@ static __global__ void __launch_bounds__(kScreenThreads) da_screen_kernel(ChainA
 // One warp per chain: the lanes add the chain's observation-block partials in
 // a fixed lane-strided order and a fixed shuffle tree (deterministic), lane 0
 // takes the decision, and the lanes copy, record and propose in parallel.
-static __global__ void da_finalize_kernel(ChainArgs A, DaArgs D, const double* __restrict__ partials,
+static __global__ void da_finalize_kernel(ChainArgs A, DaArgs D,
+                                          const double* __restrict__ partials,
                                           int CG, int total, int ntiles, int C_pad_eval) {
   const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
