@@ -719,7 +719,9 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
     // Exact folds of the paired code (an FFMA2, FMUL2 or FADD2 takes two issue
     // slots each; an operand that does not depend on the observation is
     // computed outside the loop):
-    //   -a * r            = a * -r (r a hoisted reciprocal; neg_fold)
+    //   -a * r            = a * -r (r a hoisted reciprocal; neg_fold), but not
+    //                       where -a is the linear predictor, whose own value
+    //                       the tensor cores compute (a is not evaluated there)
     //   a - p             = a + -p (p a parameter, hoisted value or constant;
     //                       a not a product, which the compiler would contract
     //                       with the sum into one rounding)
@@ -738,7 +740,8 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
         continue;
       const Node& x = g.n[i];
       if (recip(i) >= 0) {
-        if (is_pd(x.a) && g.n[x.a].op == O_NEG && uses[x.a] == 1 && x.a != root) {
+        if (is_pd(x.a) && g.n[x.a].op == O_NEG && uses[x.a] == 1 && x.a != root &&
+            x.a != tc_root) {
           neg_fold[i] = 1;
           fold_skip[x.a] = 1;
         }
@@ -795,9 +798,10 @@ int generate_model(const uint32_t* code, size_t n_code, const double* consts,
     const std::string root2 = root < 0 ? std::string("gm2(0.0f)") : ref2(root);
     s << "  (void)d; (void)pp; (void)hh;\n  return " << root2 << ";\n}\n";
 
-    // The tensor-core value path.  A linear predictor that is itself a
-    // product folded into an FFMA2 of its consumer keeps the FP32 path.
-    if (tc_root >= 0 && fused[tc_root]) tc_root = -1;
+    // The tensor-core value path.  A linear predictor that is itself folded
+    // into its consumer (a product into an FFMA2, say), whose expression then
+    // names the nodes under it, keeps the FP32 path.
+    if (tc_root >= 0 && !value_node(tc_root)) tc_root = -1;
     if (tc_root >= 0) {
       // gm_tc_tail2: the paired value with the linear predictor's pair `eta`;
       // t[k] = the k-th data column the tail reads (gm_tc_tailvals).
