@@ -125,13 +125,6 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Static shared memory of a kernel (the interpreter's operand scratch): with
-// it, a dynamic request below 48 KB can still need the opt-in attribute.
-size_t static_smem(const void* fn) {
-  cudaFuncAttributes fa{};
-  return cudaFuncGetAttributes(&fa, fn) == cudaSuccess ? fa.sharedSizeBytes : 0;
-}
-
 // Interpreter variants by peak stack depth: registers go to depth or to
 // chains per thread.
 enum Variant { V8x8 = 0, V4x16 = 1, V2x32 = 2, V16x6 = 3 };
@@ -662,9 +655,7 @@ struct gpum_b200_session {
       set_n = -1;  // unless all of it succeeds
       kc = choose(n, need_grad, pointwise);
       geo = geometry(n, kc);
-      if (geo.smem + static_smem(kc.fn) > 48 * 1024)
-        GPUM_CK(cudaFuncSetAttribute(kc.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)geo.smem));
+      GPUM_CK(allow_shared_memory(kc.fn, geo.smem));
       set_n = n;
       set_grad = need_grad;
       set_pw = pointwise;
@@ -758,9 +749,7 @@ struct gpum_b200_session {
     while (S.wpb > S.wpc && bytes() > kMax) S.wpb /= 2;
     step_smem = bytes();
     step_fn = side_draws() ? (const void*)step_kernel<false> : (const void*)step_kernel<true>;
-    if (step_smem > 48 * 1024)
-      GPUM_CK(cudaFuncSetAttribute(step_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)step_smem));
+    GPUM_CK(allow_shared_memory(step_fn, step_smem));
   }
 
   // The end of a step, after its evaluation has been launched.
@@ -2098,9 +2087,7 @@ int gpum_b200_session_train_surrogate(gpum_b200_session* s, gpum_b200_mlp* m,
     const uint32_t nchunk = std::max<uint32_t>(1, std::min<uint32_t>(64, n_tr / 2048));
     const uint32_t chunk = (n_tr + nchunk - 1) / nchunk;
     const size_t msmem = (size_t)kMomRows * (d + 1) * sizeof(double);
-    if (msmem > 48 * 1024)
-      GPUM_CK(cudaFuncSetAttribute(pairs_moments_kernel,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem));
+    GPUM_CK(allow_shared_memory((const void*)pairs_moments_kernel, msmem));
     DBuf<double> part;
     part.ensure((size_t)nchunk * NA);
     pairs_moments_kernel<<<dim3(nchunk, (NA + 255) / 256), 256, msmem, st>>>(

@@ -100,6 +100,24 @@ inline cudaError_t launch_dependent(const void* fn, dim3 grid, dim3 block, void*
   cfg.numAttrs = 1;
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
+
+// Lets kernel `fn` be launched with `smem` bytes of dynamic shared memory.  The
+// limit belongs to the kernel on its device, and sessions and threads share
+// kernels whose launches need different sizes: it is raised to all that the
+// device has, never set to one launch's size, which another's would exceed.
+inline cudaError_t allow_shared_memory(const void* fn, size_t smem) {
+  cudaFuncAttributes fa{};
+  cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+  if (e != cudaSuccess || smem <= (size_t)fa.maxDynamicSharedSizeBytes) return e;
+  int dev = 0, most = 0;
+  e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess) return e;
+  most -= (int)fa.sharedSizeBytes;
+  if (smem > (size_t)most) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
 #endif
 
 // Nanosecond clock of the GPU, for waits bounded in time as well as polls.

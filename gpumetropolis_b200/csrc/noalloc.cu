@@ -179,12 +179,7 @@ extern "C" int gpum_b200_loglik_batch_noalloc(
   int occ = 1, sms = 148, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaFuncAttributes fa{};  // the interpreter's static operand scratch counts too
-  if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess)
-    return fail(err, err_len, GPUM_ERR_CUDA, "cudaFuncGetAttributes failed");
-  if (smem + fa.sharedSizeBytes > 48 * 1024 &&
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess)
+  if (allow_shared_memory(fn, smem) != cudaSuccess)
     return fail(err, err_len, GPUM_ERR_UNSUPPORTED, "shared memory request refused");
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kThreads, smem);
   occ = std::max(occ, 1);

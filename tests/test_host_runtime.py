@@ -1,0 +1,102 @@
+"""The library's host code against a CUDA runtime that checks it (fake_cudart.c,
+preloaded into a process of its own): no GPU, kernels do nothing, and what the
+host asks for is refused or noted where the real runtime would refuse it or
+where it would be wrong on a machine this suite does not have."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from gpumetropolis_b200.build import build, nvcc
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+PREAMBLE = """
+import ctypes, os
+import numpy as np
+from gpumetropolis_b200 import _native, workloads as W
+rt = ctypes.CDLL(os.environ["LD_PRELOAD"])
+rt.fake_log.restype = ctypes.c_char_p
+rt.fake_pending.restype = ctypes.c_long
+for f in (rt.fake_largest_block, rt.fake_live_bytes):
+    f.restype = ctypes.c_size_t
+rt.fake_block.restype = ctypes.c_void_p
+rt.fake_block.argtypes = [ctypes.c_size_t]
+def log():
+    return rt.fake_log().decode().splitlines()
+def wrong():
+    return [l for l in log() if l.startswith("VIOLATION")]
+def session(p=16, n_obs=1031, engine=0):
+    w = W.make("logistic", n_obs=n_obs, p=p)
+    m = w.model
+    return _native.Session(m.loglik.code, m.loglik.consts, m.prior.code, m.prior.consts,
+                           m.n_params, w.data, m.n_cols, w.n_obs, engine=engine)
+def start(d, C, n_iter, mode=0):
+    L = np.tile(0.1 * np.eye(d), (C, 1, 1)) if mode == 2 else None
+    return np.zeros((C, d)), np.full((C, d), 0.1), np.ones(C), n_iter, 1, mode, 0.0, 0.0, L
+"""
+
+
+@pytest.fixture(scope="module")
+def runtime(tmp_path_factory):
+    lib = str(tmp_path_factory.mktemp("rt") / "fake_cudart.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(nvcc())), "include")
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-I", include,
+                    os.path.join(ROOT, "tests", "fake_cudart.c"), "-o", lib], check=True)
+    build()
+
+    def go(text):
+        env = dict(os.environ, LD_PRELOAD=lib)
+        r = subprocess.run([sys.executable, "-c", PREAMBLE + text], cwd=ROOT, env=env,
+                           capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+    return go
+
+
+def test_shared_memory_limits_of_two_sessions(runtime):
+    runtime("""
+a, b = session(), session()
+a.loglik_batch(np.zeros((512, 17)))
+b.loglik_batch(np.zeros((10, 17)))
+a.loglik_batch(np.zeros((512, 17)))
+""")
+
+
+def test_shared_memory_limits_of_two_prepared_runs(runtime):
+    runtime("""
+a, b = session(p=64), session(p=54)
+a.prepare(*start(65, 594, 6, 2))
+b.prepare(*start(55, 594, 6, 2))
+a.advance(6)
+b.advance(6)
+""")
+
+
+def test_shared_memory_limits_beside_the_no_allocation_entry(runtime):
+    # the eight-chain interpreter kernel, of programs that keep seven values
+    runtime("""
+from gpumetropolis_b200.dsl import gpum_model
+X = [f"x{j}" for j in range(16)]
+B = [f"b{j}" for j in range(16)]
+text = "~ " + "+(".join(f"b{j} * x{j}" for j in range(7)) + ")" * 6
+text += " + " + " + ".join(f"{b} * {x}" for b, x in zip(B[7:], X[7:]))
+m = gpum_model(text, params=B, data=X)
+data = np.zeros((4096, 16))
+s = _native.Session(m.loglik.code, m.loglik.consts, m.prior.code, m.prior.consts, 16, data, 16,
+                    4096, engine=0)
+s.loglik_batch(np.zeros((512, 16)))
+lib = s._lib
+cols, pts, out = np.zeros((16, 4096), np.float32), np.zeros((1, 16)), np.zeros(1)
+cols = cols.ravel()[(-cols.ctypes.data // 4) % 4:]
+code = np.ascontiguousarray(m.loglik.code, np.uint32)
+consts = np.ascontiguousarray(m.loglik.consts, np.float64)
+st, err = ctypes.c_void_p(s.stream), ctypes.create_string_buffer(256)
+rc = lib.gpum_b200_loglik_batch_noalloc(
+    code.ctypes.data_as(ctypes.POINTER(ctypes.c_uint32)), code.size,
+    consts.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), consts.size, 16,
+    ctypes.c_void_p(cols.ctypes.data), 4096, 16, 4096, ctypes.c_void_p(pts.ctypes.data), 1,
+    ctypes.c_void_p(out.ctypes.data), st, err, 256)
+assert rc == 0, err.value
+s.loglik_batch(np.zeros((512, 16)))
+""")
