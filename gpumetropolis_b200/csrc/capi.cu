@@ -177,6 +177,16 @@ int num_sms() {
   return n;
 }
 
+// CTAs of a kernel resident on an SM, at least 1.  The runtime reports none for
+// more shared memory than the kernel is allowed so far, so that comes first: a
+// kernel's first evaluation in a process has the geometry of every later one.
+int resident(const void* fn, int threads, size_t smem) {
+  int occ = 1;
+  GPUM_CK(allow_shared_memory(fn, smem));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem);
+  return std::max(occ, 1);
+}
+
 // Which kernel evaluates the current run or batch.
 struct KernelChoice {
   bool compiled = false;
@@ -574,7 +584,7 @@ struct gpum_b200_session {
   // roundings when the geometry of the others changes: 41 points x 71,864
   // observations of the 65-parameter Student-t model differed by 8e-7.
   void four_waves(int n, const KernelChoice& k, int Tk, Geometry& g) const {
-    int NCB = g.NCB, slots = 0, occ = 1;
+    int NCB = g.NCB;
     const void* fn = k.fn;
     size_t smem = g.smem;
     if (k.W > 1 && k.G == 64) {
@@ -584,9 +594,7 @@ struct gpum_b200_session {
       fn = (const void*)cm.k_grad;
       smem = skel_smem_bytes(Tk, (int)(ext(k) ? ncols_c : ncols), (int)np, 32 * WC, 32, k.W, true);
     }
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, fn == k.fn ? k.threads : kThreads,
-                                                  smem);
-    slots = num_sms() * std::max(occ, 1);
+    const int slots = num_sms() * resident(fn, fn == k.fn ? k.threads : kThreads, smem);
     const int nob = std::min(std::max(1, 4 * slots / NCB), std::max(1, g.ntiles));
     g.tiles_per_cta = g.ntiles > 0 ? (g.ntiles + nob - 1) / nob : 0;
     g.NOB = g.ntiles > 0 ? (g.ntiles + g.tiles_per_cta - 1) / g.tiles_per_cta : 1;
@@ -606,10 +614,7 @@ struct gpum_b200_session {
     g.smem = k.tc ? tc_smem_bytes(cm.tc_kp, cm.tc_ntail, cm.tc_tn, cm.tc_stages)
                   : skel_smem_bytes(Tk, (int)(ext(k) ? ncols_c : ncols), (int)np, g.CG, g.G,
                                     k.W, k.lanes, k.threads / 32);
-    int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, k.threads, g.smem);
-    if (occ < 1) occ = 1;
-    const int slots = num_sms() * occ;
+    const int slots = num_sms() * resident(k.fn, k.threads, g.smem);
     if (!sums_follow_tiles(k, Tk, k.threads / 32 / g.WC)) {
       four_waves(n, k, Tk, g);
       return g;
@@ -655,7 +660,6 @@ struct gpum_b200_session {
       set_n = -1;  // unless all of it succeeds
       kc = choose(n, need_grad, pointwise);
       geo = geometry(n, kc);
-      GPUM_CK(allow_shared_memory(kc.fn, geo.smem));
       set_n = n;
       set_grad = need_grad;
       set_pw = pointwise;
@@ -1404,11 +1408,9 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
   // device (da_obs_blocks).
   s->geo_da = g;
   {
-    int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, s->kc.fn, s->kc.threads, g.smem);
     // one wave of resident CTAs: with few survivors each CTA then takes many
     // tiles, so the per-CTA set-up is paid once per SM slot
-    s->geo_da.NCB = std::max(num_sms() * std::max(occ, 1), g.NCB);
+    s->geo_da.NCB = std::max(num_sms() * resident(s->kc.fn, s->kc.threads, g.smem), g.NCB);
     s->geo_da.NOB = 1;
   }
   const int max_nob = std::max(1, std::min(s->geo_da.NCB, std::max(g.ntiles, 1)));

@@ -100,3 +100,15 @@ rc = lib.gpum_b200_loglik_batch_noalloc(
 assert rc == 0, err.value
 s.loglik_batch(np.zeros((512, 16)))
 """)
+
+
+def test_first_evaluation_has_the_geometry_of_later_ones(runtime):
+    # 72 KB a CTA with the static part: three fit an SM, none before the limit is raised
+    runtime("""
+def grids(s):
+    rt.fake_clear()
+    s.loglik_batch(np.zeros((512, 17)))
+    return [l for l in log() if l.startswith("launch")]
+first = grids(session(n_obs=300001))
+assert first == grids(session(n_obs=300001)), first
+""")
