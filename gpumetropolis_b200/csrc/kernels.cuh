@@ -922,7 +922,9 @@ step_kernel(ChainArgs A, StepArgs S) {
   double lu = 0.0;
   const double *z = tmp + 2 * np, *inc = tmp + 3 * np;
   if constexpr (kDraw) {
-    if (L && S.stage_L) __syncthreads();  // the factors are staged
+    // The factors are staged.  A.L, not L: groups past the last chain have none,
+    // and every warp of the block takes the same barriers.
+    if (A.L && S.stage_L) __syncthreads();
     if (first) lu = draw_warp(A, c, step, A.iter[c], L, ldL, tmp + 2 * np, tmp + 3 * np, lane);
   } else if (first && !narrow) {
     const size_t o = (size_t)c * np;
