@@ -1,5 +1,5 @@
 """A block-wide barrier under a condition needs one that every thread of the
-block decides alike: made of the kernel's arguments (A., E., S., D., apply) alone."""
+block decides alike: made of the kernel's arguments (A., E., S., D., g., apply) alone."""
 import glob
 import os
 import re
@@ -15,5 +15,5 @@ def test_conditional_barriers_depend_on_arguments_only():
         for cond in re.findall(r"\bif\s*\(([^;{}]*?)\)\s*\{?\s*__syncthreads\b", text):
             seen += 1
             names = re.findall(r"[A-Za-z_]\w*(?:\.\w+)*", cond)
-            assert all(re.fullmatch(r"[AESD]\.\w+|apply", n) for n in names), (path, cond)
+            assert all(re.fullmatch(r"[AESDg]\.\w+|apply", n) for n in names), (path, cond)
     assert seen
