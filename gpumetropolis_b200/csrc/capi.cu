@@ -79,20 +79,23 @@ template <class T>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
-  void ensure(size_t count) {
+  DevMem mem;  // nothing for a part of a slab
+  bool own = true;
+  // Room for `count` elements, for the owner of stream `st`.
+  void ensure(size_t count, cudaStream_t st) {
     if (count <= n && p) return;
     release();
     if (count == 0) count = 1;
-    GPUM_CK(dev_alloc((void**)&p, count * sizeof(T)));
+    GPUM_CK(dev_alloc(&mem, count * sizeof(T), st));
+    p = static_cast<T*>(mem.p);
     n = count;
   }
   void release() {
-    if (p && own) dev_free(p, n * sizeof(T));
+    dev_free(&mem);
     p = nullptr;
     n = 0;
     own = true;
   }
-  bool own = true;
   // `count` elements of the slab at *at (nullptr: only the size), advancing it.
   void carve(char* slab, size_t* at, size_t count) {
     if (slab) {
@@ -225,6 +228,7 @@ void encode_cols_tmap(float* base, uint64_t n_obs, uint32_t n_cols, int64_t ld, 
 }
 
 struct gpum_b200_session {
+  OwnedStream owned;  // first: every buffer below goes back on it
   cudaStream_t stream = nullptr;
   UProg ll;
   std::unique_ptr<EvalProg> prog;
@@ -330,10 +334,7 @@ struct gpum_b200_session {
   ~gpum_b200_session() {
     drop_graph();
     if (pin_read) cudaEventDestroy(pin_read);
-    if (stream) {
-      cudaStreamSynchronize(stream);  // before the pinned block goes back
-      cudaStreamDestroy(stream);
-    }
+    if (stream) cudaStreamSynchronize(stream);  // before the pinned block goes back
     pinned_small().give(pin);
   }
 
@@ -410,7 +411,7 @@ struct gpum_b200_session {
         else if (!b->own) b->release();  // of a slab that may be gone
       }
       if (base) return;
-      slab.ensure(at);
+      slab.ensure(at, stream);
       base = slab.p;
     }
   }
@@ -453,8 +454,8 @@ struct gpum_b200_session {
     const long long tn = cm.tc_tn;
     long long ntl = (long long)((n_obs + (uint64_t)tn - 1) / (uint64_t)tn);
     const size_t stage = (size_t)(2 * cm.tc_kp + cm.tc_ntail) * (size_t)tn;
-    tc_data.ensure(stage * (size_t)ntl);
-    tc_flag.ensure(1);
+    tc_data.ensure(stage * (size_t)ntl, stream);
+    tc_flag.ensure(1, stream);
     GPUM_CK(cudaMemsetAsync(tc_flag.p, 0, sizeof(uint32_t), stream));
     const float* cols = cm.n_mat > 0 ? data_c.p : data.p;
     long long nobs = (long long)n_obs, lld = (long long)ld;
@@ -478,7 +479,7 @@ struct gpum_b200_session {
   void materialize() {
     ncols_c = ncols + (uint32_t)cm.n_mat;
     T_c = tile_obs(ncols_c);
-    data_c.ensure((size_t)ld * ncols_c);
+    data_c.ensure((size_t)ld * ncols_c, stream);
     GPUM_CK(cudaMemcpyAsync(data_c.p, data.p, sizeof(float) * (size_t)ld * ncols,
                             cudaMemcpyDeviceToDevice, stream));
     float* cols = data_c.p;
@@ -664,8 +665,8 @@ struct gpum_b200_session {
       set_grad = need_grad;
       set_pw = pointwise;
     }
-    params.ensure((size_t)np * geo.C_pad);
-    partials.ensure((size_t)geo.NOB * geo.C_pad * kc.W);
+    params.ensure((size_t)np * geo.C_pad, stream);
+    partials.ensure((size_t)geo.NOB * geo.C_pad * kc.W, stream);
     E = EvalArgs{};
     E.n_obs = (int)n_obs;
     E.ncols = (int)(ext(kc) ? ncols_c : ncols);
@@ -691,7 +692,7 @@ struct gpum_b200_session {
       std::memcpy(in, pts, bytes);
       src = in;
     } else {
-      points.ensure((size_t)n * np);
+      points.ensure((size_t)n * np, stream);
       GPUM_CK(cudaMemcpyAsync(points.p, pts, bytes, cudaMemcpyHostToDevice, stream));
       src = points.p;
     }
@@ -939,13 +940,14 @@ gpum_b200_session* create_session(const uint32_t* code, size_t n_code, const dou
   s->prior_code.assign(prior_code, prior_code + n_prior);
   s->prior_consts.assign(prior_consts, prior_consts + n_prior_consts);
 
-  GPUM_CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+  GPUM_CK(cudaStreamCreateWithFlags(&s->owned.s, cudaStreamNonBlocking));
+  s->stream = s->owned.s;
   GPUM_CK(cudaEventCreateWithFlags(&s->pin_read, cudaEventDisableTiming));
   s->pin = pinned_small().take();
-  s->d_err.ensure(1);
+  s->d_err.ensure(1, s->stream);
   GPUM_CK(cudaMemsetAsync(s->d_err.p, 0, sizeof(uint32_t), s->stream));
-  s->d_prior_code.ensure(std::max<size_t>(n_prior, 2));
-  s->d_prior_consts.ensure(std::max<size_t>(n_prior_consts, 1));
+  s->d_prior_code.ensure(std::max<size_t>(n_prior, 2), s->stream);
+  s->d_prior_consts.ensure(std::max<size_t>(n_prior_consts, 1), s->stream);
   if (n_prior)
     GPUM_CK(cudaMemcpyAsync(s->d_prior_code.p, prior_code, n_prior * sizeof(uint32_t),
                             cudaMemcpyHostToDevice, s->stream));
@@ -965,13 +967,13 @@ gpum_b200_session* create_session(const uint32_t* code, size_t n_code, const dou
     // Column-major f32 in HBM: each column contiguous, leading dimension
     // padded to 4 floats so every TMA row stride is a multiple of 16 bytes.
     s->ld = (int64_t)((n_obs + 3) & ~3ull);
-    s->data.ensure((size_t)s->ld * n_cols);
+    s->data.ensure((size_t)s->ld * n_cols, s->stream);
     // f64 rows through a 16 MB staging buffer (2M values per chunk; the
     // copy of a chunk follows the conversion of the previous one on the
     // stream), so a session does not allocate a second full copy.
     const int64_t rows_per_chunk = std::max<int64_t>(1, (int64_t)(2u << 20) / n_cols);
     DBuf<double> stage;
-    stage.ensure((size_t)std::min<int64_t>(rows_per_chunk, (int64_t)n_obs) * n_cols);
+    stage.ensure((size_t)std::min<int64_t>(rows_per_chunk, (int64_t)n_obs) * n_cols, s->stream);
     for (int64_t r0 = 0; r0 < (int64_t)n_obs; r0 += rows_per_chunk) {
       const int64_t nr = std::min<int64_t>(rows_per_chunk, (int64_t)n_obs - r0);
       GPUM_CK(cudaMemcpyAsync(stage.p, data + r0 * n_cols, sizeof(double) * nr * n_cols,
@@ -1015,12 +1017,12 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
   s->setup_eval((int)C, mala);
   const Geometry& g = s->geo;
   s->run_arrays(C, mala);
-  s->draws.ensure(std::max<size_t>(1, (size_t)max_iter * np * g.C_pad));
-  if (use_L) s->L.ensure((size_t)C * np * np);
+  s->draws.ensure(std::max<size_t>(1, (size_t)max_iter * np * g.C_pad), s->stream);
+  if (use_L) s->L.ensure((size_t)C * np * np, s->stream);
   if (mala && !s->kc.compiled) {  // the interpreted prior's gradient tape
     const size_t npr = std::max<size_t>(s->prior_code.size() / 2, 1);
-    s->ptape.ensure((size_t)C * 2 * npr);
-    s->ptape_i.ensure((size_t)C * 2 * npr);
+    s->ptape.ensure((size_t)C * 2 * npr, s->stream);
+    s->ptape_i.ensure((size_t)C * 2 * npr, s->stream);
   }
   cudaStream_t st = s->stream;
   if (use_L)
@@ -1077,9 +1079,9 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
     require(C % (uint32_t)s->pt_K == 0,
             "n_chains must be a multiple of the ladder length for device exchanges");
     require(mode != 4, "device exchanges are not available with de_sync");
-    s->pt_att.ensure(C);
-    s->pt_acc.ensure(C);
-    s->pt_n.ensure(1);
+    s->pt_att.ensure(C, s->stream);
+    s->pt_acc.ensure(C, s->stream);
+    s->pt_n.ensure(1, s->stream);
   }
   if (s->rec_cap > 0) {
     A.rec_theta = s->rec_theta.p;
@@ -1190,7 +1192,7 @@ void fetch(gpum_b200_session* s, float* out_draws, float* out_accept, double* ou
   if (out_last)
     GPUM_CK(cudaMemcpyAsync(last, s->cur.p, sizeof(double) * C, cudaMemcpyDeviceToHost, st));
   if (out_draws && n > 0) {
-    s->draws_out.ensure((size_t)n * C * np);
+    s->draws_out.ensure((size_t)n * C * np, s->stream);
     dim3 grid((C + 31) / 32, (n + 31) / 32, (unsigned)np);
     draws_layout_kernel<<<grid, dim3(32, 8), 0, st>>>(s->draws.p, s->draws_out.p, (int)n,
                                                       (int)np, C, s->geo.C_pad);
@@ -1240,7 +1242,7 @@ void batch(gpum_b200_session* s, const double* pts, size_t n_points, double* out
       // f32 on the device and over the bus, as they are computed; widened by
       // the host threads that copy them out.
       const size_t nv = (size_t)n * s->n_obs;
-      s->pointwise.ensure(nv);
+      s->pointwise.ensure(nv, s->stream);
       s->E.pointwise = s->pointwise.p;
       if (s->ll.empty()) {
         GPUM_CK(cudaMemsetAsync(s->pointwise.p, 0, sizeof(float) * nv, s->stream));
@@ -1281,7 +1283,7 @@ void batch(gpum_b200_session* s, const double* pts, size_t n_points, double* out
         s->report_device_error(*reinterpret_cast<volatile uint32_t*>(r));
         std::memcpy(out + p0 * width, r + 8, nv * sizeof(double));
       } else {
-        s->out64.ensure(nv);
+        s->out64.ensure(nv, s->stream);
         s->reduce(n, W, w0, s->out64.p, nullptr);
         s->result_to_host(out + p0 * width, s->out64.p, nv);
         s->check_device_error();
@@ -1378,14 +1380,16 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
   s->rec_cap = keep_cap;
   const int np = (int)s->np;
   cudaStream_t st = s->stream;
+  WaitAtExit wait{st};  // the surrogate's memory
   const Geometry& g = s->geo;
   if (lang) {
-    for (auto* b : {&s->gx, &s->gy, &s->mx, &s->my, &s->vbuf, &s->da_gs}) b->ensure((size_t)C * np);
+    for (auto* b : {&s->gx, &s->gy, &s->mx, &s->my, &s->vbuf, &s->da_gs})
+      b->ensure((size_t)C * np, s->stream);
     const size_t nt = (size_t)C * std::max<size_t>(s->prior_code.size() / 2, 1);
-    s->da_tvals.ensure(nt);
-    s->da_tadj.ensure(nt);
-    s->da_tlhs.ensure(nt);
-    s->da_trhs.ensure(nt);
+    s->da_tvals.ensure(nt, s->stream);
+    s->da_tadj.ensure(nt, s->stream);
+    s->da_tlhs.ensure(nt, s->stream);
+    s->da_trhs.ensure(nt, s->stream);
     s->A.mode = MODE_MALA;
     s->A.gx = s->gx.p;
     s->A.gy = s->gy.p;
@@ -1393,15 +1397,15 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
     s->A.my = s->my.p;
     s->A.vbuf = s->vbuf.p;
   }
-  s->sll_x.ensure(C);
-  s->sll_y.ensure(C);
-  s->prior_x.ensure(C);
-  s->prior_y.ensure(C);
-  s->da_flag.ensure(C);
-  s->da_slot.ensure(C);
-  s->da_stage1.ensure(C);
-  s->da_active.ensure(1);
-  s->da_params.ensure((size_t)np * g.C_pad);
+  s->sll_x.ensure(C, s->stream);
+  s->sll_y.ensure(C, s->stream);
+  s->prior_x.ensure(C, s->stream);
+  s->prior_y.ensure(C, s->stream);
+  s->da_flag.ensure(C, s->stream);
+  s->da_slot.ensure(C, s->stream);
+  s->da_stage1.ensure(C, s->stream);
+  s->da_active.ensure(1, s->stream);
+  s->da_params.ensure((size_t)np * g.C_pad, s->stream);
   // The exact evaluation runs a fixed 1-D grid of one CTA per resident slot
   // (at least one per chain block); the kernel splits it into (live chain
   // blocks x observation blocks) from the stage-1 survivor count on the
@@ -1414,7 +1418,7 @@ void run_da(gpum_b200_session* s, gpum_b200_mlp* mlp, const double* init, const 
     s->geo_da.NOB = 1;
   }
   const int max_nob = std::max(1, std::min(s->geo_da.NCB, std::max(g.ntiles, 1)));
-  s->da_partials.ensure((size_t)max_nob * s->geo_da.C_pad);
+  s->da_partials.ensure((size_t)max_nob * s->geo_da.C_pad, s->stream);
   GPUM_CK(cudaMemsetAsync(s->da_params.p, 0, sizeof(float) * np * g.C_pad, st));
   s->E_da = s->E;
   s->E_da.side_rows = 0;  // the loop's own kernels compute priors and draws
@@ -1784,7 +1788,7 @@ int gpum_b200_session_draw_moments(gpum_b200_session* s, uint32_t t0, uint32_t n
     require(chain_mean && chain_m2 && pool_mean && pool_m2, "output pointers are NULL");
     const int C = s->n_chains, np = (int)s->np;
     cudaStream_t st = s->stream;
-    s->mom.ensure((size_t)2 * C * np + np + (size_t)np * np);
+    s->mom.ensure((size_t)2 * C * np + np + (size_t)np * np, s->stream);
     double* dmean = s->mom.p;
     double* dm2 = dmean + (size_t)C * np;
     double* pmean = dm2 + (size_t)C * np;
@@ -1844,7 +1848,7 @@ int gpum_b200_session_set_likelihood_powers(gpum_b200_session* s, const double* 
     for (size_t c = 0; c < n_chains; ++c)
       require(std::isfinite(beta[c]) && beta[c] >= 0.0,
               "likelihood powers must be finite and non-negative");
-    s->beta.ensure(n_chains);
+    s->beta.ensure(n_chains, s->stream);
     GPUM_CK(cudaMemcpyAsync(s->beta.p, beta, sizeof(double) * n_chains, cudaMemcpyHostToDevice,
                             s->stream));
     GPUM_CK(cudaStreamSynchronize(s->stream));
@@ -1867,8 +1871,8 @@ int gpum_b200_session_record(gpum_b200_session* s, uint64_t capacity, char* err,
       s->rec_ll.release();
       return;
     }
-    s->rec_theta.ensure((size_t)capacity * s->np);
-    s->rec_ll.ensure((size_t)capacity);
+    s->rec_theta.ensure((size_t)capacity * s->np, s->stream);
+    s->rec_ll.ensure((size_t)capacity, s->stream);
   });
 }
 
@@ -2062,9 +2066,10 @@ int gpum_b200_session_train_surrogate(gpum_b200_session* s, gpum_b200_mlp* m,
     const int d = (int)s->np;
     s->check_device_error();
     cudaStream_t st = s->stream;
+    WaitAtExit wait{st};  // the surrogate's memory
     DBuf<uint32_t> pos, counts;
-    pos.ensure(n);
-    counts.ensure(2);
+    pos.ensure(n, s->stream);
+    counts.ensure(2, s->stream);
     pairs_split_kernel<<<1, kSplitThreads, 0, st>>>(s->rec_theta.p, s->rec_ll.p, n, d,
                                                     holdout_every, pos.p, counts.p);
     GPUM_CK(cudaGetLastError());
@@ -2075,10 +2080,10 @@ int gpum_b200_session_train_surrogate(gpum_b200_session* s, gpum_b200_mlp* m,
     require(n_tr >= 2, "fewer than two finite training pairs");
     DBuf<float> tr_th;
     DBuf<double> tr_ll, ho_th, ho_ll;
-    tr_th.ensure((size_t)n_tr * d);
-    tr_ll.ensure(n_tr);
-    ho_th.ensure((size_t)std::max<uint32_t>(n_ho, 1) * d);
-    ho_ll.ensure(std::max<uint32_t>(n_ho, 1));
+    tr_th.ensure((size_t)n_tr * d, s->stream);
+    tr_ll.ensure(n_tr, s->stream);
+    ho_th.ensure((size_t)std::max<uint32_t>(n_ho, 1) * d, s->stream);
+    ho_ll.ensure(std::max<uint32_t>(n_ho, 1), s->stream);
     pairs_scatter_kernel<<<(n + 255) / 256, 256, 0, st>>>(s->rec_theta.p, s->rec_ll.p, n, d,
                                                            pos.p, tr_th.p, tr_ll.p, ho_th.p,
                                                            ho_ll.p);
@@ -2091,7 +2096,7 @@ int gpum_b200_session_train_surrogate(gpum_b200_session* s, gpum_b200_mlp* m,
     const size_t msmem = (size_t)kMomRows * (d + 1) * sizeof(double);
     GPUM_CK(allow_shared_memory((const void*)pairs_moments_kernel, msmem));
     DBuf<double> part;
-    part.ensure((size_t)nchunk * NA);
+    part.ensure((size_t)nchunk * NA, s->stream);
     pairs_moments_kernel<<<dim3(nchunk, (NA + 255) / 256), 256, msmem, st>>>(
         tr_th.p, tr_ll.p, n_tr, d, chunk, part.p);
     GPUM_CK(cudaGetLastError());
@@ -2151,7 +2156,7 @@ int gpum_b200_session_train_surrogate(gpum_b200_session* s, gpum_b200_mlp* m,
     double resid_sd = std::nan("");
     if (n_ho > 0) {  // residual spread of the trained network on the held-out pairs
       DBuf<double> pred;
-      pred.ensure(n_ho);
+      pred.ensure(n_ho, s->stream);
       rc = mlp_infer(m, ho_th.p, (int)n_ho, d, pred.p, st, &e, false);
       if (rc != GPUM_OK) throw Failure{rc, e};
       std::vector<double> hpred(n_ho), hll(n_ho);

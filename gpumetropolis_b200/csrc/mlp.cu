@@ -62,14 +62,19 @@ template <class T>
 struct Buf {
   T* p = nullptr;
   size_t n = 0;
-  static size_t bytes(size_t count) { return std::max<size_t>(count, 1) * sizeof(T); }
-  void alloc(size_t count) {
-    dev_free(p, bytes(n));
+  DevMem mem;
+  // `count` elements, for the owner of stream `st`.
+  void alloc(size_t count, cudaStream_t st) {
+    dev_free(&mem);
     p = nullptr;
-    MLP_CK(dev_alloc((void**)&p, bytes(count)));
+    MLP_CK(dev_alloc(&mem, std::max<size_t>(count, 1) * sizeof(T), st));
+    p = static_cast<T*>(mem.p);
     n = count;
   }
-  ~Buf() { dev_free(p, bytes(n)); }
+  Buf() = default;
+  Buf(const Buf&) = delete;
+  Buf& operator=(const Buf&) = delete;
+  ~Buf() { dev_free(&mem); }
 };
 
 // ----------------------------------------------------------------- kernels
@@ -592,6 +597,7 @@ struct gpum_b200_mlp {
   int d = 0, dp = 0, H = 0, B = 0;
   uint32_t seed = 0;
   uint32_t steps_done = 0;  // host mirror of the device step counter
+  OwnedStream owned, owned2;  // before the buffers, which go back on the first
   cudaStream_t st = nullptr;
   // second stream and events: the dW2 GEMM runs beside the dZ1 -> dW1 chain
   cudaStream_t st2 = nullptr;
@@ -632,11 +638,10 @@ struct gpum_b200_mlp {
   bool fused_inference() const { return dp == 64 && (H == 128 || H == 256); }
 
   ~gpum_b200_mlp() {
+    if (st) cudaStreamSynchronize(st);
     if (st2) cudaStreamSynchronize(st2);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
-    if (st2) cudaStreamDestroy(st2);
-    if (st) cudaStreamDestroy(st);
   }
 
   // `pdl`: may start while the kernel before it in the stream runs.
@@ -811,8 +816,8 @@ void upload_pairs(gpum_b200_mlp* m, const double* theta, const double* ll, size_
                   Buf<float>& dth, Buf<double>& dll) {
   const size_t total = n * m->d, per = std::min<size_t>(total, (size_t)2 << 20);
   Buf<double> stage;
-  stage.alloc(per);
-  dth.alloc(total);
+  stage.alloc(per, m->st);
+  dth.alloc(total, m->st);
   for (size_t at = 0; at < total; at += per) {
     const size_t k = std::min(per, total - at);
     MLP_CK(cudaMemcpyAsync(stage.p, theta + at, k * sizeof(double), cudaMemcpyHostToDevice,
@@ -821,7 +826,7 @@ void upload_pairs(gpum_b200_mlp* m, const double* theta, const double* ll, size_
     MLP_CK(cudaGetLastError());
   }
   if (ll) {
-    dll.alloc(n);
+    dll.alloc(n, m->st);
     MLP_CK(cudaMemcpyAsync(dll.p, ll, n * sizeof(double), cudaMemcpyHostToDevice, m->st));
   }
   MLP_CK(cudaStreamSynchronize(m->st));
@@ -968,8 +973,10 @@ int gpum_b200_mlp_create(uint32_t d, uint32_t hidden, uint32_t batch, uint32_t s
     m->H = (int)hidden;
     m->B = (int)batch;
     m->seed = seed;
-    MLP_CK(cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking));
-    MLP_CK(cudaStreamCreateWithFlags(&m->st2, cudaStreamNonBlocking));
+    MLP_CK(cudaStreamCreateWithFlags(&m->owned.s, cudaStreamNonBlocking));
+    m->st = m->owned.s;
+    MLP_CK(cudaStreamCreateWithFlags(&m->owned2.s, cudaStreamNonBlocking));
+    m->st2 = m->owned2.s;
     MLP_CK(cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming));
     MLP_CK(cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming));
     const int H = m->H, dp = m->dp, B = m->B;
@@ -983,34 +990,34 @@ int gpum_b200_mlp_create(uint32_t d, uint32_t hidden, uint32_t batch, uint32_t s
     L.ow3 = L.ob2 + H;
     L.ob3 = L.ow3 + H;
     L.n = L.ob3 + 1;
-    for (auto* b : {&m->P, &m->Mm, &m->V, &m->G}) b->alloc(L.n);
-    m->W1h.alloc((size_t)H * dp);
-    m->W1Th.alloc((size_t)dp * H);
-    m->W2h.alloc((size_t)H * H);
-    m->W2Th.alloc((size_t)H * H);
+    for (auto* b : {&m->P, &m->Mm, &m->V, &m->G}) b->alloc(L.n, m->st);
+    m->W1h.alloc((size_t)H * dp, m->st);
+    m->W1Th.alloc((size_t)dp * H, m->st);
+    m->W2h.alloc((size_t)H * H, m->st);
+    m->W2Th.alloc((size_t)H * H, m->st);
     for (int k = 0; k < 2; ++k) {
-      m->Xh[k].alloc((size_t)B * dp);
-      m->XTh[k].alloc((size_t)dp * B);
-      m->t[k].alloc(B);
+      m->Xh[k].alloc((size_t)B * dp, m->st);
+      m->XTh[k].alloc((size_t)dp * B, m->st);
+      m->t[k].alloc(B, m->st);
     }
-    for (auto* b : {&m->A1h, &m->dZ2h}) b->alloc((size_t)B * H);
-    for (auto* b : {&m->A1Th, &m->dZ2Th, &m->dZ1Th}) b->alloc((size_t)H * B);
-    m->Z1.alloc((size_t)B * H);
-    m->yhat.alloc(B);
-    m->dX.alloc((size_t)B * dp);
+    for (auto* b : {&m->A1h, &m->dZ2h}) b->alloc((size_t)B * H, m->st);
+    for (auto* b : {&m->A1Th, &m->dZ2Th, &m->dZ1Th}) b->alloc((size_t)H * B, m->st);
+    m->Z1.alloc((size_t)B * H, m->st);
+    m->yhat.alloc(B, m->st);
+    m->dX.alloc((size_t)B * dp, m->st);
     m->S2 = split_k(B, (H / 128) * (H / 64), sms, 16);
     m->S1 = split_k(B, (H / 128) * (dp / 64), sms, 64);
-    m->pW2.alloc((size_t)m->S2 * H * H);
-    m->pW1.alloc((size_t)m->S1 * H * dp);
+    m->pW2.alloc((size_t)m->S2 * H * H, m->st);
+    m->pW1.alloc((size_t)m->S1 * H * dp, m->st);
     const int nct = B / kGemmBM;
-    m->colhead.alloc((size_t)2 * nct * H);
-    m->colb1.alloc((size_t)nct * H);
-    m->rowpart.alloc((size_t)2 * nct);
-    m->ctr.alloc(2);
-    m->xmean.alloc(d);
-    m->xinv.alloc(d);
-    m->xw.alloc((size_t)d * d);
-    m->err.alloc(1);
+    m->colhead.alloc((size_t)2 * nct * H, m->st);
+    m->colb1.alloc((size_t)nct * H, m->st);
+    m->rowpart.alloc((size_t)2 * nct, m->st);
+    m->ctr.alloc(2, m->st);
+    m->xmean.alloc(d, m->st);
+    m->xinv.alloc(d, m->st);
+    m->xw.alloc((size_t)d * d, m->st);
+    m->err.alloc(1, m->st);
     MLP_CK(cudaMemsetAsync(m->err.p, 0, sizeof(uint32_t), m->st));
     MLP_CK(cudaMemsetAsync(m->ctr.p, 0, 2 * sizeof(uint32_t), m->st));
     // zero moments, biases and the (padded) batch buffers
@@ -1113,7 +1120,8 @@ uint64_t schedule_steps(uint32_t n_stages, const uint32_t* steps, const double* 
 void train_on_device(gpum_b200_mlp* m, const float* dth, const double* dll, size_t n_pairs,
                      uint32_t n_stages, const uint32_t* steps, const double* lrs, uint64_t total,
                      float* out_loss) {
-  m->losses.alloc(total);
+  WaitAtExit wait{m->st}, wait2{m->st2};  // the pairs, on both
+  m->losses.alloc(total, m->st);
   const uint32_t base = m->steps_done;
   // The schedule in device memory: one captured graph serves all its steps.
   std::vector<uint32_t> ends;
@@ -1125,8 +1133,8 @@ void train_on_device(gpum_b200_mlp* m, const float* dth, const double* dll, size
     ends.push_back(at);
     rates.push_back((float)lrs[k]);
   }
-  m->ends.alloc(ends.size());
-  m->lrs.alloc(rates.size());
+  m->ends.alloc(ends.size(), m->st);
+  m->lrs.alloc(rates.size(), m->st);
   MLP_CK(cudaMemcpyAsync(m->ends.p, ends.data(), ends.size() * sizeof(uint32_t),
                          cudaMemcpyHostToDevice, m->st));
   MLP_CK(cudaMemcpyAsync(m->lrs.p, rates.data(), rates.size() * sizeof(float),
@@ -1243,8 +1251,8 @@ int gpum_b200_mlp_predict(gpum_b200_mlp* m, const double* theta, size_t n, doubl
     if (n == 0) return;
     // The same device path as the delayed-acceptance loop (mlp_infer).
     Buf<double> dth, dout;
-    dth.alloc(n * m->d);
-    dout.alloc(n);
+    dth.alloc(n * m->d, m->st);
+    dout.alloc(n, m->st);
     MLP_CK(cudaMemcpyAsync(dth.p, theta, n * m->d * sizeof(double), cudaMemcpyHostToDevice,
                            m->st));
     std::string e;
@@ -1264,9 +1272,9 @@ int gpum_b200_mlp_predict_grad(gpum_b200_mlp* m, const double* theta, size_t n, 
     if (n == 0) return;
     // The same device path as the delayed-acceptance Langevin loop.
     Buf<double> dth, dout, dgrad;
-    dth.alloc(n * m->d);
-    dout.alloc(n);
-    dgrad.alloc(n * m->d);
+    dth.alloc(n * m->d, m->st);
+    dout.alloc(n, m->st);
+    dgrad.alloc(n * m->d, m->st);
     MLP_CK(cudaMemcpyAsync(dth.p, theta, n * m->d * sizeof(double), cudaMemcpyHostToDevice,
                            m->st));
     std::string e;
@@ -1289,7 +1297,7 @@ int gpum_b200_mlp_gradients(gpum_b200_mlp* m, const double* theta, const double*
     Buf<double> dll;
     upload_pairs(m, theta, ll, n, dth, dll);
     Buf<float> loss1;
-    loss1.alloc(1);
+    loss1.alloc(1, m->st);
     mlp_gather<<<m->B / kGatherRows, 32 * kGatherRows, 0, m->st>>>(
         dth.p, dll.p, n, m->d, m->dp, m->B, 0, 0, m->ctr.p, 0,
                                         m->xmean.p, m->xinv.p, m->xw_or_null(), m->ymean,
@@ -1328,13 +1336,14 @@ int gpum_b200_mlp_gemm_check(uint32_t M, uint32_t N, uint32_t K, const float* A,
     for (size_t i = 0; i < ah.size(); ++i) ah[i] = __float2bfloat16(A[i]);
     for (size_t i = 0; i < bh.size(); ++i) bh[i] = __float2bfloat16(B[i]);
     gpum_b200_mlp tmp;
-    MLP_CK(cudaStreamCreateWithFlags(&tmp.st, cudaStreamNonBlocking));
+    MLP_CK(cudaStreamCreateWithFlags(&tmp.owned.s, cudaStreamNonBlocking));
+    tmp.st = tmp.owned.s;
     Buf<bf16> da, db;
     Buf<float> dc;
-    da.alloc(ah.size());
-    db.alloc(bh.size());
-    dc.alloc((size_t)M * N);
-    tmp.err.alloc(1);
+    da.alloc(ah.size(), tmp.st);
+    db.alloc(bh.size(), tmp.st);
+    dc.alloc((size_t)M * N, tmp.st);
+    tmp.err.alloc(1, tmp.st);
     MLP_CK(cudaMemsetAsync(tmp.err.p, 0, sizeof(uint32_t), tmp.st));
     MLP_CK(cudaMemcpyAsync(da.p, ah.data(), ah.size() * 2, cudaMemcpyHostToDevice, tmp.st));
     MLP_CK(cudaMemcpyAsync(db.p, bh.data(), bh.size() * 2, cudaMemcpyHostToDevice, tmp.st));

@@ -85,15 +85,20 @@ inline PinnedBlocks& pinned_chunks() {
 
 // ------------------------------------------------------------ device memory
 // Allocations up to kPoolMax come from a memory pool of the current device
-// that keeps at most kPoolKeep when nothing is allocated.  The pool's own
-// stream orders them; as with cudaMalloc and cudaFree the memory is usable on
-// every stream at once, and freeing it waits for the device first.
+// that keeps at most kPoolKeep when nothing is allocated.  As with cudaMalloc
+// the memory is usable on every stream at once.  It goes back to the pool and
+// device that it came from, whatever device is current: on the pool's stream when
+// its owner's stream is idle, so that the next allocation may take it at once,
+// else on its owner's, and the pool hands it out again when that is done.
+// Nothing here waits for a device: another thread may be capturing a graph, and
+// CUDA allows no such wait meanwhile.
 constexpr size_t kPoolMax = 32u << 20;
 constexpr uint64_t kPoolKeep = 64ull << 20;
 
 struct DevicePool {
   cudaMemPool_t pool = nullptr;
   cudaStream_t st = nullptr;
+  int dev = -1;
 };
 inline DevicePool* device_pool() {
   static std::mutex* mu = new std::mutex();
@@ -104,13 +109,17 @@ inline DevicePool* device_pool() {
   auto it = pools->find(dev);
   if (it == pools->end()) {
     DevicePool d;
+    d.dev = dev;
     cudaMemPoolProps pp{};
     pp.allocType = cudaMemAllocationTypePinned;
     pp.location.type = cudaMemLocationTypeDevice;
     pp.location.id = dev;
     uint64_t keep = kPoolKeep;
+    int wait = 0;  // an allocation does not queue behind other owners' work
     if (cudaMemPoolCreate(&d.pool, &pp) != cudaSuccess ||
         cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+        cudaMemPoolSetAttribute(d.pool, cudaMemPoolReuseAllowInternalDependencies, &wait) !=
+            cudaSuccess ||
         cudaStreamCreateWithFlags(&d.st, cudaStreamNonBlocking) != cudaSuccess) {
       cudaGetLastError();
       d = DevicePool{};  // plain allocations on this device
@@ -119,23 +128,61 @@ inline DevicePool* device_pool() {
   }
   return it->second.pool ? &it->second : nullptr;
 }
-inline cudaError_t dev_alloc(void** p, size_t bytes) {
+
+// An allocation, and where it goes back.
+struct DevMem {
+  void* p = nullptr;
+  DevicePool* pool = nullptr;  // that it came from; nullptr: plain
+  cudaStream_t st = nullptr;   // the owner's stream
+};
+// For the owner of stream `st`, which outlives the allocation.
+inline cudaError_t dev_alloc(DevMem* m, size_t bytes, cudaStream_t st) {
+  *m = DevMem{};
+  m->st = st;
   DevicePool* d = bytes <= kPoolMax ? device_pool() : nullptr;
-  if (!d) return cudaMalloc(p, bytes);
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, d->pool, d->st);
+  if (!d) return cudaMalloc(&m->p, bytes);
+  m->pool = d;
+  cudaError_t e = cudaMallocFromPoolAsync(&m->p, bytes, d->pool, d->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(d->st);
   return e;
 }
-inline void dev_free(void* p, size_t bytes) {
-  if (!p) return;
-  DevicePool* d = bytes <= kPoolMax ? device_pool() : nullptr;
-  if (!d) {
-    cudaFree(p);
-    return;
+inline void dev_free(DevMem* m) {
+  if (!m->p) return;
+  if (!m->pool) {
+    cudaFree(m->p);  // which waits for its device
+  } else {
+    int dev = m->pool->dev;
+    cudaGetDevice(&dev);
+    if (dev != m->pool->dev) cudaSetDevice(m->pool->dev);
+    const bool idle = cudaStreamQuery(m->st) == cudaSuccess;
+    if (cudaFreeAsync(m->p, idle ? m->pool->st : m->st) != cudaSuccess) {
+      // Without a stream's order: after a wait for the owner's, or, if that fails
+      // too (the context is lost), not at all.
+      if (cudaStreamSynchronize(m->st) == cudaSuccess) cudaFree(m->p);
+    }
+    cudaGetLastError();
+    if (dev != m->pool->dev) cudaSetDevice(dev);
   }
-  cudaDeviceSynchronize();
-  cudaFreeAsync(p, d->st);
+  *m = DevMem{};
 }
+
+// A stream that outlives the buffers declared after it.
+struct OwnedStream {
+  cudaStream_t s = nullptr;
+  OwnedStream() = default;
+  OwnedStream(const OwnedStream&) = delete;
+  OwnedStream& operator=(const OwnedStream&) = delete;
+  ~OwnedStream() {
+    if (s) cudaStreamDestroy(s);
+  }
+};
+
+// Waits for a stream on the way out, errors included: where work on it uses
+// memory of another owner, who may give it back next.
+struct WaitAtExit {
+  cudaStream_t st;
+  ~WaitAtExit() { cudaStreamSynchronize(st); }
+};
 
 // ---------------------------------------------------------- large transfers
 inline void convert_copy(float* dst, const float* src, size_t n) {

@@ -123,6 +123,9 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s) {
   stream_of(s)->done = stream_of(s)->submitted;
   return cudaSuccess;
 }
+cudaError_t cudaStreamQuery(cudaStream_t s) {
+  return stream_of(s)->done == stream_of(s)->submitted ? cudaSuccess : cudaErrorNotReady;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f) {
   (void)s, (void)e, (void)f;
   return cudaSuccess;

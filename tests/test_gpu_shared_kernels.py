@@ -1,6 +1,7 @@
 """Sessions alive together whose launches of one kernel need different amounts
 of shared memory: what one of them sets up leaves the other's calls as they
 were."""
+import threading
 
 import numpy as np
 import pytest
@@ -53,3 +54,47 @@ def test_prepared_runs_of_two_sessions(gpu):
     assert n == 6
     assert np.array_equal(np.ravel(draws), np.ravel(alone[0]))
     assert np.array_equal(acc, alone[1]) and np.array_equal(last, alone[2])
+
+
+def test_runs_beside_a_thread_that_opens_and_closes_sessions(gpu):
+    # runs of 64 iterations capture a graph in each new session, training steps
+    # in each call; the other thread allocates, grows and frees meanwhile
+    w = W.make("logistic", n_obs=2000, p=5)
+    d = w.model.n_params
+    args = (np.tile(w.truth["beta"], (8, 1)), np.full((8, d), 0.05), np.ones(8), 64, 3, 0)
+    pts = np.random.default_rng(0).normal(0, 1, (1000, d))
+    stop, wrong, opened = threading.Event(), [], [0]
+
+    def other():
+        try:
+            while not stop.is_set():
+                with _session(gpu, w) as s:
+                    for n in (4, 1000):
+                        s.loglik_batch(pts[:n])
+                    s.run(*args[:3], 5, 3, 0)
+                opened[0] += 1
+        except Exception as e:  # reported by the test below
+            wrong.append(e)
+
+    def once():
+        net = gpu.Surrogate(d, hidden=128, batch=256, seed=1)
+        with _session(gpu, w) as s:
+            run = s.run(*args)
+        net.train(pts, -np.sum(pts ** 2, axis=1), steps=40, lr=1e-3)
+        params = net.params()
+        net.close()
+        return [*run, params]
+
+    first = once()
+    t = threading.Thread(target=other)
+    t.start()
+    try:
+        runs = [once() for _ in range(30)]
+    finally:
+        stop.set()
+        t.join()
+    assert not wrong, wrong
+    assert opened[0] > 0
+    for r in runs:
+        for x, y in zip(first, r):
+            assert np.array_equal(x, y)

@@ -112,3 +112,55 @@ def grids(s):
 first = grids(session(n_obs=300001))
 assert first == grids(session(n_obs=300001)), first
 """)
+
+
+def test_memory_goes_back_without_waiting_for_the_device(runtime):
+    # another thread captures a graph: buffers grow with work pending, sessions
+    # and surrogates come and go
+    runtime("""
+s = session()
+net = _native.Surrogate(17, hidden=128, batch=256, seed=1)
+rt.fake_capture_elsewhere(1)
+s.prepare(*start(17, 8, 6))
+s.advance(5)
+s.prepare(*start(17, 1000, 6))
+s.advance(5)
+s.loglik_batch(np.zeros((5000, 17)))
+net.close()
+s.close()
+session().close()
+assert not wrong(), wrong()
+assert rt.fake_live_bytes() == 0
+""")
+
+
+def test_memory_goes_back_to_its_own_device(runtime):
+    runtime("""
+s = session()
+s.loglik_batch(np.zeros((10, 17)))
+net = _native.Surrogate(17, hidden=128, batch=256, seed=1)
+rt.fake_set_device(1)
+other = session()
+s.close()
+net.close()
+assert rt.fake_device() == 1
+other.loglik_batch(np.zeros((10, 17)))
+rt.fake_set_device(0)
+other.close()
+assert rt.fake_device() == 0
+assert not wrong(), wrong()
+assert rt.fake_live_bytes() == 0
+""")
+
+
+def test_a_refused_free_waits_for_the_owner(runtime):
+    runtime("""
+s = session()
+s.prepare(*start(17, 8, 6))
+s.advance(5)
+rt.fake_fail_frees(1)
+s.prepare(*start(17, 1000, 6))
+s.close()
+assert not wrong(), wrong()
+assert rt.fake_live_bytes() == 0
+""")
