@@ -1173,8 +1173,11 @@ void fetch(gpum_b200_session* s, float* out_draws, float* out_accept, double* ou
   const uint32_t n = s->n_done;
   const int C = s->n_chains;
   const size_t np = s->np;
-  if (n_done) *n_done = n;
-  if (!out_draws && !out_accept && !out_last) return;  // the count alone: nothing to wait for
+  if (!out_draws && !out_accept && !out_last) {  // the count alone, of a run without failure
+    s->check_device_error();
+    if (n_done) *n_done = n;
+    return;
+  }
   cudaStream_t st = s->stream;
   // The small results first, so that a failed run copies no draws: the error
   // word, the log posteriors and the acceptance counts, one wait for all.
@@ -1213,6 +1216,7 @@ void fetch(gpum_b200_session* s, float* out_draws, float* out_accept, double* ou
     GPUM_CK(cudaStreamSynchronize(st));
   }
   s->report_device_error(*err);
+  if (n_done) *n_done = n;
   if (out_last) std::memcpy(out_last, last, sizeof(double) * C);
   if (out_accept)
     for (int c = 0; c < C; ++c) out_accept[c] = n == 0 ? 0.0f : (float)acc[c] / (float)n;

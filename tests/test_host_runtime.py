@@ -164,3 +164,33 @@ s.close()
 assert not wrong(), wrong()
 assert rt.fake_live_bytes() == 0
 """)
+
+
+FETCH = """
+s = session()
+s.prepare(*start(17, {C}, 6))
+s.advance(5)
+err = ctypes.create_string_buffer(256)
+draws = np.full(5 * {C} * 17, 7, np.float32)
+acc, last = np.full({C}, 7, np.float32), np.full({C}, 7.0)
+n = ctypes.c_uint32(99)
+def fetch(*out):
+    return s._lib.gpum_b200_session_fetch(s._h, *out, ctypes.byref(n), err, 256)
+f32, f64 = ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_double)
+everything = [draws.ctypes.data_as(f32), acc.ctypes.data_as(f32), last.ctypes.data_as(f64)]
+def fail_kernels():  # as a kernel whose wait ran out does: the session's error word
+    ctypes.c_uint32.from_address(rt.fake_block(4)).value = 1
+"""
+
+
+def test_the_count_alone_waits_and_reports_a_failed_run(runtime):
+    runtime(FETCH.format(C=8) + """
+assert rt.fake_pending() > 0
+assert fetch(None, None, None) == 0 and n.value == 5
+assert rt.fake_pending() == 0
+n.value = 99
+fail_kernels()
+assert fetch(None, None, None) == _native.ERR_DEVICE, err.value
+assert n.value == 99
+assert fetch(None, None, None) == 0 and n.value == 5
+""")
