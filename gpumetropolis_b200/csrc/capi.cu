@@ -1179,12 +1179,15 @@ void fetch(gpum_b200_session* s, float* out_draws, float* out_accept, double* ou
     return;
   }
   cudaStream_t st = s->stream;
-  // The small results first, so that a failed run copies no draws: the error
-  // word, the log posteriors and the acceptance counts, one wait for all.
+  // The small results first: the error word, the log posteriors and the
+  // acceptance counts, with draws that fit the pinned block too.  A failed run
+  // writes nothing to the caller's arrays, and larger draws are copied only after
+  // the wait for these.
   std::vector<char> own;
-  char* r = s->pinned_results((size_t)C * 12 + 8);
+  const size_t small = (size_t)C * 12 + 8;
+  char* r = s->pinned_results(small);
   if (!r) {
-    own.resize((size_t)C * 12 + 8);
+    own.resize(small);
     r = own.data();
   }
   uint32_t* err = reinterpret_cast<uint32_t*>(r);
@@ -1194,29 +1197,30 @@ void fetch(gpum_b200_session* s, float* out_draws, float* out_accept, double* ou
   GPUM_CK(cudaMemcpyAsync(acc, s->accepts.p, sizeof(uint32_t) * C, cudaMemcpyDeviceToHost, st));
   if (out_last)
     GPUM_CK(cudaMemcpyAsync(last, s->cur.p, sizeof(double) * C, cudaMemcpyDeviceToHost, st));
-  if (out_draws && n > 0) {
-    s->draws_out.ensure((size_t)n * C * np, s->stream);
+  const size_t nd = out_draws ? (size_t)n * C * np : 0;
+  const char* dr = nullptr;
+  if (nd > 0) {
+    s->draws_out.ensure(nd, s->stream);
     dim3 grid((C + 31) / 32, (n + 31) / 32, (unsigned)np);
     draws_layout_kernel<<<grid, dim3(32, 8), 0, st>>>(s->draws.p, s->draws_out.p, (int)n,
                                                       (int)np, C, s->geo.C_pad);
     GPUM_CK(cudaGetLastError());
     ++s->launches;
-    const size_t nd = (size_t)n * C * np;
-    char* dr = s->pinned_results((size_t)C * 12 + 8 + nd * sizeof(float));
-    if (dr) {  // small draws share the wait
-      dr += ((size_t)C * 12 + 8);
-      GPUM_CK(cudaMemcpyAsync(dr, s->draws_out.p, sizeof(float) * nd, cudaMemcpyDeviceToHost, st));
-      GPUM_CK(cudaStreamSynchronize(st));
-      std::memcpy(out_draws, dr, sizeof(float) * nd);
-    } else {
-      s->result_to_host(out_draws, s->draws_out.p, nd);
-      GPUM_CK(cudaStreamSynchronize(st));
+    if (s->pinned_results(small + nd * sizeof(float))) {
+      GPUM_CK(cudaMemcpyAsync(r + small, s->draws_out.p, sizeof(float) * nd,
+                              cudaMemcpyDeviceToHost, st));
+      dr = r + small;
     }
-  } else {
-    GPUM_CK(cudaStreamSynchronize(st));
   }
+  GPUM_CK(cudaStreamSynchronize(st));
   s->report_device_error(*err);
   if (n_done) *n_done = n;
+  if (dr) {
+    std::memcpy(out_draws, dr, sizeof(float) * nd);
+  } else if (nd > 0) {
+    s->result_to_host(out_draws, s->draws_out.p, nd);
+    GPUM_CK(cudaStreamSynchronize(st));
+  }
   if (out_last) std::memcpy(out_last, last, sizeof(double) * C);
   if (out_accept)
     for (int c = 0; c < C; ++c) out_accept[c] = n == 0 ? 0.0f : (float)acc[c] / (float)n;

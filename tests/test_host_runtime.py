@@ -194,3 +194,15 @@ assert fetch(None, None, None) == _native.ERR_DEVICE, err.value
 assert n.value == 99
 assert fetch(None, None, None) == 0 and n.value == 5
 """)
+
+
+@pytest.mark.parametrize("C", [8, 2000])
+def test_a_failed_run_leaves_the_outputs_alone(runtime, C):
+    # draws that share the pinned block, and draws of their own copy
+    runtime(FETCH.format(C=C) + """
+fail_kernels()
+assert fetch(*everything) == _native.ERR_DEVICE, err.value
+assert np.all(draws == 7) and np.all(acc == 7) and np.all(last == 7) and n.value == 99
+assert fetch(*everything) == 0 and n.value == 5
+assert not draws.any() and not acc.any() and not last.any()
+""")
