@@ -397,19 +397,22 @@ struct gpum_b200_session {
     return std::vector<char>(b, b + sizeof k);
   }
 
-  // The chains' arrays of a run of C chains in one allocation.
-  void run_arrays(size_t C, bool mala) {
+  // The chains' arrays of a run of C chains in one allocation; `side`: with those
+  // of the side rows' draws (side_draws).
+  void run_arrays(size_t C, bool mala, bool side) {
     for (char* base = nullptr;;) {
       size_t at = 0;
-      for (auto* b : {&state, &prop, &snap, &sd, &zbuf, &side_z, &side_inc})
-        b->carve(base, &at, C * np);
-      for (auto* b : {&temp, &cur, &last_eval, &prior_v, &side_lu}) b->carve(base, &at, C);
+      auto part = [&](DBuf<double>& b, bool used, size_t count) {
+        if (used) b.carve(base, &at, count);
+        else if (!b.own) b.release();  // of a slab that may be gone
+      };
+      for (auto* b : {&state, &prop, &snap, &sd, &zbuf}) b->carve(base, &at, C * np);
+      for (auto* b : {&temp, &cur, &last_eval, &prior_v}) b->carve(base, &at, C);
       for (auto* b : {&ctr, &accepts, &iter}) b->carve(base, &at, C);
       vars.carve(base, &at, 1);
-      for (auto* b : {&gx, &gy, &mx, &my, &vbuf, &prior_g}) {
-        if (mala) b->carve(base, &at, C * np);
-        else if (!b->own) b->release();  // of a slab that may be gone
-      }
+      for (auto* b : {&gx, &gy, &mx, &my, &vbuf, &prior_g}) part(*b, mala, C * np);
+      for (auto* b : {&side_z, &side_inc}) part(*b, side, C * np);
+      part(side_lu, side, C);
       if (base) return;
       slab.ensure(at, stream);
       base = slab.p;
@@ -718,9 +721,10 @@ struct gpum_b200_session {
   // hold an SM's shared memory (2,048 x 65 DE on 2^18 observations: 14.1 ms
   // for 20 steps, 13.4 with the draws in the step kernel; 8 Gaussian chains:
   // 5.0 us per step, 6.2).
-  bool side_draws() const {
-    return A.mode != MODE_DESYNC && warps_per_chain(n_chains) == kWarps;
+  static bool side_draws(int mode, int n) {
+    return mode != MODE_DESYNC && warps_per_chain(n) == kWarps;
   }
+  bool side_draws() const { return side_draws(A.mode, n_chains); }
   // The row of the priors, and the rows of the normals: one a thread, up to
   // eight rows.
   int side_rows() const {
@@ -1016,7 +1020,12 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
   s->n_chains = (int)C;
   s->setup_eval((int)C, mala);
   const Geometry& g = s->geo;
-  s->run_arrays(C, mala);
+  const int kind = mode == 0 ? MODE_RWM
+                 : mode == 2 ? MODE_CHOL
+                 : mala      ? MODE_MALA
+                 : mode == 4 ? MODE_DESYNC
+                             : MODE_DE;
+  s->run_arrays(C, mala, s->side_draws(kind, (int)C));
   s->draws.ensure(std::max<size_t>(1, (size_t)max_iter * np * g.C_pad), s->stream);
   if (use_L) s->L.ensure((size_t)C * np * np, s->stream);
   if (mala && !s->kc.compiled) {  // the interpreted prior's gradient tape
@@ -1046,11 +1055,7 @@ void prepare(gpum_b200_session* s, const double* init, const double* sd, const d
   A.draws = s->draws.p;
   A.n_iter = max_iter;
   A.seed = seed;
-  A.mode = mode == 0 ? MODE_RWM
-         : mode == 2 ? MODE_CHOL
-         : mala      ? MODE_MALA
-         : mode == 4 ? MODE_DESYNC
-                     : MODE_DE;
+  A.mode = kind;
   A.rng = rng;
   A.gamma = gamma;
   A.de_noise = de_noise;

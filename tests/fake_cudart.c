@@ -167,6 +167,7 @@ static cudaError_t allocate(void** p, size_t bytes, int dev, int pooled) {
   b->dev = dev;
   b->pooled = pooled;
   b->live = 1;
+  note("allocated %zu", bytes);
   return cudaSuccess;
 }
 static Block* block_of(void* p) {

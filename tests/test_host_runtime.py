@@ -206,3 +206,17 @@ assert np.all(draws == 7) and np.all(acc == 7) and np.all(last == 7) and n.value
 assert fetch(*everything) == 0 and n.value == 5
 assert not draws.any() and not acc.any() and not last.any()
 """)
+
+
+@pytest.mark.parametrize("C,arrays", [(444, 7), (445, 5), (20000, 5)])
+def test_arrays_of_a_run(runtime, C, arrays):
+    # states, proposals, snapshot, scales and scratch, and up to 444 chains the
+    # draws made ahead: chains x 17 doubles each; five values of 8 bytes and three
+    # of 4 a chain, and 16 alignments, at most beside them
+    runtime(f"""
+s = session()
+s.prepare(*start(17, {C}, 1))
+sizes = [int(l.split()[1]) for l in log() if l.startswith("allocated")]
+one = {C} * 17 * 8
+assert any({arrays} * one <= b < {arrays} * one + 64 * {C} + 16 * 256 for b in sizes), sizes
+""")
