@@ -139,8 +139,15 @@ struct DevMem {
 inline cudaError_t dev_alloc(DevMem* m, size_t bytes, cudaStream_t st) {
   *m = DevMem{};
   m->st = st;
-  DevicePool* d = bytes <= kPoolMax ? device_pool() : nullptr;
-  if (!d) return cudaMalloc(&m->p, bytes);
+  DevicePool* d = device_pool();
+  if (!d || bytes > kPoolMax) {
+    cudaError_t e = cudaMalloc(&m->p, bytes);
+    if (e == cudaErrorMemoryAllocation && d && cudaMemPoolTrimTo(d->pool, 0) == cudaSuccess) {
+      cudaGetLastError();
+      e = cudaMalloc(&m->p, bytes);  // with what the pool kept
+    }
+    return e;
+  }
   m->pool = d;
   cudaError_t e = cudaMallocFromPoolAsync(&m->p, bytes, d->pool, d->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(d->st);

@@ -31,7 +31,8 @@ typedef struct {
 static Stream streams[MAX_ITEMS];
 static Block blocks[MAX_ITEMS];
 static Limit limits[DEVICES][MAX_ITEMS];
-static int n_streams, n_blocks, n_limits[DEVICES], current, captures_elsewhere, fail_frees;
+static int n_streams, n_blocks, n_limits[DEVICES], current, captures_elsewhere, fail_frees,
+    pool_keeps_last;
 static char log_text[1 << 20];
 static size_t log_len;
 
@@ -53,6 +54,7 @@ void fake_set_device(int d) { current = d; }
 int fake_device(void) { return current; }
 void fake_capture_elsewhere(int on) { captures_elsewhere = on; }
 void fake_fail_frees(int on) { fail_frees = on; }
+void fake_pool_keeps_last(int on) { pool_keeps_last = on; } /* until it is trimmed */
 long fake_pending(void) {
   long n = 0;
   for (int i = 0; i < n_streams; ++i)
@@ -176,7 +178,13 @@ static Block* block_of(void* p) {
   note("VIOLATION: free of an unknown pointer");
   return 0;
 }
-cudaError_t cudaMalloc(void** p, size_t bytes) { return allocate(p, bytes, current, 0); }
+cudaError_t cudaMalloc(void** p, size_t bytes) {
+  return pool_keeps_last ? cudaErrorMemoryAllocation : allocate(p, bytes, current, 0);
+}
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t p, size_t keep) {
+  (void)p, (void)keep;
+  return pool_keeps_last = 0, cudaSuccess;
+}
 cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned f) {
   (void)f;
   *p = calloc(bytes, 1);

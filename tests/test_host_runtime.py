@@ -220,3 +220,11 @@ sizes = [int(l.split()[1]) for l in log() if l.startswith("allocated")]
 one = {C} * 17 * 8
 assert any({arrays} * one <= b < {arrays} * one + 64 * {C} + 16 * 256 for b in sizes), sizes
 """)
+
+
+def test_what_the_pool_keeps_serves_a_large_allocation(runtime):
+    runtime("""
+session().close()
+rt.fake_pool_keeps_last(1)
+session(p=64, n_obs=200000)  # 52 MB of data
+""")
