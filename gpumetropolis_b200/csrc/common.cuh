@@ -305,7 +305,9 @@ __device__ __forceinline__ double stream_normal_at(const Stream& rs, uint32_t i0
   return sqrt(-2.0 * log(u1)) * cos(6.283185307179586 * u2);
 }
 // The stream of chain c for this step's acceptance uniform, and, past it, for
-// the next proposal's draws (advance_stream: past those, too).
+// the next proposal's draws: three uniforms with DE (de_difference), then 2 np
+// for the normals.  The step kernel's draws_used advances the triple32 counter by
+// the same counts.
 __device__ __forceinline__ Stream accept_stream(const ChainArgs& A, int c, uint32_t t) {
   Stream rs = make_stream(A, c);
   if (A.rng != RNG_TRIPLE32) {
@@ -346,8 +348,11 @@ __device__ __forceinline__ double de_difference(const ChainArgs& A, const Stream
 // latencies and SMs are free) also the logs of the acceptance uniforms, and
 // the other rows, a share of the chain block's chains each, the next
 // proposals' normals and L z or the DE differences: in the step kernel they
-// were 2 of the 6.2 us of an iteration of 8 Gaussian chains.  (Inlined: as a
-// function of its own it returned wrong values in the tensor-core kernel.)
+// were 2 of the 6.2 us of an iteration of 8 Gaussian chains.  Inlined: as a
+// function of its own it returned wrong values in the tensor-core kernel, for a
+// reason that reading and the compiler's statistics (96 registers, 480 bytes of
+// stack) do not show.  test_gpu_tensor_cores.py compares that kernel's runs, side
+// rows included, with the FP32 kernel's.
 template <class Prior>
 __device__ __forceinline__ void side_block(const EvalArgs& E, ChainArgs A, int cb, int CG,
                                            int phase, int nthreads) {
