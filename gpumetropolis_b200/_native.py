@@ -530,17 +530,20 @@ class Session:
     def fetch(self, want_draws=True):
         n = C.c_uint32(0)
         err = C.create_string_buffer(_ERRLEN)
-        # First call learns n_done without copying draws.
-        _check(self._lib.gpum_b200_session_fetch(self._h, None, None, None, C.byref(n), err,
-                                                 _ERRLEN), err)
-        nd = n.value
-        draws = np.empty(max(nd * self.n_chains * self.n_params, 1), np.float32)
         acc = np.empty(self.n_chains, np.float32)
         last = np.empty(self.n_chains, np.float64)
+        per = self.n_chains * self.n_params
+        draws = None
+        if want_draws:  # a first call learns n_done without copying draws
+            _check(self._lib.gpum_b200_session_fetch(self._h, None, None, None, C.byref(n), err,
+                                                     _ERRLEN), err)
+            draws = np.empty(max(n.value * per, 1), np.float32)
         _check(self._lib.gpum_b200_session_fetch(
-            self._h, _p(draws, C.c_float) if want_draws else None, _p(acc, C.c_float),
-            _p(last, C.c_double), C.byref(n), err, _ERRLEN), err)
-        return draws[: nd * self.n_chains * self.n_params], acc, last, nd
+            self._h, _p(draws, C.c_float), _p(acc, C.c_float), _p(last, C.c_double), C.byref(n),
+            err, _ERRLEN), err)
+        if draws is None:
+            draws = np.empty(max(n.value * per, 1), np.float32)
+        return draws[: n.value * per], acc, last, n.value
 
     def loglik_batch(self, points):
         pts = _f64(points)

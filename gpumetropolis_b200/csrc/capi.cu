@@ -645,9 +645,12 @@ struct gpum_b200_session {
   }
 
   void check_device_error() {
-    uint32_t e = 0;
-    GPUM_CK(cudaMemcpyAsync(&e, d_err.p, sizeof e, cudaMemcpyDeviceToHost, stream));
+    uint32_t own = 0, e = 0;
+    char* r = pinned_results(sizeof e);
+    if (!r) r = reinterpret_cast<char*>(&own);
+    GPUM_CK(cudaMemcpyAsync(r, d_err.p, sizeof e, cudaMemcpyDeviceToHost, stream));
     GPUM_CK(cudaStreamSynchronize(stream));
+    std::memcpy(&e, r, sizeof e);
     report_device_error(e);
   }
   void report_device_error(uint32_t e) {
