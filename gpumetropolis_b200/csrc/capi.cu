@@ -496,14 +496,63 @@ struct gpum_b200_session {
   }
   bool ext(const KernelChoice& k) const { return k.compiled && cm.n_mat > 0; }
 
+  // The gradient kernel of the compiled engine for n points, out of one chain per
+  // lane (eight warps of 32 chains) and, where the model has them, two (four or
+  // eight warps of 64).  A chain's FP32 blocks are the same on each: as many warps
+  // share it (8, 4, 2, 1 up to 32, 64, 128 points and above).
+  //
+  // Two chains per lane halve the column loads per chain and double its registers.
+  // On a full GPU they run at 1.05 to 1.3 times the speed of one where as many warps
+  // stay resident on an SM (1, 4, 6, 17, 24, 32 parameters), at 1.0 with three
+  // quarters of the warps (8 parameters) and 0.8 to 0.95 with half (a mixture's 5,
+  // 12): taken as 0.5 + 0.65 x the share of warps.  A block of four warps alone on
+  // its SM takes 1.25 times as long as eight of one chain per lane, and neither may
+  // leave SMs or the last wave idle: so each geometry's waves x (tiles x time of a
+  // tile + 1), in units of a full SM's tile of one chain per lane.  That picks the
+  // fastest of the three within 0.5 % on average over 945 calls (9 models, 33 to
+  // 4,000 points, 3,000 to 600,000 observations).  Against eight warps of 64 above
+  // 256 points and four above 32 always: 1.12 on average; 600 points x 131,072
+  // observations of the mixture 632 -> 404 us, 400 x 3,000 of the 17-parameter
+  // logistic model 125 -> 92.
+  KernelChoice choose_gradient(int n) const {
+    KernelChoice one;
+    one.compiled = true;
+    one.fn = (const void*)cm.k_grad;
+    one.lanes = cm.lanes_grad;
+    one.G = one.lanes ? 32 : cm.GG;
+    one.W = 1 + (int)np;
+    if (!cm.k_grad2 || n <= 32 || n_obs == 0) return one;
+    KernelChoice best = one, four = one, eight = one;
+    four.fn = (const void*)cm.k_grad2h;
+    four.G = eight.G = 64;
+    four.threads = 128;
+    eight.fn = (const void*)cm.k_grad2;
+    int full = 1;  // resident CTAs of one chain per lane
+    double least = 0.0;
+    auto consider = [&](const KernelChoice& k) {
+      const Geometry g = geometry(n, k);
+      const int occ = resident(k.fn, k.threads, g.smem), sms = num_sms();
+      if (k.G == 32) full = occ;
+      const double share = (double)occ * k.threads / (full * kThreads);
+      const double gain = 0.5 + 0.65 * std::min(1.0, share);
+      const int ctas = g.NCB * g.NOB, waves = (ctas + sms * occ - 1) / (sms * occ);
+      const int r = std::min(occ, (ctas + sms - 1) / sms);  // on an SM at once
+      const double t = k.G == 32                ? r
+                       : k.threads == kThreads ? 2 * r / gain
+                                               : std::max(1.25, r / gain);
+      const double cost = waves * (g.tiles_per_cta * t / full + 1.0);
+      if (k.G != 32 && cost >= least * (1.0 - 1e-9)) return;
+      least = cost;
+      best = k;
+    };
+    consider(one);
+    if (n > 256) consider(eight);  // before four: one fill of a tile for 512 chains
+    consider(four);
+    return best;
+  }
+
   // `pointwise`: per-observation output, which the tensor-core value kernel
-  // does not write.  Gradients of more than 256 points run two chains per lane:
-  // its eight warps of 64 then share no chain, as the eight of 32 share none
-  // above 224, so every chain's FP32 blocks are the same on either kernel.
-  // From 33 to 256 points its form with four warps shares a chain among as many
-  // warps as the eight of 32 do (4, 2 or 1).  The kernel on 65,537 observations,
-  // eight warps of 32 -> four of 64: 250 points of 17 parameters 96 -> 83 us, of
-  // 24 83 -> 66, 100 points of 24 43 -> 35, 64 of 17 28 -> 25.
+  // does not write.
   KernelChoice choose(int n, bool need_grad, bool pointwise = false) {
     KernelChoice k;
     // Gradients: the compiled engine's adjoint unless the interpreter engine
@@ -529,20 +578,13 @@ struct gpum_b200_session {
         throw Failure{GPUM_ERR_UNSUPPORTED,
                       std::string(need_grad ? "gradients need" : "engine=compiled needs") +
                           " the compiled engine: " + cm_error};
+      if (need_grad) return choose_gradient(n);
       k.compiled = true;
-      k.fn = need_grad ? (const void*)cm.k_grad : (const void*)cm.k_value;
-      k.lanes = need_grad ? cm.lanes_grad : cm.lanes;
-      k.G = k.lanes ? 32 : (need_grad ? cm.GG : cm.G);
-      if (need_grad && cm.k_grad2 && n > 256) {
-        k.fn = (const void*)cm.k_grad2;
-        k.G = 64;
-      } else if (need_grad && cm.k_grad2h && n > 32) {
-        k.fn = (const void*)cm.k_grad2h;
-        k.G = 64;
-        k.threads = 128;
-      }
-      k.W = need_grad ? 1 + (int)np : 1;
-      if (!need_grad && !pointwise && tc_ok) {
+      k.fn = (const void*)cm.k_value;
+      k.lanes = cm.lanes;
+      k.G = k.lanes ? 32 : cm.G;
+      k.W = 1;
+      if (!pointwise && tc_ok) {
         k.tc = true;
         k.fn = (const void*)cm.k_value_tc;
         k.lanes = false;

@@ -455,8 +455,9 @@ gm_iter_grad(const __grid_constant__ gpum::TmapDesc tmap, gpum::EvalArgs E, gpum
 }
 
 #if GM_GRAD2
-// The gradient kernel with two chains per lane (64 per warp): eight warps for
-// batches above 256 points, four (two CTAs per SM) for those above 32.
+// The gradient kernel with two chains per lane (64 per warp), with eight warps
+// and with four (two CTAs per SM); the host chooses among these and one chain per
+// lane.
 extern "C" __global__ void __launch_bounds__(gpum::kThreads, 1)
 gm_iter_grad2(const __grid_constant__ gpum::TmapDesc tmap, gpum::EvalArgs E, gpum::ChainArgs A,
               int phase) {

@@ -27,12 +27,18 @@ typedef struct {
   const void* fn;
   int limit;
 } Limit;
+typedef struct {
+  char name[64];
+  int regs;
+} Kernel; /* of a library, which fake_registers names beforehand */
 
 static Stream streams[MAX_ITEMS];
 static Block blocks[MAX_ITEMS];
 static Limit limits[DEVICES][MAX_ITEMS];
 static int n_streams, n_blocks, n_limits[DEVICES], current, captures_elsewhere, fail_frees,
     pool_keeps_last;
+static Kernel kernels[64];
+static int n_kernels;
 static char log_text[1 << 20];
 static size_t log_len;
 
@@ -55,6 +61,10 @@ int fake_device(void) { return current; }
 void fake_capture_elsewhere(int on) { captures_elsewhere = on; }
 void fake_fail_frees(int on) { fail_frees = on; }
 void fake_pool_keeps_last(int on) { pool_keeps_last = on; } /* until it is trimmed */
+void fake_registers(const char* name, int regs) {
+  snprintf(kernels[n_kernels].name, 64, "%s", name);
+  kernels[n_kernels++].regs = regs;
+}
 long fake_pending(void) {
   long n = 0;
   for (int i = 0; i < n_streams; ++i)
@@ -262,38 +272,46 @@ cudaError_t cudaGetSymbolAddress(void** p, const void* sym) {
 }
 
 /* ---- kernels */
+static const Kernel* kernel_of(const void* fn) {
+  const Kernel* k = fn;
+  return k >= kernels && k < kernels + n_kernels ? k : 0;
+}
+static int static_smem(const void* fn) { return kernel_of(fn) ? 0 : STATIC_SMEM; }
 static int* limit_of(const void* fn) {
   int i;
   for (i = 0; i < n_limits[current]; ++i)
     if (limits[current][i].fn == fn) return &limits[current][i].limit;
   limits[current][i].fn = fn;
-  limits[current][i].limit = 49152 - STATIC_SMEM;
+  limits[current][i].limit = 49152 - static_smem(fn);
   ++n_limits[current];
   return &limits[current][i].limit;
 }
 cudaError_t cudaFuncGetAttributes(struct cudaFuncAttributes* a, const void* fn) {
   memset(a, 0, sizeof *a);
-  a->sharedSizeBytes = STATIC_SMEM;
+  a->sharedSizeBytes = static_smem(fn);
   a->maxDynamicSharedSizeBytes = *limit_of(fn);
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void* fn, enum cudaFuncAttribute a, int v) {
   if (a != cudaFuncAttributeMaxDynamicSharedMemorySize) return cudaSuccess;
-  if (v + STATIC_SMEM > OPTIN) return cudaErrorInvalidValue;
+  if (v + static_smem(fn) > OPTIN) return cudaErrorInvalidValue;
   *limit_of(fn) = v;
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void* fn, int threads,
                                                           size_t smem) {
-  const int by_smem = (int)(OPTIN / (smem + STATIC_SMEM + 1024)), by_threads = 1024 / threads;
-  *n = (long)smem > *limit_of(fn) ? 0 : by_smem < by_threads ? by_smem : by_threads;
+  const Kernel* k = kernel_of(fn);
+  const int by_smem = (int)(OPTIN / (smem + static_smem(fn) + 1024));
+  const int by_regs = k ? 65536 / (((k->regs + 7) & ~7) * threads) : 1024 / threads;
+  *n = (long)smem > *limit_of(fn) ? 0 : by_smem < by_regs ? by_smem : by_regs;
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernel(const void* fn, dim3 g, dim3 b, void** args, size_t smem,
                              cudaStream_t st) {
   (void)args;
   if ((long)smem > *limit_of(fn)) return cudaErrorInvalidValue;
-  note("launch grid %u %u %u block %u smem %zu", g.x, g.y, g.z, b.x, smem);
+  note("launch %s grid %u %u %u block %u smem %zu", kernel_of(fn) ? kernel_of(fn)->name : "-",
+       g.x, g.y, g.z, b.x, smem);
   if (!stream_of(st)->capturing) ++stream_of(st)->submitted;
   return cudaSuccess;
 }
@@ -323,11 +341,14 @@ void __cudaRegisterVar(void) {}
 cudaError_t cudaLibraryLoadData(cudaLibrary_t* l, const void* c, enum cudaJitOption* jo, void** jv,
                                 unsigned nj, enum cudaLibraryOption* lo, void** lv, unsigned nl) {
   (void)l, (void)c, (void)jo, (void)jv, (void)nj, (void)lo, (void)lv, (void)nl;
-  return cudaErrorNotSupported;
+  return n_kernels ? cudaSuccess : cudaErrorNotSupported;
 }
-cudaError_t cudaLibraryGetKernel(cudaKernel_t* k, cudaLibrary_t l, const char* n) {
-  (void)k, (void)l, (void)n;
-  return cudaErrorNotSupported;
+cudaError_t cudaLibraryGetKernel(cudaKernel_t* k, cudaLibrary_t l, const char* name) {
+  (void)l;
+  for (int i = 0; i < n_kernels; ++i)
+    if (!strcmp(kernels[i].name, name)) return *k = (cudaKernel_t)&kernels[i], cudaSuccess;
+  fake_registers(name, 64);
+  return *k = (cudaKernel_t)&kernels[n_kernels - 1], cudaSuccess;
 }
 cudaError_t cudaLibraryUnload(cudaLibrary_t l) { return (void)l, cudaSuccess; }
 

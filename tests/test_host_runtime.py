@@ -228,3 +228,53 @@ session().close()
 rt.fake_pool_keeps_last(1)
 session(p=64, n_obs=200000)  # 52 MB of data
 """)
+
+
+# Registers of the gradient kernels as compiled for sm_100a: one chain per lane,
+# two.  With 148 and 234 two chains per lane keep eight warps on an SM (in one block
+# or in two of four warps), with 113 and 196 they halve the sixteen.
+@pytest.mark.parametrize("model,regs,n_obs,points,kernel", [
+    ("logistic", (148, 234), 600000, 32, "gm_iter_grad"),
+    ("logistic", (148, 234), 600000, 33, "gm_iter_grad2h"),
+    ("logistic", (148, 234), 600000, 256, "gm_iter_grad2h"),
+    ("logistic", (148, 234), 600000, 257, "gm_iter_grad2"),
+    ("logistic", (148, 234), 600000, 600, "gm_iter_grad2h"),
+    ("logistic", (148, 234), 600000, 2048, "gm_iter_grad2"),
+    # a block per SM at most: four warps of it are slower than eight
+    ("logistic", (148, 234), 3000, 256, "gm_iter_grad"),
+    ("logistic", (148, 234), 3000, 1025, "gm_iter_grad"),
+    ("logistic", (148, 234), 0, 300, "gm_iter_grad"),
+    ("mixture", (113, 196), 600000, 300, "gm_iter_grad"),
+    ("mixture", (113, 196), 600000, 2048, "gm_iter_grad"),
+])
+def test_choice_of_the_gradient_kernel(runtime, model, regs, n_obs, points, kernel):
+    runtime(f"""
+for name in ("gm_iter_grad2", "gm_iter_grad2h"):
+    rt.fake_registers(name.encode(), {regs[1]})
+rt.fake_registers(b"gm_iter_grad", {regs[0]})
+kw = dict(p=16) if {model!r} == "logistic" else dict()
+m = W.make({model!r}, n_obs=16, **kw).model
+data = np.zeros(({n_obs}, m.n_cols))
+s = _native.Session(m.loglik.code, m.loglik.consts, m.prior.code, m.prior.consts, m.n_params,
+                    data, m.n_cols, {n_obs})
+s.grad_batch(np.zeros(({points}, m.n_params)))
+names = [l.split()[1] for l in log() if l.startswith("launch")]
+assert [n for n in names if n.startswith("gm_iter_grad")] == [{kernel!r}], names
+""")
+
+
+def test_eight_warps_of_two_chains_where_two_blocks_do_not_fit(runtime):
+    # 33 parameters: 67 KB of sums and 67 KB of data a block of four warps, so one
+    # block an SM; a block of eight warps is as many as with one chain per lane
+    runtime("""
+for name in ("gm_iter_grad2", "gm_iter_grad2h"):
+    rt.fake_registers(name.encode(), 242)
+rt.fake_registers(b"gm_iter_grad", 254)
+m = W.make("logistic", n_obs=16, p=31).model
+s = _native.Session(m.loglik.code, m.loglik.consts, m.prior.code, m.prior.consts, m.n_params,
+                    np.zeros((300000, m.n_cols)), m.n_cols, 300000)
+for n in (200, 300, 600, 2048):
+    s.grad_batch(np.zeros((n, m.n_params)))
+names = [l.split()[1] for l in log() if l.startswith("launch gm_iter_grad")]
+assert names == ["gm_iter_grad", "gm_iter_grad2", "gm_iter_grad", "gm_iter_grad2"], names
+""")
