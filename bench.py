@@ -184,8 +184,8 @@ def cpu_sample(w, seconds, chains_cap):
 
 
 class Clocks:
-    """nvidia-smi sampled every 100 ms; the summary keeps the samples whose
-    timestamps fall inside the marked (timed) window."""
+    """nvidia-smi sampled every 10 ms (the default run's timed region takes 40); the
+    summary keeps the samples whose timestamps fall inside the marked (timed) window."""
 
     Q = ("timestamp,index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
          "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -206,7 +206,7 @@ class Clocks:
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--id={self.index}", f"--query-gpu={self.Q}",
-                 "--format=csv,noheader,nounits", "-lms", "100"],
+                 "--format=csv,noheader,nounits", "-lms", "10"],
                 stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
         except OSError:
             self.proc = None
