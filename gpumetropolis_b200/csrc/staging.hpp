@@ -94,8 +94,7 @@ inline PinnedBlocks& pinned_chunks() {
 // CUDA allows no such wait meanwhile.
 // 96 MB hold three sessions of 65,537 x 17 values, packed copy and partial sums
 // included; with 64 MB a new one's first gradient call allocated anew (500 us,
-// 200 without).  With 128 MB kept, large allocations after it lay elsewhere, and the
-// random-walk steps on 2^20 observations took 1.2 % longer, the mixture's 1.7 % less.
+// 200 without).
 constexpr size_t kPoolMax = 32u << 20;
 constexpr uint64_t kPoolKeep = 96ull << 20;
 
