@@ -242,7 +242,8 @@ GPUM_API int gpum_b200_session_advance(gpum_b200_session* s, uint32_t n_iter, ch
 GPUM_API int gpum_b200_session_sync(gpum_b200_session* s, char* err, size_t err_len);
 /* Copies draws of the iterations advanced so far (n_done <= max_iter) in the
  * reference layout with n_iter = n_done, accept rates over n_done, last
- * log posteriors.  Any output pointer may be NULL. */
+ * log posteriors.  Any output pointer may be NULL.  Waits for the iterations;
+ * a run that failed on the device (GPUM_ERR_DEVICE) writes nothing. */
 GPUM_API int gpum_b200_session_fetch(gpum_b200_session* s, float* out_draws, float* out_accept,
                             double* out_last_logpost, uint32_t* n_done, char* err,
                             size_t err_len);
